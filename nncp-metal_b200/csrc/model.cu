@@ -254,7 +254,7 @@ template <typename TC>
 static int mm_nt_impl(nncu_model *m, int M, int N, int K, const float *A, long lda, size_t w_off,
                       TC *C, long ldc, const float *bias, int bias_n)
 {
-    return gemm_simt<float, float, TC>(m->st, GEMM_NT, M, N, K, A, lda, m->W + w_off, K, C, ldc, bias, 0,
+    return gemm_simt<float, float, TC>(m->st, GEMM_NT, M, N, K, A, lda, m->W + w_off, K, C, ldc, bias, (const TC *)nullptr,
                                        bias_n);
 }
 template <typename TC>
@@ -264,7 +264,7 @@ static int mm_nt_impl(nncu_model *m, int M, int N, int K, const bf16 *A, long ld
     const bf16 *Wt = m->Wb + w_off;
     if (m->use_tc && tc::usable(A, lda, Wt, K, K))
         return tc::gemm_nt<TC>(m->st, M, N, K, A, lda, Wt, K, C, ldc, bias, nullptr, m->err_flag, bias_n);
-    return gemm_simt<bf16, bf16, TC>(m->st, GEMM_NT, M, N, K, A, lda, Wt, K, C, ldc, bias, 0, bias_n);
+    return gemm_simt<bf16, bf16, TC>(m->st, GEMM_NT, M, N, K, A, lda, Wt, K, C, ldc, bias, (const TC *)nullptr, bias_n);
 }
 // bias (if any) is added to output columns n < bias_n only
 template <typename AT, typename TC>
@@ -289,11 +289,8 @@ static bool tc_mn_major()
 static int mm_nn(nncu_model *m, int M, int Kin, int Nout, const float *dY, long ldy, size_t w_off,
                  float *C, long ldc, const float *addsrc)
 {
-    if (addsrc && addsrc != C)
-        CUDA_TRY(cudaMemcpy2DAsync(C, ldc * 4, addsrc, ldc * 4, (size_t)Kin * 4, M,
-                                   cudaMemcpyDeviceToDevice, m->st));
     return gemm_simt<float, float, float>(m->st, GEMM_NN, M, Kin, Nout, dY, ldy, m->W + w_off, Kin,
-                                          C, ldc, nullptr, addsrc ? 1 : 0);
+                                          C, ldc, nullptr, addsrc);
 }
 static int mm_nn(nncu_model *m, int M, int Kin, int Nout, const bf16 *dY, long ldy, size_t w_off,
                  bf16 *C, long ldc, const bf16 *addsrc)
@@ -318,11 +315,8 @@ static int mm_nn(nncu_model *m, int M, int Kin, int Nout, const bf16 *dY, long l
     if (m->use_tc && tc::usable(dY, ldy, WT, Nout, Nout))
         return tc::gemm_nt<bf16>(m->st, M, Kin, Nout, dY, ldy, WT, Nout, C, ldc, nullptr, addsrc,
                                  m->err_flag);
-    if (addsrc && addsrc != C)
-        CUDA_TRY(cudaMemcpy2DAsync(C, ldc * 2, addsrc, ldc * 2, (size_t)Kin * 2, M,
-                                   cudaMemcpyDeviceToDevice, m->st));
     return gemm_simt<bf16, bf16, bf16>(m->st, GEMM_NN, M, Kin, Nout, dY, ldy, m->Wb + w_off, Kin, C,
-                                       ldc, nullptr, addsrc ? 1 : 0);
+                                       ldc, nullptr, addsrc);
 }
 
 // dW = dY^T X: G[Nout][Kin] = sum over R rows of dY[r][Nout] X[r][Kin]   (fp32 result)
@@ -361,7 +355,7 @@ static int mm_tn(nncu_model *m, int Nout, int Kin, int R, const float *dY, long 
                  long ldx, float *Gout)
 {
     return gemm_simt<float, float, float>(side_fork(m), GEMM_TN, Nout, Kin, R, dY, ldy, X, ldx, Gout, Kin,
-                                          nullptr, 0);
+                                          nullptr, (const float *)nullptr);
 }
 static int mm_tn(nncu_model *m, int Nout, int Kin, int R, const bf16 *dY, long ldy, const bf16 *X,
                  long ldx, float *Gout)
@@ -383,7 +377,7 @@ static int mm_tn(nncu_model *m, int Nout, int Kin, int R, const bf16 *dY, long l
                                   m->err_flag);
     }
     return gemm_simt<bf16, bf16, float>(side_fork(m), GEMM_TN, Nout, Kin, R, dY, ldy, X, ldx, Gout, Kin,
-                                        nullptr, 0);
+                                        nullptr, (const float *)nullptr);
 }
 
 // The column and stream reductions of the backward pass only write gradient buffers, which nobody
@@ -2415,8 +2409,8 @@ int nncu_gemm_bf16(int backend, int mode, int M, int N, int K, const void *A, in
     cudaStream_t st = (cudaStream_t)cuda_stream;
     const bf16 *a = (const bf16 *)A, *b = (const bf16 *)B;
     if (backend == NNCU_GEMM_SIMT)
-        return c_is_f32 ? gemm_simt<bf16, bf16, float>(st, mode, M, N, K, a, lda, b, ldb, (float *)C, ldc, nullptr, 0)
-                        : gemm_simt<bf16, bf16, bf16>(st, mode, M, N, K, a, lda, b, ldb, (bf16 *)C, ldc, nullptr, 0);
+        return c_is_f32 ? gemm_simt<bf16, bf16, float>(st, mode, M, N, K, a, lda, b, ldb, (float *)C, ldc, nullptr, (const float *)nullptr)
+                        : gemm_simt<bf16, bf16, bf16>(st, mode, M, N, K, a, lda, b, ldb, (bf16 *)C, ldc, nullptr, (const bf16 *)nullptr);
     int *flag = nullptr;
     NNCU_TRY(gemm_flag(&flag));
     int rc;
@@ -2443,8 +2437,8 @@ int nncu_gemm_bf16_nt(int backend, int M, int N, int K, const void *A, int lda, 
     cudaStream_t st = (cudaStream_t)cuda_stream;
     const bf16 *a = (const bf16 *)A, *b = (const bf16 *)B;
     if (backend == NNCU_GEMM_SIMT) {
-        return c_is_f32 ? gemm_simt<bf16, bf16, float>(st, GEMM_NT, M, N, K, a, lda, b, ldb, (float *)C, ldc, bias, 0)
-                        : gemm_simt<bf16, bf16, bf16>(st, GEMM_NT, M, N, K, a, lda, b, ldb, (bf16 *)C, ldc, bias, 0);
+        return c_is_f32 ? gemm_simt<bf16, bf16, float>(st, GEMM_NT, M, N, K, a, lda, b, ldb, (float *)C, ldc, bias, (const float *)nullptr)
+                        : gemm_simt<bf16, bf16, bf16>(st, GEMM_NT, M, N, K, a, lda, b, ldb, (bf16 *)C, ldc, bias, (const bf16 *)nullptr);
     }
     int *flag = nullptr;
     NNCU_TRY(gemm_flag(&flag));
