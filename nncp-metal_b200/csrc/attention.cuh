@@ -24,20 +24,70 @@ struct AttnArgs {
     void *o, *dq, *dkv;
     float *lse, *dwr_part, *dbr_part;
     int B, H, dk, T, M, L, P, attn_len, t0, t1, qchunk;
+    int smem_pitch; // row pitch of the staged K and table rows (CUDA-core kernels)
     int qp, kvp, dqp, dkvp; // row pitches (elements) of q, kv, dq, dkv; K then V inside a kv row
     float br_scale, inv_sqrt;
 };
 
-template <typename T> struct SmemRow; // padded row strides that avoid bank conflicts
-template <> struct SmemRow<float> { static __host__ __device__ int stride(int dk) { return dk + 1; } };
-template <> struct SmemRow<bf16> { static __host__ __device__ int stride(int dk) { return dk + 2; } };
+// Row pitch (elements) of the K and table rows in shared memory.  Head sizes that are a multiple of
+// four go through four-element loads: a pitch of dk + 4 puts the rows of eight neighbouring keys on
+// different bank groups; where that does not fit, dk alone; any other head size keeps dk + an odd
+// word and single-element loads.
+template <typename T> struct SmemRow {
+    static __host__ __device__ int wide(int dk) { return dk % 4 == 0 ? dk + 4 : dk + (sizeof(T) == 4 ? 1 : 2); }
+    static __host__ __device__ int tight(int dk) { return dk % 4 == 0 ? dk : wide(dk); }
+};
+
+__device__ __forceinline__ float4 load_f4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
+__device__ __forceinline__ float4 load_f4(const bf16 *p)
+{
+    const uint2 u = *reinterpret_cast<const uint2 *>(p);
+    const __nv_bfloat162 a = *reinterpret_cast<const __nv_bfloat162 *>(&u.x), b = *reinterpret_cast<const __nv_bfloat162 *>(&u.y);
+    return make_float4(__low2float(a), __high2float(a), __low2float(b), __high2float(b));
+}
+__device__ __forceinline__ void store_f4(float *p, float4 v) { *reinterpret_cast<float4 *>(p) = v; }
+__device__ __forceinline__ void store_f4(bf16 *p, float4 v)
+{
+    const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
+    *reinterpret_cast<uint2 *>(p) = make_uint2(*reinterpret_cast<const uint32_t *>(&a), *reinterpret_cast<const uint32_t *>(&b));
+}
+
+// rows x dk elements (row pitch ld) into shared memory (row pitch lds), converted from S to D
+template <typename D, typename S>
+__device__ __forceinline__ void stage_rows(D *dst, int lds, const S *src, size_t ld, int rows, int dk)
+{
+    if (dk % 4 == 0 && ld % 4 == 0 && lds % 4 == 0 && (reinterpret_cast<uintptr_t>(src) & (4 * sizeof(S) - 1)) == 0) {
+        const int cpr = dk / 4;
+#pragma unroll 4
+        for (int idx = threadIdx.x; idx < rows * cpr; idx += blockDim.x) {
+            const int r = idx / cpr, e = (idx - r * cpr) * 4;
+            store_f4(dst + (size_t)r * lds + e, load_f4(src + (size_t)r * ld + e));
+        }
+    } else {
+        for (int idx = threadIdx.x; idx < rows * dk; idx += blockDim.x) {
+            const int r = idx / dk, e = idx - r * dk;
+            dst[(size_t)r * lds + e] = from_f<D>(to_f(src[(size_t)r * ld + e]));
+        }
+    }
+}
 
 template <typename T>
 __device__ __forceinline__ float dot_q(const float *__restrict__ qf, const T *__restrict__ row, int dk)
 {
     float s = 0.0f;
-    for (int e = 0; e < dk; e++)
-        s = fmaf(qf[e], to_f(row[e]), s);
+    if (dk % 4 == 0) {
+#pragma unroll 4
+        for (int e = 0; e < dk; e += 4) {
+            const float4 a = load_f4(qf + e), b = load_f4(row + e);
+            s = fmaf(a.x, b.x, s);
+            s = fmaf(a.y, b.y, s);
+            s = fmaf(a.z, b.z, s);
+            s = fmaf(a.w, b.w, s);
+        }
+    } else {
+        for (int e = 0; e < dk; e++)
+            s = fmaf(qf[e], to_f(row[e]), s);
+    }
     return s;
 }
 
@@ -63,15 +113,17 @@ __device__ __forceinline__ void key_range(const AttnArgs &a, int i, int &jlo, in
     jlo = max(0, i + a.M - a.attn_len + 1);      // (i+M)-j < attn_len
 }
 
+// floats a warp of the forward kernel keeps: the query row and its scores
+__host__ __device__ inline int warp_floats(int dk, int L) { return dk % 4 == 0 ? (dk + L + 3) & ~3 : dk + L; }
+
 template <typename T>
-size_t attn_fwd_smem(int L, int P, int dk, bool has_wr)
+size_t attn_fwd_smem(int L, int P, int dk, bool has_wr, int ks)
 {
-    int ks = SmemRow<T>::stride(dk);
     size_t b = (size_t)L * ks * sizeof(T) + (size_t)L * dk * sizeof(T);
     if (has_wr)
         b += (size_t)P * ks * sizeof(T);
     b = (b + 15) & ~(size_t)15;
-    b += 8 * ((size_t)dk + L) * sizeof(float);
+    b += 8 * (size_t)warp_floats(dk, L) * sizeof(float);
     return b;
 }
 
@@ -79,7 +131,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) attn_fwd_kernel(AttnArgs a)
 {
     extern __shared__ __align__(16) unsigned char smraw[];
-    const int ks = SmemRow<T>::stride(a.dk);
+    const int ks = a.smem_pitch;
     T *Ks = reinterpret_cast<T *>(smraw);
     T *Vs = Ks + (size_t)a.L * ks;
     T *Rs = Vs + (size_t)a.L * a.dk;
@@ -87,8 +139,10 @@ __global__ void __launch_bounds__(256) attn_fwd_kernel(AttnArgs a)
     off = (off + 15) & ~(size_t)15;
     float *fs = reinterpret_cast<float *>(smraw + off);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    float *qf = fs + (size_t)warp * (a.dk + a.L);
+    float *qf = fs + (size_t)warp * warp_floats(a.dk, a.L);
     float *ps = qf + a.dk;
+    pdl_trigger();
+    pdl_wait();
 
     const int b = blockIdx.x / a.H, h = blockIdx.x % a.H;
     const int HD = a.H * a.dk;
@@ -100,20 +154,12 @@ __global__ void __launch_bounds__(256) attn_fwd_kernel(AttnArgs a)
     key_range(a, i_first, jlo_all, tmp);
     key_range(a, i_last, tmp, jhi_all);
 
-    const T *kv = reinterpret_cast<const T *>(a.kv);
+    const T *kv = reinterpret_cast<const T *>(a.kv) + ((size_t)jlo_all * a.B + b) * a.kvp + h * a.dk;
     const int nj = jhi_all - jlo_all + 1;
-    for (int idx = threadIdx.x; idx < nj * a.dk; idx += blockDim.x) {
-        int j = jlo_all + idx / a.dk, e = idx % a.dk;
-        const T *src = kv + ((size_t)j * a.B + b) * a.kvp + h * a.dk + e;
-        Ks[(size_t)j * ks + e] = src[0];
-        Vs[(size_t)j * a.dk + e] = src[HD];
-    }
-    if (a.w_r) {
-        for (int idx = threadIdx.x; idx < a.P * a.dk; idx += blockDim.x) {
-            int p = idx / a.dk, e = idx % a.dk;
-            Rs[(size_t)p * ks + e] = from_f<T>(a.w_r[((size_t)h * a.P + p) * a.dk + e]);
-        }
-    }
+    stage_rows(Ks + (size_t)jlo_all * ks, ks, kv, (size_t)a.B * a.kvp, nj, a.dk);
+    stage_rows(Vs + (size_t)jlo_all * a.dk, a.dk, kv + HD, (size_t)a.B * a.kvp, nj, a.dk);
+    if (a.w_r)
+        stage_rows(Rs, ks, a.w_r + (size_t)h * a.P * a.dk, (size_t)a.dk, a.P, a.dk);
     __syncthreads();
 
     const T *q = reinterpret_cast<const T *>(a.q);
@@ -143,6 +189,7 @@ __global__ void __launch_bounds__(256) attn_fwd_kernel(AttnArgs a)
         __syncwarp();
         for (int e = lane; e < a.dk; e += 32) {
             float acc = 0.0f;
+#pragma unroll 8
             for (int j = jlo; j <= jhi; j++)
                 acc = fmaf(ps[j] * rs, to_f(Vs[(size_t)j * a.dk + e]), acc);
             o[((size_t)i * a.B + b) * HD + h * a.dk + e] = from_f<T>(acc);
@@ -154,10 +201,10 @@ __global__ void __launch_bounds__(256) attn_fwd_kernel(AttnArgs a)
 }
 
 template <typename T>
-size_t attn_bwd_smem(int T_, int L, int P, int dk, bool has_wr)
+size_t attn_bwd_smem(int T_, int L, int P, int dk, bool has_wr, int ks)
 {
-    int ks = SmemRow<T>::stride(dk);
-    size_t b = (size_t)L * ks * sizeof(T) + (size_t)L * dk * sizeof(T);
+    const int vs = dk % 4 == 0 ? ks : dk; // row pitch of V
+    size_t b = (size_t)L * ks * sizeof(T) + (size_t)L * vs * sizeof(T);
     if (has_wr)
         b += (size_t)P * ks * sizeof(T);
     b = (b + 15) & ~(size_t)15;
@@ -165,132 +212,188 @@ size_t attn_bwd_smem(int T_, int L, int P, int dk, bool has_wr)
     return b;
 }
 
-template <typename T>
+// W consecutive elements of a shared-memory row as floats (W = 4: one vector load)
+template <int W, typename T> __device__ __forceinline__ void load_w(const T *p, float (&v)[W])
+{
+    if constexpr (W == 4) {
+        const float4 x = load_f4(p);
+        v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
+    } else {
+        v[0] = to_f(p[0]);
+    }
+}
+template <int W, typename T> __device__ __forceinline__ void store_w(T *p, const float (&v)[W], bool vec)
+{
+    if constexpr (W == 4) {
+        if (vec) {
+            store_f4(p, make_float4(v[0], v[1], v[2], v[3]));
+            return;
+        }
+    }
+#pragma unroll
+    for (int w = 0; w < W; w++)
+        p[w] = from_f<T>(v[w]);
+}
+
+// One CTA per (stream, head): the whole problem sits in shared memory and what bounds it is the rate
+// of shared-memory reads, so every inner loop reads W = 4 elements per access (head sizes that are
+// a multiple of four; W = 1 otherwise) and each gradient row is a register tile of W columns.
+template <typename T, int W>
 __global__ void __launch_bounds__(256) attn_bwd_kernel(AttnArgs a)
 {
     extern __shared__ __align__(16) unsigned char smraw[];
-    const int ks = SmemRow<T>::stride(a.dk);
+    const int ks = a.smem_pitch;
     const int Tn = a.T, L = a.L, dk = a.dk, P = a.P, M = a.M;
+    const int vs = dk % 4 == 0 ? ks : dk;
     T *Ks = reinterpret_cast<T *>(smraw);
     T *Vs = Ks + (size_t)L * ks;
-    T *Rs = Vs + (size_t)L * dk;
-    size_t off = ((size_t)L * ks + (size_t)L * dk + (a.w_r ? (size_t)P * ks : 0)) * sizeof(T);
+    T *Rs = Vs + (size_t)L * vs;
+    size_t off = ((size_t)L * ks + (size_t)L * vs + (a.w_r ? (size_t)P * ks : 0)) * sizeof(T);
     off = (off + 15) & ~(size_t)15;
     float *qs = reinterpret_cast<float *>(smraw + off); // [T][dk]
     float *dos = qs + (size_t)Tn * dk;                  // [T][dk]
     float *Pm = dos + (size_t)Tn * dk;                  // [T][L+1]
     float *dS = Pm + (size_t)Tn * (L + 1);              // [T][L+1]
-    float *Dr = dS + (size_t)Tn * (L + 1);              // [T]
+    float *Dr = dS + (size_t)Tn * (L + 1);              // [T]: D_i, later the row's sum over the left pad
     const int ls = L + 1;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int b = blockIdx.x / a.H, h = blockIdx.x % a.H;
     const int HD = a.H * dk;
+    pdl_trigger();
+    pdl_wait();
 
-    const T *kv = reinterpret_cast<const T *>(a.kv);
-    const T *q = reinterpret_cast<const T *>(a.q);
-    const T *outp = reinterpret_cast<const T *>(a.out);
-    const T *dout = reinterpret_cast<const T *>(a.dout);
-    for (int idx = threadIdx.x; idx < L * dk; idx += blockDim.x) {
-        int j = idx / dk, e = idx % dk;
-        const T *src = kv + ((size_t)j * a.B + b) * a.kvp + h * dk + e;
-        Ks[(size_t)j * ks + e] = src[0];
-        Vs[(size_t)j * dk + e] = src[HD];
-    }
+    const T *kv = reinterpret_cast<const T *>(a.kv) + (size_t)b * a.kvp + h * dk;
+    const T *q = reinterpret_cast<const T *>(a.q) + (size_t)b * a.qp + h * dk;
+    const T *outp = reinterpret_cast<const T *>(a.out) + (size_t)b * HD + h * dk;
+    const T *dout = reinterpret_cast<const T *>(a.dout) + (size_t)b * HD + h * dk;
+    stage_rows(Ks, ks, kv, (size_t)a.B * a.kvp, L, dk);
+    stage_rows(Vs, vs, kv + HD, (size_t)a.B * a.kvp, L, dk);
+    stage_rows(qs, dk, q, (size_t)a.B * a.qp, Tn, dk);
+    stage_rows(dos, dk, dout, (size_t)a.B * HD, Tn, dk);
     if (a.w_r)
-        for (int idx = threadIdx.x; idx < P * dk; idx += blockDim.x) {
-            int p = idx / dk, e = idx % dk;
-            Rs[(size_t)p * ks + e] = from_f<T>(a.w_r[((size_t)h * P + p) * dk + e]);
-        }
-    for (int idx = threadIdx.x; idx < Tn * dk; idx += blockDim.x) {
-        int i = idx / dk, e = idx % dk;
-        qs[idx] = to_f(q[((size_t)i * a.B + b) * a.qp + h * dk + e]);
-        dos[idx] = to_f(dout[((size_t)i * a.B + b) * HD + h * dk + e]);
-    }
-    for (int idx = threadIdx.x; idx < Tn * ls; idx += blockDim.x) {
-        Pm[idx] = 0.0f;
-        dS[idx] = 0.0f;
-    }
+        stage_rows(Rs, ks, a.w_r + (size_t)h * P * dk, (size_t)dk, P, dk);
     __syncthreads();
-    // D_i = dO_i . O_i  (= sum_j P_ij dP_ij)
+    // P and dS, zero where the pair is masked
     for (int i = warp; i < Tn; i += 8) {
-        float s = 0.0f;
+        // D_i = dO_i . O_i  (= sum_j P_ij dP_ij)
+        float D = 0.0f;
         for (int e = lane; e < dk; e += 32)
-            s += dos[(size_t)i * dk + e] * to_f(outp[((size_t)i * a.B + b) * HD + h * dk + e]);
-        s = warp_sum(s);
-        if (lane == 0)
-            Dr[i] = s;
-    }
-    __syncthreads();
-    // P and dS
-    for (int i = warp; i < Tn; i += 8) {
+            D += dos[(size_t)i * dk + e] * to_f(outp[(size_t)i * a.B * HD + e]);
+        D = warp_sum(D);
         int jlo, jhi;
         key_range(a, i, jlo, jhi);
         const float lse = a.lse[((size_t)b * a.H + h) * Tn + i];
         const float *qf = qs + (size_t)i * dk, *dof = dos + (size_t)i * dk;
-        for (int j = jlo + lane; j <= jhi; j += 32) {
-            float s = score_ij<T>(a, h, i, j, qf, Ks, Rs, ks);
-            float p = expf(s - lse);
-            float dp = 0.0f;
-            for (int e = 0; e < dk; e++)
-                dp = fmaf(dof[e], to_f(Vs[(size_t)j * dk + e]), dp);
+        const int jpad = L - P - (Tn - 1) + i; // keys up to here share table row 0 (the left pad)
+        float pad = 0.0f;
+        for (int j = lane; j < L; j += 32) {
+            float p = 0.0f, d = 0.0f;
+            if (j >= jlo && j <= jhi) {
+                p = expf(score_ij<T>(a, h, i, j, qf, Ks, Rs, ks) - lse);
+                d = p * (dot_q<T>(dof, Vs + (size_t)j * vs, dk) - D) * a.inv_sqrt;
+            }
             Pm[(size_t)i * ls + j] = p;
-            dS[(size_t)i * ls + j] = p * (dp - Dr[i]) * a.inv_sqrt;
+            dS[(size_t)i * ls + j] = d;
+            if (j <= jpad)
+                pad += d;
         }
+        pad = warp_sum(pad);
+        if (lane == 0)
+            Dr[i] = pad;
     }
     __syncthreads();
-    // dV[j] = sum_i P_ij dO_i ; dK[j] = sum_i dS_ij q_i     (i ascending)
-    T *dkv = reinterpret_cast<T *>(a.dkv);
-    for (int idx = threadIdx.x; idx < L * dk; idx += blockDim.x) {
-        int j = idx / dk, e = idx % dk;
-        float av = 0.0f, ak = 0.0f;
-        for (int i = max(0, j - M); i < Tn; i++) {
-            av = fmaf(Pm[(size_t)i * ls + j], dos[(size_t)i * dk + e], av);
-            ak = fmaf(dS[(size_t)i * ls + j], qs[(size_t)i * dk + e], ak);
+    const int nw = dk / W; // column groups
+    const bool vec = (reinterpret_cast<uintptr_t>(a.dkv) & (4 * sizeof(T) - 1)) == 0 && (reinterpret_cast<uintptr_t>(a.dq) & (4 * sizeof(T) - 1)) == 0 &&
+                     a.dkvp % 4 == 0 && a.dqp % 4 == 0;
+    // dV[j] = sum_i P_ij dO_i ; dK[j] = sum_i dS_ij q_i     (i ascending), two keys per thread
+    T *dkv = reinterpret_cast<T *>(a.dkv) + (size_t)b * a.dkvp + h * dk;
+    const int half = (L + 1) / 2;
+    for (int idx = threadIdx.x; idx < half * nw; idx += blockDim.x) {
+        const int j0 = idx / nw, e = (idx - j0 * nw) * W, j1 = j0 + half < L ? j0 + half : j0;
+        float av[2][W] = {}, ak[2][W] = {};
+#pragma unroll 4
+        for (int i = max(0, j0 - M); i < Tn; i++) {
+            float x[W], y[W];
+            load_w<W>(dos + (size_t)i * dk + e, x);
+            load_w<W>(qs + (size_t)i * dk + e, y);
+            const float p0 = Pm[(size_t)i * ls + j0], p1 = Pm[(size_t)i * ls + j1];
+            const float d0 = dS[(size_t)i * ls + j0], d1 = dS[(size_t)i * ls + j1];
+#pragma unroll
+            for (int w = 0; w < W; w++) {
+                av[0][w] = fmaf(p0, x[w], av[0][w]);
+                av[1][w] = fmaf(p1, x[w], av[1][w]);
+                ak[0][w] = fmaf(d0, y[w], ak[0][w]);
+                ak[1][w] = fmaf(d1, y[w], ak[1][w]);
+            }
         }
-        T *dst = dkv + ((size_t)j * a.B + b) * a.dkvp + h * dk + e;
-        dst[0] = from_f<T>(ak);
-        dst[HD] = from_f<T>(av);
+        T *dst = dkv + (size_t)j0 * a.B * a.dkvp + e;
+        store_w<W>(dst, ak[0], vec);
+        store_w<W>(dst + HD, av[0], vec && HD % 4 == 0);
+        if (j1 != j0) {
+            dst = dkv + (size_t)j1 * a.B * a.dkvp + e;
+            store_w<W>(dst, ak[1], vec);
+            store_w<W>(dst + HD, av[1], vec && HD % 4 == 0);
+        }
     }
     // dQ[i] = sum_j dS_ij (k_j + w_r[pi(i,j)])               (j ascending)
-    T *dq = reinterpret_cast<T *>(a.dq);
-    for (int idx = threadIdx.x; idx < Tn * dk; idx += blockDim.x) {
-        int i = idx / dk, e = idx % dk;
+    T *dq = reinterpret_cast<T *>(a.dq) + (size_t)b * a.dqp + h * dk;
+    for (int idx = threadIdx.x; idx < Tn * nw; idx += blockDim.x) {
+        const int i = idx / nw, e = (idx - i * nw) * W;
         int jlo, jhi;
         key_range(a, i, jlo, jhi);
-        float acc = 0.0f;
+        float acc[W] = {};
+#pragma unroll 4
         for (int j = jlo; j <= jhi; j++) {
-            float w = to_f(Ks[(size_t)j * ks + e]);
+            float x[W];
+            load_w<W>(Ks + (size_t)j * ks + e, x);
             if (a.w_r) {
                 int pi = j + (Tn - 1) - i - (L - P);
                 pi = pi < 0 ? 0 : pi;
-                w += to_f(Rs[(size_t)pi * ks + e]);
+                float y[W];
+                load_w<W>(Rs + (size_t)pi * ks + e, y);
+#pragma unroll
+                for (int w = 0; w < W; w++)
+                    x[w] += y[w];
             }
-            acc = fmaf(dS[(size_t)i * ls + j], w, acc);
+            const float d = dS[(size_t)i * ls + j];
+#pragma unroll
+            for (int w = 0; w < W; w++)
+                acc[w] = fmaf(d, x[w], acc[w]);
         }
-        dq[((size_t)i * a.B + b) * a.dqp + h * dk + e] = from_f<T>(acc);
+        store_w<W>(dq + (size_t)i * a.B * a.dqp + e, acc, vec);
     }
-    // table gradients of this (stream, head): slot r collects pairs (i, j = r-(T-1-i))
+    // table gradients of this (stream, head): table row p collects the pairs (i, j = p + L - P - (T-1) + i),
+    // row 0 the whole left pad
     if (a.w_r && a.dwr_part) {
         float *dst = a.dwr_part + ((size_t)b * a.H + h) * P * dk;
-        for (int idx = threadIdx.x; idx < P * dk; idx += blockDim.x) {
-            int p = idx / dk, e = idx % dk;
-            int rlo = (p == 0) ? 0 : p + (L - P), rhi = p + (L - P);
-            float acc = 0.0f;
-            for (int r = rlo; r <= rhi; r++)
-                for (int i = 0; i < Tn; i++) {
-                    int j = r - (Tn - 1 - i);
-                    if (j >= 0 && j < L)
-                        acc = fmaf(dS[(size_t)i * ls + j], qs[(size_t)i * dk + e], acc);
-                }
-            dst[idx] = acc;
+        for (int idx = threadIdx.x; idx < P * nw; idx += blockDim.x) {
+            const int p = idx / nw, e = (idx - p * nw) * W, j0 = p + L - P - (Tn - 1);
+            float acc[W] = {};
+#pragma unroll 4
+            for (int i = 0; i < Tn; i++) {
+                const int j = j0 + i;
+                float y[W], d = 0.0f;
+                if (p == 0)
+                    d = Dr[i];
+                else if (j >= 0 && j < L)
+                    d = dS[(size_t)i * ls + j];
+                load_w<W>(qs + (size_t)i * dk + e, y);
+#pragma unroll
+                for (int w = 0; w < W; w++)
+                    acc[w] = fmaf(d, y[w], acc[w]);
+            }
+#pragma unroll
+            for (int w = 0; w < W; w++)
+                dst[(size_t)p * dk + e + w] = acc[w];
         }
     }
     if (a.dbr_part) {
         float *dst = a.dbr_part + ((size_t)b * a.H + h) * L;
         for (int r = threadIdx.x; r < L; r += blockDim.x) {
             float acc = 0.0f;
+#pragma unroll 4
             for (int i = 0; i < Tn; i++) {
-                int j = r - (Tn - 1 - i);
+                const int j = r - (Tn - 1) + i;
                 if (j >= 0 && j < L)
                     acc += dS[(size_t)i * ls + j];
             }
@@ -352,6 +455,24 @@ static AttnArgs attn_args(const nncu_attn_shape *s, const AttnPitch *pt = nullpt
     return a;
 }
 
+// the row pitch for a shape and the shared memory it takes
+template <typename T> static int fwd_pitch(const AttnArgs &a, bool has_wr, size_t &smem)
+{
+    int ks = SmemRow<T>::wide(a.dk);
+    if (attn_fwd_smem<T>(a.L, a.P, a.dk, has_wr, ks) > 227 * 1024)
+        ks = SmemRow<T>::tight(a.dk);
+    smem = attn_fwd_smem<T>(a.L, a.P, a.dk, has_wr, ks);
+    return ks;
+}
+template <typename T> static int bwd_pitch(const AttnArgs &a, bool has_wr, size_t &smem)
+{
+    int ks = SmemRow<T>::wide(a.dk);
+    if (attn_bwd_smem<T>(a.T, a.L, a.P, a.dk, has_wr, ks) > 227 * 1024)
+        ks = SmemRow<T>::tight(a.dk);
+    smem = attn_bwd_smem<T>(a.T, a.L, a.P, a.dk, has_wr, ks);
+    return ks;
+}
+
 template <typename T>
 static int attn_forward_t(const nncu_attn_shape *s, const void *q, const void *kv, const float *w_r,
                           const float *b_r, void *out, float *lse, cudaStream_t st,
@@ -364,11 +485,12 @@ static int attn_forward_t(const nncu_attn_shape *s, const void *q, const void *k
     int chunks = max(1, min(ceil_div(nq, 8), ceil_div(2 * 148, a.B * a.H)));
     a.qchunk = ceil_div(nq, chunks);
     chunks = ceil_div(nq, a.qchunk);
-    size_t smem = attn_fwd_smem<T>(a.L, a.P, a.dk, w_r != nullptr);
+    size_t smem = 0;
+    a.smem_pitch = fwd_pitch<T>(a, w_r != nullptr, smem);
     if (smem > 227 * 1024)
         return nncu_fail(NNCU_ERR_RANGE, "attention forward: %zu bytes of shared memory needed", smem);
     CUDA_TRY(cudaFuncSetAttribute(attn_fwd_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    attn_fwd_kernel<T><<<dim3(a.B * a.H, chunks), 256, smem, st>>>(a);
+    launch_k(attn_fwd_kernel<T>, dim3(a.B * a.H, chunks), dim3(256), smem, st, a);
     KERNEL_CHECK();
     return NNCU_OK;
 }
@@ -384,11 +506,13 @@ static int attn_backward_t(const nncu_attn_shape *s, const void *q, const void *
         return nncu_fail(NNCU_ERR_INVALID, "attention backward runs over the whole segment");
     a.q = q; a.kv = kv; a.w_r = w_r; a.b_r = b_r; a.out = out; a.lse = const_cast<float *>(lse);
     a.dout = dout; a.dq = dq; a.dkv = dkv; a.dwr_part = dwr_part; a.dbr_part = dbr_part;
-    size_t smem = attn_bwd_smem<T>(a.T, a.L, a.P, a.dk, w_r != nullptr);
+    size_t smem = 0;
+    a.smem_pitch = bwd_pitch<T>(a, w_r != nullptr, smem);
     if (smem > 227 * 1024)
         return nncu_fail(NNCU_ERR_RANGE, "attention backward: %zu bytes of shared memory needed", smem);
-    CUDA_TRY(cudaFuncSetAttribute(attn_bwd_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    attn_bwd_kernel<T><<<a.B * a.H, 256, smem, st>>>(a);
+    auto kernel = a.dk % 4 == 0 ? attn_bwd_kernel<T, 4> : attn_bwd_kernel<T, 1>;
+    CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    launch_k(kernel, dim3(a.B * a.H), dim3(256), smem, st, a);
     KERNEL_CHECK();
     return NNCU_OK;
 }

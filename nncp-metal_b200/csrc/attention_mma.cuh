@@ -930,7 +930,8 @@ static int attn_shape_supported(const nncu_attn_shape *s, bool has_wr)
     AttnArgs a = attn_args(s, nullptr);
     const bool mma = sizeof(T) == 2 && !attn_force_simt();
     if (!(mma && amma::supported(a, false))) {
-        const size_t smem = attn_fwd_smem<T>(a.L, a.P, a.dk, has_wr);
+        size_t smem = 0;
+        fwd_pitch<T>(a, has_wr, smem);
         if (smem > 227 * 1024)
             return nncu_fail(NNCU_ERR_RANGE,
                              "attention forward of this shape (%d keys, d_pos %d, d_key %d) needs %zu bytes of "
@@ -938,7 +939,8 @@ static int attn_shape_supported(const nncu_attn_shape *s, bool has_wr)
                              a.L, a.P, a.dk, smem, 227 * 1024);
     }
     if (!(mma && amma::supported(a, true))) {
-        const size_t smem = attn_bwd_smem<T>(a.T, a.L, a.P, a.dk, has_wr);
+        size_t smem = 0;
+        bwd_pitch<T>(a, has_wr, smem);
         if (smem > 227 * 1024)
             return nncu_fail(NNCU_ERR_RANGE,
                              "attention backward of this shape (seg_len %d, %d keys, d_pos %d, d_key %d) needs %zu "
