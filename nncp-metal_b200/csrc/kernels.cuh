@@ -139,181 +139,238 @@ norm_bwd_kernel(const T *__restrict__ dy, const T *__restrict__ x, const float *
     }
 }
 
-// ---- bf16 rows of NC * 256 elements held in registers: 16-byte accesses, one pass over memory.
-// Lane l owns elements c*256 + l*8 .. +7 of every 256-element chunk c.
-template <int NC>
-__device__ __forceinline__ void row_load(const bf16 *row, int lane, float (&v)[NC][8])
+// ---- rows held in registers: 16-byte accesses, one pass over memory, one warp per row.  Lane l owns
+// the W = 16 / sizeof(T) elements from c * 32 * W + l * W of every chunk c; D is a multiple of W and at
+// most NC * 32 * W, what lies past D reads as zero and is not written.
+template <typename T> struct RowVec {
+    static constexpr int W = 16 / (int)sizeof(T), CHUNK = 32 * W;
+};
+template <typename T, int NC, int W>
+__device__ __forceinline__ void row_load(const T *row, int lane, int D, float (&v)[NC][W])
 {
 #pragma unroll
     for (int c = 0; c < NC; c++) {
-        const uint4 u = *reinterpret_cast<const uint4 *>(row + c * 256 + lane * 8);
-        const bf16 *h = reinterpret_cast<const bf16 *>(&u);
+        const int at = c * 32 * W + lane * W;
+        uint4 u = make_uint4(0u, 0u, 0u, 0u);
+        if (at < D)
+            u = *reinterpret_cast<const uint4 *>(row + at);
+        const T *h = reinterpret_cast<const T *>(&u);
 #pragma unroll
-        for (int e = 0; e < 8; e++)
+        for (int e = 0; e < W; e++)
             v[c][e] = to_f(h[e]);
     }
 }
-template <int NC>
-__device__ __forceinline__ void row_store(bf16 *row, int lane, const float (&v)[NC][8])
+template <typename T, int NC, int W>
+__device__ __forceinline__ void row_store(T *row, int lane, int D, const float (&v)[NC][W])
 {
 #pragma unroll
     for (int c = 0; c < NC; c++) {
+        const int at = c * 32 * W + lane * W;
         uint4 u;
-        bf16 *h = reinterpret_cast<bf16 *>(&u);
+        T *h = reinterpret_cast<T *>(&u);
 #pragma unroll
-        for (int e = 0; e < 8; e++)
-            h[e] = from_f<bf16>(v[c][e]);
-        *reinterpret_cast<uint4 *>(row + c * 256 + lane * 8) = u;
+        for (int e = 0; e < W; e++)
+            h[e] = from_f<T>(v[c][e]);
+        if (at < D)
+            *reinterpret_cast<uint4 *>(row + at) = u;
     }
 }
-template <int NC>
-__device__ __forceinline__ void vec_load_f32(const float *p, int lane, float (&v)[NC][8])
+template <int NC, int W>
+__device__ __forceinline__ void vec_load_f32(const float *p, int lane, int D, float (&v)[NC][W])
 {
 #pragma unroll
     for (int c = 0; c < NC; c++) {
-        const float4 a = *reinterpret_cast<const float4 *>(p + c * 256 + lane * 8);
-        const float4 b = *reinterpret_cast<const float4 *>(p + c * 256 + lane * 8 + 4);
-        v[c][0] = a.x; v[c][1] = a.y; v[c][2] = a.z; v[c][3] = a.w;
-        v[c][4] = b.x; v[c][5] = b.y; v[c][6] = b.z; v[c][7] = b.w;
+        const int at = c * 32 * W + lane * W;
+#pragma unroll
+        for (int e = 0; e < W; e += 4) {
+            const float4 a = at < D ? *reinterpret_cast<const float4 *>(p + at + e) : make_float4(0.f, 0.f, 0.f, 0.f);
+            v[c][e] = a.x; v[c][e + 1] = a.y; v[c][e + 2] = a.z; v[c][e + 3] = a.w;
+        }
     }
 }
 
-// residual_norm_kernel for bf16 rows of D = NC * 256 elements; same arguments and rounding
-// points (s is rounded to bf16 before the statistics), sums taken per lane, then over the warp.
-template <int NC>
+// residual_norm_kernel with the row in registers; same arguments and rounding points (s is rounded
+// to the storage type before the statistics), sums taken per lane, then over the warp.
+template <typename T, int NC>
 __global__ void __launch_bounds__(128)
-residual_norm_vec_kernel(const bf16 *__restrict__ a, const bf16 *__restrict__ res, bf16 *__restrict__ s_out,
-                         bf16 *__restrict__ y, const float *__restrict__ g, const float *__restrict__ b,
-                         float *__restrict__ stats, int rows, int mode)
+residual_norm_vec_kernel(const T *__restrict__ a, const T *__restrict__ res, T *__restrict__ s_out,
+                         T *__restrict__ y, const float *__restrict__ g, const float *__restrict__ b,
+                         float *__restrict__ stats, int rows, int D, int mode)
 {
     pdl_trigger();
     pdl_wait();
-    constexpr int D = NC * 256;
+    constexpr int W = RowVec<T>::W;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int r = blockIdx.x * 4 + warp;
     if (r >= rows)
         return;
-    float v[NC][8];
-    row_load<NC>(a + (size_t)r * D, lane, v);
+    float v[NC][W];
+    row_load<T, NC, W>(a + (size_t)r * D, lane, D, v);
     if (res) {
-        float w[NC][8];
-        row_load<NC>(res + (size_t)r * D, lane, w);
+        float w[NC][W];
+        row_load<T, NC, W>(res + (size_t)r * D, lane, D, w);
 #pragma unroll
         for (int c = 0; c < NC; c++)
 #pragma unroll
-            for (int e = 0; e < 8; e++)
-                v[c][e] = round_to<bf16>(v[c][e] + w[c][e]);
+            for (int e = 0; e < W; e++)
+                v[c][e] = round_to<T>(v[c][e] + w[c][e]);
     }
     if (s_out)
-        row_store<NC>(s_out + (size_t)r * D, lane, v);
+        row_store<T, NC, W>(s_out + (size_t)r * D, lane, D, v);
     if (mode == 0) {
-        row_store<NC>(y + (size_t)r * D, lane, v);
+        row_store<T, NC, W>(y + (size_t)r * D, lane, D, v);
         return;
     }
+    float gv[NC][W], bv[NC][W];
+    vec_load_f32<NC, W>(g, lane, D, gv);
+    vec_load_f32<NC, W>(b, lane, D, bv);
     float mu = 0.0f;
     if (mode == 1) {
         float sum = 0.0f;
 #pragma unroll
         for (int c = 0; c < NC; c++)
 #pragma unroll
-            for (int e = 0; e < 8; e++)
+            for (int e = 0; e < W; e++)
                 sum += v[c][e];
         mu = warp_sum(sum) / (float)D;
     }
     float var = 0.0f;
 #pragma unroll
-    for (int c = 0; c < NC; c++)
+    for (int c = 0; c < NC; c++) {
+        float part = 0.0f;
 #pragma unroll
-        for (int e = 0; e < 8; e++)
-            var += (v[c][e] - mu) * (v[c][e] - mu);
+        for (int e = 0; e < W; e++)
+            part += (v[c][e] - mu) * (v[c][e] - mu);
+        var += c * 32 * W + lane * W < D ? part : 0.0f;
+    }
     var = warp_sum(var) / (float)D;
     const float rstd = 1.0f / sqrtf(var + 1e-5f);
     if (stats && lane == 0) {
         stats[2 * r] = mu;
         stats[2 * r + 1] = rstd;
     }
-    float gv[NC][8], bv[NC][8];
-    vec_load_f32<NC>(g, lane, gv);
-    vec_load_f32<NC>(b, lane, bv);
 #pragma unroll
     for (int c = 0; c < NC; c++)
 #pragma unroll
-        for (int e = 0; e < 8; e++)
+        for (int e = 0; e < W; e++)
             v[c][e] = (v[c][e] - mu) * rstd * gv[c][e] + bv[c][e];
-    row_store<NC>(y + (size_t)r * D, lane, v);
+    row_store<T, NC, W>(y + (size_t)r * D, lane, D, v);
 }
 
-// norm_bwd_kernel for bf16 rows of D = NC * 256 elements: one row per warp, eight rows per block,
-// the block's column sums (dg, db, and the sums of the dx just written) go to part[block][3][D].
-template <int NC>
+// norm_bwd_kernel with the row in registers: every warp walks rpb / 8 rows and keeps its lanes'
+// column sums (dg, db and, if asked, the sums of the dx just written) in registers; the block's
+// sums go to part[block][3][D].  Several rows per warp keep the number of partial rows that the
+// reduction launch has to read near two per SM.
+template <typename T, int NC>
 __global__ void __launch_bounds__(256)
-norm_bwd_vec_kernel(const bf16 *__restrict__ dy, const bf16 *__restrict__ x, const float *__restrict__ g,
-                    const float *__restrict__ stats, const bf16 *__restrict__ base, bf16 *__restrict__ dx,
-                    float *__restrict__ part, int rows, int mode, int want_sum)
+norm_bwd_vec_kernel(const T *__restrict__ dy, const T *__restrict__ x, const float *__restrict__ g,
+                    const float *__restrict__ stats, const T *__restrict__ base, T *__restrict__ dx,
+                    float *__restrict__ part, int rows, int D, int mode, int rpb, int want_sum)
 {
     pdl_trigger();
     pdl_wait();
-    constexpr int D = NC * 256;
-    extern __shared__ float sm[]; // [8][3][D]
+    constexpr int W = RowVec<T>::W;
+    extern __shared__ float sm[]; // [8][D]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    float *mine = sm + (size_t)warp * 3 * D;
-    const int r = blockIdx.x * 8 + warp;
-    float xh[NC][8], d[NC][8], o[NC][8];
-    if (r < rows) {
+    // The row's operands stay packed as they came (NC 16-byte pieces each) and are unpacked at each use,
+    // and the gains are read again from the L1 cache: the sums alone are 3 * NC * W registers.
+    float dg[NC][W], db[NC][W], ds[NC][W];
+#pragma unroll
+    for (int c = 0; c < NC; c++)
+#pragma unroll
+        for (int e = 0; e < W; e++)
+            dg[c][e] = db[c][e] = ds[c][e] = 0.0f;
+    auto gain = [&](int c, int e4) {
+        const int at = c * 32 * W + lane * W + e4;
+        return at < D ? __ldg(reinterpret_cast<const float4 *>(g + at)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+    const int r_end = min(rows, (int)(blockIdx.x + 1) * rpb);
+    for (int r = blockIdx.x * rpb + warp; r < r_end; r += 8) {
+        uint4 xu[NC], du[NC], bu[NC];
         const float mu = stats[2 * r], rstd = stats[2 * r + 1];
-        float gv[NC][8];
-        row_load<NC>(x + (size_t)r * D, lane, xh);
-        row_load<NC>(dy + (size_t)r * D, lane, d);
-        vec_load_f32<NC>(g, lane, gv);
+#pragma unroll
+        for (int c = 0; c < NC; c++) {
+            const int at = c * 32 * W + lane * W;
+            xu[c] = du[c] = bu[c] = make_uint4(0u, 0u, 0u, 0u);
+            if (at < D) {
+                xu[c] = *reinterpret_cast<const uint4 *>(x + (size_t)r * D + at);
+                du[c] = *reinterpret_cast<const uint4 *>(dy + (size_t)r * D + at);
+                if (base)
+                    bu[c] = *reinterpret_cast<const uint4 *>(base + (size_t)r * D + at);
+            }
+        }
         float s1 = 0.0f, s2 = 0.0f;
 #pragma unroll
-        for (int c = 0; c < NC; c++)
+        for (int c = 0; c < NC; c++) {
+            const T *xp = reinterpret_cast<const T *>(&xu[c]), *dp = reinterpret_cast<const T *>(&du[c]);
 #pragma unroll
-            for (int e = 0; e < 8; e++) {
-                xh[c][e] = (xh[c][e] - mu) * rstd;
-                gv[c][e] *= d[c][e]; // dxh
-                s1 += gv[c][e];
-                s2 += gv[c][e] * xh[c][e];
+            for (int e4 = 0; e4 < W; e4 += 4) {
+                const float4 g4 = gain(c, e4);
+                const float gg[4] = {g4.x, g4.y, g4.z, g4.w};
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    const int e = e4 + k;
+                    const float xh = (to_f(xp[e]) - mu) * rstd, d = to_f(dp[e]), dxh = gg[k] * d;
+                    s1 += dxh;
+                    s2 += dxh * xh;
+                    dg[c][e] += xh * d;
+                    db[c][e] += d;
+                }
             }
+        }
         s1 = warp_sum(s1) / (float)D;
         s2 = warp_sum(s2) / (float)D;
         if (mode == 2)
             s1 = 0.0f;
-        if (base)
-            row_load<NC>(base + (size_t)r * D, lane, o);
 #pragma unroll
-        for (int c = 0; c < NC; c++)
+        for (int c = 0; c < NC; c++) {
+            const T *xp = reinterpret_cast<const T *>(&xu[c]), *dp = reinterpret_cast<const T *>(&du[c]),
+                    *bp = reinterpret_cast<const T *>(&bu[c]);
+            uint4 ou;
+            T *op = reinterpret_cast<T *>(&ou);
 #pragma unroll
-            for (int e = 0; e < 8; e++) {
-                const float vv = rstd * (gv[c][e] - s1 - xh[c][e] * s2);
-                o[c][e] = round_to<bf16>(base ? vv + o[c][e] : vv);
-                xh[c][e] *= d[c][e]; // dg contribution
+            for (int e4 = 0; e4 < W; e4 += 4) {
+                const float4 g4 = gain(c, e4);
+                const float gg[4] = {g4.x, g4.y, g4.z, g4.w};
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    const int e = e4 + k;
+                    const float xh = (to_f(xp[e]) - mu) * rstd;
+                    const float vv = rstd * (gg[k] * to_f(dp[e]) - s1 - xh * s2);
+                    op[e] = from_f<T>(base ? vv + to_f(bp[e]) : vv);
+                    ds[c][e] += to_f(op[e]);
+                }
             }
-        row_store<NC>(dx + (size_t)r * D, lane, o);
-    } else {
-#pragma unroll
-        for (int c = 0; c < NC; c++)
-#pragma unroll
-            for (int e = 0; e < 8; e++)
-                xh[c][e] = d[c][e] = o[c][e] = 0.0f;
-    }
-#pragma unroll
-    for (int c = 0; c < NC; c++)
-#pragma unroll
-        for (int e = 0; e < 8; e++) {
-            const int col = c * 256 + lane * 8 + e;
-            mine[col] = xh[c][e];
-            mine[D + col] = d[c][e];
-            mine[2 * D + col] = want_sum ? o[c][e] : 0.0f;
+            if (c * 32 * W + lane * W < D)
+                *reinterpret_cast<uint4 *>(dx + (size_t)r * D + c * 32 * W + lane * W) = ou;
         }
-    __syncthreads();
-    for (int i = threadIdx.x; i < 3 * D; i += blockDim.x) {
-        float s = 0.0f;
-#pragma unroll
-        for (int w = 0; w < 8; w++)
-            s += sm[(size_t)w * 3 * D + i];
-        part[(size_t)blockIdx.x * 3 * D + i] = s;
     }
+    // the eight warps' sums, one quantity after the other through one buffer
+    float *mine = sm + (size_t)warp * D;
+    auto fold = [&](const float (&v)[NC][W], int q) {
+        if (q)
+            __syncthreads();
+#pragma unroll
+        for (int c = 0; c < NC; c++) {
+            const int at = c * 32 * W + lane * W;
+            if (at < D)
+#pragma unroll
+                for (int e = 0; e < W; e += 4)
+                    *reinterpret_cast<float4 *>(mine + at + e) = make_float4(v[c][e], v[c][e + 1], v[c][e + 2], v[c][e + 3]);
+        }
+        __syncthreads();
+        for (int i = threadIdx.x; i < D; i += 256) {
+            float s = 0.0f;
+#pragma unroll
+            for (int w = 0; w < 8; w++)
+                s += sm[(size_t)w * D + i];
+            part[((size_t)blockIdx.x * 3 + q) * D + i] = s;
+        }
+    };
+    fold(dg, 0);
+    fold(db, 1);
+    if (want_sum)
+        fold(ds, 2);
 }
 
 // out[i] = ws[0][i] + ws[1][i] + ... (in that order) for the partial products of a split-K GEMM;
@@ -587,18 +644,26 @@ __global__ void act_fwd_vec_kernel(const bf16 *__restrict__ hpre, bf16 *__restri
 }
 
 // Adjoint of the activation, and (part != NULL) per-chunk column sums of the result for the
-// ff_bias1 gradient: part[chunk][F1].  grid (ceil(F/128), ceil(rows/32)); one column per thread.
+// ff_bias1 gradient: part[chunk][F1].  grid (ceil(F/128), ceil(rows/ACT_BWD_ROWS)); one column per
+// thread, short chains of rows (see act_bwd_vec_kernel).
+constexpr int ACT_BWD_ROWS = 8;
 template <typename T>
 __global__ void __launch_bounds__(128)
 act_bwd_kernel(const T *__restrict__ hpre, const T *__restrict__ dhact, T *__restrict__ dhpre,
                float *__restrict__ part, int rows, int F, int F1, int act)
 {
+    pdl_trigger();
+    pdl_wait();
     const int i = blockIdx.x * 128 + threadIdx.x;
     if (i >= F)
         return;
-    const int r0 = blockIdx.y * 32, r1 = min(rows, r0 + 32);
+    const int r0 = blockIdx.y * ACT_BWD_ROWS;
     float s0 = 0.0f, s1 = 0.0f;
-    for (int r = r0; r < r1; r++) {
+#pragma unroll
+    for (int rr = 0; rr < ACT_BWD_ROWS; rr++) {
+        const int r = r0 + rr;
+        if (r >= rows)
+            break;
         float a = to_f(hpre[(size_t)r * F1 + i]), d = to_f(dhact[(size_t)r * F + i]);
         if (act == NNCU_FF_RELU || act == NNCU_FF_GELU) {
             T o = from_f<T>(act == NNCU_FF_RELU ? (a > 0.0f ? d : 0.0f) : d * gelu_grad_f(a));
@@ -623,7 +688,6 @@ act_bwd_kernel(const T *__restrict__ hpre, const T *__restrict__ dhact, T *__res
 // Two columns per thread (4-byte accesses), ACT_BWD_ROWS rows per block (short serial chains:
 // the kernel is bound by the latency of its per-element math, not by bytes); element
 // arithmetic as in act_bwd_kernel.  F even; grid (ceil(F/256), ceil(rows/ACT_BWD_ROWS)).
-constexpr int ACT_BWD_ROWS = 8;
 __global__ void __launch_bounds__(128)
 act_bwd_vec_kernel(const bf16 *__restrict__ hpre, const bf16 *__restrict__ dhact, bf16 *__restrict__ dhpre,
                    float *__restrict__ part, int rows, int F, int F1, int act)
@@ -862,6 +926,7 @@ __global__ void colsum_part_kernel(const T *__restrict__ A, long lda, int R, int
         return;
     int r0 = blockIdx.y * rows_per, r1 = min(R, r0 + rows_per);
     float s = 0.0f;
+#pragma unroll 16 // the loads of sixteen rows are in flight together
     for (int r = r0; r < r1; r++)
         s += to_f(A[(long)r * lda + n]);
     part[(size_t)blockIdx.y * N + n] = s;

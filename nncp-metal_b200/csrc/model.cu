@@ -427,28 +427,39 @@ static int colsum(nncu_model *m, const AT *A, long lda, int R, int N, float *out
     return reduce_cols(m, part, chunks, N, N, out, 0);
 }
 
+// Rows whose length is a multiple of 16 bytes and that fit a warp's registers (16 KB of them over the
+// lanes: up to 2048 bf16 or 1024 fp32 elements) go through the one-pass kernels; f(NC) launches the one
+// for NC 512-byte chunks.
+template <typename AT> static bool norm_in_registers(int D, int max_chunks)
+{
+    return D % RowVec<AT>::W == 0 && D <= max_chunks * RowVec<AT>::CHUNK;
+}
+template <typename AT, typename F> static void with_chunks(int D, F f)
+{
+    switch (ceil_div(D, RowVec<AT>::CHUNK)) {
+    case 1: f(std::integral_constant<int, 1>()); break;
+    case 2: f(std::integral_constant<int, 2>()); break;
+    case 3: f(std::integral_constant<int, 3>()); break;
+    case 4: f(std::integral_constant<int, 4>()); break;
+    case 5: case 6: f(std::integral_constant<int, 6>()); break;
+    default: f(std::integral_constant<int, 8>()); break;
+    }
+}
+
 template <typename AT>
 static int norm_fwd(nncu_model *m, const AT *a, const AT *res, AT *s_out, AT *y, size_t g_off,
                     size_t b_off, float *stats, int rows, bool do_norm)
 {
     int mode = !do_norm ? 0 : ((m->p.ln_flags & NNCU_LN_RMSNORM) ? 2 : 1);
     const float *g = do_norm ? m->W + g_off : nullptr, *b = do_norm ? m->W + b_off : nullptr;
-    if (sizeof(AT) == 2 && (m->D == 256 || m->D == 512 || m->D == 1024 || m->D == 2048)) {
-        // rows that fit in a warp's registers: one pass, 16-byte accesses
-        const bf16 *a16 = (const bf16 *)a, *r16 = (const bf16 *)res;
-        bf16 *s16 = (bf16 *)s_out, *y16 = (bf16 *)y;
-        const dim3 grid(ceil_div(rows, 4)), block(128);
-        switch (m->D / 256) {
-        case 1: launch_k(residual_norm_vec_kernel<1>, grid, block, 0, m->st, a16, r16, s16, y16, g, b, stats, rows, mode); break;
-        case 2: launch_k(residual_norm_vec_kernel<2>, grid, block, 0, m->st, a16, r16, s16, y16, g, b, stats, rows, mode); break;
-        case 4: launch_k(residual_norm_vec_kernel<4>, grid, block, 0, m->st, a16, r16, s16, y16, g, b, stats, rows, mode); break;
-        default: launch_k(residual_norm_vec_kernel<8>, grid, block, 0, m->st, a16, r16, s16, y16, g, b, stats, rows, mode); break;
-        }
-        KERNEL_CHECK();
-        return NNCU_OK;
-    }
-    launch_k(residual_norm_kernel<AT>, dim3(ceil_div(rows, 4)), dim3(128), 0, m->st, a, res, s_out, y, g, b, stats,
-             rows, m->D, mode);
+    if (norm_in_registers<AT>(m->D, 8))
+        with_chunks<AT>(m->D, [&](auto nc) {
+            launch_k(residual_norm_vec_kernel<AT, decltype(nc)::value>, dim3(ceil_div(rows, 4)), dim3(128), 0, m->st, a, res,
+                     s_out, y, g, b, stats, rows, m->D, mode);
+        });
+    else
+        launch_k(residual_norm_kernel<AT>, dim3(ceil_div(rows, 4)), dim3(128), 0, m->st, a, res, s_out, y, g, b, stats,
+                 rows, m->D, mode);
     KERNEL_CHECK();
     return NNCU_OK;
 }
@@ -457,25 +468,22 @@ template <typename AT>
 static int norm_bwd(nncu_model *m, const AT *dy, const AT *x, size_t g_off, size_t b_off,
                     const float *stats, const AT *base, AT *dx, int rows, float *dxsum = nullptr)
 {
-    const int rpb = 8;
-    int blocks = ceil_div(rows, rpb);
     int mode = (m->p.ln_flags & NNCU_LN_RMSNORM) ? 2 : 1;
-    size_t smem = (size_t)8 * 3 * m->D * sizeof(float);
     float *part = part_slot(m);
-    if (sizeof(AT) == 2 && (m->D == 256 || m->D == 512 || m->D == 1024)) {
-        const bf16 *dy16 = (const bf16 *)dy, *x16 = (const bf16 *)x, *b16 = (const bf16 *)base;
-        bf16 *dx16 = (bf16 *)dx;
-        const float *g = m->W + g_off;
-        const int ws = dxsum ? 1 : 0;
-        switch (m->D / 256) {
-        case 1: launch_k(norm_bwd_vec_kernel<1>, dim3(blocks), dim3(256), smem, m->st, dy16, x16, g, stats, b16, dx16, part, rows, mode, ws); break;
-        case 2: launch_k(norm_bwd_vec_kernel<2>, dim3(blocks), dim3(256), smem, m->st, dy16, x16, g, stats, b16, dx16, part, rows, mode, ws); break;
-        default: launch_k(norm_bwd_vec_kernel<4>, dim3(blocks), dim3(256), smem, m->st, dy16, x16, g, stats, b16, dx16, part, rows, mode, ws); break;
-        }
-    } else {
-        launch_k(norm_bwd_kernel<AT>, dim3(blocks), dim3(256), smem, m->st, dy, x, m->W + g_off, stats, base, dx, part,
-                 rows, m->D, mode, rpb, dxsum ? 1 : 0);
-    }
+    const float *g = m->W + g_off;
+    const int ws = dxsum ? 1 : 0;
+    // eight warps a block, one row each, until the blocks are two per SM; then more rows per warp
+    const int rpb = 8 * std::max(1, ceil_div(rows, 8 * 2 * 148));
+    const int blocks = ceil_div(rows, rpb);
+    if (norm_in_registers<AT>(m->D, 4))
+        with_chunks<AT>(m->D, [&](auto nc) {
+            constexpr int NC = decltype(nc)::value <= 4 ? decltype(nc)::value : 4;
+            launch_k(norm_bwd_vec_kernel<AT, NC>, dim3(blocks), dim3(256), (size_t)8 * m->D * sizeof(float), m->st, dy, x, g,
+                     stats, base, dx, part, rows, m->D, mode, rpb, ws);
+        });
+    else
+        launch_k(norm_bwd_kernel<AT>, dim3(blocks), dim3(256), (size_t)8 * 3 * m->D * sizeof(float), m->st, dy, x, g, stats,
+                 base, dx, part, rows, m->D, mode, rpb, ws);
     KERNEL_CHECK();
     return reduce_cols(m, part, blocks, 3 * m->D, m->D, gf(m, g_off), 0, gf(m, b_off), m->D, dxsum, 2 * m->D);
 }
@@ -855,13 +863,13 @@ static int backward(nncu_model *m)
         NNCU_TRY(mm_nn(m, TB, F, D, dt2, D, o.ff2, dh, F, (const AT *)nullptr));
         float *apart = o.ff_bias1 != NONE ? part_slot(m) : nullptr;
         const bool act_vec = sizeof(AT) == 2 && F % 2 == 0;
-        const int act_rows = act_vec ? ACT_BWD_ROWS : 32;
+        const int act_rows = ACT_BWD_ROWS;
         if (act_vec)
             launch_k(act_bwd_vec_kernel, dim3(ceil_div(F, 256), ceil_div(TB, act_rows)), dim3(128), 0, m->st,
                      (const bf16 *)atc<AT>(a.hpre, 0), (const bf16 *)dh, (bf16 *)dhp, apart, TB, F, F1, p.ff_act);
         else
-            act_bwd_kernel<AT><<<dim3(ceil_div(F, 128), ceil_div(TB, act_rows)), 128, 0, m->st>>>(
-                atc<AT>(a.hpre, 0), dh, dhp, apart, TB, F, F1, p.ff_act);
+            launch_k(act_bwd_kernel<AT>, dim3(ceil_div(F, 128), ceil_div(TB, act_rows)), dim3(128), 0, m->st,
+                     atc<AT>(a.hpre, 0), (const AT *)dh, dhp, apart, TB, F, F1, p.ff_act);
         KERNEL_CHECK();
         if (apart)
             NNCU_TRY(reduce_cols(m, apart, ceil_div(TB, act_rows), F1, F1, gf(m, o.ff_bias1), 0));
@@ -1426,8 +1434,6 @@ int nncu_create(const nncu_params *p, nncu_model **out)
     if ((size_t)8 * 3 * D * 4 > 48 * 1024) {
         cudaFuncSetAttribute(norm_bwd_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * 3 * D * 4);
         cudaFuncSetAttribute(norm_bwd_kernel<bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * 3 * D * 4);
-        if (D == 1024)
-            cudaFuncSetAttribute(norm_bwd_vec_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * 3 * D * 4);
     }
     if ((size_t)2 * V * 4 > 48 * 1024 && (size_t)2 * V * 4 <= 200 * 1024) {
         cudaFuncSetAttribute(coder_paths_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * V * 4);
