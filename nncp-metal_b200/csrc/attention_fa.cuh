@@ -1,0 +1,1070 @@
+// attention_fa.cuh -- bf16 relative-position attention for head sizes 16, 32, 64 and 128 on
+// warp-level tensor-core instructions (mma.sync m16n8k16, fp32 accumulation).
+//
+// Same math as attention.cuh (nncp.c:722-800 and its adjoint).  Per (stream, head) the
+// contractions are 64 queries x 64-key blocks x head size, a few hundred warp-level products; what
+// bounds the op is the chain load -> scores -> softmax -> product, not the tensor rate (measured
+// 544 TFLOP/s for mma.sync on this part, of which the op needs a quarter).  A warp's products need
+// no hand-off through tensor memory and barriers, two CTAs share an SM, and the relative shift is a
+// 3 KB round trip through shared memory private to the warp.  The tcgen05 kernels these replace
+// spent 47 k cycles per 128-key block of a stream pair (64 streams x 16 heads, 320 keys: backward
+// 330 us, forward 70 us a launch).
+//
+// Geometry.  Keys go in blocks of 64 counted from key 0, queries in groups of 64 rows, a warp owns
+// 16 rows.  Query i0 + ii and key j0 + jj meet table row max(wlo + w, 0), w = jj + 63 - ii, with
+// wlo = j0 - i0 + P - M - 64: the window of a block is 128 table rows (rows below the table are
+// loaded as row 0, which is what the left pad duplicates), and the next block's window starts 64
+// rows further on.
+//
+// Association, the same for every launch: a block's maximum, sum and output are taken by
+// themselves (probabilities relative to the block's own maximum, output chain over the block's
+// keys from zero), even and odd blocks are merged in ascending order into two running results, and
+// the odd result is merged into the even one.  A block in which a row sees nothing leaves the
+// running result unchanged bit for bit.  So whole segments and single queries, which go through
+// different kernels, give the same bits.
+#pragma once
+#include "attention.cuh"
+
+namespace fa {
+
+constexpr int KB = 64;  // keys per block
+constexpr int ESC = 52; // floats per row of a warp's skew scratch (48 used)
+
+__device__ __forceinline__ uint32_t smem_addr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void ldsm4(uint32_t (&r)[4], const bf16 *p)
+{
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(smem_addr(p)));
+}
+__device__ __forceinline__ void ldsm4t(uint32_t (&r)[4], const bf16 *p)
+{
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(smem_addr(p)));
+}
+__device__ __forceinline__ void mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1)
+{
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 "
+                 "{%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ uint32_t pack2(float lo, float hi)
+{
+    const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t *>(&h);
+}
+__device__ __forceinline__ float ex2(float x)
+{
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ void cp16(void *dst, const void *src, bool valid)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_addr(dst)), "l"(src), "r"(valid ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// 4 x 4 transpose of 32-bit values over the four lanes of a quad: lane t ends with what lane u held in
+// v[t] at v[u] (turns four 4-byte column pairs per lane into one 16-byte run per lane)
+__device__ __forceinline__ void quad_transpose(uint32_t (&v)[4], int t)
+{
+    const bool o1 = t & 1, o2 = t & 2;
+    uint32_t a = o1 ? v[0] : v[1], b = o1 ? v[2] : v[3];
+    a = __shfl_xor_sync(0xffffffffu, a, 1);
+    b = __shfl_xor_sync(0xffffffffu, b, 1);
+    if (o1) { v[0] = a; v[2] = b; } else { v[1] = a; v[3] = b; }
+    a = o2 ? v[0] : v[2];
+    b = o2 ? v[1] : v[3];
+    a = __shfl_xor_sync(0xffffffffu, a, 2);
+    b = __shfl_xor_sync(0xffffffffu, b, 2);
+    if (o2) { v[0] = a; v[1] = b; } else { v[2] = a; v[3] = b; }
+}
+
+// One row of a warp tile out as bf16: lane t of the quad holds columns nt * 8 + 2t, + 1 of the N / 8
+// column groups in x[nt][c], x[nt][c + 1].  Rows of 32 columns and more leave in 16-byte pieces.
+template <int NT> __device__ __forceinline__ void store_row(bf16 *dst, const float (&x)[NT][4], int c, int t, bool act)
+{
+    if constexpr (NT % 4 == 0) {
+#pragma unroll
+        for (int n4 = 0; n4 < NT; n4 += 4) {
+            uint32_t v[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++)
+                v[u] = pack2(x[n4 + u][c], x[n4 + u][c + 1]);
+            quad_transpose(v, t);
+            if (act)
+                *reinterpret_cast<uint4 *>(dst + (n4 + t) * 8) = make_uint4(v[0], v[1], v[2], v[3]);
+        }
+    } else {
+#pragma unroll
+        for (int nt = 0; nt < NT; nt++)
+            if (act)
+                *reinterpret_cast<uint32_t *>(dst + nt * 8 + 2 * t) = pack2(x[nt][c], x[nt][c + 1]);
+    }
+}
+
+// rows [0, rows) of a bf16 matrix (row pitch `pitch`) -> shared tile, zero where !valid(r)
+template <int DK, typename F>
+__device__ __forceinline__ void load_rows(bf16 *dst, const bf16 *src, size_t pitch, int rows, int tid, int nthr, F valid)
+{
+    constexpr int LD = DK + 8, CPR = DK / 8;
+    for (int idx = tid; idx < rows * CPR; idx += nthr) {
+        const int r = idx / CPR, c = (idx % CPR) * 8;
+        const bool ok = valid(r);
+        cp16(dst + r * LD + c, ok ? src + (size_t)r * pitch + c : src, ok);
+    }
+}
+// rows x0 .. x0 + rows - 1 of one head's position table, clamped to [0, P)
+template <int DK>
+__device__ __forceinline__ void load_table(bf16 *dst, const AttnArgs &a, int h, int x0, int rows, int tid, int nthr)
+{
+    constexpr int LD = DK + 8, CPR = DK / 8;
+    const bf16 *w16 = reinterpret_cast<const bf16 *>(a.w_r16) + (size_t)h * a.P * DK;
+    const float *w32 = a.w_r + (size_t)h * a.P * DK;
+    for (int idx = tid; idx < rows * CPR; idx += nthr) {
+        const int r = idx / CPR, c = (idx % CPR) * 8;
+        const int x = min(max(x0 + r, 0), a.P - 1);
+        if (a.w_r16) {
+            cp16(dst + r * LD + c, w16 + (size_t)x * DK + c, true);
+        } else {
+            const float4 u = *reinterpret_cast<const float4 *>(w32 + (size_t)x * DK + c);
+            const float4 v = *reinterpret_cast<const float4 *>(w32 + (size_t)x * DK + c + 4);
+            *reinterpret_cast<uint4 *>(dst + r * LD + c) = make_uint4(pack2(u.x, u.y), pack2(u.z, u.w), pack2(v.x, v.y), pack2(v.z, v.w));
+        }
+    }
+}
+
+struct Blocks {
+    int lo, hi; // first and last key block with a visible pair for query rows [t0, t1)
+};
+__host__ __device__ inline Blocks blocks_of(int M, int L, int attn_len, int t0, int t1)
+{
+    int jlo = t0 + M - attn_len + 1, jhi = t1 - 1 + M;
+    jlo = jlo < 0 ? 0 : jlo;
+    jhi = jhi > L - 1 ? L - 1 : jhi;
+    return Blocks{jlo / KB, jhi / KB};
+}
+
+// (m, l, o) <- (m, l, o) merged with a block's (mb, lb, ob); scale() gives the two factors
+struct Merge {
+    float al, be;
+};
+__device__ __forceinline__ Merge merge_scale(float &m, float &l, float mb, float lb)
+{
+    const float mn = fmaxf(m, mb), mu = mn == -INFINITY ? 0.0f : mn;
+    Merge s;
+    s.al = ex2(__fsub_rn(m, mu));
+    s.be = ex2(__fsub_rn(mb, mu));
+    l = __fmaf_rn(l, s.al, __fmul_rn(lb, s.be));
+    m = mn;
+    return s;
+}
+__device__ __forceinline__ float merge_o(float o, float ob, const Merge &s) { return __fmaf_rn(o, s.al, __fmul_rn(ob, s.be)); }
+
+// b_r of one head in the log2 domain, [0, L)
+__device__ __forceinline__ void load_br(float *brs, const AttnArgs &a, int h, int tid, int nthr)
+{
+    const float f = a.inv_sqrt * 1.4426950408889634f;
+    for (int r = tid; r < a.L; r += nthr)
+        brs[r] = __fmul_rn(__fmul_rn(a.br_scale, a.b_r[(size_t)h * a.L + r]), f);
+}
+
+// E of a warp's 16 rows (16 * qt ..) against 32 keys (32 * hf ..) of a block, skewed into the layout
+// of the score fragments: e[nt][c] belongs to key 32 hf + 8 nt + 2 t + (c & 1), row g + 8 (c >> 1).
+// window(p): the 16 rows of piece p of the block's window (row 16 p).
+template <int DK, typename W>
+__device__ __forceinline__ void skewed_positions(float (&e)[4][4], const bf16 *Qt, W window, int qt, int hf, float *es, int lane)
+{
+    constexpr int LD = DK + 8;
+    const int g = lane >> 2, t = lane & 3;
+    float x[6][4];
+#pragma unroll
+    for (int n = 0; n < 6; n++)
+#pragma unroll
+        for (int c = 0; c < 4; c++)
+            x[n][c] = 0.0f;
+#pragma unroll
+    for (int ks = 0; ks < DK / 16; ks++) {
+        uint32_t q[4];
+        ldsm4(q, Qt + (lane & 15) * LD + ks * 16 + (lane >> 4) * 8);
+#pragma unroll
+        for (int p = 0; p < 3; p++) {
+            uint32_t b[4];
+            ldsm4(b, window(2 * hf + 3 - qt + p) + ((lane & 7) + (lane >> 4) * 8) * LD + ks * 16 + ((lane >> 3) & 1) * 8);
+            mma(x[2 * p], q, b[0], b[1]);
+            mma(x[2 * p + 1], q, b[2], b[3]);
+        }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int n = 0; n < 6; n++) {
+        *reinterpret_cast<float2 *>(es + g * ESC + n * 8 + 2 * t) = make_float2(x[n][0], x[n][1]);
+        *reinterpret_cast<float2 *>(es + (g + 8) * ESC + n * 8 + 2 * t) = make_float2(x[n][2], x[n][3]);
+    }
+    __syncwarp();
+#pragma unroll
+    for (int n = 0; n < 4; n++)
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            const int row = g + (c >> 1) * 8;
+            e[n][c] = es[row * ESC + n * 8 + 2 * t + (c & 1) + 15 - row];
+        }
+}
+
+// s[nt][c] (same layout) = rows of At (16 rows) against 32 rows of Bt
+template <int DK>
+__device__ __forceinline__ void product_16x32(float (&s)[4][4], const bf16 *At, const bf16 *Bt, int lane)
+{
+    constexpr int LD = DK + 8;
+#pragma unroll
+    for (int n = 0; n < 4; n++)
+#pragma unroll
+        for (int c = 0; c < 4; c++)
+            s[n][c] = 0.0f;
+#pragma unroll
+    for (int ks = 0; ks < DK / 16; ks++) {
+        uint32_t q[4];
+        ldsm4(q, At + (lane & 15) * LD + ks * 16 + (lane >> 4) * 8);
+#pragma unroll
+        for (int p = 0; p < 2; p++) {
+            uint32_t b[4];
+            ldsm4(b, Bt + (p * 16 + (lane & 7) + (lane >> 4) * 8) * LD + ks * 16 + ((lane >> 3) & 1) * 8);
+            mma(s[2 * p], q, b[0], b[1]);
+            mma(s[2 * p + 1], q, b[2], b[3]);
+        }
+    }
+}
+
+// ---------------- forward, a group of queries ----------------
+//
+// One CTA per (stream, head, 64 queries): warps 0-3 take the even key blocks, warps 4-7 the odd ones,
+// each warp one 16-row tile.  102 KB of shared memory at head size 64, so two CTAs share an SM.
+template <int DK> struct FwdSmem {
+    static constexpr int LD = DK + 8, TILE = 64 * LD * 2;
+    static constexpr int Q = 0, K = TILE, V = K + 2 * TILE, R = V + 2 * TILE, ES = R + 3 * TILE, BRS = ES + 8 * 16 * ESC * 4;
+    static size_t bytes(int L) { return (size_t)BRS + (size_t)((L + 3) & ~3) * 4; }
+};
+
+template <int DK>
+__global__ void __launch_bounds__(256, DK <= 64 ? 2 : 1) attn_fwd_kernel(const __grid_constant__ AttnArgs a)
+{
+    using SM = FwdSmem<DK>;
+    constexpr int LD = SM::LD, NT = DK / 8;
+    extern __shared__ __align__(16) unsigned char sm[];
+    bf16 *Qs = reinterpret_cast<bf16 *>(sm + SM::Q), *Ks = reinterpret_cast<bf16 *>(sm + SM::K),
+         *Vs = reinterpret_cast<bf16 *>(sm + SM::V), *Rs = reinterpret_cast<bf16 *>(sm + SM::R);
+    float *brs = reinterpret_cast<float *>(sm + SM::BRS);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int qt = warp & 3, set = warp >> 2;
+    const int b = blockIdx.x / a.H, h = blockIdx.x % a.H, HD = a.H * DK, T = a.T, M = a.M, L = a.L;
+    const int i0 = (a.t0 & ~63) + blockIdx.y * 64;
+    const int ta = max(i0, a.t0), tb = min(i0 + 64, a.t1);
+    const Blocks blk = blocks_of(M, L, a.attn_len, ta, tb);
+    float *es = reinterpret_cast<float *>(sm + SM::ES) + warp * 16 * ESC;
+    pdl_trigger();
+    pdl_wait();
+
+    const bf16 *q = reinterpret_cast<const bf16 *>(a.q) + ((size_t)i0 * a.B + b) * a.qp + h * DK;
+    const bf16 *kv = reinterpret_cast<const bf16 *>(a.kv) + (size_t)b * a.kvp + h * DK;
+    load_rows<DK>(Qs, q, (size_t)a.B * a.qp, 64, threadIdx.x, 256, [&](int r) { return i0 + r >= a.t0 && i0 + r < a.t1; });
+    load_br(brs, a, h, threadIdx.x, 256);
+    const float sc2 = a.inv_sqrt * 1.4426950408889634f;
+    const int iA = i0 + qt * 16 + g, iB = iA + 8; // this thread's two rows
+    const bool active = i0 + qt * 16 < a.t1 && i0 + qt * 16 + 16 > a.t0;
+
+    float o[NT][4], mA = -INFINITY, mB = -INFINITY, lA = 0.0f, lB = 0.0f;
+#pragma unroll
+    for (int n = 0; n < NT; n++)
+#pragma unroll
+        for (int c = 0; c < 4; c++)
+            o[n][c] = 0.0f;
+
+    for (int pr = blk.lo >> 1; pr <= blk.hi >> 1; pr++) {
+        const int j00 = pr * 2 * KB;
+        if (pr != blk.lo >> 1)
+            __syncthreads(); // the pair before has been read
+        for (int s = 0; s < 2; s++) {
+            const int j0 = j00 + s * KB;
+            if (pr * 2 + s < blk.lo || pr * 2 + s > blk.hi)
+                continue;
+            load_rows<DK>(Ks + s * 64 * LD, kv + (size_t)j0 * a.B * a.kvp, (size_t)a.B * a.kvp, 64, threadIdx.x, 256,
+                          [&](int r) { return j0 + r < L; });
+            load_rows<DK>(Vs + s * 64 * LD, kv + HD + (size_t)j0 * a.B * a.kvp, (size_t)a.B * a.kvp, 64, threadIdx.x, 256,
+                          [&](int r) { return j0 + r < L; });
+        }
+        if (a.w_r)
+            load_table<DK>(Rs, a, h, j00 - i0 + a.P - M - 64, 192, threadIdx.x, 256);
+        cp_commit();
+        cp_wait<0>();
+        __syncthreads();
+        const int kb = pr * 2 + set, j0 = kb * KB;
+        if (!active || kb < blk.lo || kb > blk.hi)
+            continue;
+        // scores of 16 rows x 64 keys, log2 domain, masked
+        uint32_t pf[4][4]; // probabilities as the A fragments of the value product
+        float s[2][4][4], mbA = -INFINITY, mbB = -INFINITY;
+#pragma unroll
+        for (int hf = 0; hf < 2; hf++) {
+            product_16x32<DK>(s[hf], Qs + qt * 16 * LD, Ks + (set * 64 + hf * 32) * LD, lane);
+            if (a.w_r) {
+                float e[4][4];
+                skewed_positions<DK>(e, Qs + qt * 16 * LD, [&](int p) { return Rs + (set * 64 + p * 16) * LD; }, qt, hf, es, lane);
+#pragma unroll
+                for (int n = 0; n < 4; n++)
+#pragma unroll
+                    for (int c = 0; c < 4; c++)
+                        s[hf][n][c] = __fadd_rn(s[hf][n][c], e[n][c]);
+            }
+#pragma unroll
+            for (int n = 0; n < 4; n++)
+#pragma unroll
+                for (int c = 0; c < 4; c++) {
+                    const int j = j0 + hf * 32 + n * 8 + 2 * t + (c & 1), i = c < 2 ? iA : iB;
+                    const int d = i + M - j; // visible iff 0 <= d < attn_len
+                    const float v = __fmaf_rn(s[hf][n][c], sc2, brs[min(max(j + T - 1 - i, 0), L - 1)]);
+                    s[hf][n][c] = (unsigned)d < (unsigned)a.attn_len ? v : -INFINITY;
+                }
+#pragma unroll
+            for (int n = 0; n < 4; n++) {
+                mbA = fmaxf(mbA, fmaxf(s[hf][n][0], s[hf][n][1]));
+                mbB = fmaxf(mbB, fmaxf(s[hf][n][2], s[hf][n][3]));
+            }
+        }
+        mbA = fmaxf(mbA, __shfl_xor_sync(0xffffffffu, mbA, 1));
+        mbB = fmaxf(mbB, __shfl_xor_sync(0xffffffffu, mbB, 1));
+        mbA = fmaxf(mbA, __shfl_xor_sync(0xffffffffu, mbA, 2));
+        mbB = fmaxf(mbB, __shfl_xor_sync(0xffffffffu, mbB, 2));
+        const float uA = mbA == -INFINITY ? 0.0f : mbA, uB = mbB == -INFINITY ? 0.0f : mbB;
+        float sumA = 0.0f, sumB = 0.0f;
+#pragma unroll
+        for (int n = 0; n < 8; n++) {
+            float(&x)[4] = s[n >> 2][n & 3];
+            x[0] = ex2(__fsub_rn(x[0], uA));
+            x[1] = ex2(__fsub_rn(x[1], uA));
+            x[2] = ex2(__fsub_rn(x[2], uB));
+            x[3] = ex2(__fsub_rn(x[3], uB));
+            sumA = __fadd_rn(sumA, __fadd_rn(x[0], x[1]));
+            sumB = __fadd_rn(sumB, __fadd_rn(x[2], x[3]));
+            pf[n >> 1][(n & 1) * 2] = pack2(x[0], x[1]);
+            pf[n >> 1][(n & 1) * 2 + 1] = pack2(x[2], x[3]);
+        }
+        sumA = __fadd_rn(sumA, __shfl_xor_sync(0xffffffffu, sumA, 1));
+        sumB = __fadd_rn(sumB, __shfl_xor_sync(0xffffffffu, sumB, 1));
+        sumA = __fadd_rn(sumA, __shfl_xor_sync(0xffffffffu, sumA, 2));
+        sumB = __fadd_rn(sumB, __shfl_xor_sync(0xffffffffu, sumB, 2));
+        const Merge fA = merge_scale(mA, lA, mbA, sumA), fB = merge_scale(mB, lB, mbB, sumB);
+        // the block's output, 32 columns (16 at head size 16) at a time
+        constexpr int NP = NT < 4 ? NT : 4;
+#pragma unroll
+        for (int n0 = 0; n0 < NT; n0 += NP) {
+            float ob[NP][4];
+#pragma unroll
+            for (int n = 0; n < NP; n++)
+#pragma unroll
+                for (int c = 0; c < 4; c++)
+                    ob[n][c] = 0.0f;
+#pragma unroll
+            for (int ks = 0; ks < 4; ks++)
+#pragma unroll
+                for (int p = 0; p < NP / 2; p++) {
+                    uint32_t bb[4];
+                    ldsm4t(bb, Vs + (set * 64 + ks * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * LD + n0 * 8 + p * 16 + (lane >> 4) * 8);
+                    mma(ob[2 * p], pf[ks], bb[0], bb[1]);
+                    mma(ob[2 * p + 1], pf[ks], bb[2], bb[3]);
+                }
+#pragma unroll
+            for (int n = 0; n < NP; n++) {
+                o[n0 + n][0] = merge_o(o[n0 + n][0], ob[n][0], fA);
+                o[n0 + n][1] = merge_o(o[n0 + n][1], ob[n][1], fA);
+                o[n0 + n][2] = merge_o(o[n0 + n][2], ob[n][2], fB);
+                o[n0 + n][3] = merge_o(o[n0 + n][3], ob[n][3], fB);
+            }
+        }
+    }
+    // the odd blocks' result goes to the warps of the even ones through the K tiles
+    __syncthreads();
+    float *xo = reinterpret_cast<float *>(sm + SM::K) + qt * 32 * (NT * 4 + 4);
+    if (set == 1) {
+#pragma unroll
+        for (int n = 0; n < NT; n++)
+#pragma unroll
+            for (int c = 0; c < 4; c++)
+                xo[(n * 4 + c) * 32 + lane] = o[n][c];
+        xo[(NT * 4) * 32 + lane] = mA;
+        xo[(NT * 4 + 1) * 32 + lane] = mB;
+        xo[(NT * 4 + 2) * 32 + lane] = lA;
+        xo[(NT * 4 + 3) * 32 + lane] = lB;
+    }
+    __syncthreads();
+    if (set == 1 || !active)
+        return;
+    const float m1A = xo[(NT * 4) * 32 + lane], m1B = xo[(NT * 4 + 1) * 32 + lane];
+    const Merge fA = merge_scale(mA, lA, m1A, xo[(NT * 4 + 2) * 32 + lane]), fB = merge_scale(mB, lB, m1B, xo[(NT * 4 + 3) * 32 + lane]);
+    const float rA = __fdiv_rn(1.0f, lA), rB = __fdiv_rn(1.0f, lB);
+#pragma unroll
+    for (int n = 0; n < NT; n++)
+#pragma unroll
+        for (int c = 0; c < 4; c++)
+            o[n][c] = __fmul_rn(merge_o(o[n][c], xo[(n * 4 + c) * 32 + lane], c < 2 ? fA : fB), c < 2 ? rA : rB);
+    bf16 *out = reinterpret_cast<bf16 *>(a.o) + ((size_t)iA * a.B + b) * HD + h * DK;
+    const bool okA = iA >= a.t0 && iA < a.t1, okB = iB >= a.t0 && iB < a.t1;
+    store_row<NT>(out, o, 0, t, okA);
+    store_row<NT>(out + (size_t)8 * a.B * HD, o, 2, t, okB);
+    if (t == 0 && a.lse) {
+        float *lse = a.lse + ((size_t)b * a.H + h) * T;
+        if (okA)
+            lse[iA] = (mA + __log2f(lA)) * 0.6931471805599453f;
+        if (okB)
+            lse[iB] = (mB + __log2f(lB)) * 0.6931471805599453f;
+    }
+}
+
+// ---------------- forward, one query ----------------
+//
+// A decoding step: one query per stream, so the op is a stream of K and V through the chip (126 MB a
+// layer at 128 streams x 8 heads x 576 keys) and what bounds it is HBM.  One CTA of four warps per
+// (stream, head); a warp takes every fourth key block by itself (its own tiles, no barrier), so that
+// 220 KB an SM are in flight.  The operand roles are exchanged: keys (and table rows, of which a
+// single query needs exactly one per key) fill the 16 rows of a product, the query is the other
+// operand, broadcast to its 8 columns; a product of 16 terms gives the same bits either way round.
+template <int DK> struct OneSmem {
+    static constexpr int LD = DK + 8, TILE = 64 * LD * 2;
+    static constexpr int W = 3 * TILE + 64 * 4; // a warp's K, V, table rows and probabilities
+    static constexpr int RES = 4 * W;
+    static size_t bytes(int nb) { return (size_t)RES + (size_t)nb * (DK + 2) * 4; }
+};
+
+template <int DK>
+__global__ void __launch_bounds__(128) attn_one_kernel(const __grid_constant__ AttnArgs a)
+{
+    using SM = OneSmem<DK>;
+    constexpr int LD = SM::LD;
+    extern __shared__ __align__(16) unsigned char sm[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    bf16 *Ks = reinterpret_cast<bf16 *>(sm + warp * SM::W), *Vs = Ks + 64 * LD, *Rs = Vs + 64 * LD;
+    float *ps = reinterpret_cast<float *>(Rs + 64 * LD);
+    float *res = reinterpret_cast<float *>(sm + SM::RES);
+    const int b = blockIdx.x / a.H, h = blockIdx.x % a.H, HD = a.H * DK, T = a.T, M = a.M, L = a.L, i = a.t0;
+    const Blocks blk = blocks_of(M, L, a.attn_len, i, i + 1);
+    const int nb = blk.hi - blk.lo + 1;
+    pdl_trigger();
+    pdl_wait();
+    const bf16 *kv = reinterpret_cast<const bf16 *>(a.kv) + (size_t)b * a.kvp + h * DK;
+    const float sc2 = a.inv_sqrt * 1.4426950408889634f;
+    auto fetch = [&](int kb) {
+        const int j0 = kb * KB;
+        load_rows<DK>(Ks, kv + (size_t)j0 * a.B * a.kvp, (size_t)a.B * a.kvp, 64, lane, 32, [&](int r) { return j0 + r < L; });
+        load_rows<DK>(Vs, kv + HD + (size_t)j0 * a.B * a.kvp, (size_t)a.B * a.kvp, 64, lane, 32, [&](int r) { return j0 + r < L; });
+        if (a.w_r)
+            load_table<DK>(Rs, a, h, j0 - i + a.P - M - 1, 64, lane, 32);
+        cp_commit();
+    };
+    if (warp < nb)
+        fetch(blk.lo + warp);
+    // the query as the second operand: k = 2t, 2t + 1 (+ 8) of every 16-wide slice, the same for all columns
+    uint32_t qf[DK / 16][2];
+    {
+        const bf16 *q = reinterpret_cast<const bf16 *>(a.q) + ((size_t)i * a.B + b) * a.qp + h * DK;
+#pragma unroll
+        for (int ks = 0; ks < DK / 16; ks++) {
+            qf[ks][0] = *reinterpret_cast<const uint32_t *>(q + ks * 16 + 2 * t);
+            qf[ks][1] = *reinterpret_cast<const uint32_t *>(q + ks * 16 + 8 + 2 * t);
+        }
+    }
+    for (int kbi = warp; kbi < nb; kbi += 4) {
+        const int j0 = (blk.lo + kbi) * KB;
+        cp_wait<0>();
+        __syncwarp();
+        float s[4][2], mb = -INFINITY; // keys 16 m + g, + 8
+#pragma unroll
+        for (int m = 0; m < 4; m++) {
+            float x[4] = {0.0f, 0.0f, 0.0f, 0.0f}, e[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+            for (int ks = 0; ks < DK / 16; ks++) {
+                uint32_t k4[4];
+                ldsm4(k4, Ks + (m * 16 + (lane & 15)) * LD + ks * 16 + (lane >> 4) * 8);
+                mma(x, k4, qf[ks][0], qf[ks][1]);
+                if (a.w_r) {
+                    ldsm4(k4, Rs + (m * 16 + (lane & 15)) * LD + ks * 16 + (lane >> 4) * 8);
+                    mma(e, k4, qf[ks][0], qf[ks][1]);
+                }
+            }
+#pragma unroll
+            for (int c = 0; c < 2; c++) {
+                const int j = j0 + m * 16 + g + c * 8, d = i + M - j, r = min(max(j + T - 1 - i, 0), L - 1);
+                float v = x[2 * c];
+                if (a.w_r)
+                    v = __fadd_rn(v, e[2 * c]);
+                const float br = __fmul_rn(__fmul_rn(a.br_scale, __ldg(a.b_r + (size_t)h * L + r)), sc2);
+                v = __fmaf_rn(v, sc2, br);
+                s[m][c] = (unsigned)d < (unsigned)a.attn_len ? v : -INFINITY;
+                mb = fmaxf(mb, s[m][c]);
+            }
+        }
+        mb = fmaxf(mb, __shfl_xor_sync(0xffffffffu, mb, 4));
+        mb = fmaxf(mb, __shfl_xor_sync(0xffffffffu, mb, 8));
+        mb = fmaxf(mb, __shfl_xor_sync(0xffffffffu, mb, 16));
+        const float u = mb == -INFINITY ? 0.0f : mb;
+#pragma unroll
+        for (int m = 0; m < 4; m++)
+#pragma unroll
+            for (int c = 0; c < 2; c++)
+                if (t == 0)
+                    ps[m * 16 + g + c * 8] = ex2(__fsub_rn(s[m][c], u));
+        __syncwarp();
+        // the sum in the order of the 16-row kernel: column pairs of a lane, then the quad
+        float sum = 0.0f;
+        uint32_t pf[4][2];
+#pragma unroll
+        for (int n = 0; n < 8; n++) {
+            const float2 x = *reinterpret_cast<const float2 *>(ps + n * 8 + 2 * t);
+            sum = __fadd_rn(sum, __fadd_rn(x.x, x.y));
+            pf[n >> 1][n & 1] = pack2(x.x, x.y);
+        }
+        sum = __fadd_rn(sum, __shfl_xor_sync(0xffffffffu, sum, 1));
+        sum = __fadd_rn(sum, __shfl_xor_sync(0xffffffffu, sum, 2));
+        float *rb = res + (size_t)kbi * (DK + 2);
+#pragma unroll
+        for (int m = 0; m < DK / 16; m++) {
+            float x[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+            for (int ks = 0; ks < 4; ks++) {
+                uint32_t v4[4]; // V^T: rows are columns of V, so the 8 x 8 blocks come transposed
+                ldsm4t(v4, Vs + (ks * 16 + (lane & 7) + (lane >> 4) * 8) * LD + m * 16 + ((lane >> 3) & 1) * 8);
+                mma(x, v4, pf[ks][0], pf[ks][1]);
+            }
+            if (t == 0) {
+                rb[m * 16 + g] = x[0];
+                rb[m * 16 + g + 8] = x[2];
+            }
+        }
+        if (lane == 0) {
+            rb[DK] = mb;
+            rb[DK + 1] = sum;
+        }
+        __syncwarp(); // the tiles have been read
+        if (kbi + 4 < nb)
+            fetch(blk.lo + kbi + 4);
+    }
+    __syncthreads();
+    for (int d = threadIdx.x; d < DK; d += 128) {
+        auto chain = [&](int par, float &m, float &l) { // the blocks of one parity, ascending
+            float o = 0.0f;
+            m = -INFINITY;
+            l = 0.0f;
+            for (int kbi = (blk.lo ^ par) & 1; kbi < nb; kbi += 2) {
+                const float *rb = res + (size_t)kbi * (DK + 2);
+                const Merge f = merge_scale(m, l, rb[DK], rb[DK + 1]);
+                o = merge_o(o, rb[d], f);
+            }
+            return o;
+        };
+        float m0, l0, m1, l1;
+        const float o0 = chain(0, m0, l0), o1 = chain(1, m1, l1);
+        const Merge f = merge_scale(m0, l0, m1, l1);
+        const float v = __fmul_rn(merge_o(o0, o1, f), __fdiv_rn(1.0f, l0));
+        reinterpret_cast<bf16 *>(a.o)[((size_t)i * a.B + b) * HD + h * DK + d] = __float2bfloat16_rn(v);
+        if (d == 0 && a.lse)
+            a.lse[((size_t)b * a.H + h) * T + i] = (m0 + __log2f(l0)) * 0.6931471805599453f;
+    }
+}
+
+// ---------------- backward ----------------
+//
+// One CTA of eight warps per (stream, head), key blocks in ascending order; per block
+//
+//   A   warp (q tile, key half): scores and table products again, P = exp(a - lse), dP = dO V^T,
+//       dS = P (dP - D) / sqrt(dk); P, dS and the inverse-skewed dE (row ii, window column jj + 63 - ii)
+//       go to shared memory as bf16
+//   B1  dQ += dS K + dE Rwin                 (registers over all blocks; 16 rows x half the columns)
+//   B2  dV = P^T dO, dK = dS^T Q             (complete for the block: stored)
+//       dR += dE^T Q and the column sums of dE, per 64-row group of the table
+//
+// A table group is touched by two consecutive blocks only (upper half of one window, lower half of
+// the next), so warps 0-3 keep the even groups' sums in registers and warps 4-7 the odd ones', and
+// every table row is stored once; nothing is read back.  Rows that stand for table row 0 (the
+// left pad) are folded into it at the end.  K, the table window and V of the next block are fetched
+// as soon as phases B1 and A have read the present ones.  109 KB of shared memory at head size 64:
+// two CTAs per SM.
+template <int DK> struct BwdSmem {
+    static constexpr int LD = DK + 8, TILE = 64 * LD * 2;
+    static constexpr int LPS = 152, LDE = 136; // row pitches: [P 64 | pad 8 | dS 64 | pad 16], dE window
+    static constexpr int Q = 0, DO = Q + TILE, K = DO + TILE, V = K + TILE, R = V + TILE, PS = R + 2 * TILE,
+                         DE = PS + 64 * LPS * 2, ES = DE + 64 * LDE * 2, ROW = ES + 4 * 16 * ESC * 4, PAD = ROW + 2 * 64 * 4, BRS = PAD + 8 * DK * 4;
+    static size_t bytes(int L) { return (size_t)BRS + (size_t)((L + 3) & ~3) * 4; }
+};
+
+template <int DK>
+__global__ void __launch_bounds__(256, DK <= 64 ? 2 : 1) attn_bwd_kernel(const __grid_constant__ AttnArgs a)
+{
+    using SM = BwdSmem<DK>;
+    constexpr int LD = SM::LD, LPS = SM::LPS, LDE = SM::LDE;
+    constexpr int NCH = DK >= 32 ? 2 : 1, NTC = DK / 8 / NCH; // column halves of dQ, dV, dK; 8-column groups in one
+    constexpr int NT = DK / 8;
+    extern __shared__ __align__(16) unsigned char sm[];
+    bf16 *Qs = reinterpret_cast<bf16 *>(sm + SM::Q), *Os = reinterpret_cast<bf16 *>(sm + SM::DO),
+         *Ks = reinterpret_cast<bf16 *>(sm + SM::K), *Vs = reinterpret_cast<bf16 *>(sm + SM::V),
+         *Rs = reinterpret_cast<bf16 *>(sm + SM::R), *PS = reinterpret_cast<bf16 *>(sm + SM::PS),
+         *DE = reinterpret_cast<bf16 *>(sm + SM::DE);
+    float *lse2 = reinterpret_cast<float *>(sm + SM::ROW), *Dr = lse2 + 64, *brs = reinterpret_cast<float *>(sm + SM::BRS);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int qt = warp & 3, hf = warp >> 2; // phase A: q tile, key half; B: row tile, column half or table set
+    const int b = blockIdx.x / a.H, h = blockIdx.x % a.H, HD = a.H * DK, T = a.T, M = a.M, L = a.L, P = a.P;
+    const Blocks blk = blocks_of(M, L, a.attn_len, 0, T);
+    const int nqt = (T + 15) >> 4; // q tiles in use
+    // skew scratch: the warps of key half 0 use their tile's rows of PS (written after both warps of the tile
+    // have read their scratch), the others an area of their own
+    float *es = hf == 0 ? reinterpret_cast<float *>(PS + qt * 16 * LPS) : reinterpret_cast<float *>(sm + SM::ES) + qt * 16 * ESC;
+    pdl_trigger();
+    pdl_wait();
+
+    const bf16 *kv = reinterpret_cast<const bf16 *>(a.kv) + (size_t)b * a.kvp + h * DK;
+    const bf16 *dout = reinterpret_cast<const bf16 *>(a.dout) + (size_t)b * HD + h * DK;
+    const bf16 *outp = reinterpret_cast<const bf16 *>(a.out) + (size_t)b * HD + h * DK;
+    bf16 *dkv = reinterpret_cast<bf16 *>(a.dkv) + (size_t)b * a.dkvp + h * DK;
+    float *dwr = (a.w_r && a.dwr_part) ? a.dwr_part + ((size_t)b * a.H + h) * P * DK : nullptr;
+    float *dbr = a.dbr_part ? a.dbr_part + ((size_t)b * a.H + h) * L : nullptr;
+    auto window0 = [&](int kb) { return kb * KB + P - M - 64; }; // table row of window row 0
+    auto fetch_k = [&](int kb) {
+        const int j0 = kb * KB;
+        load_rows<DK>(Ks, kv + (size_t)j0 * a.B * a.kvp, (size_t)a.B * a.kvp, 64, threadIdx.x, 256, [&](int r) { return j0 + r < L; });
+    };
+    auto fetch_v = [&](int kb) {
+        const int j0 = kb * KB;
+        load_rows<DK>(Vs, kv + HD + (size_t)j0 * a.B * a.kvp, (size_t)a.B * a.kvp, 64, threadIdx.x, 256, [&](int r) { return j0 + r < L; });
+    };
+    // table group gr (window rows 0-63 of block gr, 64-127 of block gr - 1) into its slot of the two
+    auto fetch_r = [&](int gr) {
+        if (a.w_r)
+            load_table<DK>(Rs + (gr & 1) * 64 * LD, a, h, window0(gr), 64, threadIdx.x, 256);
+    };
+    load_rows<DK>(Qs, reinterpret_cast<const bf16 *>(a.q) + (size_t)b * a.qp + h * DK, (size_t)a.B * a.qp, 64, threadIdx.x, 256,
+                  [&](int r) { return r < T; });
+    load_rows<DK>(Os, dout, (size_t)a.B * HD, 64, threadIdx.x, 256, [&](int r) { return r < T; });
+    fetch_k(blk.lo);
+    fetch_v(blk.lo);
+    fetch_r(blk.lo);
+    fetch_r(blk.lo + 1);
+    cp_commit();
+    load_br(brs, a, h, threadIdx.x, 256);
+    // D_i = dO_i . O_i and the log-sum-exp in the log2 domain: four lanes a row
+    {
+        const int r = threadIdx.x >> 2;
+        float D = 0.0f;
+        if (r < T) {
+            const bf16 *x = outp + (size_t)r * a.B * HD, *y = dout + (size_t)r * a.B * HD;
+#pragma unroll
+            for (int e = (threadIdx.x & 3) * 4; e < DK; e += 16) {
+                const float4 u = load_f4(x + e), v = load_f4(y + e);
+                D += (u.x * v.x + u.y * v.y) + (u.z * v.z + u.w * v.w);
+            }
+        }
+        D += __shfl_xor_sync(0xffffffffu, D, 1);
+        D += __shfl_xor_sync(0xffffffffu, D, 2);
+        if ((threadIdx.x & 3) == 0) {
+            Dr[r] = D;
+            lse2[r] = r < T ? a.lse[((size_t)b * a.H + h) * T + r] * 1.4426950408889634f : 0.0f;
+        }
+    }
+    // outside the rows' bands the dE window is zero for every block; unused q tiles of P, dS and dE stay zero
+    for (int idx = threadIdx.x; idx < (64 * LPS + 64 * LDE) / 8; idx += 256)
+        reinterpret_cast<uint4 *>(PS)[idx] = make_uint4(0u, 0u, 0u, 0u);
+    // what no block reaches: keys' gradients, table rows, b_r slots
+    for (int kb = 0; kb * KB < L; kb++) {
+        if (kb >= blk.lo && kb <= blk.hi)
+            continue;
+        for (int idx = threadIdx.x; idx < 64 * (DK / 8); idx += 256) {
+            const int j = kb * KB + idx / (DK / 8), c = (idx % (DK / 8)) * 8;
+            if (j < L) {
+                *reinterpret_cast<uint4 *>(dkv + (size_t)j * a.B * a.dkvp + c) = make_uint4(0u, 0u, 0u, 0u);
+                *reinterpret_cast<uint4 *>(dkv + (size_t)j * a.B * a.dkvp + HD + c) = make_uint4(0u, 0u, 0u, 0u);
+            }
+        }
+    }
+    const int x_lo = window0(blk.lo), x_hi = window0(blk.hi) + 127, r_off = T - P + M; // b_r slot = table row + r_off
+    if (dwr)
+        for (int idx = threadIdx.x; idx < P * DK / 4; idx += 256) {
+            const int x = idx / (DK / 4);
+            if (x < x_lo || x > x_hi)
+                reinterpret_cast<float4 *>(dwr)[idx] = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    if (dbr)
+        for (int r = threadIdx.x; r < L; r += 256)
+            if (r < x_lo + r_off || r > x_hi + r_off)
+                dbr[r] = 0.0f;
+
+    const float sc2 = a.inv_sqrt * 1.4426950408889634f;
+    float dq[NTC][4], dr[NT][4], cs[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+    for (int n = 0; n < NTC; n++)
+#pragma unroll
+        for (int c = 0; c < 4; c++)
+            dq[n][c] = 0.0f;
+#pragma unroll
+    for (int n = 0; n < NT; n++)
+#pragma unroll
+        for (int c = 0; c < 4; c++)
+            dr[n][c] = 0.0f;
+    // this warp's share of table row 0: its window rows at or below it
+    float *pad = reinterpret_cast<float *>(sm + SM::PAD) + warp * DK;
+    for (int d = lane; d < DK; d += 32)
+        pad[d] = 0.0f;
+    // the finished sums of table group gr (this warp: its rows 16 qt ..) out, and the registers cleared
+    auto store_group = [&](int gr) {
+        const int xA = window0(gr) + qt * 16 + g, xB = xA + 8;
+        if (dwr) {
+#pragma unroll
+            for (int n = 0; n < NT; n++) {
+                if (xA > 0 && xA < P)
+                    *reinterpret_cast<float2 *>(dwr + (size_t)xA * DK + n * 8 + 2 * t) = make_float2(dr[n][0], dr[n][1]);
+                if (xB > 0 && xB < P)
+                    *reinterpret_cast<float2 *>(dwr + (size_t)xB * DK + n * 8 + 2 * t) = make_float2(dr[n][2], dr[n][3]);
+            }
+            if (window0(gr) + qt * 16 <= 0) { // the same for the whole warp
+#pragma unroll
+                for (int n = 0; n < NT; n++)
+#pragma unroll
+                    for (int c = 0; c < 2; c++) {
+                        float v = (xA <= 0 ? dr[n][c] : 0.0f) + (xB <= 0 ? dr[n][c + 2] : 0.0f);
+                        v += __shfl_xor_sync(0xffffffffu, v, 4);
+                        v += __shfl_xor_sync(0xffffffffu, v, 8);
+                        v += __shfl_xor_sync(0xffffffffu, v, 16);
+                        if (g == 0)
+                            pad[n * 8 + 2 * t + c] += v;
+                    }
+            }
+        }
+        if (dbr && t == 0) {
+            const int rA = xA + r_off, rB = xB + r_off;
+            if (rA >= 0 && rA < L)
+                dbr[rA] = a.br_scale * cs[0];
+            if (rB >= 0 && rB < L)
+                dbr[rB] = a.br_scale * cs[2];
+        }
+#pragma unroll
+        for (int n = 0; n < NT; n++)
+#pragma unroll
+            for (int c = 0; c < 4; c++)
+                dr[n][c] = 0.0f;
+        cs[0] = cs[1] = cs[2] = cs[3] = 0.0f;
+    };
+    const int iA = qt * 16 + g, iB = iA + 8;
+    cp_wait<0>();
+    __syncthreads();
+
+    for (int kb = blk.lo; kb <= blk.hi; kb++) {
+        const int j0 = kb * KB;
+        auto window = [&](int p) { return Rs + (((kb + (p >> 2)) & 1) * 64 + (p & 3) * 16) * LD; }; // piece p of the window
+        // ---- A
+        if (qt < nqt) {
+            float s[4][4], e[4][4];
+            product_16x32<DK>(s, Qs + qt * 16 * LD, Ks + hf * 32 * LD, lane);
+            if (a.w_r) {
+                skewed_positions<DK>(e, Qs + qt * 16 * LD, window, qt, hf, es, lane);
+#pragma unroll
+                for (int n = 0; n < 4; n++)
+#pragma unroll
+                    for (int c = 0; c < 4; c++)
+                        s[n][c] = __fadd_rn(s[n][c], e[n][c]);
+            }
+            const float lA = lse2[iA], lB = lse2[iB], DA = Dr[iA], DB = Dr[iB];
+#pragma unroll
+            for (int n = 0; n < 4; n++)
+#pragma unroll
+                for (int c = 0; c < 4; c++) {
+                    const int j = j0 + hf * 32 + n * 8 + 2 * t + (c & 1), i = c < 2 ? iA : iB, d = i + M - j;
+                    const float v = __fmaf_rn(s[n][c], sc2, brs[min(max(j + T - 1 - i, 0), L - 1)]);
+                    const bool vis = (unsigned)d < (unsigned)a.attn_len && i < T;
+                    s[n][c] = vis ? ex2(v - (c < 2 ? lA : lB)) : 0.0f;
+                }
+            product_16x32<DK>(e, Os + qt * 16 * LD, Vs + hf * 32 * LD, lane); // dP
+            asm volatile("bar.sync %0, 64;" ::"r"(1 + qt) : "memory"); // both warps of the tile are done with their scratch
+            bf16 *pA = PS + (qt * 16 + g) * LPS + hf * 32 + 2 * t, *pB = pA + 8 * LPS;
+#pragma unroll
+            for (int n = 0; n < 4; n++) {
+                const uint32_t wA = pack2(s[n][0], s[n][1]), wB = pack2(s[n][2], s[n][3]);
+                *reinterpret_cast<uint32_t *>(pA + n * 8) = wA;
+                *reinterpret_cast<uint32_t *>(pB + n * 8) = wB;
+                // dS with the probabilities as the products see them
+                const __nv_bfloat162 hA = *reinterpret_cast<const __nv_bfloat162 *>(&wA), hB = *reinterpret_cast<const __nv_bfloat162 *>(&wB);
+                const __nv_bfloat162 dA = __floats2bfloat162_rn(__low2float(hA) * (e[n][0] - DA) * a.inv_sqrt,
+                                                                __high2float(hA) * (e[n][1] - DA) * a.inv_sqrt);
+                const __nv_bfloat162 dB = __floats2bfloat162_rn(__low2float(hB) * (e[n][2] - DB) * a.inv_sqrt,
+                                                                __high2float(hB) * (e[n][3] - DB) * a.inv_sqrt);
+                *reinterpret_cast<__nv_bfloat162 *>(pA + 72 + n * 8) = dA;
+                *reinterpret_cast<__nv_bfloat162 *>(pB + 72 + n * 8) = dB;
+                // window column of key jj is jj + 63 - ii: odd rows' pairs are aligned, even rows' are not
+                const int w = hf * 32 + n * 8 + 2 * t + 63 - iA;
+                bf16 *eA = DE + iA * LDE + w, *eB = DE + iB * LDE + w - 8;
+                if (iA & 1) {
+                    *reinterpret_cast<__nv_bfloat162 *>(eA) = dA;
+                    *reinterpret_cast<__nv_bfloat162 *>(eB) = dB;
+                } else {
+                    eA[0] = dA.x; eA[1] = dA.y;
+                    eB[0] = dB.x; eB[1] = dB.y;
+                }
+            }
+        }
+        __syncthreads(); // P, dS, dE complete; V has been read
+        if (kb < blk.hi)
+            fetch_v(kb + 1);
+        // ---- B1: dQ of rows 16 qt .., columns of half hf
+        if (qt < nqt && hf < NCH) {
+            const bf16 *arow = PS + (qt * 16 + (lane & 15)) * LPS + 72 + (lane >> 4) * 8;
+            const int vrow = (lane & 7) + ((lane >> 3) & 1) * 8, vcol = hf * (DK / 2) * (NCH - 1) + (lane >> 4) * 8;
+#pragma unroll
+            for (int ks = 0; ks < 4; ks++) {
+                uint32_t x[4];
+                ldsm4(x, arow + ks * 16);
+#pragma unroll
+                for (int p = 0; p < NTC / 2; p++) {
+                    uint32_t bb[4];
+                    ldsm4t(bb, Ks + (ks * 16 + vrow) * LD + vcol + p * 16);
+                    mma(dq[2 * p], x, bb[0], bb[1]);
+                    mma(dq[2 * p + 1], x, bb[2], bb[3]);
+                }
+            }
+            if (a.w_r) {
+                const bf16 *erow = DE + (qt * 16 + (lane & 15)) * LDE + (lane >> 4) * 8;
+#pragma unroll
+                for (int pc = 0; pc < 5; pc++) { // the five pieces of the window that the tile's band touches
+                    const int pp = 3 - qt + pc;
+                    uint32_t x[4];
+                    ldsm4(x, erow + pp * 16);
+                    const bf16 *rw = window(pp) + vrow * LD + vcol;
+#pragma unroll
+                    for (int p = 0; p < NTC / 2; p++) {
+                        uint32_t bb[4];
+                        ldsm4t(bb, rw + p * 16);
+                        mma(dq[2 * p], x, bb[0], bb[1]);
+                        mma(dq[2 * p + 1], x, bb[2], bb[3]);
+                    }
+                }
+            }
+        }
+        __syncthreads(); // K and the table window have been read
+        if (kb < blk.hi) {
+            fetch_k(kb + 1);
+            fetch_r(kb + 2); // the slot of group kb
+        }
+        cp_commit();
+        // ---- B2: dV and dK of keys j0 + 16 qt .., columns of half hf
+        if (hf < NCH) {
+            const bf16 *pcol = PS + ((lane & 7) + (lane >> 4) * 8) * LPS + qt * 16 + ((lane >> 3) & 1) * 8;
+            const int vrow = (lane & 7) + ((lane >> 3) & 1) * 8, vcol = hf * (DK / 2) * (NCH - 1) + (lane >> 4) * 8;
+#pragma unroll
+            for (int which = 0; which < 2; which++) { // 0: dV = P^T dO, 1: dK = dS^T Q
+                const bf16 *ac = pcol + which * 72, *bm = (which ? Qs : Os) + vrow * LD + vcol;
+                float acc[NTC][4];
+#pragma unroll
+                for (int n = 0; n < NTC; n++)
+#pragma unroll
+                    for (int c = 0; c < 4; c++)
+                        acc[n][c] = 0.0f;
+                for (int ks = 0; ks < nqt; ks++) {
+                    uint32_t x[4];
+                    ldsm4t(x, ac + ks * 16 * LPS);
+#pragma unroll
+                    for (int p = 0; p < NTC / 2; p++) {
+                        uint32_t bb[4];
+                        ldsm4t(bb, bm + ks * 16 * LD + p * 16);
+                        mma(acc[2 * p], x, bb[0], bb[1]);
+                        mma(acc[2 * p + 1], x, bb[2], bb[3]);
+                    }
+                }
+                const int jA = j0 + qt * 16 + g, jB = jA + 8;
+                bf16 *dst = dkv + (which ? 0 : HD) + hf * (DK / 2) * (NCH - 1) + (size_t)(jA < L ? jA : 0) * a.B * a.dkvp;
+                store_row<NTC>(dst, acc, 0, t, jA < L);
+                dst += (size_t)(jB < L ? 8 : 0) * a.B * a.dkvp;
+                store_row<NTC>(dst, acc, 2, t, jB < L);
+            }
+        }
+        // dR and the column sums of one table group: the lower one (window columns 0-63) belongs to the warps of
+        // set kb & 1, the upper one to the others
+        {
+            const bool upper = hf != (kb & 1);
+            const int piece = (upper ? 4 : 0) + qt, k0 = upper ? 0 : 3 - qt, k1 = min(nqt, upper ? 4 - qt : 4); // q tiles whose band meets the piece
+            const bf16 *ecol = DE + ((lane & 7) + (lane >> 4) * 8) * LDE + piece * 16 + ((lane >> 3) & 1) * 8;
+            const bf16 *qrow = Qs + ((lane & 7) + ((lane >> 3) & 1) * 8) * LD + (lane >> 4) * 8;
+            for (int ks = k0; ks < k1; ks++) {
+                uint32_t x[4];
+                ldsm4t(x, ecol + ks * 16 * LDE);
+                mma(cs, x, 0x3F803F80u, 0x3F803F80u);
+                if (dwr) {
+#pragma unroll
+                    for (int p = 0; p < NT / 2; p++) {
+                        uint32_t bb[4];
+                        ldsm4t(bb, qrow + ks * 16 * LD + p * 16);
+                        mma(dr[2 * p], x, bb[0], bb[1]);
+                        mma(dr[2 * p + 1], x, bb[2], bb[3]);
+                    }
+                }
+            }
+            if (!upper)
+                store_group(kb);
+            else if (kb == blk.hi)
+                store_group(kb + 1);
+        }
+        cp_wait<0>();
+        __syncthreads(); // the next block's tiles have landed; P, dS and dE may be written again
+    }
+    if (qt < nqt && hf < NCH) {
+        bf16 *dst = reinterpret_cast<bf16 *>(a.dq) + ((size_t)(iA < T ? iA : 0) * a.B + b) * a.dqp + h * DK + hf * (DK / 2) * (NCH - 1);
+        store_row<NTC>(dst, dq, 0, t, iA < T);
+        dst += (size_t)(iB < T ? 8 : 0) * a.B * a.dqp;
+        store_row<NTC>(dst, dq, 2, t, iB < T);
+    }
+    if (dwr && x_lo <= 0) // table row 0: the warps' shares, in warp order (the loop's last barrier is behind them)
+        for (int d = threadIdx.x; d < DK; d += 256) {
+            const float *all = reinterpret_cast<const float *>(sm + SM::PAD);
+            float v = 0.0f;
+#pragma unroll
+            for (int w = 0; w < 8; w++)
+                v += all[w * DK + d];
+            dwr[d] = v;
+        }
+}
+
+// ---------------- host side ----------------
+
+// head sizes and operand placements the kernels take (16-byte loads and stores everywhere)
+inline bool head_size(int dk) { return dk == 16 || dk == 32 || dk == 64 || dk == 128; }
+inline bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+inline bool supported(const AttnArgs &a)
+{
+    return head_size(a.dk) && a.qp % 8 == 0 && a.kvp % 8 == 0 && aligned16(a.q) && aligned16(a.kv) && aligned16(a.o) &&
+           aligned16(a.w_r) && aligned16(a.w_r16);
+}
+inline bool supported_bwd(const AttnArgs &a)
+{
+    return supported(a) && a.T <= 64 && a.t0 == 0 && a.t1 == a.T && a.dqp % 8 == 0 && a.dkvp % 8 == 0 && aligned16(a.dq) &&
+           aligned16(a.dkv) && aligned16(a.dout) && aligned16(a.out) && aligned16(a.dwr_part) && a.lse;
+}
+// shared memory both kernels of a shape need
+inline bool fits(int dk, int L)
+{
+    const size_t most = 227 * 1024;
+    switch (dk) {
+    case 16: return FwdSmem<16>::bytes(L) <= most && BwdSmem<16>::bytes(L) <= most;
+    case 32: return FwdSmem<32>::bytes(L) <= most && BwdSmem<32>::bytes(L) <= most;
+    case 64: return FwdSmem<64>::bytes(L) <= most && BwdSmem<64>::bytes(L) <= most;
+    default: return FwdSmem<128>::bytes(L) <= most && BwdSmem<128>::bytes(L) <= most;
+    }
+}
+
+template <int DK> static int forward_dk(const AttnArgs &a, cudaStream_t st)
+{
+    const Blocks one = blocks_of(a.M, a.L, a.attn_len, a.t0, a.t1);
+    const size_t smem1 = OneSmem<DK>::bytes(one.hi - one.lo + 1), smem = FwdSmem<DK>::bytes(a.L);
+    static bool attr_done = false;
+    if (!attr_done) {
+        CUDA_TRY(cudaFuncSetAttribute(attn_fwd_kernel<DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+        CUDA_TRY(cudaFuncSetAttribute(attn_one_kernel<DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+        attr_done = true;
+    }
+    if (a.t1 - a.t0 == 1 && smem1 <= 227 * 1024)
+        launch_k(attn_one_kernel<DK>, dim3(a.B * a.H), dim3(128), smem1, st, a);
+    else
+        launch_k(attn_fwd_kernel<DK>, dim3(a.B * a.H, (a.t1 - (a.t0 & ~63) + 63) / 64), dim3(256), smem, st, a);
+    KERNEL_CHECK();
+    return NNCU_OK;
+}
+template <int DK> static int backward_dk(const AttnArgs &a, cudaStream_t st)
+{
+    static bool attr_done = false;
+    if (!attr_done) {
+        CUDA_TRY(cudaFuncSetAttribute(attn_bwd_kernel<DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+        attr_done = true;
+    }
+    launch_k(attn_bwd_kernel<DK>, dim3(a.B * a.H), dim3(256), BwdSmem<DK>::bytes(a.L), st, a);
+    KERNEL_CHECK();
+    return NNCU_OK;
+}
+static int forward(const AttnArgs &a, cudaStream_t st)
+{
+    switch (a.dk) {
+    case 16: return forward_dk<16>(a, st);
+    case 32: return forward_dk<32>(a, st);
+    case 64: return forward_dk<64>(a, st);
+    default: return forward_dk<128>(a, st);
+    }
+}
+static int backward(const AttnArgs &a, cudaStream_t st)
+{
+    switch (a.dk) {
+    case 16: return backward_dk<16>(a, st);
+    case 32: return backward_dk<32>(a, st);
+    case 64: return backward_dk<64>(a, st);
+    default: return backward_dk<128>(a, st);
+    }
+}
+
+} // namespace fa
+
+// ---- dispatch: bf16 goes to the tensor-core kernels when the shape allows, everything else to the
+// CUDA-core kernels of attention.cuh.  The choice depends on the shape only, never on the query
+// range, so one-symbol steps and whole segments take the same arithmetic.
+template <typename T>
+static int attn_forward_any(const nncu_attn_shape *s, const void *q, const void *kv, const float *w_r,
+                            const float *b_r, void *out, float *lse, cudaStream_t st,
+                            const AttnPitch *pt = nullptr, const void *w_r16 = nullptr)
+{
+    if (sizeof(T) == 2) {
+        AttnArgs a = attn_args(s, pt);
+        a.q = q; a.kv = kv; a.w_r = w_r; a.b_r = b_r; a.o = out; a.lse = lse;
+        a.w_r16 = w_r ? w_r16 : nullptr;
+        if (fa::supported(a) && fa::fits(a.dk, a.L))
+            return fa::forward(a, st);
+    }
+    return attn_forward_t<T>(s, q, kv, w_r, b_r, out, lse, st, pt);
+}
+
+template <typename T>
+static int attn_backward_any(const nncu_attn_shape *s, const void *q, const void *kv, const float *w_r,
+                             const float *b_r, const void *out, const float *lse, const void *dout,
+                             void *dq, void *dkv, float *dwr_part, float *dbr_part, cudaStream_t st,
+                             const AttnPitch *pt = nullptr, const void *w_r16 = nullptr)
+{
+    if (sizeof(T) == 2) {
+        AttnArgs a = attn_args(s, pt);
+        a.w_r16 = w_r ? w_r16 : nullptr;
+        a.q = q; a.kv = kv; a.w_r = w_r; a.b_r = b_r; a.out = out; a.lse = const_cast<float *>(lse);
+        a.dout = dout; a.dq = dq; a.dkv = dkv; a.dwr_part = dwr_part; a.dbr_part = dbr_part;
+        if (fa::supported_bwd(a) && fa::fits(a.dk, a.L))
+            return fa::backward(a, st);
+    }
+    return attn_backward_t<T>(s, q, kv, w_r, b_r, out, lse, dout, dq, dkv, dwr_part, dbr_part, st, pt);
+}
+
+// Whether some kernel pair can run the forward and the backward pass of this shape (asked once,
+// when a model is created, so that an unsupported shape is refused there and not in the middle
+// of a file).  Mirrors the dispatch of attn_forward_any / attn_backward_any.
+template <typename T>
+static int attn_shape_supported(const nncu_attn_shape *s, bool has_wr)
+{
+    AttnArgs a = attn_args(s, nullptr);
+    const bool tensor = sizeof(T) == 2 && fa::head_size(a.dk) && fa::fits(a.dk, a.L);
+    if (!tensor) {
+        size_t smem = 0;
+        fwd_pitch<T>(a, has_wr, smem);
+        if (smem > 227 * 1024)
+            return nncu_fail(NNCU_ERR_RANGE,
+                             "attention forward of this shape (%d keys, d_pos %d, d_key %d) needs %zu bytes of "
+                             "shared memory; the limit is %d",
+                             a.L, a.P, a.dk, smem, 227 * 1024);
+    }
+    if (!(tensor && a.T <= 64)) {
+        size_t smem = 0;
+        bwd_pitch<T>(a, has_wr, smem);
+        if (smem > 227 * 1024)
+            return nncu_fail(NNCU_ERR_RANGE,
+                             "attention backward of this shape (seg_len %d, %d keys, d_pos %d, d_key %d) needs %zu "
+                             "bytes of shared memory; the limit is %d",
+                             a.T, a.L, a.P, a.dk, smem, 227 * 1024);
+    }
+    return NNCU_OK;
+}

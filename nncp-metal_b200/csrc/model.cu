@@ -1,7 +1,7 @@
 // model.cu -- the Transformer-XL train step behind the C ABI of include/nncu.h.
 //
 // Host-side orchestration only; every number is produced by the kernels in
-// gemm_simt.cuh, gemm_tc.cuh, attention.cuh, kernels.cuh and coder.cuh.
+// gemm_simt.cuh, gemm_tc.cuh, attention.cuh, attention_fa.cuh, kernels.cuh and coder.cuh.
 //
 //   forward_range    trf_eval            nncp.c:581-1029
 //   backward         trf_eval_gradient   nncp.c:1099-1193 (hand-derived adjoint)
@@ -28,7 +28,7 @@
 #include <string>
 #include <vector>
 
-#include "attention_mma.cuh"
+#include "attention_fa.cuh"
 #include "coder.cuh"
 
 // ceil(log2 V): the depth of the coder's tree for any alphabet (its heap has 1 << depth slots per row)
@@ -598,7 +598,7 @@ static int forward_range(nncu_model *m, int t0, int t1)
         const AttnPitch pt = {3 * HD, 3 * HD, 3 * HD, 3 * HD};
         NNCU_TRY(attn_forward_any<AT>(&s, at<AT>(a.qkv, (size_t)M * B * 3 * HD), at<AT>(a.qkv, HD),
                                       wf(m, o.w_r), m->W + o.b_r, a.o, a.lse, m->st, &pt,
-                                      (m->bf && o.w_r != NONE) ? m->Wb + o.w_r : nullptr, m->err_flag));
+                                      (m->bf && o.w_r != NONE) ? m->Wb + o.w_r : nullptr));
         // output projection, residual, post-LN (nncp.c:865-920)
         if (o.alpha != NONE) { // LN_COEF: the projection is kept as it is for the backward pass, tmp = alpha * it
             AT *ao = at<AT>(a.ao, (size_t)r0 * D);
@@ -903,7 +903,7 @@ static int backward(nncu_model *m)
         nncu_attn_shape s = attn_shape(m, l, 0, m->T);
         NNCU_TRY(attn_backward_any<AT>(&s, at<AT>(a.qkv, (size_t)M * B * 3 * HD), at<AT>(a.qkv, HD), wf(m, o.w_r),
                                        m->W + o.b_r, a.o, a.lse, dof, dq, dkv, m->dwr_part, m->dbr_part, m->st,
-                                       &pt, (m->bf && o.w_r != NONE) ? m->Wb + o.w_r : nullptr, m->err_flag));
+                                       &pt, (m->bf && o.w_r != NONE) ? m->Wb + o.w_r : nullptr));
         {
             // the partials are next written after the join at the layer's end
             size_t nb = (size_t)m->H * m->L;
@@ -2386,14 +2386,6 @@ static int gemm_flag_check(int *flag, cudaStream_t st)
     return NNCU_OK;
 }
 
-#ifdef NNCU_ATTN_TRACE
-extern "C" int nncu_attn_trace(long long *dev_buf)
-{
-    CUDA_TRY(cudaMemcpyToSymbol(amma::g_attn_trace, &dev_buf, sizeof(dev_buf)));
-    CUDA_TRY(cudaMemcpyToSymbol(attc::g_trace, &dev_buf, sizeof(dev_buf)));
-    return NNCU_OK;
-}
-#endif
 #ifdef NNCU_GEMM_TRACE
 extern "C" int nncu_gemm_trace(long long *dev_buf)
 {
