@@ -16,12 +16,11 @@
 // loaded as row 0, which is what the left pad duplicates), and the next block's window starts 64
 // rows further on.
 //
-// Association, the same for every launch: a block's maximum, sum and output are taken by
-// themselves (probabilities relative to the block's own maximum, output chain over the block's
-// keys from zero), even and odd blocks are merged in ascending order into two running results, and
-// the odd result is merged into the even one.  A block in which a row sees nothing leaves the
-// running result unchanged bit for bit.  So whole segments and single queries, which go through
-// different kernels, give the same bits.
+// Association, the same for every launch: key blocks in ascending order; a block's probabilities are
+// taken relative to the running maximum, the running output is rescaled and the block's products
+// continue its chain (16 keys a step), a row's sum is kept in four parts (columns 2t, 2t + 1 of every
+// eight) that meet at the end.  A block in which a row sees nothing changes no bit.  So whole
+// segments and single queries, which go through different kernels, give the same bits.
 #pragma once
 #include "attention.cuh"
 
@@ -54,12 +53,6 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi)
 {
     const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<const uint32_t *>(&h);
-}
-__device__ __forceinline__ float ex2(float x)
-{
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
 }
 __device__ __forceinline__ void cp16(void *dst, const void *src, bool valid)
 {
@@ -149,28 +142,17 @@ __host__ __device__ inline Blocks blocks_of(int M, int L, int attn_len, int t0, 
     return Blocks{jlo / KB, jhi / KB};
 }
 
-// (m, l, o) <- (m, l, o) merged with a block's (mb, lb, ob); scale() gives the two factors
-struct Merge {
-    float al, be;
-};
-__device__ __forceinline__ Merge merge_scale(float &m, float &l, float mb, float lb)
-{
-    const float mn = fmaxf(m, mb), mu = mn == -INFINITY ? 0.0f : mn;
-    Merge s;
-    s.al = ex2(__fsub_rn(m, mu));
-    s.be = ex2(__fsub_rn(mb, mu));
-    l = __fmaf_rn(l, s.al, __fmul_rn(lb, s.be));
-    m = mn;
-    return s;
-}
-__device__ __forceinline__ float merge_o(float o, float ob, const Merge &s) { return __fmaf_rn(o, s.al, __fmul_rn(ob, s.be)); }
-
-// b_r of one head in the log2 domain, [0, L)
+// b_r of one head, scaled, [0, L)
 __device__ __forceinline__ void load_br(float *brs, const AttnArgs &a, int h, int tid, int nthr)
 {
-    const float f = a.inv_sqrt * 1.4426950408889634f;
     for (int r = tid; r < a.L; r += nthr)
-        brs[r] = __fmul_rn(__fmul_rn(a.br_scale, a.b_r[(size_t)h * a.L + r]), f);
+        brs[r] = __fmul_rn(a.br_scale, a.b_r[(size_t)h * a.L + r]);
+}
+// the score of a pair, masked
+__device__ __forceinline__ float score_of(float s, float e, float br, bool visible, const AttnArgs &a)
+{
+    const float v = __fmul_rn(__fadd_rn(s, __fadd_rn(br, e)), a.inv_sqrt);
+    return visible ? v : -INFINITY;
 }
 
 // E of a warp's 16 rows (16 * qt ..) against 32 keys (32 * hf ..) of a block, skewed into the layout
@@ -241,11 +223,15 @@ __device__ __forceinline__ void product_16x32(float (&s)[4][4], const bf16 *At, 
 
 // ---------------- forward, a group of queries ----------------
 //
-// One CTA per (stream, head, 64 queries): warps 0-3 take the even key blocks, warps 4-7 the odd ones,
-// each warp one 16-row tile.  102 KB of shared memory at head size 64, so two CTAs share an SM.
+// One CTA of eight warps per (stream, head, 64 queries).  Per key block, warp (q tile, half) takes the
+// scores of 16 rows x 32 keys and then the value product of all 64 keys into half of the columns; the two
+// warps of a tile exchange maxima and probabilities through shared memory under a barrier of
+// their own.  The next block's tiles are fetched under the present block.  109 KB of shared memory at
+// head size 64: two CTAs per SM.
 template <int DK> struct FwdSmem {
     static constexpr int LD = DK + 8, TILE = 64 * LD * 2;
-    static constexpr int Q = 0, K = TILE, V = K + 2 * TILE, R = V + 2 * TILE, ES = R + 3 * TILE, BRS = ES + 8 * 16 * ESC * 4;
+    static constexpr int Q = 0, K = TILE, V = K + 2 * TILE, R = V + 2 * TILE, ES = R + 3 * TILE, PF = ES + 8 * 16 * ESC * 4,
+                         MX = PF + 4 * 4 * 512, BRS = MX + 4 * 6 * 32 * 4;
     static size_t bytes(int L) { return (size_t)BRS + (size_t)((L + 3) & ~3) * 4; }
 };
 
@@ -253,218 +239,236 @@ template <int DK>
 __global__ void __launch_bounds__(256, DK <= 64 ? 2 : 1) attn_fwd_kernel(const __grid_constant__ AttnArgs a)
 {
     using SM = FwdSmem<DK>;
-    constexpr int LD = SM::LD, NT = DK / 8;
+    constexpr int LD = SM::LD, NCH = DK >= 32 ? 2 : 1, NTC = DK / 8 / NCH; // column halves, 8-column groups in one
     extern __shared__ __align__(16) unsigned char sm[];
     bf16 *Qs = reinterpret_cast<bf16 *>(sm + SM::Q), *Ks = reinterpret_cast<bf16 *>(sm + SM::K),
          *Vs = reinterpret_cast<bf16 *>(sm + SM::V), *Rs = reinterpret_cast<bf16 *>(sm + SM::R);
     float *brs = reinterpret_cast<float *>(sm + SM::BRS);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    const int qt = warp & 3, set = warp >> 2;
+    const int qt = warp & 3, hf = warp >> 2;
     const int b = blockIdx.x / a.H, h = blockIdx.x % a.H, HD = a.H * DK, T = a.T, M = a.M, L = a.L;
     const int i0 = (a.t0 & ~63) + blockIdx.y * 64;
-    const int ta = max(i0, a.t0), tb = min(i0 + 64, a.t1);
-    const Blocks blk = blocks_of(M, L, a.attn_len, ta, tb);
+    const Blocks blk = blocks_of(M, L, a.attn_len, max(i0, a.t0), min(i0 + 64, a.t1));
     float *es = reinterpret_cast<float *>(sm + SM::ES) + warp * 16 * ESC;
+    // of this tile: [half][row A, row B][8] maxima, then [row A, row B][32] sums of half 0
+    float *mx = reinterpret_cast<float *>(sm + SM::MX) + qt * 6 * 32, *sums = mx + 32;
+    uint4 *pfs = reinterpret_cast<uint4 *>(sm + SM::PF) + qt * 4 * 32; // A fragments of the tile's probabilities, [16-key step][lane]
     pdl_trigger();
     pdl_wait();
 
     const bf16 *q = reinterpret_cast<const bf16 *>(a.q) + ((size_t)i0 * a.B + b) * a.qp + h * DK;
     const bf16 *kv = reinterpret_cast<const bf16 *>(a.kv) + (size_t)b * a.kvp + h * DK;
+    auto fetch_r = [&](int gr) { // table group gr: window rows 0-63 of block gr, 64-127 of block gr - 1
+        if (a.w_r)
+            load_table<DK>(Rs + (gr % 3) * 64 * LD, a, h, gr * KB - i0 + a.P - M - 64, 64, threadIdx.x, 256);
+    };
+    auto fetch = [&](int kb) {
+        const int j0 = kb * KB;
+        load_rows<DK>(Ks + (kb & 1) * 64 * LD, kv + (size_t)j0 * a.B * a.kvp, (size_t)a.B * a.kvp, 64, threadIdx.x, 256,
+                      [&](int r) { return j0 + r < L; });
+        load_rows<DK>(Vs + (kb & 1) * 64 * LD, kv + HD + (size_t)j0 * a.B * a.kvp, (size_t)a.B * a.kvp, 64, threadIdx.x, 256,
+                      [&](int r) { return j0 + r < L; });
+        fetch_r(kb + 1);
+    };
     load_rows<DK>(Qs, q, (size_t)a.B * a.qp, 64, threadIdx.x, 256, [&](int r) { return i0 + r >= a.t0 && i0 + r < a.t1; });
+    fetch_r(blk.lo);
+    fetch(blk.lo);
+    cp_commit();
     load_br(brs, a, h, threadIdx.x, 256);
-    const float sc2 = a.inv_sqrt * 1.4426950408889634f;
     const int iA = i0 + qt * 16 + g, iB = iA + 8; // this thread's two rows
     const bool active = i0 + qt * 16 < a.t1 && i0 + qt * 16 + 16 > a.t0;
 
-    float o[NT][4], mA = -INFINITY, mB = -INFINITY, lA = 0.0f, lB = 0.0f;
+    float o[NTC][4], mA = -INFINITY, mB = -INFINITY, lA = 0.0f, lB = 0.0f;
 #pragma unroll
-    for (int n = 0; n < NT; n++)
+    for (int n = 0; n < NTC; n++)
 #pragma unroll
         for (int c = 0; c < 4; c++)
             o[n][c] = 0.0f;
 
-    for (int pr = blk.lo >> 1; pr <= blk.hi >> 1; pr++) {
-        const int j00 = pr * 2 * KB;
-        if (pr != blk.lo >> 1)
-            __syncthreads(); // the pair before has been read
-        for (int s = 0; s < 2; s++) {
-            const int j0 = j00 + s * KB;
-            if (pr * 2 + s < blk.lo || pr * 2 + s > blk.hi)
-                continue;
-            load_rows<DK>(Ks + s * 64 * LD, kv + (size_t)j0 * a.B * a.kvp, (size_t)a.B * a.kvp, 64, threadIdx.x, 256,
-                          [&](int r) { return j0 + r < L; });
-            load_rows<DK>(Vs + s * 64 * LD, kv + HD + (size_t)j0 * a.B * a.kvp, (size_t)a.B * a.kvp, 64, threadIdx.x, 256,
-                          [&](int r) { return j0 + r < L; });
-        }
-        if (a.w_r)
-            load_table<DK>(Rs, a, h, j00 - i0 + a.P - M - 64, 192, threadIdx.x, 256);
-        cp_commit();
+    for (int kb = blk.lo; kb <= blk.hi; kb++) {
+        const int j0 = kb * KB;
         cp_wait<0>();
-        __syncthreads();
-        const int kb = pr * 2 + set, j0 = kb * KB;
-        if (!active || kb < blk.lo || kb > blk.hi)
+        __syncthreads(); // this block's tiles have landed, the one before has been read
+        if (kb < blk.hi)
+            fetch(kb + 1);
+        cp_commit();
+        if (!active)
             continue;
-        // scores of 16 rows x 64 keys, log2 domain, masked
-        uint32_t pf[4][4]; // probabilities as the A fragments of the value product
-        float s[2][4][4], mbA = -INFINITY, mbB = -INFINITY;
-#pragma unroll
-        for (int hf = 0; hf < 2; hf++) {
-            product_16x32<DK>(s[hf], Qs + qt * 16 * LD, Ks + (set * 64 + hf * 32) * LD, lane);
-            if (a.w_r) {
-                float e[4][4];
-                skewed_positions<DK>(e, Qs + qt * 16 * LD, [&](int p) { return Rs + (set * 64 + p * 16) * LD; }, qt, hf, es, lane);
-#pragma unroll
-                for (int n = 0; n < 4; n++)
-#pragma unroll
-                    for (int c = 0; c < 4; c++)
-                        s[hf][n][c] = __fadd_rn(s[hf][n][c], e[n][c]);
-            }
+        float s[4][4], mbA = -INFINITY, mbB = -INFINITY;
+        {
+            float e[4][4] = {};
+            product_16x32<DK>(s, Qs + qt * 16 * LD, Ks + ((kb & 1) * 64 + hf * 32) * LD, lane);
+            if (a.w_r)
+                skewed_positions<DK>(e, Qs + qt * 16 * LD, [&](int p) { return Rs + (((kb + (p >> 2)) % 3) * 64 + (p & 3) * 16) * LD; },
+                                     qt, hf, es, lane);
 #pragma unroll
             for (int n = 0; n < 4; n++)
 #pragma unroll
                 for (int c = 0; c < 4; c++) {
-                    const int j = j0 + hf * 32 + n * 8 + 2 * t + (c & 1), i = c < 2 ? iA : iB;
-                    const int d = i + M - j; // visible iff 0 <= d < attn_len
-                    const float v = __fmaf_rn(s[hf][n][c], sc2, brs[min(max(j + T - 1 - i, 0), L - 1)]);
-                    s[hf][n][c] = (unsigned)d < (unsigned)a.attn_len ? v : -INFINITY;
+                    const int j = j0 + hf * 32 + n * 8 + 2 * t + (c & 1), i = c < 2 ? iA : iB, d = i + M - j; // visible iff 0 <= d < attn_len
+                    s[n][c] = score_of(s[n][c], e[n][c], brs[min(max(j + T - 1 - i, 0), L - 1)], (unsigned)d < (unsigned)a.attn_len, a);
                 }
+        }
 #pragma unroll
-            for (int n = 0; n < 4; n++) {
-                mbA = fmaxf(mbA, fmaxf(s[hf][n][0], s[hf][n][1]));
-                mbB = fmaxf(mbB, fmaxf(s[hf][n][2], s[hf][n][3]));
-            }
+        for (int n = 0; n < 4; n++) {
+            mbA = fmaxf(mbA, fmaxf(s[n][0], s[n][1]));
+            mbB = fmaxf(mbB, fmaxf(s[n][2], s[n][3]));
         }
         mbA = fmaxf(mbA, __shfl_xor_sync(0xffffffffu, mbA, 1));
         mbB = fmaxf(mbB, __shfl_xor_sync(0xffffffffu, mbB, 1));
         mbA = fmaxf(mbA, __shfl_xor_sync(0xffffffffu, mbA, 2));
         mbB = fmaxf(mbB, __shfl_xor_sync(0xffffffffu, mbB, 2));
-        const float uA = mbA == -INFINITY ? 0.0f : mbA, uB = mbB == -INFINITY ? 0.0f : mbB;
-        float sumA = 0.0f, sumB = 0.0f;
-#pragma unroll
-        for (int n = 0; n < 8; n++) {
-            float(&x)[4] = s[n >> 2][n & 3];
-            x[0] = ex2(__fsub_rn(x[0], uA));
-            x[1] = ex2(__fsub_rn(x[1], uA));
-            x[2] = ex2(__fsub_rn(x[2], uB));
-            x[3] = ex2(__fsub_rn(x[3], uB));
-            sumA = __fadd_rn(sumA, __fadd_rn(x[0], x[1]));
-            sumB = __fadd_rn(sumB, __fadd_rn(x[2], x[3]));
-            pf[n >> 1][(n & 1) * 2] = pack2(x[0], x[1]);
-            pf[n >> 1][(n & 1) * 2 + 1] = pack2(x[2], x[3]);
+        if (t == 0) {
+            mx[hf * 16 + g] = mbA;
+            mx[hf * 16 + 8 + g] = mbB;
         }
-        sumA = __fadd_rn(sumA, __shfl_xor_sync(0xffffffffu, sumA, 1));
-        sumB = __fadd_rn(sumB, __shfl_xor_sync(0xffffffffu, sumB, 1));
-        sumA = __fadd_rn(sumA, __shfl_xor_sync(0xffffffffu, sumA, 2));
-        sumB = __fadd_rn(sumB, __shfl_xor_sync(0xffffffffu, sumB, 2));
-        const Merge fA = merge_scale(mA, lA, mbA, sumA), fB = merge_scale(mB, lB, mbB, sumB);
-        // the block's output, 32 columns (16 at head size 16) at a time
-        constexpr int NP = NT < 4 ? NT : 4;
+        asm volatile("bar.sync %0, 64;" ::"r"(1 + qt) : "memory");
+        mbA = fmaxf(mbA, mx[(hf ^ 1) * 16 + g]);
+        mbB = fmaxf(mbB, mx[(hf ^ 1) * 16 + 8 + g]);
+        const float nA = fmaxf(mA, mbA), nB = fmaxf(mB, mbB);
+        const float uA = nA == -INFINITY ? 0.0f : nA, uB = nB == -INFINITY ? 0.0f : nB;
+        const float scA = __expf(__fsub_rn(mA, uA)), scB = __expf(__fsub_rn(mB, uB));
+        mA = nA;
+        mB = nB;
+        float sA = 0.0f, sB = 0.0f, xA[4], xB[4];
 #pragma unroll
-        for (int n0 = 0; n0 < NT; n0 += NP) {
-            float ob[NP][4];
+        for (int n = 0; n < 4; n++) {
+            s[n][0] = __expf(__fsub_rn(s[n][0], uA));
+            s[n][1] = __expf(__fsub_rn(s[n][1], uA));
+            s[n][2] = __expf(__fsub_rn(s[n][2], uB));
+            s[n][3] = __expf(__fsub_rn(s[n][3], uB));
+            xA[n] = __fadd_rn(s[n][0], s[n][1]);
+            xB[n] = __fadd_rn(s[n][2], s[n][3]);
+            sA = __fadd_rn(sA, xA[n]);
+            sB = __fadd_rn(sB, xB[n]);
+        }
 #pragma unroll
-            for (int n = 0; n < NP; n++)
+        for (int ks = 0; ks < 2; ks++)
+            pfs[(hf * 2 + ks) * 32 + lane] = make_uint4(pack2(s[2 * ks][0], s[2 * ks][1]), pack2(s[2 * ks][2], s[2 * ks][3]),
+                                                        pack2(s[2 * ks + 1][0], s[2 * ks + 1][1]), pack2(s[2 * ks + 1][2], s[2 * ks + 1][3]));
+        if (hf == 0) {
+            sums[lane] = sA;
+            sums[32 + lane] = sB;
+        }
+        asm volatile("bar.sync %0, 64;" ::"r"(1 + qt) : "memory");
+        if (hf == 1) { // the row's sum runs over the keys in order: half 1 carries on from half 0
+            sA = sums[lane];
+            sB = sums[32 + lane];
 #pragma unroll
-                for (int c = 0; c < 4; c++)
-                    ob[n][c] = 0.0f;
+            for (int n = 0; n < 4; n++) {
+                sA = __fadd_rn(sA, xA[n]);
+                sB = __fadd_rn(sB, xB[n]);
+            }
+            lA = __fmaf_rn(lA, scA, sA);
+            lB = __fmaf_rn(lB, scB, sB);
+        }
+        if (hf < NCH) {
 #pragma unroll
-            for (int ks = 0; ks < 4; ks++)
+            for (int n = 0; n < NTC; n++) {
+                o[n][0] = __fmul_rn(o[n][0], scA);
+                o[n][1] = __fmul_rn(o[n][1], scA);
+                o[n][2] = __fmul_rn(o[n][2], scB);
+                o[n][3] = __fmul_rn(o[n][3], scB);
+            }
+            const bf16 *vb = Vs + ((kb & 1) * 64 + (lane & 7) + ((lane >> 3) & 1) * 8) * LD + hf * (DK / 2) * (NCH - 1) + (lane >> 4) * 8;
 #pragma unroll
-                for (int p = 0; p < NP / 2; p++) {
+            for (int ks = 0; ks < 4; ks++) {
+                const uint4 u = pfs[ks * 32 + lane];
+                const uint32_t pf[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+                for (int p = 0; p < NTC / 2; p++) {
                     uint32_t bb[4];
-                    ldsm4t(bb, Vs + (set * 64 + ks * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * LD + n0 * 8 + p * 16 + (lane >> 4) * 8);
-                    mma(ob[2 * p], pf[ks], bb[0], bb[1]);
-                    mma(ob[2 * p + 1], pf[ks], bb[2], bb[3]);
+                    ldsm4t(bb, vb + ks * 16 * LD + p * 16);
+                    mma(o[2 * p], pf, bb[0], bb[1]);
+                    mma(o[2 * p + 1], pf, bb[2], bb[3]);
                 }
-#pragma unroll
-            for (int n = 0; n < NP; n++) {
-                o[n0 + n][0] = merge_o(o[n0 + n][0], ob[n][0], fA);
-                o[n0 + n][1] = merge_o(o[n0 + n][1], ob[n][1], fA);
-                o[n0 + n][2] = merge_o(o[n0 + n][2], ob[n][2], fB);
-                o[n0 + n][3] = merge_o(o[n0 + n][3], ob[n][3], fB);
             }
         }
     }
-    // the odd blocks' result goes to the warps of the even ones through the K tiles
-    __syncthreads();
-    float *xo = reinterpret_cast<float *>(sm + SM::K) + qt * 32 * (NT * 4 + 4);
-    if (set == 1) {
-#pragma unroll
-        for (int n = 0; n < NT; n++)
-#pragma unroll
-            for (int c = 0; c < 4; c++)
-                xo[(n * 4 + c) * 32 + lane] = o[n][c];
-        xo[(NT * 4) * 32 + lane] = mA;
-        xo[(NT * 4 + 1) * 32 + lane] = mB;
-        xo[(NT * 4 + 2) * 32 + lane] = lA;
-        xo[(NT * 4 + 3) * 32 + lane] = lB;
-    }
-    __syncthreads();
-    if (set == 1 || !active)
+    if (!active)
         return;
-    const float m1A = xo[(NT * 4) * 32 + lane], m1B = xo[(NT * 4 + 1) * 32 + lane];
-    const Merge fA = merge_scale(mA, lA, m1A, xo[(NT * 4 + 2) * 32 + lane]), fB = merge_scale(mB, lB, m1B, xo[(NT * 4 + 3) * 32 + lane]);
-    const float rA = __fdiv_rn(1.0f, lA), rB = __fdiv_rn(1.0f, lB);
-#pragma unroll
-    for (int n = 0; n < NT; n++)
-#pragma unroll
-        for (int c = 0; c < 4; c++)
-            o[n][c] = __fmul_rn(merge_o(o[n][c], xo[(n * 4 + c) * 32 + lane], c < 2 ? fA : fB), c < 2 ? rA : rB);
-    bf16 *out = reinterpret_cast<bf16 *>(a.o) + ((size_t)iA * a.B + b) * HD + h * DK;
+    if (hf == 1) {
+        lA = __fadd_rn(lA, __shfl_xor_sync(0xffffffffu, lA, 1));
+        lB = __fadd_rn(lB, __shfl_xor_sync(0xffffffffu, lB, 1));
+        lA = __fadd_rn(lA, __shfl_xor_sync(0xffffffffu, lA, 2));
+        lB = __fadd_rn(lB, __shfl_xor_sync(0xffffffffu, lB, 2));
+        sums[lane] = lA;
+        sums[32 + lane] = lB;
+    }
+    asm volatile("bar.sync %0, 64;" ::"r"(1 + qt) : "memory");
+    lA = sums[lane];
+    lB = sums[32 + lane];
     const bool okA = iA >= a.t0 && iA < a.t1, okB = iB >= a.t0 && iB < a.t1;
-    store_row<NT>(out, o, 0, t, okA);
-    store_row<NT>(out + (size_t)8 * a.B * HD, o, 2, t, okB);
-    if (t == 0 && a.lse) {
+    if (hf < NCH) {
+        const float rA = __fdiv_rn(1.0f, lA), rB = __fdiv_rn(1.0f, lB);
+#pragma unroll
+        for (int n = 0; n < NTC; n++) {
+            o[n][0] = __fmul_rn(o[n][0], rA);
+            o[n][1] = __fmul_rn(o[n][1], rA);
+            o[n][2] = __fmul_rn(o[n][2], rB);
+            o[n][3] = __fmul_rn(o[n][3], rB);
+        }
+        bf16 *out = reinterpret_cast<bf16 *>(a.o) + ((size_t)iA * a.B + b) * HD + h * DK + hf * (DK / 2) * (NCH - 1);
+        store_row<NTC>(out, o, 0, t, okA);
+        store_row<NTC>(out + (size_t)8 * a.B * HD, o, 2, t, okB);
+    }
+    if (hf == 0 && t == 0 && a.lse) {
         float *lse = a.lse + ((size_t)b * a.H + h) * T;
         if (okA)
-            lse[iA] = (mA + __log2f(lA)) * 0.6931471805599453f;
+            lse[iA] = mA + logf(lA);
         if (okB)
-            lse[iB] = (mB + __log2f(lB)) * 0.6931471805599453f;
+            lse[iB] = mB + logf(lB);
     }
 }
 
 // ---------------- forward, one query ----------------
 //
-// A decoding step: one query per stream, so the op is a stream of K and V through the chip (126 MB a
+// A decoding step: one query per stream, so the op is a stream of K and V through the chip (151 MB a
 // layer at 128 streams x 8 heads x 576 keys) and what bounds it is HBM.  One CTA of four warps per
-// (stream, head); a warp takes every fourth key block by itself (its own tiles, no barrier), so that
-// 220 KB an SM are in flight.  The operand roles are exchanged: keys (and table rows, of which a
-// single query needs exactly one per key) fill the 16 rows of a product, the query is the other
-// operand, broadcast to its 8 columns; a product of 16 terms gives the same bits either way round.
+// (stream, head), four key blocks a round: a warp takes one block's scores from tiles of its own, then
+// the four share the round's value products by 16-column slices.  The next round's K and table rows are
+// fetched as soon as the scores are taken; 220 KB an SM are in flight.  The operand roles are
+// exchanged: keys (and table rows, of which a single query needs exactly one per key) fill the 16 rows
+// of a product, the query is the other operand, broadcast to its 8 columns; a product of 16 terms gives
+// the same bits either way round.
 template <int DK> struct OneSmem {
     static constexpr int LD = DK + 8, TILE = 64 * LD * 2;
-    static constexpr int W = 3 * TILE + 64 * 4; // a warp's K, V, table rows and probabilities
-    static constexpr int RES = 4 * W;
-    static size_t bytes(int nb) { return (size_t)RES + (size_t)nb * (DK + 2) * 4; }
+    static constexpr int K = 0, R = 4 * TILE, V = 8 * TILE, S = 12 * TILE, MB = S + 4 * 64 * 4, L4 = MB + 16, TOTAL = L4 + 16;
 };
 
 template <int DK>
 __global__ void __launch_bounds__(128) attn_one_kernel(const __grid_constant__ AttnArgs a)
 {
     using SM = OneSmem<DK>;
-    constexpr int LD = SM::LD;
+    constexpr int LD = SM::LD, MT = DK / 16, MW = (MT + 3) / 4; // 16-column slices, and those of one warp
     extern __shared__ __align__(16) unsigned char sm[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    bf16 *Ks = reinterpret_cast<bf16 *>(sm + warp * SM::W), *Vs = Ks + 64 * LD, *Rs = Vs + 64 * LD;
-    float *ps = reinterpret_cast<float *>(Rs + 64 * LD);
-    float *res = reinterpret_cast<float *>(sm + SM::RES);
+    bf16 *Ks = reinterpret_cast<bf16 *>(sm + SM::K) + warp * 64 * LD, *Rs = reinterpret_cast<bf16 *>(sm + SM::R) + warp * 64 * LD,
+         *Vall = reinterpret_cast<bf16 *>(sm + SM::V);
+    float *sc = reinterpret_cast<float *>(sm + SM::S), *mbs = reinterpret_cast<float *>(sm + SM::MB); // [4][64] scores, [4] maxima
     const int b = blockIdx.x / a.H, h = blockIdx.x % a.H, HD = a.H * DK, T = a.T, M = a.M, L = a.L, i = a.t0;
     const Blocks blk = blocks_of(M, L, a.attn_len, i, i + 1);
-    const int nb = blk.hi - blk.lo + 1;
     pdl_trigger();
     pdl_wait();
     const bf16 *kv = reinterpret_cast<const bf16 *>(a.kv) + (size_t)b * a.kvp + h * DK;
-    const float sc2 = a.inv_sqrt * 1.4426950408889634f;
-    auto fetch = [&](int kb) {
+    auto fetch_kr = [&](int kb) { // this warp's block of a round
         const int j0 = kb * KB;
+        if (kb > blk.hi)
+            return;
         load_rows<DK>(Ks, kv + (size_t)j0 * a.B * a.kvp, (size_t)a.B * a.kvp, 64, lane, 32, [&](int r) { return j0 + r < L; });
-        load_rows<DK>(Vs, kv + HD + (size_t)j0 * a.B * a.kvp, (size_t)a.B * a.kvp, 64, lane, 32, [&](int r) { return j0 + r < L; });
         if (a.w_r)
             load_table<DK>(Rs, a, h, j0 - i + a.P - M - 1, 64, lane, 32);
-        cp_commit();
     };
-    if (warp < nb)
-        fetch(blk.lo + warp);
+    auto fetch_v = [&](int kb) {
+        const int j0 = kb * KB;
+        if (kb <= blk.hi)
+            load_rows<DK>(Vall + warp * 64 * LD, kv + HD + (size_t)j0 * a.B * a.kvp, (size_t)a.B * a.kvp, 64, lane, 32,
+                          [&](int r) { return j0 + r < L; });
+    };
+    fetch_kr(blk.lo + warp);
+    cp_commit();
+    fetch_v(blk.lo + warp);
+    cp_commit();
     // the query as the second operand: k = 2t, 2t + 1 (+ 8) of every 16-wide slice, the same for all columns
     uint32_t qf[DK / 16][2];
     {
@@ -475,102 +479,101 @@ __global__ void __launch_bounds__(128) attn_one_kernel(const __grid_constant__ A
             qf[ks][1] = *reinterpret_cast<const uint32_t *>(q + ks * 16 + 8 + 2 * t);
         }
     }
-    for (int kbi = warp; kbi < nb; kbi += 4) {
-        const int j0 = (blk.lo + kbi) * KB;
-        cp_wait<0>();
+    float o[MW][4], m_run = -INFINITY, l = 0.0f; // l: the part of the sum that lane t of a quad keeps
+#pragma unroll
+    for (int w = 0; w < MW; w++)
+#pragma unroll
+        for (int c = 0; c < 4; c++)
+            o[w][c] = 0.0f;
+    for (int kb0 = blk.lo; kb0 <= blk.hi; kb0 += 4) {
+        const int kb = kb0 + warp, j0 = kb * KB, nb = min(4, blk.hi - kb0 + 1);
+        cp_wait<1>(); // K and the table rows
         __syncwarp();
-        float s[4][2], mb = -INFINITY; // keys 16 m + g, + 8
+        if (kb <= blk.hi) {
+            float mb = -INFINITY;
 #pragma unroll
-        for (int m = 0; m < 4; m++) {
-            float x[4] = {0.0f, 0.0f, 0.0f, 0.0f}, e[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            for (int m = 0; m < 4; m++) {
+                float x[4] = {0.0f, 0.0f, 0.0f, 0.0f}, e[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
-            for (int ks = 0; ks < DK / 16; ks++) {
-                uint32_t k4[4];
-                ldsm4(k4, Ks + (m * 16 + (lane & 15)) * LD + ks * 16 + (lane >> 4) * 8);
-                mma(x, k4, qf[ks][0], qf[ks][1]);
-                if (a.w_r) {
-                    ldsm4(k4, Rs + (m * 16 + (lane & 15)) * LD + ks * 16 + (lane >> 4) * 8);
-                    mma(e, k4, qf[ks][0], qf[ks][1]);
+                for (int ks = 0; ks < DK / 16; ks++) {
+                    uint32_t k4[4];
+                    ldsm4(k4, Ks + (m * 16 + (lane & 15)) * LD + ks * 16 + (lane >> 4) * 8);
+                    mma(x, k4, qf[ks][0], qf[ks][1]);
+                    if (a.w_r) {
+                        ldsm4(k4, Rs + (m * 16 + (lane & 15)) * LD + ks * 16 + (lane >> 4) * 8);
+                        mma(e, k4, qf[ks][0], qf[ks][1]);
+                    }
+                }
+#pragma unroll
+                for (int c = 0; c < 2; c++) {
+                    const int j = j0 + m * 16 + g + c * 8, d = i + M - j, r = min(max(j + T - 1 - i, 0), L - 1);
+                    const float br = __fmul_rn(a.br_scale, __ldg(a.b_r + (size_t)h * L + r));
+                    const float v = score_of(x[2 * c], e[2 * c], br, (unsigned)d < (unsigned)a.attn_len, a);
+                    mb = fmaxf(mb, v);
+                    if (t == 0)
+                        sc[warp * 64 + m * 16 + g + c * 8] = v;
                 }
             }
-#pragma unroll
-            for (int c = 0; c < 2; c++) {
-                const int j = j0 + m * 16 + g + c * 8, d = i + M - j, r = min(max(j + T - 1 - i, 0), L - 1);
-                float v = x[2 * c];
-                if (a.w_r)
-                    v = __fadd_rn(v, e[2 * c]);
-                const float br = __fmul_rn(__fmul_rn(a.br_scale, __ldg(a.b_r + (size_t)h * L + r)), sc2);
-                v = __fmaf_rn(v, sc2, br);
-                s[m][c] = (unsigned)d < (unsigned)a.attn_len ? v : -INFINITY;
-                mb = fmaxf(mb, s[m][c]);
-            }
+            mb = fmaxf(mb, __shfl_xor_sync(0xffffffffu, mb, 4));
+            mb = fmaxf(mb, __shfl_xor_sync(0xffffffffu, mb, 8));
+            mb = fmaxf(mb, __shfl_xor_sync(0xffffffffu, mb, 16));
+            if (lane == 0)
+                mbs[warp] = mb;
         }
-        mb = fmaxf(mb, __shfl_xor_sync(0xffffffffu, mb, 4));
-        mb = fmaxf(mb, __shfl_xor_sync(0xffffffffu, mb, 8));
-        mb = fmaxf(mb, __shfl_xor_sync(0xffffffffu, mb, 16));
-        const float u = mb == -INFINITY ? 0.0f : mb;
-#pragma unroll
-        for (int m = 0; m < 4; m++)
-#pragma unroll
-            for (int c = 0; c < 2; c++)
-                if (t == 0)
-                    ps[m * 16 + g + c * 8] = ex2(__fsub_rn(s[m][c], u));
         __syncwarp();
-        // the sum in the order of the 16-row kernel: column pairs of a lane, then the quad
-        float sum = 0.0f;
-        uint32_t pf[4][2];
+        if (kb0 + 4 <= blk.hi)
+            fetch_kr(kb + 4);
+        cp_commit();
+        cp_wait<1>(); // V
+        __syncthreads(); // scores, maxima and V of the round are there for everyone
+        for (int s = 0; s < nb; s++) {
+            const float n = fmaxf(m_run, mbs[s]), u = n == -INFINITY ? 0.0f : n, scale = __expf(__fsub_rn(m_run, u));
+            m_run = n;
+            float sum = 0.0f;
+            uint32_t pf[4][2];
 #pragma unroll
-        for (int n = 0; n < 8; n++) {
-            const float2 x = *reinterpret_cast<const float2 *>(ps + n * 8 + 2 * t);
-            sum = __fadd_rn(sum, __fadd_rn(x.x, x.y));
-            pf[n >> 1][n & 1] = pack2(x.x, x.y);
-        }
-        sum = __fadd_rn(sum, __shfl_xor_sync(0xffffffffu, sum, 1));
-        sum = __fadd_rn(sum, __shfl_xor_sync(0xffffffffu, sum, 2));
-        float *rb = res + (size_t)kbi * (DK + 2);
-#pragma unroll
-        for (int m = 0; m < DK / 16; m++) {
-            float x[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll
-            for (int ks = 0; ks < 4; ks++) {
-                uint32_t v4[4]; // V^T: rows are columns of V, so the 8 x 8 blocks come transposed
-                ldsm4t(v4, Vs + (ks * 16 + (lane & 7) + (lane >> 4) * 8) * LD + m * 16 + ((lane >> 3) & 1) * 8);
-                mma(x, v4, pf[ks][0], pf[ks][1]);
+            for (int k = 0; k < 8; k++) {
+                const float2 v = *reinterpret_cast<const float2 *>(sc + s * 64 + k * 8 + 2 * t);
+                const float p0 = __expf(__fsub_rn(v.x, u)), p1 = __expf(__fsub_rn(v.y, u));
+                sum = __fadd_rn(sum, __fadd_rn(p0, p1));
+                pf[k >> 1][k & 1] = pack2(p0, p1);
             }
-            if (t == 0) {
-                rb[m * 16 + g] = x[0];
-                rb[m * 16 + g + 8] = x[2];
+            l = __fmaf_rn(l, scale, sum);
+#pragma unroll
+            for (int w = 0; w < MW; w++) {
+                const int m = warp + 4 * w;
+                if (MT % 4 != 0 && m >= MT)
+                    break;
+#pragma unroll
+                for (int c = 0; c < 4; c++)
+                    o[w][c] = __fmul_rn(o[w][c], scale);
+#pragma unroll
+                for (int ks = 0; ks < 4; ks++) {
+                    uint32_t v4[4]; // V^T: rows are columns of V, so the 8 x 8 blocks come transposed
+                    ldsm4t(v4, Vall + (s * 64 + ks * 16 + (lane & 7) + (lane >> 4) * 8) * LD + m * 16 + ((lane >> 3) & 1) * 8);
+                    mma(o[w], v4, pf[ks][0], pf[ks][1]);
+                }
             }
         }
-        if (lane == 0) {
-            rb[DK] = mb;
-            rb[DK + 1] = sum;
-        }
-        __syncwarp(); // the tiles have been read
-        if (kbi + 4 < nb)
-            fetch(blk.lo + kbi + 4);
+        __syncthreads(); // the round has been read
+        if (kb0 + 4 <= blk.hi)
+            fetch_v(kb + 4);
+        cp_commit();
     }
-    __syncthreads();
-    for (int d = threadIdx.x; d < DK; d += 128) {
-        auto chain = [&](int par, float &m, float &l) { // the blocks of one parity, ascending
-            float o = 0.0f;
-            m = -INFINITY;
-            l = 0.0f;
-            for (int kbi = (blk.lo ^ par) & 1; kbi < nb; kbi += 2) {
-                const float *rb = res + (size_t)kbi * (DK + 2);
-                const Merge f = merge_scale(m, l, rb[DK], rb[DK + 1]);
-                o = merge_o(o, rb[d], f);
-            }
-            return o;
-        };
-        float m0, l0, m1, l1;
-        const float o0 = chain(0, m0, l0), o1 = chain(1, m1, l1);
-        const Merge f = merge_scale(m0, l0, m1, l1);
-        const float v = __fmul_rn(merge_o(o0, o1, f), __fdiv_rn(1.0f, l0));
-        reinterpret_cast<bf16 *>(a.o)[((size_t)i * a.B + b) * HD + h * DK + d] = __float2bfloat16_rn(v);
-        if (d == 0 && a.lse)
-            a.lse[((size_t)b * a.H + h) * T + i] = (m0 + __log2f(l0)) * 0.6931471805599453f;
+    l = __fadd_rn(l, __shfl_xor_sync(0xffffffffu, l, 1));
+    l = __fadd_rn(l, __shfl_xor_sync(0xffffffffu, l, 2));
+    const float inv = __fdiv_rn(1.0f, l);
+    bf16 *out = reinterpret_cast<bf16 *>(a.o) + ((size_t)i * a.B + b) * HD + h * DK;
+#pragma unroll
+    for (int w = 0; w < MW; w++) {
+        const int m = warp + 4 * w;
+        if (t == 0 && (MT % 4 == 0 || m < MT)) {
+            out[m * 16 + g] = __float2bfloat16_rn(__fmul_rn(o[w][0], inv));
+            out[m * 16 + g + 8] = __float2bfloat16_rn(__fmul_rn(o[w][2], inv));
+        }
     }
+    if (threadIdx.x == 0 && a.lse)
+        a.lse[((size_t)b * a.H + h) * T + i] = m_run + logf(l);
 }
 
 // ---------------- backward ----------------
@@ -610,7 +613,7 @@ __global__ void __launch_bounds__(256, DK <= 64 ? 2 : 1) attn_bwd_kernel(const _
          *Ks = reinterpret_cast<bf16 *>(sm + SM::K), *Vs = reinterpret_cast<bf16 *>(sm + SM::V),
          *Rs = reinterpret_cast<bf16 *>(sm + SM::R), *PS = reinterpret_cast<bf16 *>(sm + SM::PS),
          *DE = reinterpret_cast<bf16 *>(sm + SM::DE);
-    float *lse2 = reinterpret_cast<float *>(sm + SM::ROW), *Dr = lse2 + 64, *brs = reinterpret_cast<float *>(sm + SM::BRS);
+    float *lses = reinterpret_cast<float *>(sm + SM::ROW), *Dr = lses + 64, *brs = reinterpret_cast<float *>(sm + SM::BRS);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const int qt = warp & 3, hf = warp >> 2; // phase A: q tile, key half; B: row tile, column half or table set
     const int b = blockIdx.x / a.H, h = blockIdx.x % a.H, HD = a.H * DK, T = a.T, M = a.M, L = a.L, P = a.P;
@@ -651,23 +654,21 @@ __global__ void __launch_bounds__(256, DK <= 64 ? 2 : 1) attn_bwd_kernel(const _
     fetch_r(blk.lo + 1);
     cp_commit();
     load_br(brs, a, h, threadIdx.x, 256);
-    // D_i = dO_i . O_i and the log-sum-exp in the log2 domain: four lanes a row
-    {
-        const int r = threadIdx.x >> 2;
+    // D_i = dO_i . O_i and the log-sum-exp, a warp for eight rows
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        const int r = warp * 8 + k;
         float D = 0.0f;
         if (r < T) {
-            const bf16 *x = outp + (size_t)r * a.B * HD, *y = dout + (size_t)r * a.B * HD;
+            const bf16 *x = dout + (size_t)r * a.B * HD, *y = outp + (size_t)r * a.B * HD;
 #pragma unroll
-            for (int e = (threadIdx.x & 3) * 4; e < DK; e += 16) {
-                const float4 u = load_f4(x + e), v = load_f4(y + e);
-                D += (u.x * v.x + u.y * v.y) + (u.z * v.z + u.w * v.w);
-            }
+            for (int e = lane; e < DK; e += 32)
+                D = __fmaf_rn(to_f(x[e]), to_f(y[e]), D);
         }
-        D += __shfl_xor_sync(0xffffffffu, D, 1);
-        D += __shfl_xor_sync(0xffffffffu, D, 2);
-        if ((threadIdx.x & 3) == 0) {
+        D = warp_sum(D);
+        if (lane == 0) {
             Dr[r] = D;
-            lse2[r] = r < T ? a.lse[((size_t)b * a.H + h) * T + r] * 1.4426950408889634f : 0.0f;
+            lses[r] = r < T ? a.lse[((size_t)b * a.H + h) * T + r] : 0.0f;
         }
     }
     // outside the rows' bands the dE window is zero for every block; unused q tiles of P, dS and dE stay zero
@@ -697,13 +698,12 @@ __global__ void __launch_bounds__(256, DK <= 64 ? 2 : 1) attn_bwd_kernel(const _
             if (r < x_lo + r_off || r > x_hi + r_off)
                 dbr[r] = 0.0f;
 
-    const float sc2 = a.inv_sqrt * 1.4426950408889634f;
-    float dq[NTC][4], dr[NT][4], cs[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    float dq[NTC][4], dqr[NTC][4], dr[NT][4], cs[4] = {0.0f, 0.0f, 0.0f, 0.0f}; // dq: through the keys, dqr: through the table
 #pragma unroll
     for (int n = 0; n < NTC; n++)
 #pragma unroll
         for (int c = 0; c < 4; c++)
-            dq[n][c] = 0.0f;
+            dq[n][c] = dqr[n][c] = 0.0f;
 #pragma unroll
     for (int n = 0; n < NT; n++)
 #pragma unroll
@@ -761,40 +761,29 @@ __global__ void __launch_bounds__(256, DK <= 64 ? 2 : 1) attn_bwd_kernel(const _
         auto window = [&](int p) { return Rs + (((kb + (p >> 2)) & 1) * 64 + (p & 3) * 16) * LD; }; // piece p of the window
         // ---- A
         if (qt < nqt) {
-            float s[4][4], e[4][4];
+            float s[4][4], e[4][4] = {};
             product_16x32<DK>(s, Qs + qt * 16 * LD, Ks + hf * 32 * LD, lane);
-            if (a.w_r) {
+            if (a.w_r)
                 skewed_positions<DK>(e, Qs + qt * 16 * LD, window, qt, hf, es, lane);
-#pragma unroll
-                for (int n = 0; n < 4; n++)
-#pragma unroll
-                    for (int c = 0; c < 4; c++)
-                        s[n][c] = __fadd_rn(s[n][c], e[n][c]);
-            }
-            const float lA = lse2[iA], lB = lse2[iB], DA = Dr[iA], DB = Dr[iB];
+            const float lA = lses[iA], lB = lses[iB], DA = Dr[iA], DB = Dr[iB];
 #pragma unroll
             for (int n = 0; n < 4; n++)
 #pragma unroll
                 for (int c = 0; c < 4; c++) {
                     const int j = j0 + hf * 32 + n * 8 + 2 * t + (c & 1), i = c < 2 ? iA : iB, d = i + M - j;
-                    const float v = __fmaf_rn(s[n][c], sc2, brs[min(max(j + T - 1 - i, 0), L - 1)]);
-                    const bool vis = (unsigned)d < (unsigned)a.attn_len && i < T;
-                    s[n][c] = vis ? ex2(v - (c < 2 ? lA : lB)) : 0.0f;
+                    const float v = score_of(s[n][c], e[n][c], brs[min(max(j + T - 1 - i, 0), L - 1)],
+                                             (unsigned)d < (unsigned)a.attn_len && i < T, a);
+                    s[n][c] = __expf(__fsub_rn(v, c < 2 ? lA : lB));
                 }
             product_16x32<DK>(e, Os + qt * 16 * LD, Vs + hf * 32 * LD, lane); // dP
             asm volatile("bar.sync %0, 64;" ::"r"(1 + qt) : "memory"); // both warps of the tile are done with their scratch
             bf16 *pA = PS + (qt * 16 + g) * LPS + hf * 32 + 2 * t, *pB = pA + 8 * LPS;
 #pragma unroll
             for (int n = 0; n < 4; n++) {
-                const uint32_t wA = pack2(s[n][0], s[n][1]), wB = pack2(s[n][2], s[n][3]);
-                *reinterpret_cast<uint32_t *>(pA + n * 8) = wA;
-                *reinterpret_cast<uint32_t *>(pB + n * 8) = wB;
-                // dS with the probabilities as the products see them
-                const __nv_bfloat162 hA = *reinterpret_cast<const __nv_bfloat162 *>(&wA), hB = *reinterpret_cast<const __nv_bfloat162 *>(&wB);
-                const __nv_bfloat162 dA = __floats2bfloat162_rn(__low2float(hA) * (e[n][0] - DA) * a.inv_sqrt,
-                                                                __high2float(hA) * (e[n][1] - DA) * a.inv_sqrt);
-                const __nv_bfloat162 dB = __floats2bfloat162_rn(__low2float(hB) * (e[n][2] - DB) * a.inv_sqrt,
-                                                                __high2float(hB) * (e[n][3] - DB) * a.inv_sqrt);
+                *reinterpret_cast<uint32_t *>(pA + n * 8) = pack2(s[n][0], s[n][1]);
+                *reinterpret_cast<uint32_t *>(pB + n * 8) = pack2(s[n][2], s[n][3]);
+                const __nv_bfloat162 dA = __floats2bfloat162_rn(s[n][0] * (e[n][0] - DA) * a.inv_sqrt, s[n][1] * (e[n][1] - DA) * a.inv_sqrt);
+                const __nv_bfloat162 dB = __floats2bfloat162_rn(s[n][2] * (e[n][2] - DB) * a.inv_sqrt, s[n][3] * (e[n][3] - DB) * a.inv_sqrt);
                 *reinterpret_cast<__nv_bfloat162 *>(pA + 72 + n * 8) = dA;
                 *reinterpret_cast<__nv_bfloat162 *>(pB + 72 + n * 8) = dB;
                 // window column of key jj is jj + 63 - ii: odd rows' pairs are aligned, even rows' are not
@@ -840,8 +829,8 @@ __global__ void __launch_bounds__(256, DK <= 64 ? 2 : 1) attn_bwd_kernel(const _
                     for (int p = 0; p < NTC / 2; p++) {
                         uint32_t bb[4];
                         ldsm4t(bb, rw + p * 16);
-                        mma(dq[2 * p], x, bb[0], bb[1]);
-                        mma(dq[2 * p + 1], x, bb[2], bb[3]);
+                        mma(dqr[2 * p], x, bb[0], bb[1]);
+                        mma(dqr[2 * p + 1], x, bb[2], bb[3]);
                     }
                 }
             }
@@ -913,6 +902,11 @@ __global__ void __launch_bounds__(256, DK <= 64 ? 2 : 1) attn_bwd_kernel(const _
         __syncthreads(); // the next block's tiles have landed; P, dS and dE may be written again
     }
     if (qt < nqt && hf < NCH) {
+#pragma unroll
+        for (int n = 0; n < NTC; n++)
+#pragma unroll
+            for (int c = 0; c < 4; c++)
+                dq[n][c] = __fadd_rn(dq[n][c], dqr[n][c]);
         bf16 *dst = reinterpret_cast<bf16 *>(a.dq) + ((size_t)(iA < T ? iA : 0) * a.B + b) * a.dqp + h * DK + hf * (DK / 2) * (NCH - 1);
         store_row<NTC>(dst, dq, 0, t, iA < T);
         dst += (size_t)(iB < T ? 8 : 0) * a.B * a.dqp;
@@ -958,15 +952,14 @@ inline bool fits(int dk, int L)
 
 template <int DK> static int forward_dk(const AttnArgs &a, cudaStream_t st)
 {
-    const Blocks one = blocks_of(a.M, a.L, a.attn_len, a.t0, a.t1);
-    const size_t smem1 = OneSmem<DK>::bytes(one.hi - one.lo + 1), smem = FwdSmem<DK>::bytes(a.L);
+    const size_t smem1 = OneSmem<DK>::TOTAL, smem = FwdSmem<DK>::bytes(a.L);
     static bool attr_done = false;
     if (!attr_done) {
         CUDA_TRY(cudaFuncSetAttribute(attn_fwd_kernel<DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
         CUDA_TRY(cudaFuncSetAttribute(attn_one_kernel<DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
         attr_done = true;
     }
-    if (a.t1 - a.t0 == 1 && smem1 <= 227 * 1024)
+    if (a.t1 - a.t0 == 1)
         launch_k(attn_one_kernel<DK>, dim3(a.B * a.H), dim3(128), smem1, st, a);
     else
         launch_k(attn_fwd_kernel<DK>, dim3(a.B * a.H, (a.t1 - (a.t0 & ~63) + 63) / 64), dim3(256), smem, st, a);

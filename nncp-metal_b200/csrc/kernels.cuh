@@ -236,13 +236,11 @@ residual_norm_vec_kernel(const T *__restrict__ a, const T *__restrict__ res, T *
     }
     float var = 0.0f;
 #pragma unroll
-    for (int c = 0; c < NC; c++) {
-        float part = 0.0f;
+    for (int c = 0; c < NC; c++)
+        if (c * 32 * W + lane * W < D)
 #pragma unroll
-        for (int e = 0; e < W; e++)
-            part += (v[c][e] - mu) * (v[c][e] - mu);
-        var += c * 32 * W + lane * W < D ? part : 0.0f;
-    }
+            for (int e = 0; e < W; e++)
+                var += (v[c][e] - mu) * (v[c][e] - mu);
     var = warp_sum(var) / (float)D;
     const float rstd = 1.0f / sqrtf(var + 1e-5f);
     if (stats && lane == 0) {

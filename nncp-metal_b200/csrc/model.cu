@@ -565,9 +565,10 @@ static int forward_range(nncu_model *m, int t0, int t1)
     const nncu_params &p = m->p;
     const int D = m->D, HD = m->HD, F = m->F, F1 = m->F1, B = m->B, M = m->M, V = m->V;
     const int r0 = t0 * B, nr = (t1 - t0) * B;
-    const bool pre = p.ln_flags & NNCU_LN_PRE, post = p.ln_flags & NNCU_LN_POST;
+    const bool pre = p.ln_flags & NNCU_LN_PRE, post = p.ln_flags & NNCU_LN_POST, final = p.ln_flags & NNCU_LN_FINAL;
     const float emul = sqrtf((float)D) * p.embed_mult;
     AT *tmp = reinterpret_cast<AT *>(m->pool[0]); // [TB][D] scratch
+    AT *xf = at<AT>(final ? m->xf : m->xlast, (size_t)r0 * D); // what the output head reads
 
     launch_k(embed_kernel<AT>, dim3(nr), dim3(128), 0, m->st, m->ids_dev + r0, m->W + m->embed,
                                             at<AT>(m->act[0].xin, (size_t)r0 * D), nr, D, emul, V);
@@ -578,7 +579,9 @@ static int forward_range(nncu_model *m, int t0, int t1)
         AT *hc = reinterpret_cast<AT *>(hcat_layer(m, m->cur, l));
         AT *x1 = hc + ((size_t)M * B + r0) * D;   // attention input of these rows (train_h)
         AT *xin = at<AT>(a.xin, (size_t)r0 * D);  // residual-stream input
-        if (pre)
+        // a pre-LN residual sum and the norm behind it share a launch (one rounding point each, as before);
+        // only the first layer's norm stands alone
+        if (pre && l == 0)
             NNCU_TRY(norm_fwd<AT>(m, xin, nullptr, nullptr, x1, o.ln_g1, o.ln_b1, a.st_pre1 + 2 * r0, nr, true));
         // fused projections over [memory ; segment]: Q for the segment rows, K|V for the
         // memory rows (once per segment) and the segment rows (nncp.c:659-695)
@@ -610,14 +613,13 @@ static int forward_range(nncu_model *m, int t0, int t1)
             NNCU_TRY((mm_nt<AT, AT>(m, nr, D, HD, at<AT>(a.o, (size_t)r0 * HD), HD, o.w_o, tmp, D, nullptr)));
         }
         AT *yy = at<AT>(a.y, (size_t)r0 * D);
-        NNCU_TRY(norm_fwd<AT>(m, tmp, xin, post ? at<AT>(a.s1, (size_t)r0 * D) : nullptr, yy, o.ln_g1,
-                              o.ln_b1, a.st_1 + 2 * r0, nr, post));
         // feed-forward (nncp.c:925-986)
-        AT *u = yy;
-        if (pre) {
-            u = at<AT>(a.u, (size_t)r0 * D);
-            NNCU_TRY(norm_fwd<AT>(m, yy, nullptr, nullptr, u, o.ln_g2, o.ln_b2, a.st_pre2 + 2 * r0, nr, true));
-        }
+        AT *u = pre ? at<AT>(a.u, (size_t)r0 * D) : yy;
+        if (pre)
+            NNCU_TRY(norm_fwd<AT>(m, tmp, xin, yy, u, o.ln_g2, o.ln_b2, a.st_pre2 + 2 * r0, nr, true));
+        else
+            NNCU_TRY(norm_fwd<AT>(m, tmp, xin, post ? at<AT>(a.s1, (size_t)r0 * D) : nullptr, yy, o.ln_g1, o.ln_b1,
+                                  a.st_1 + 2 * r0, nr, post));
         AT *hpre = at<AT>(a.hpre, (size_t)r0 * F1), *hact = at<AT>(a.hact, (size_t)r0 * F);
         NNCU_TRY((mm_nt<AT, AT>(m, nr, F1, D, u, D, o.ff1, hpre, F1, wf(m, o.ff_bias1))));
         if (sizeof(AT) == 2 && F % 8 == 0 && F1 % 8 == 0)
@@ -637,15 +639,20 @@ static int forward_range(nncu_model *m, int t0, int t1)
         }
         AT *xout = (l + 1 < m->nl) ? at<AT>(m->act[l + 1].xin, (size_t)r0 * D)
                                    : at<AT>(m->xlast, (size_t)r0 * D);
-        NNCU_TRY(norm_fwd<AT>(m, tmp, yy, post ? at<AT>(a.s2, (size_t)r0 * D) : nullptr, xout, o.ln_g2,
-                              o.ln_b2, a.st_2 + 2 * r0, nr, post));
+        if (pre && l + 1 < m->nl) {
+            AT *next = reinterpret_cast<AT *>(hcat_layer(m, m->cur, l + 1)) + ((size_t)M * B + r0) * D;
+            NNCU_TRY(norm_fwd<AT>(m, tmp, yy, xout, next, m->lo[l + 1].ln_g1, m->lo[l + 1].ln_b1, m->act[l + 1].st_pre1 + 2 * r0,
+                                  nr, true));
+        } else if (pre && final) {
+            NNCU_TRY(norm_fwd<AT>(m, tmp, yy, xout, xf, m->ln_g, m->ln_b, m->st_f + 2 * r0, nr, true));
+        } else {
+            NNCU_TRY(norm_fwd<AT>(m, tmp, yy, post ? at<AT>(a.s2, (size_t)r0 * D) : nullptr, xout, o.ln_g2,
+                                  o.ln_b2, a.st_2 + 2 * r0, nr, post));
+        }
     }
-    AT *xf = at<AT>(m->xlast, (size_t)r0 * D);
-    if (p.ln_flags & NNCU_LN_FINAL) {
-        xf = at<AT>(m->xf, (size_t)r0 * D);
+    if (final && !pre)
         NNCU_TRY(norm_fwd<AT>(m, at<AT>(m->xlast, (size_t)r0 * D), nullptr, nullptr, xf, m->ln_g, m->ln_b,
                               m->st_f + 2 * r0, nr, true));
-    }
     float *pr = m->probs + (size_t)r0 * V;
     NNCU_TRY((mm_nt<AT, float>(m, nr, V, D, xf, D, m->embed_out, pr, V, wf(m, m->out_bias))));
     // the output kernel: probabilities for the coder, and p / (T * B) for the backward pass
@@ -817,6 +824,10 @@ static int backward(nncu_model *m)
     launch_k(loss_sum_kernel, dim3(1), dim3(256), 0, m->st, (const float *)m->logp, TB, m->loss_dev, m->dz_fixed);
     KERNEL_CHECK();
     const AT *xf = (p.ln_flags & NNCU_LN_FINAL) ? atc<AT>(m->xf, 0) : atc<AT>(m->xlast, 0);
+    // the column sums of a residual gradient are the ff_bias2 gradient of the layer it enters from above;
+    // the norm that produces it takes them along
+    auto bias2_of = [&](int l) { return l >= 0 && m->lo[l].ff_bias2 != NONE && m->lo[l].alpha == NONE ? gf(m, m->lo[l].ff_bias2) : nullptr; };
+    bool bias2_done = false;
     if (m->out_bias != NONE)
         NNCU_TRY(colsum<AT>(m, dz, V, TB, V, gf(m, m->out_bias)));
     NNCU_TRY(mm_tn(m, V, D, TB, dz, V, xf, D, gf(m, m->embed_out)));
@@ -824,7 +835,9 @@ static int backward(nncu_model *m)
     NNCU_TRY(mm_nn(m, TB, D, V, dz, V, m->embed_out, dx, D, (const AT *)nullptr));
     if (p.ln_flags & NNCU_LN_FINAL) {
         AT *t = pick<AT>(m, {dx});
-        NNCU_TRY(norm_bwd<AT>(m, dx, atc<AT>(m->xlast, 0), m->ln_g, m->ln_b, m->st_f, nullptr, t, TB));
+        NNCU_TRY(norm_bwd<AT>(m, dx, atc<AT>(m->xlast, 0), m->ln_g, m->ln_b, m->st_f, nullptr, t, TB,
+                              pre ? bias2_of(m->nl - 1) : nullptr));
+        bias2_done = pre;
         dx = t;
     }
     // tied tables collect the contributions of every layer
@@ -842,10 +855,8 @@ static int backward(nncu_model *m)
         const bool coef = o.alpha != NONE;
         if (post) {
             ds2 = pick<AT>(m, {dx});
-            // the column sums of ds2 are the ff_bias2 gradient: taken in the same pass
-            NNCU_TRY(norm_bwd<AT>(m, dx, atc<AT>(a.s2, 0), o.ln_g2, o.ln_b2, a.st_2, nullptr, ds2, TB,
-                                  (o.ff_bias2 != NONE && !coef) ? gf(m, o.ff_bias2) : nullptr));
-        } else if (o.ff_bias2 != NONE && !coef) {
+            NNCU_TRY(norm_bwd<AT>(m, dx, atc<AT>(a.s2, 0), o.ln_g2, o.ln_b2, a.st_2, nullptr, ds2, TB, bias2_of(l)));
+        } else if (o.ff_bias2 != NONE && !coef && !bias2_done) {
             NNCU_TRY(colsum<AT>(m, ds2, D, TB, D, gf(m, o.ff_bias2)));
         }
         // LN_COEF: the branch sees alpha * ds2 (its own buffer: the weight-gradient GEMMs read it until the
@@ -922,7 +933,9 @@ static int backward(nncu_model *m)
         if (pre) {
             AT *dx1 = pick<AT>(m, {ds1, ds2, dxn});
             NNCU_TRY(mm_nn(m, TB, D, 3 * HD, dq, 3 * HD, o.w_q, dx1, D, (const AT *)nullptr));
-            NNCU_TRY(norm_bwd<AT>(m, dx1, atc<AT>(a.xin, 0), o.ln_g1, o.ln_b1, a.st_pre1, ds1, dxn, TB));
+            NNCU_TRY(norm_bwd<AT>(m, dx1, atc<AT>(a.xin, 0), o.ln_g1, o.ln_b1, a.st_pre1, ds1, dxn, TB,
+                                  bias2_of(l - 1)));
+            bias2_done = true;
         } else {
             NNCU_TRY(mm_nn(m, TB, D, 3 * HD, dq, 3 * HD, o.w_q, dxn, D, (const AT *)ds1));
         }
