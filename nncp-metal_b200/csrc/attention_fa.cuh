@@ -142,17 +142,44 @@ __host__ __device__ inline Blocks blocks_of(int M, int L, int attn_len, int t0, 
     return Blocks{jlo / KB, jhi / KB};
 }
 
-// b_r of one head, scaled, [0, L)
+// b_r of one head, scaled, with room on both sides for the slots that masked pairs name
+constexpr int BR_LO = 64, BR_PAD = BR_LO + 128;
 __device__ __forceinline__ void load_br(float *brs, const AttnArgs &a, int h, int tid, int nthr)
 {
-    for (int r = tid; r < a.L; r += nthr)
-        brs[r] = __fmul_rn(a.br_scale, a.b_r[(size_t)h * a.L + r]);
+    for (int r = tid; r < a.L + BR_PAD; r += nthr) {
+        const int x = r - BR_LO;
+        brs[r] = x >= 0 && x < a.L ? __fmul_rn(a.br_scale, a.b_r[(size_t)h * a.L + x]) : 0.0f;
+    }
 }
-// the score of a pair, masked
-__device__ __forceinline__ float score_of(float s, float e, float br, bool visible, const AttnArgs &a)
+inline size_t br_bytes(int L) { return (size_t)((L + BR_PAD + 3) & ~3) * 4; }
+// the score of a pair
+__device__ __forceinline__ float score_of(float s, float e, float br, const AttnArgs &a)
 {
-    const float v = __fmul_rn(__fadd_rn(s, __fadd_rn(br, e)), a.inv_sqrt);
-    return visible ? v : -INFINITY;
+    return __fmul_rn(__fadd_rn(s, __fadd_rn(br, e)), a.inv_sqrt);
+}
+// The scores of a warp's 16 x 32 pairs in place over s; first row i_w, first key j_w; rows from i_end on see
+// nothing.  Whether a warp's pairs are all visible is the same for the whole warp, and for most tiles
+// it is so: no masking there.
+__device__ __forceinline__ void scores_16x32(float (&s)[4][4], const float (&e)[4][4], const float *brs, const AttnArgs &a, int i_w,
+                                             int j_w, int i_end, int lane)
+{
+    const int g = lane >> 2, t = lane & 3, d0 = i_w + g + a.M - j_w - 2 * t; // query - key distance of element (0, 0)
+    const float *br = brs + BR_LO + j_w + 2 * t + a.T - 1 - i_w - g;
+#pragma unroll
+    for (int n = 0; n < 4; n++)
+#pragma unroll
+        for (int c = 0; c < 4; c++)
+            s[n][c] = score_of(s[n][c], e[n][c], br[n * 8 + (c & 1) - (c >> 1) * 8], a);
+    if (j_w + 31 <= i_w + a.M && j_w > i_w + 15 + a.M - a.attn_len && i_w + 16 <= i_end)
+        return;
+#pragma unroll
+    for (int n = 0; n < 4; n++)
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            const int d = d0 - n * 8 - (c & 1) + (c >> 1) * 8; // visible iff 0 <= d < attn_len
+            if ((unsigned)d >= (unsigned)a.attn_len || i_w + g + (c >> 1) * 8 >= i_end)
+                s[n][c] = -INFINITY;
+        }
 }
 
 // E of a warp's 16 rows (16 * qt ..) against 32 keys (32 * hf ..) of a block, skewed into the layout
@@ -232,7 +259,7 @@ template <int DK> struct FwdSmem {
     static constexpr int LD = DK + 8, TILE = 64 * LD * 2;
     static constexpr int Q = 0, K = TILE, V = K + 2 * TILE, R = V + 2 * TILE, ES = R + 3 * TILE, PF = ES + 8 * 16 * ESC * 4,
                          MX = PF + 4 * 4 * 512, BRS = MX + 4 * 6 * 32 * 4;
-    static size_t bytes(int L) { return (size_t)BRS + (size_t)((L + 3) & ~3) * 4; }
+    static size_t bytes(int L) { return (size_t)BRS + br_bytes(L); }
 };
 
 template <int DK>
@@ -301,13 +328,7 @@ __global__ void __launch_bounds__(256, DK <= 64 ? 2 : 1) attn_fwd_kernel(const _
             if (a.w_r)
                 skewed_positions<DK>(e, Qs + qt * 16 * LD, [&](int p) { return Rs + (((kb + (p >> 2)) % 3) * 64 + (p & 3) * 16) * LD; },
                                      qt, hf, es, lane);
-#pragma unroll
-            for (int n = 0; n < 4; n++)
-#pragma unroll
-                for (int c = 0; c < 4; c++) {
-                    const int j = j0 + hf * 32 + n * 8 + 2 * t + (c & 1), i = c < 2 ? iA : iB, d = i + M - j; // visible iff 0 <= d < attn_len
-                    s[n][c] = score_of(s[n][c], e[n][c], brs[min(max(j + T - 1 - i, 0), L - 1)], (unsigned)d < (unsigned)a.attn_len, a);
-                }
+            scores_16x32(s, e, brs, a, i0 + qt * 16, j0 + hf * 32, 1 << 30, lane);
         }
 #pragma unroll
         for (int n = 0; n < 4; n++) {
@@ -508,7 +529,7 @@ __global__ void __launch_bounds__(128) attn_one_kernel(const __grid_constant__ A
                 for (int c = 0; c < 2; c++) {
                     const int j = j0 + m * 16 + g + c * 8, d = i + M - j, r = min(max(j + T - 1 - i, 0), L - 1);
                     const float br = __fmul_rn(a.br_scale, __ldg(a.b_r + (size_t)h * L + r));
-                    const float v = score_of(x[2 * c], e[2 * c], br, (unsigned)d < (unsigned)a.attn_len, a);
+                    const float v = (unsigned)d < (unsigned)a.attn_len ? score_of(x[2 * c], e[2 * c], br, a) : -INFINITY;
                     mb = fmaxf(mb, v);
                     if (t == 0)
                         sc[warp * 64 + m * 16 + g + c * 8] = v;
@@ -598,7 +619,7 @@ template <int DK> struct BwdSmem {
     static constexpr int LPS = 152, LDE = 136; // row pitches: [P 64 | pad 8 | dS 64 | pad 16], dE window
     static constexpr int Q = 0, DO = Q + TILE, K = DO + TILE, V = K + TILE, R = V + TILE, PS = R + 2 * TILE,
                          DE = PS + 64 * LPS * 2, ES = DE + 64 * LDE * 2, ROW = ES + 4 * 16 * ESC * 4, PAD = ROW + 2 * 64 * 4, BRS = PAD + 8 * DK * 4;
-    static size_t bytes(int L) { return (size_t)BRS + (size_t)((L + 3) & ~3) * 4; }
+    static size_t bytes(int L) { return (size_t)BRS + br_bytes(L); }
 };
 
 template <int DK>
@@ -766,15 +787,12 @@ __global__ void __launch_bounds__(256, DK <= 64 ? 2 : 1) attn_bwd_kernel(const _
             if (a.w_r)
                 skewed_positions<DK>(e, Qs + qt * 16 * LD, window, qt, hf, es, lane);
             const float lA = lses[iA], lB = lses[iB], DA = Dr[iA], DB = Dr[iB];
+            scores_16x32(s, e, brs, a, qt * 16, j0 + hf * 32, T, lane);
 #pragma unroll
             for (int n = 0; n < 4; n++)
 #pragma unroll
-                for (int c = 0; c < 4; c++) {
-                    const int j = j0 + hf * 32 + n * 8 + 2 * t + (c & 1), i = c < 2 ? iA : iB, d = i + M - j;
-                    const float v = score_of(s[n][c], e[n][c], brs[min(max(j + T - 1 - i, 0), L - 1)],
-                                             (unsigned)d < (unsigned)a.attn_len && i < T, a);
-                    s[n][c] = __expf(__fsub_rn(v, c < 2 ? lA : lB));
-                }
+                for (int c = 0; c < 4; c++)
+                    s[n][c] = __expf(__fsub_rn(s[n][c], c < 2 ? lA : lB));
             product_16x32<DK>(e, Os + qt * 16 * LD, Vs + hf * 32 * LD, lane); // dP
             asm volatile("bar.sync %0, 64;" ::"r"(1 + qt) : "memory"); // both warps of the tile are done with their scratch
             bf16 *pA = PS + (qt * 16 + g) * LPS + hf * 32 + 2 * t, *pB = pA + 8 * LPS;

@@ -47,6 +47,8 @@ __global__ void __launch_bounds__(256)
 coder_paths_kernel(const float *__restrict__ probs, const int32_t *__restrict__ sym,
                    uint16_t *__restrict__ out, int V, int n_bits)
 {
+    pdl_trigger();
+    pdl_wait();
     extern __shared__ float S[];
     const int row = blockIdx.x;
     build_sum_tree(S, probs + (size_t)row * V, V);
@@ -76,6 +78,8 @@ __global__ void __launch_bounds__(256)
 coder_paths_fast_kernel(const float *__restrict__ probs, const int32_t *__restrict__ sym,
                         uint16_t *__restrict__ out, int V, int n_bits)
 {
+    pdl_trigger();
+    pdl_wait();
     __shared__ float heap[256]; // top of the tree: entries [1, 2*NW), NW = V/128 <= 128
     __shared__ float p0s[16];
     const int row = blockIdx.x, tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
@@ -137,6 +141,8 @@ coder_paths_fast_kernel(const float *__restrict__ probs, const int32_t *__restri
 __global__ void __launch_bounds__(256)
 coder_trees_kernel(const float *__restrict__ probs, uint16_t *__restrict__ out, int V)
 {
+    pdl_trigger();
+    pdl_wait();
     extern __shared__ float S[];
     const int row = blockIdx.x;
     build_sum_tree(S, probs + (size_t)row * V, V);
@@ -210,6 +216,8 @@ __global__ void __launch_bounds__(256)
 coder_paths_any_kernel(const float *__restrict__ probs, const int32_t *__restrict__ sym,
                        uint16_t *__restrict__ out, int V, int P, int L)
 {
+    pdl_trigger();
+    pdl_wait();
     extern __shared__ float S[];
     const int row = blockIdx.x;
     build_sum_tree_any(S, probs + (size_t)row * V, V, P);
@@ -243,6 +251,8 @@ coder_paths_any_kernel(const float *__restrict__ probs, const int32_t *__restric
 __global__ void __launch_bounds__(256)
 coder_trees_any_kernel(const float *__restrict__ probs, uint16_t *__restrict__ out, int V, int P)
 {
+    pdl_trigger();
+    pdl_wait();
     extern __shared__ float S[];
     const int row = blockIdx.x;
     build_sum_tree_any(S, probs + (size_t)row * V, V, P);

@@ -58,6 +58,8 @@ decode_step_kernel(const uint16_t *__restrict__ trees, const uint8_t *__restrict
                    int32_t *__restrict__ sym_out, int32_t *__restrict__ ids_next, int t, int limit_t, int limit_b,
                    int B, int V, int P, int nb, int ring, int *err_flag)
 {
+    pdl_trigger();
+    pdl_wait();
     extern __shared__ __align__(128) uint8_t dsm[];
     uint64_t *bars = reinterpret_cast<uint64_t *>(dsm);           // [MAX_RING] of 8 bytes, 128 reserved
     uint16_t *slots = reinterpret_cast<uint16_t *>(dsm + 128);    // [ring][P]

@@ -376,6 +376,7 @@ norm_bwd_vec_kernel(const T *__restrict__ dy, const T *__restrict__ x, const flo
 template <typename TO>
 __global__ void splitk_reduce_kernel(const float *__restrict__ ws, int ksplit, size_t n, TO *__restrict__ out)
 {
+    pdl_trigger();
     pdl_wait();
     const size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
     if (i >= n)
@@ -991,6 +992,8 @@ __global__ void f32_to_bf16_kernel(const float *__restrict__ src, bf16 *__restri
 // them, in ascending order, into the four columns it owns; the other blocks leave after two loads.
 __global__ void first_rows_kernel(const int32_t *__restrict__ ids, int rows, int V, int *__restrict__ first)
 {
+    pdl_trigger();
+    pdl_wait();
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= rows)
         return;
