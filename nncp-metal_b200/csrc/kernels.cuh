@@ -371,6 +371,12 @@ norm_bwd_vec_kernel(const T *__restrict__ dy, const T *__restrict__ x, const flo
         fold(ds, 2);
 }
 
+__device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi)
+{
+    __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<uint32_t *>(&h);
+}
+
 // out[i] = ws[0][i] + ws[1][i] + ... (in that order) for the partial products of a split-K GEMM;
 // n a multiple of 4.
 template <typename TO>
@@ -386,10 +392,12 @@ __global__ void splitk_reduce_kernel(const float *__restrict__ ws, int ksplit, s
         const float4 v = *reinterpret_cast<const float4 *>(ws + (size_t)z * n + i);
         acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
     }
-    out[i] = from_f<TO>(acc.x);
-    out[i + 1] = from_f<TO>(acc.y);
-    out[i + 2] = from_f<TO>(acc.z);
-    out[i + 3] = from_f<TO>(acc.w);
+    if constexpr (sizeof(TO) == 4) {
+        *reinterpret_cast<float4 *>(out + i) = acc;
+    } else {
+        const uint2 pk = make_uint2(pack_bf16x2(acc.x, acc.y), pack_bf16x2(acc.z, acc.w));
+        *reinterpret_cast<uint2 *>(out + i) = pk;
+    }
 }
 
 // Column reduction of partial sums, fixed order: out_k[c] = sum_p part[p*stride + off_k + c].
@@ -592,6 +600,8 @@ template <typename T>
 __global__ void act_fwd_kernel(const T *__restrict__ hpre, T *__restrict__ hact, int rows, int F,
                                int F1, int act)
 {
+    pdl_trigger();
+    pdl_wait();
     size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= (size_t)rows * F)
         return;
@@ -765,12 +775,6 @@ __device__ __forceinline__ float block_max_256(float v, float *red)
     for (int w = 1; w < 8; w++)
         s = fmaxf(s, red[w]);
     return s;
-}
-
-__device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi)
-{
-    __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
-    return *reinterpret_cast<uint32_t *>(&h);
 }
 
 // in-place softmax over the V symbols of each row of fp32 logits (nc_soft_max, nncp.c:1008).

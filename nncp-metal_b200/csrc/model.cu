@@ -43,6 +43,7 @@ static int coder_depth(int V)
 #include "gemm_simt.cuh"
 #include "gemm_tc.cuh"
 #include "kernels.cuh"
+#include "gemm_tc2.cuh"
 #include "decoder.cuh"
 
 thread_local char g_nncu_err[512] = "";
@@ -245,33 +246,32 @@ static int check_err_flag(nncu_model *m)
     return NNCU_OK;
 }
 
-// y = x W^T (+bias): C[M][N] = A[M][K] . Wt[N][K]^T
-template <typename AT, typename TC>
-static int mm_nt(nncu_model *m, int M, int N, int K, const AT *A, long lda, size_t w_off, TC *C,
-                 long ldc, const float *bias, int bias_n = 1 << 30);
-
+// y = x W^T (+bias): C[M][N] = A[M][K] . Wt[N][K]^T; bias (if any) is added to output columns n < bias_n
+// only.  Of the extras, what is only a saving (the hole) may be ignored; *did_act says whether
+// the second output was written.
 template <typename TC>
 static int mm_nt_impl(nncu_model *m, int M, int N, int K, const float *A, long lda, size_t w_off,
-                      TC *C, long ldc, const float *bias, int bias_n)
+                      TC *C, long ldc, const float *bias, int bias_n, const tc2::Extra &, bool *)
 {
-    return gemm_simt<float, float, TC>(m->st, GEMM_NT, M, N, K, A, lda, m->W + w_off, K, C, ldc, bias, (const TC *)nullptr,
-                                       bias_n);
+    return gemm_simt<float, float, TC>(m->st, GEMM_NT, M, N, K, A, lda, m->W + w_off, K, C, ldc, bias,
+                                           (const TC *)nullptr, bias_n);
 }
 template <typename TC>
 static int mm_nt_impl(nncu_model *m, int M, int N, int K, const bf16 *A, long lda, size_t w_off,
-                      TC *C, long ldc, const float *bias, int bias_n)
+                      TC *C, long ldc, const float *bias, int bias_n, const tc2::Extra &x, bool *did_act)
 {
     const bf16 *Wt = m->Wb + w_off;
     if (m->use_tc && tc::usable(A, lda, Wt, K, K))
-        return tc::gemm_nt<TC>(m->st, M, N, K, A, lda, Wt, K, C, ldc, bias, nullptr, m->err_flag, bias_n);
+        return tc2::gemm<TC, false, false>(m->st, M, N, K, A, lda, Wt, K, C, ldc, bias, nullptr, m->err_flag, bias_n, x, did_act);
     return gemm_simt<bf16, bf16, TC>(m->st, GEMM_NT, M, N, K, A, lda, Wt, K, C, ldc, bias, (const TC *)nullptr, bias_n);
 }
-// bias (if any) is added to output columns n < bias_n only
 template <typename AT, typename TC>
 static int mm_nt(nncu_model *m, int M, int N, int K, const AT *A, long lda, size_t w_off, TC *C,
-                 long ldc, const float *bias, int bias_n)
+                 long ldc, const float *bias, int bias_n = 1 << 30, const tc2::Extra &x = tc2::Extra(), bool *did_act = nullptr)
 {
-    return mm_nt_impl<TC>(m, M, N, K, A, lda, w_off, C, ldc, bias, bias_n);
+    if (did_act)
+        *did_act = false;
+    return mm_nt_impl<TC>(m, M, N, K, A, lda, w_off, C, ldc, bias, bias_n, x, did_act);
 }
 
 // MN-major tensor-core operands (default) or explicit transposes (NNCU_TC_TRANSPOSE=1)
@@ -308,7 +308,7 @@ static int mm_nn(nncu_model *m, int M, int Kin, int Nout, const bf16 *dY, long l
             KERNEL_CHECK();
             return NNCU_OK;
         }
-        return tc::gemm<bf16, false, true>(m->st, M, Kin, Nout, dY, ldy, m->Wb + w_off, Kin, C, ldc, nullptr,
+        return tc2::gemm<bf16, false, true>(m->st, M, Kin, Nout, dY, ldy, m->Wb + w_off, Kin, C, ldc, nullptr,
                                            addsrc, m->err_flag);
     }
     const bf16 *WT = m->WbT + w_off; // [Kin][Nout]
@@ -351,19 +351,41 @@ static float *part_slot(nncu_model *m)
     return p;
 }
 
+// dY rows below skip_r are zero in the first skip_n columns (the q gradients of memory rows)
 static int mm_tn(nncu_model *m, int Nout, int Kin, int R, const float *dY, long ldy, const float *X,
-                 long ldx, float *Gout)
+                 long ldx, float *Gout, int = 0, int = 0)
 {
     return gemm_simt<float, float, float>(side_fork(m), GEMM_TN, Nout, Kin, R, dY, ldy, X, ldx, Gout, Kin,
                                           nullptr, (const float *)nullptr);
 }
 static int mm_tn(nncu_model *m, int Nout, int Kin, int R, const bf16 *dY, long ldy, const bf16 *X,
-                 long ldx, float *Gout)
+                 long ldx, float *Gout, int skip_r = 0, int skip_n = 0)
 {
-    if (m->use_tc && tc_mn_major() && tc::usable(dY, ldy, X, ldx, R))
+    if (m->use_tc && tc_mn_major() && tc::usable(dY, ldy, X, ldx, R)) {
         // dY is [R][Nout] = [k][m], X is [R][Kin] = [k][n]: both MN-major, read in place
-        return tc::gemm<float, true, true>(side_fork(m), Nout, Kin, R, dY, ldy, X, ldx, Gout, Kin, nullptr,
-                                           nullptr, m->err_flag);
+        cudaStream_t st = side_fork(m);
+        tc2::Extra x;
+        x.skip_m = skip_n;
+        x.skip_k = skip_r;
+        // A long contraction into few tiles (the projection's weight gradient over all memory rows) is split
+        // over the idle pairs; the parts are added in order.  1536 x 512 x 73728: 176 us with one CTA per
+        // 128 x 64 tile, 12 tiles of 256 x 256 on 74 pairs in six parts 78.
+        const int tiles = tc2::tile_count(Nout, Kin, 256, x), parts = tiles ? tc2::PAIRS / tiles : 1;
+        if (R >= 8192 && parts >= 2 && Nout % 256 == 0 && Kin % 4 == 0 && m->skw) {
+            x.ksplit = std::min(parts, 8);
+            const size_t n = (size_t)Nout * Kin;
+            if (n * x.ksplit <= m->skw_floats) {
+                NNCU_TRY((tc2::launch<256, float, true, true>(st, Nout, Kin, R, dY, ldy, X, ldx, m->skw, Kin, nullptr, nullptr, m->err_flag,
+                                                              1 << 30, x)));
+                launch_k(splitk_reduce_kernel<float>, dim3((unsigned)ceil_div((long long)(n / 4), 256)), dim3(256), 0, st, m->skw, x.ksplit, n,
+                         Gout);
+                KERNEL_CHECK();
+                return NNCU_OK;
+            }
+            x.ksplit = 1;
+        }
+        return tc2::gemm<float, true, true>(st, Nout, Kin, R, dY, ldy, X, ldx, Gout, Kin, nullptr, nullptr, m->err_flag, 1 << 30, x);
+    }
     if (m->use_tc && (R % 8) == 0) {
         // both operands become K-major by an explicit transpose (the contraction runs over rows)
         bf16 *tA = reinterpret_cast<bf16 *>(m->tA), *tB = reinterpret_cast<bf16 *>(m->tB);
@@ -591,10 +613,13 @@ static int forward_range(nncu_model *m, int t0, int t1)
         // all layers on the side stream at the start of the pass, the main chain projecting the segment
         // rows only -- 2.686 against 2.594 ms per step: twelve more launches competing for SMs cost the
         // latency-bound main chain more than the shorter projection saves.
-        if (t0 == 0 && M > 0)
+        if (t0 == 0 && M > 0) {
+            tc2::Extra x; // the memory rows need no q: whole tiles of them are left out
+            x.hole_m = M * B;
+            x.hole_n = HD;
             NNCU_TRY((mm_nt<AT, AT>(m, M * B + nr, 3 * HD, D, hc, D, o.w_q, at<AT>(a.qkv, 0), 3 * HD,
-                                    wf(m, o.b_q), HD)));
-        else
+                                    wf(m, o.b_q), HD, x)));
+        } else
             NNCU_TRY((mm_nt<AT, AT>(m, nr, 3 * HD, D, x1, D, o.w_q,
                                     at<AT>(a.qkv, ((size_t)M * B + r0) * 3 * HD), 3 * HD, wf(m, o.b_q), HD)));
         nncu_attn_shape s = attn_shape(m, l, t0, t1);
@@ -621,13 +646,22 @@ static int forward_range(nncu_model *m, int t0, int t1)
             NNCU_TRY(norm_fwd<AT>(m, tmp, xin, post ? at<AT>(a.s1, (size_t)r0 * D) : nullptr, yy, o.ln_g1, o.ln_b1,
                                   a.st_1 + 2 * r0, nr, post));
         AT *hpre = at<AT>(a.hpre, (size_t)r0 * F1), *hact = at<AT>(a.hact, (size_t)r0 * F);
-        NNCU_TRY((mm_nt<AT, AT>(m, nr, F1, D, u, D, o.ff1, hpre, F1, wf(m, o.ff_bias1))));
-        if (sizeof(AT) == 2 && F % 8 == 0 && F1 % 8 == 0)
-            launch_k(act_fwd_vec_kernel, dim3(ceil_div((long long)nr * (F / 8), 256)), dim3(256), 0, m->st,
-                     (const bf16 *)hpre, (bf16 *)hact, nr, F, F1, p.ff_act);
-        else
-            act_fwd_kernel<AT><<<ceil_div((long long)nr * F, 256), 256, 0, m->st>>>(hpre, hact, nr, F, F1, p.ff_act);
-        KERNEL_CHECK();
+        bool did_act = false;
+        tc2::Extra xa; // the pair kernel writes the activation of an ungated feed-forward beside its argument
+        if (F1 == F && (p.ff_act == NNCU_FF_RELU || p.ff_act == NNCU_FF_GELU)) {
+            xa.C2 = hact;
+            xa.act = p.ff_act;
+        }
+        NNCU_TRY((mm_nt<AT, AT>(m, nr, F1, D, u, D, o.ff1, hpre, F1, wf(m, o.ff_bias1), 1 << 30, xa, &did_act)));
+        if (!did_act) {
+            if (sizeof(AT) == 2 && F % 8 == 0 && F1 % 8 == 0)
+                launch_k(act_fwd_vec_kernel, dim3(ceil_div((long long)nr * (F / 8), 256)), dim3(256), 0, m->st, (const bf16 *)hpre,
+                         (bf16 *)hact, nr, F, F1, p.ff_act);
+            else
+                launch_k(act_fwd_kernel<AT>, dim3(ceil_div((long long)nr * F, 256)), dim3(256), 0, m->st, (const AT *)hpre, hact, nr, F,
+                         F1, p.ff_act);
+            KERNEL_CHECK();
+        }
         if (o.alpha != NONE) {
             AT *aff = at<AT>(a.aff, (size_t)r0 * D);
             NNCU_TRY((mm_nt<AT, AT>(m, nr, D, F, hact, F, o.ff2, aff, D, wf(m, o.ff_bias2))));
@@ -925,7 +959,7 @@ static int backward(nncu_model *m)
             }
         }
         // d[w_q ; w_kv] = [dq | dk | dv]^T [memory ; segment] in one contraction over all L*B rows
-        NNCU_TRY(mm_tn(m, 3 * HD, D, LB, dqkv, 3 * HD, hc, D, gf(m, o.w_q)));
+        NNCU_TRY(mm_tn(m, 3 * HD, D, LB, dqkv, 3 * HD, hc, D, gf(m, o.w_q), M * B, HD));
         if (o.b_q != NONE)
             NNCU_TRY(colsum<AT>(m, dq, 3 * HD, TB, HD, gf(m, o.b_q)));
         // d(attention input) = [dq | dk | dv](segment rows) [w_q ; w_kv]; the memory rows get no gradient
@@ -1351,7 +1385,8 @@ int nncu_create(const nncu_params *p, nncu_model **out)
     part_floats = std::max(part_floats, (size_t)ceil_div(TB, ACT_BWD_ROWS) * F1);
     size_t oPart = take(part_floats * 4 * PART_SLOTS);
     m->part_floats = part_floats;
-    const size_t skw_floats = (m->use_tc && V >= SPLITK_MIN_K) ? (size_t)SPLITK * TB * D : 0;
+    // split-K workspace: the output head's dX (SPLITK parts) and the projections' weight gradients (up to 8)
+    const size_t skw_floats = !m->use_tc ? 0 : std::max(V >= SPLITK_MIN_K ? (size_t)SPLITK * TB * D : 0, LB >= 8192 ? (size_t)8 * 3 * HD * D : 0);
     size_t oSkw = take(skw_floats * 4 + 256);
     size_t oLogp = take((size_t)TB * 4), oLoss = take(256);
     size_t oIds = take((size_t)TB * 4), oTgt = take((size_t)TB * 4), oErr = take(256), oHash = take(256);
@@ -2426,14 +2461,14 @@ int nncu_gemm_bf16(int backend, int mode, int M, int N, int K, const void *A, in
     NNCU_TRY(gemm_flag(&flag));
     int rc;
     if (mode == GEMM_NT)
-        rc = c_is_f32 ? tc::gemm<float, false, false>(st, M, N, K, a, lda, b, ldb, (float *)C, ldc, nullptr, nullptr, flag)
-                      : tc::gemm<bf16, false, false>(st, M, N, K, a, lda, b, ldb, (bf16 *)C, ldc, nullptr, nullptr, flag);
+        rc = c_is_f32 ? tc2::gemm<float, false, false>(st, M, N, K, a, lda, b, ldb, (float *)C, ldc, nullptr, nullptr, flag)
+                      : tc2::gemm<bf16, false, false>(st, M, N, K, a, lda, b, ldb, (bf16 *)C, ldc, nullptr, nullptr, flag);
     else if (mode == GEMM_NN)
-        rc = c_is_f32 ? tc::gemm<float, false, true>(st, M, N, K, a, lda, b, ldb, (float *)C, ldc, nullptr, nullptr, flag)
-                      : tc::gemm<bf16, false, true>(st, M, N, K, a, lda, b, ldb, (bf16 *)C, ldc, nullptr, nullptr, flag);
+        rc = c_is_f32 ? tc2::gemm<float, false, true>(st, M, N, K, a, lda, b, ldb, (float *)C, ldc, nullptr, nullptr, flag)
+                      : tc2::gemm<bf16, false, true>(st, M, N, K, a, lda, b, ldb, (bf16 *)C, ldc, nullptr, nullptr, flag);
     else
-        rc = c_is_f32 ? tc::gemm<float, true, true>(st, M, N, K, a, lda, b, ldb, (float *)C, ldc, nullptr, nullptr, flag)
-                      : tc::gemm<bf16, true, true>(st, M, N, K, a, lda, b, ldb, (bf16 *)C, ldc, nullptr, nullptr, flag);
+        rc = c_is_f32 ? tc2::gemm<float, true, true>(st, M, N, K, a, lda, b, ldb, (float *)C, ldc, nullptr, nullptr, flag)
+                      : tc2::gemm<bf16, true, true>(st, M, N, K, a, lda, b, ldb, (bf16 *)C, ldc, nullptr, nullptr, flag);
     if (rc != NNCU_OK)
         return rc;
     return gemm_flag_check(flag, st);
@@ -2453,8 +2488,8 @@ int nncu_gemm_bf16_nt(int backend, int M, int N, int K, const void *A, int lda, 
     }
     int *flag = nullptr;
     NNCU_TRY(gemm_flag(&flag));
-    int rc = c_is_f32 ? tc::gemm_nt<float>(st, M, N, K, a, lda, b, ldb, (float *)C, ldc, bias, nullptr, flag)
-                      : tc::gemm_nt<bf16>(st, M, N, K, a, lda, b, ldb, (bf16 *)C, ldc, bias, nullptr, flag);
+    int rc = c_is_f32 ? tc2::gemm<float, false, false>(st, M, N, K, a, lda, b, ldb, (float *)C, ldc, bias, nullptr, flag)
+                      : tc2::gemm<bf16, false, false>(st, M, N, K, a, lda, b, ldb, (bf16 *)C, ldc, bias, nullptr, flag);
     if (rc != NNCU_OK)
         return rc;
     return gemm_flag_check(flag, st);

@@ -1,0 +1,97 @@
+"""Kernels at the sizes where they can go wrong: edges of tiles, remainders, one-tile and many-tile
+launches, through the C ABI."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from conftest import rel_err
+from test_gpu_parity import _attn_case
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("mode,M,N,K", [(0, 20480, 1544, 520), (0, 33000, 768, 64), (0, 20481, 1000, 1096), (1, 20483, 1032, 136),
+                                        (2, 5000, 5008, 72), (2, 6144, 1032, 2056), (0, 19200, 1024, 8)])
+@pytest.mark.parametrize("c_f32", [0, 1])
+def test_many_tile_gemm_vs_fp32(pkg, mode, M, N, K, c_f32):
+    """More output tiles than CTA pairs: ragged last rows, columns and k-blocks, one k-block alone (no
+    odd chain), every operand arrangement, both output types."""
+    lib = pkg.library()
+    g = torch.Generator(device="cuda").manual_seed(M + N + K + mode)
+    a = torch.randn((K, M) if mode == 2 else (M, K), generator=g, device="cuda").bfloat16()
+    if mode == 2 and M % 8:
+        pytest.skip("rows of a transposed operand are 16-byte aligned")
+    b = torch.randn((N, K) if mode == 0 else (K, N), generator=g, device="cuda").bfloat16()
+    ref = (a.float().T if mode == 2 else a.float()) @ (b.float().T if mode == 0 else b.float())
+    c = torch.full((M, N), float("nan"), device="cuda", dtype=torch.float32 if c_f32 else torch.bfloat16)
+    assert lib.nncu_gemm_bf16(pkg.abi.GEMM_TCGEN05, mode, M, N, K, a.data_ptr(), a.shape[1], b.data_ptr(), b.shape[1],
+                              c.data_ptr(), N, c_f32, None) == 0, lib.nncu_last_error()
+    assert (c.float() - ref).abs().max().item() < (5e-5 if c_f32 else 5e-3) * ref.abs().max().item()
+    if mode == 0:   # the rows of a one-tile launch, which takes the other kernel, are the same bits
+        part = torch.zeros(40, N, device="cuda", dtype=c.dtype)
+        off = M - 40
+        assert lib.nncu_gemm_bf16(pkg.abi.GEMM_TCGEN05, 0, 40, N, K, a[off:].data_ptr(), K, b.data_ptr(), K,
+                                  part.data_ptr(), N, c_f32, None) == 0, lib.nncu_last_error()
+        assert torch.equal(part, c[off:])
+
+
+@pytest.mark.parametrize("B,H,dk,T,M,P,alen", [(1, 1, 64, 1, 1, 2, 0), (2, 1, 64, 64, 65, 129, 0), (1, 2, 32, 16, 48, 33, 0),
+                                               (2, 1, 128, 64, 256, 300, 0), (3, 1, 16, 17, 64, 81, 30), (1, 2, 128, 64, 1, 65, 2)])
+def test_attention_edges_bf16(pkg, oracle, B, H, dk, T, M, P, alen):
+    """One query, one key more than the blocks hold, a table that ends inside the left pad, a window of two keys."""
+    _attn_case(pkg, oracle, B, H, dk, T, M, P, alen, True, 7)
+
+
+@pytest.mark.parametrize("dk,T,M,P,alen", [(16, 20, 100, 50, 0), (32, 64, 300, 364, 0), (64, 64, 513, 577, 0), (64, 70, 64, 90, 100),
+                                           (128, 33, 256, 289, 200)])
+def test_attention_single_queries_equal_the_segment_bitwise(pkg, dk, T, M, P, alen):
+    """The one-query kernel against the segment kernel, every query: output and log-sum-exp bit for bit."""
+    lib = pkg.library()
+    B, H, L = 3, 2, T + M
+    g = torch.Generator(device="cuda").manual_seed(dk + T + M)
+    q = torch.randn(T * B, H * dk, generator=g, device="cuda").bfloat16()
+    kv = torch.randn(L * B, 2 * H * dk, generator=g, device="cuda").bfloat16()
+    w_r = 0.1 * torch.randn(H, P, dk, generator=g, device="cuda")
+    b_r = 0.1 * torch.randn(H, L, generator=g, device="cuda")
+    outs = []
+    for ranges in ([(0, T)], [(t, t + 1) for t in range(T)]):
+        out, lse = torch.zeros_like(q), torch.zeros(B * H, T, device="cuda")
+        for t0, t1 in ranges:
+            shp = pkg.abi.AttnShape(B, H, dk, T, M, P, alen, t0, t1, float(np.sqrt(dk * 512.0)), 1)
+            assert lib.nncu_attention_forward(C.byref(shp), q.data_ptr(), kv.data_ptr(), w_r.data_ptr(), b_r.data_ptr(),
+                                              out.data_ptr(), lse.data_ptr(), None) == 0, lib.nncu_last_error()
+        torch.cuda.synchronize()
+        outs.append((out, lse))
+    assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
+
+
+def test_attention_edges_fp32(pkg, oracle):
+    """The CUDA-core kernels: a head size that is no multiple of four, one that fills the shared memory up
+    to the narrow row pitch, a left pad of most of the table."""
+    for B, H, dk, T, M, P, alen in ((2, 2, 6, 7, 9, 16, 0), (1, 1, 64, 32, 120, 152, 0), (2, 1, 32, 31, 40, 3, 20)):
+        _attn_case(pkg, oracle, B, H, dk, T, M, P, alen, False, 8)
+
+
+@pytest.mark.parametrize("ln,act,D,n_head", [(1, 1, 256, 4), (2 | 4 | 16, 2, 384, 3)])
+def test_gradients_of_a_long_memory_match_the_other_engine(pkg, ln, act, D, n_head):
+    """Projection gradients over 9216 rows: the memory rows' query part is left out in both passes, the
+    contraction is split over idle CTA pairs; rows that are no multiple of 512 bytes go through the norms."""
+    kw = dict(n_layer=1, d_model=D, n_head=n_head, d_key=D // n_head, d_inner=2 * D, d_pos=192, mem_len=128, seg_len=64,
+              n_streams=48, n_symbols=512, use_bf16=1, init_range=0.05, ln_flags=ln, ff_act=act)
+    rng = np.random.default_rng(3)
+    ids, tg = (rng.integers(0, 512, (3, 64, 48)).astype(np.int32) for _ in range(2))
+    got = []
+    for backend in (1, 2):
+        m = pkg.TrfModel(pkg.abi.make_params(gemm_backend=backend, **kw))
+        m.reset()
+        for s in range(3):
+            m.eval(-1, ids[s], read=False)
+            loss = m.eval_gradient(tg[s])
+            m.memory_shift()
+        got.append(({n: m.get_grad(n) for n in m.info}, loss))
+        m.close()
+    assert abs(got[0][1] - got[1][1]) < 1e-3 * abs(got[0][1])
+    for n in got[0][0]:
+        assert rel_err(got[1][0][n], got[0][0][n]) < 2e-2, n
