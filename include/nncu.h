@@ -146,6 +146,9 @@ int nncu_destroy(nncu_model *m);
    stream the whole-segment forward and the backward pass are captured into CUDA graphs on
    their second use and replayed afterwards (same results, fewer launch gaps). */
 int nncu_set_stream(nncu_model *m, void *cuda_stream);
+/* The same with a stream that the model makes for itself and destroys with itself (what the file-level
+   host code binds: no other stream has to see its launches). */
+int nncu_own_stream(nncu_model *m);
 
 /* ---- the 13-pointer plugin surface (nncp.c:49-69) ---- */
 /* model_reset: zero the memory of every layer (nncp.c:1195-1203). */

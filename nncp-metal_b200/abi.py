@@ -82,6 +82,7 @@ PROTOTYPES = {
     "nncu_create": (_i, [C.POINTER(Params), C.POINTER(_vp)]),
     "nncu_destroy": (_i, [_vp]),
     "nncu_set_stream": (_i, [_vp, _vp]),
+    "nncu_own_stream": (_i, [_vp]),
     "nncu_reset": (_i, [_vp]),
     "nncu_set_lr": (_i, [_vp, C.c_float]),
     "nncu_eval": (_i, [_vp, _i, _vp]),

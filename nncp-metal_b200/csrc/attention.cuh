@@ -91,26 +91,64 @@ __device__ __forceinline__ float dot_q(const float *__restrict__ qf, const T *__
     return s;
 }
 
-// score of (query i, key j) for an unmasked pair
+// score of (query i, key j) for an unmasked pair; br: the head's row of b_r, Rs NULL without a table
 template <typename T>
-__device__ __forceinline__ float score_ij(const AttnArgs &a, int h, int i, int j, const float *qf,
-                                          const T *Ks, const T *Rs, int ks)
+__device__ __forceinline__ float score_ij(int i, int j, int Tn, int L, int P, int dk, float inv_sqrt, float br_scale,
+                                          const float *qf, const T *Ks, const T *Rs, int ks, const float *br)
 {
-    float s = dot_q<T>(qf, Ks + (size_t)j * ks, a.dk);
-    int r = j + (a.T - 1) - i;
-    float z = a.br_scale * a.b_r[(size_t)h * a.L + r];
-    if (a.w_r) {
-        int pi = r - (a.L - a.P);
+    const float s = dot_q<T>(qf, Ks + (size_t)j * ks, dk);
+    const int r = j + (Tn - 1) - i;
+    float z = __fmul_rn(br_scale, br[r]);
+    if (Rs) {
+        int pi = r - (L - P);
         pi = pi < 0 ? 0 : pi;
-        z += dot_q<T>(qf, Rs + (size_t)pi * ks, a.dk);
+        z = __fadd_rn(z, dot_q<T>(qf, Rs + (size_t)pi * ks, dk));
     }
-    return (s + z) * a.inv_sqrt;
+    return __fmul_rn(__fadd_rn(s, z), inv_sqrt);
+}
+__device__ __forceinline__ void attn_key_range(int L, int M, int attn_len, int i, int &jlo, int &jhi)
+{
+    jhi = min(L - 1, i + M);                 // (i+M)-j >= 0
+    jlo = max(0, i + M - attn_len + 1);      // (i+M)-j < attn_len
+}
+
+// One query row by one warp: keys [jlo, jhi] over the lanes, output column e to out(e, value), log-sum-exp
+// in lse.  qf: the query as floats; ps: scratch for the scores, indexed by key.
+template <typename T, typename F>
+__device__ __forceinline__ void attn_row(int i, int jlo, int jhi, int Tn, int L, int P, int dk, float inv_sqrt, float br_scale,
+                                         const float *qf, const T *Ks, const T *Rs, int ks, const T *Vs, const float *br, float *ps,
+                                         int lane, float &lse, F out)
+{
+    float mx = -INFINITY;
+    for (int j = jlo + lane; j <= jhi; j += 32) {
+        float s = score_ij<T>(i, j, Tn, L, P, dk, inv_sqrt, br_scale, qf, Ks, Rs, ks, br);
+        ps[j] = s;
+        mx = fmaxf(mx, s);
+    }
+    mx = warp_max(mx);
+    float sum = 0.0f;
+    for (int j = jlo + lane; j <= jhi; j += 32) {
+        float p = expf(__fsub_rn(ps[j], mx));
+        ps[j] = p;
+        sum = __fadd_rn(sum, p);
+    }
+    sum = warp_sum(sum);
+    const float rs = __fdiv_rn(1.0f, sum);
+    __syncwarp();
+    for (int e = lane; e < dk; e += 32) {
+        float acc = 0.0f;
+#pragma unroll 8
+        for (int j = jlo; j <= jhi; j++)
+            acc = fmaf(__fmul_rn(ps[j], rs), to_f(Vs[(size_t)j * dk + e]), acc);
+        out(e, acc);
+    }
+    lse = __fadd_rn(mx, logf(sum));
+    __syncwarp();
 }
 
 __device__ __forceinline__ void key_range(const AttnArgs &a, int i, int &jlo, int &jhi)
 {
-    jhi = min(a.L - 1, i + a.M);                 // (i+M)-j >= 0
-    jlo = max(0, i + a.M - a.attn_len + 1);      // (i+M)-j < attn_len
+    attn_key_range(a.L, a.M, a.attn_len, i, jlo, jhi);
 }
 
 // floats a warp of the forward kernel keeps: the query row and its scores
@@ -171,32 +209,12 @@ __global__ void __launch_bounds__(256) attn_fwd_kernel(AttnArgs a)
         __syncwarp();
         int jlo, jhi;
         key_range(a, i, jlo, jhi);
-        float mx = -INFINITY;
-        for (int j = jlo + lane; j <= jhi; j += 32) {
-            float s = score_ij<T>(a, h, i, j, qf, Ks, Rs, ks);
-            ps[j] = s;
-            mx = fmaxf(mx, s);
-        }
-        mx = warp_max(mx);
-        float sum = 0.0f;
-        for (int j = jlo + lane; j <= jhi; j += 32) {
-            float p = expf(ps[j] - mx);
-            ps[j] = p;
-            sum += p;
-        }
-        sum = warp_sum(sum);
-        const float rs = 1.0f / sum;
-        __syncwarp();
-        for (int e = lane; e < a.dk; e += 32) {
-            float acc = 0.0f;
-#pragma unroll 8
-            for (int j = jlo; j <= jhi; j++)
-                acc = fmaf(ps[j] * rs, to_f(Vs[(size_t)j * a.dk + e]), acc);
-            o[((size_t)i * a.B + b) * HD + h * a.dk + e] = from_f<T>(acc);
-        }
+        float lse;
+        attn_row<T>(i, jlo, jhi, a.T, a.L, a.P, a.dk, a.inv_sqrt, a.br_scale, qf, Ks, a.w_r ? Rs : nullptr, ks, Vs,
+                    a.b_r + (size_t)h * a.L, ps, lane, lse,
+                    [&](int e, float v) { o[((size_t)i * a.B + b) * HD + h * a.dk + e] = from_f<T>(v); });
         if (lane == 0 && a.lse)
-            a.lse[((size_t)b * a.H + h) * a.T + i] = mx + logf(sum);
-        __syncwarp();
+            a.lse[((size_t)b * a.H + h) * a.T + i] = lse;
     }
 }
 
@@ -289,7 +307,7 @@ __global__ void __launch_bounds__(256) attn_bwd_kernel(AttnArgs a)
         for (int j = lane; j < L; j += 32) {
             float p = 0.0f, d = 0.0f;
             if (j >= jlo && j <= jhi) {
-                p = expf(score_ij<T>(a, h, i, j, qf, Ks, Rs, ks) - lse);
+                p = expf(score_ij<T>(i, j, Tn, L, P, dk, a.inv_sqrt, a.br_scale, qf, Ks, a.w_r ? Rs : nullptr, ks, a.b_r + (size_t)h * L) - lse);
                 d = p * (dot_q<T>(dof, Vs + (size_t)j * vs, dk) - D) * a.inv_sqrt;
             }
             Pm[(size_t)i * ls + j] = p;

@@ -30,7 +30,7 @@ __device__ __forceinline__ int prob0_of(float p0, float p)
 }
 
 // builds S[1..2V) in shared memory from one row of probabilities
-__device__ __forceinline__ void build_sum_tree(float *S, const float *__restrict__ prob, int V)
+__device__ __forceinline__ void build_sum_tree(float *S, const float *prob, int V)
 {
     for (int i = threadIdx.x; i < V; i += blockDim.x)
         S[V + i] = prob[i];
@@ -137,16 +137,15 @@ coder_paths_fast_kernel(const float *__restrict__ probs, const int32_t *__restri
     }
 }
 
-// one block per row: prob0 of every internal node, heap order, entry 0 unused
-__global__ void __launch_bounds__(256)
-coder_trees_kernel(const float *__restrict__ probs, uint16_t *__restrict__ out, int V)
+// Threads of a tree block: a row's tree is a division a node and two passes of log2 P barriers, bound by
+// the divisions for large alphabets (16384 symbols, 128 rows on 128 SMs: 42 us with 256 threads) and by
+// the barriers for small ones.
+static inline int tree_threads(int P) { return P >= 4096 ? 1024 : 256; }
+
+// prob0 of every internal node of one row's tree, heap order, entry 0 unused; S: 2 V floats of shared memory
+__device__ __forceinline__ void coder_tree_row(float *S, const float *prob, uint16_t *__restrict__ o, int V)
 {
-    pdl_trigger();
-    pdl_wait();
-    extern __shared__ float S[];
-    const int row = blockIdx.x;
-    build_sum_tree(S, probs + (size_t)row * V, V);
-    uint16_t *o = out + (size_t)row * V;
+    build_sum_tree(S, prob, V);
     if (threadIdx.x == 0) {
         S[1] = 1.0f; // running mass p at the root
         o[0] = 0;
@@ -161,6 +160,14 @@ coder_trees_kernel(const float *__restrict__ probs, uint16_t *__restrict__ out, 
         }
         __syncthreads();
     }
+}
+__global__ void __launch_bounds__(1024)
+coder_trees_kernel(const float *__restrict__ probs, uint16_t *__restrict__ out, int V)
+{
+    pdl_trigger();
+    pdl_wait();
+    extern __shared__ float S[];
+    coder_tree_row(S, probs + (size_t)blockIdx.x * V, out + (size_t)blockIdx.x * V, V);
 }
 
 // ---------------------------------------------------------------- any alphabet size
@@ -186,7 +193,7 @@ __device__ __forceinline__ void node_range(unsigned k, int V, int &lo, int &n)
 }
 
 // S[1..2P): sums of the nodes; a one-symbol node at depth L-1 has no children (their slots are 0)
-__device__ __forceinline__ void build_sum_tree_any(float *S, const float *__restrict__ prob, int V, int P)
+__device__ __forceinline__ void build_sum_tree_any(float *S, const float *prob, int V, int P)
 {
     for (int k = (P >> 1) + threadIdx.x; k < P; k += blockDim.x) {
         int lo, n;
@@ -246,17 +253,11 @@ coder_paths_any_kernel(const float *__restrict__ probs, const int32_t *__restric
     }
 }
 
-// one block per row: prob0 of every internal node in heap order, P entries per row (entry 0 and the
-// one-symbol nodes of depth L-1 hold 0)
-__global__ void __launch_bounds__(256)
-coder_trees_any_kernel(const float *__restrict__ probs, uint16_t *__restrict__ out, int V, int P)
+// prob0 of every internal node in heap order, P entries per row (entry 0 and the one-symbol nodes of
+// depth L-1 hold 0); S: 2 P floats of shared memory
+__device__ __forceinline__ void coder_tree_row_any(float *S, const float *prob, uint16_t *__restrict__ o, int V, int P)
 {
-    pdl_trigger();
-    pdl_wait();
-    extern __shared__ float S[];
-    const int row = blockIdx.x;
-    build_sum_tree_any(S, probs + (size_t)row * V, V, P);
-    uint16_t *o = out + (size_t)row * P;
+    build_sum_tree_any(S, prob, V, P);
     if (threadIdx.x == 0) {
         S[1] = 1.0f; // running mass p at the root
         o[0] = 0;
@@ -276,4 +277,12 @@ coder_trees_any_kernel(const float *__restrict__ probs, uint16_t *__restrict__ o
         }
         __syncthreads();
     }
+}
+__global__ void __launch_bounds__(1024)
+coder_trees_any_kernel(const float *__restrict__ probs, uint16_t *__restrict__ out, int V, int P)
+{
+    pdl_trigger();
+    pdl_wait();
+    extern __shared__ float S[];
+    coder_tree_row_any(S, probs + (size_t)blockIdx.x * V, out + (size_t)blockIdx.x * P, V, P);
 }

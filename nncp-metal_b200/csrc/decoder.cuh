@@ -5,10 +5,11 @@
 // cp_utils.c:326-349) bit for bit: split = (range * prob0) >> 15, bit = low >= split,
 // renormalisation one byte at a time while range < 0xFF01, zero bytes past the end of the input.
 // The streams of one step share ONE bit stream, so their symbols decode strictly one after the
-// other: a single thread walks the trees.  What can run ahead is the data movement: a ring of
-// shared-memory slots is filled with the next streams' trees by bulk copies (2 V bytes each,
-// completion on an mbarrier) while the current one is walked, and the payload bytes the step can
-// consume at most (two per bit) are staged in shared memory by the whole warp up front.
+// other: a single thread walks the trees, and its chain of operations per bit bounds the step.  What
+// can run ahead is the data movement: a second warp fills a ring of shared-memory slots with the next
+// streams' trees by bulk copies (2 V bytes each, completion on an mbarrier) while the current one is
+// walked, and the payload bytes the step can consume at most (two per bit) are staged in shared memory
+// up front.  128 streams of 14 bits: 156 us with one load of prob0 behind every decision.
 //
 // An alphabet that is not a power of two has the uneven tree of write_sym (a node of n symbols
 // sends n >> 1 left): the walk then carries the node's range beside its heap index and ends when
@@ -53,73 +54,80 @@ inline size_t smem_bytes(int B, int P, int nb, int ring) { return (size_t)ring *
 // (when not null) receive the decoded symbol, 0 for the streams past the end of the block: those at
 // step `t` are b >= limit_b when t == limit_t, and all of them when t > limit_t.
 template <bool ANY>
-__global__ void __launch_bounds__(32)
+__global__ void __launch_bounds__(64)
 decode_step_kernel(const uint16_t *__restrict__ trees, const uint8_t *__restrict__ payload, State *state,
                    int32_t *__restrict__ sym_out, int32_t *__restrict__ ids_next, int t, int limit_t, int limit_b,
                    int B, int V, int P, int nb, int ring, int *err_flag)
 {
-    pdl_trigger();
     pdl_wait();
+    pdl_trigger_late(); // a successor that was launched to overlap this kernel may start on what does not depend on it
     extern __shared__ __align__(128) uint8_t dsm[];
-    uint64_t *bars = reinterpret_cast<uint64_t *>(dsm);           // [MAX_RING] of 8 bytes, 128 reserved
+    uint64_t *bars = reinterpret_cast<uint64_t *>(dsm);           // [2][MAX_RING] of 8 bytes: 128
     uint16_t *slots = reinterpret_cast<uint16_t *>(dsm + 128);    // [ring][P]
     uint8_t *win = dsm + 128 + (size_t)ring * P * 2;              // payload window
     __shared__ int abort_s;
-    const int lane = threadIdx.x;
+    __shared__ int issued_s;
+    const int tid = threadIdx.x;
     const int n_act = t < limit_t ? B : (t == limit_t ? min(limit_b, B) : 0);
     const uint32_t slot_bytes = (uint32_t)P * 2u;
-    unsigned long long pos = state->pos;
-    const unsigned long long len = state->len, pos0 = pos;
-    uint32_t low = state->low, range = state->range;
+    const unsigned long long pos0 = state->pos, len = state->len;
+    uint64_t *done = bars + MAX_RING; // the walker has left a slot
 
-    if (lane == 0) {
+    if (tid == 0) {
         abort_s = 0;
-        for (int i = 0; i < ring; i++)
+        for (int i = 0; i < ring; i++) {
             tc::mbar_init(tc::smem_u32(bars + i), 1);
+            tc::mbar_init(tc::smem_u32(done + i), 1);
+        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    __syncwarp();
-    if (lane == 0) {
-        for (int b = 0; b < ring && b < n_act; b++) {
-            tc::mbar_expect_tx(tc::smem_u32(bars + b), slot_bytes);
-            bulk_load(tc::smem_u32(slots + (size_t)b * P), trees + (size_t)b * P, slot_bytes, tc::smem_u32(bars + b));
-        }
-    }
     const int wbytes = window_bytes(B, nb);
-    for (int i = lane; i < wbytes; i += 32)
+    for (int i = tid; i < wbytes; i += 64)
         win[i] = (pos0 + i < len) ? payload[pos0 + i] : (uint8_t)0;
-    __syncwarp();
+    __syncthreads();
 
-    if (lane == 0) {
-        bool ok = true;
-        int issued = min(ring, n_act); // streams whose copy has been issued
+    if (tid == 32) { // the copies, on a warp of their own: the walk does not stop to issue them
+        int b = 0;
+        for (; b < n_act; b++) {
+            const int s = b % ring;
+            if (b >= ring && !tc::mbar_wait(tc::smem_u32(done + s), (uint32_t)((b / ring - 1) & 1), &abort_s, err_flag, 43))
+                break;
+            tc::mbar_expect_tx(tc::smem_u32(bars + s), slot_bytes);
+            bulk_load(tc::smem_u32(slots + (size_t)s * P), trees + (size_t)b * P, slot_bytes, tc::smem_u32(bars + s));
+        }
+        issued_s = b;
+    }
+    int walked = 0;
+    bool ok = true;
+    if (tid == 0) {
+        uint32_t low = state->low, range = state->range, used = 0;
+        const uint32_t left = (uint32_t)min(len - pos0, (unsigned long long)wbytes); // payload bytes in the window
+        const uint32_t half = (uint32_t)P / 2u;
         for (int b = 0; b < B; b++) {
             int c = 0;
             if (b < n_act && ok) {
                 const int s = b % ring;
                 ok = tc::mbar_wait(tc::smem_u32(bars + s), (uint32_t)((b / ring) & 1), &abort_s, err_flag, 41);
                 if (ok) {
-                    const uint16_t *tree = slots + (size_t)s * P;
-                    int k = 1;
-                    auto next_bit = [&]() { // get_bit at node k: the branch taken, low / range / pos advanced
-                        const uint32_t prob0 = tree[k];
-                        const uint32_t split = (uint32_t)(((unsigned long long)range * prob0) >> 15);
+                    // Node k's prob0 is in hand, and its children's (one 32-bit word) are on their way, before the
+                    // branch at k is known: what a bit costs is the chain product - compare - select.
+                    // (range * prob0) >> 15 is the high word of (range << 8) * (prob0 << 9): range stays below 2^24.
+                    const uint32_t *pairs = reinterpret_cast<const uint32_t *>(slots + (size_t)s * P);
+                    uint32_t k = 1, p0 = pairs[0] >> 16, kids = pairs[1];
+                    auto next_bit = [&]() { // get_bit at node k: the branch taken, low / range / used advanced
+                        const uint32_t split = __umulhi(range << 8, p0 << 9);
                         const bool bit = low >= split;
-                        if (bit) {
-                            low -= split;
-                            range -= split;
-                        } else {
-                            range = split;
-                        }
+                        k = 2 * k + (bit ? 1u : 0u);
+                        p0 = bit ? kids >> 16 : kids & 0xffffu;
+                        kids = pairs[min(k, half - 1)];
+                        low = bit ? low - split : low;
+                        range = bit ? range - split : split;
                         while (range < R_LOW) {
                             range <<= 8;
                             low <<= 8;
-                            if (pos < len) {
-                                low += win[pos - pos0];
-                                pos++;
-                            }
+                            if (used < left)
+                                low += win[used++];
                         }
-                        k = 2 * k + (bit ? 1 : 0);
                         return bit;
                     };
                     if constexpr (ANY) {
@@ -137,32 +145,26 @@ decode_step_kernel(const uint16_t *__restrict__ trees, const uint8_t *__restrict
                     } else {
                         for (int lvl = 0; lvl < nb; lvl++)
                             next_bit();
-                        c = k - V;
+                        c = (int)k - V;
                     }
-                    if (issued < n_act) { // the slot just walked takes the tree of stream b + ring
-                        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                        tc::mbar_expect_tx(tc::smem_u32(bars + s), slot_bytes);
-                        bulk_load(tc::smem_u32(slots + (size_t)s * P), trees + (size_t)issued * P, slot_bytes,
-                                  tc::smem_u32(bars + s));
-                        issued++;
-                    }
+                    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc::smem_u32(done + s)) : "memory");
+                    walked = b + 1;
                 }
             }
             sym_out[b] = c;
             if (ids_next)
                 ids_next[b] = c;
         }
-        if (!ok) {
-            // copies still in flight land in this CTA's shared memory: give each a bounded chance to finish
-            for (int b2 = max(issued - ring, 0); b2 < issued; b2++)
-                tc::mbar_wait(tc::smem_u32(bars + b2 % ring), (uint32_t)((b2 / ring) & 1), &abort_s, err_flag, 42);
-            state->err = 1;
-        }
-        state->pos = pos;
+        state->pos = pos0 + used;
         state->low = low;
         state->range = range;
+        if (!ok)
+            state->err = 1;
     }
-    __syncwarp();
+    __syncthreads();
+    if (tid == 0 && !ok) // copies still in flight land in this CTA's shared memory: each gets a bounded chance to finish
+        for (int b = walked; b < issued_s; b++)
+            tc::mbar_wait(tc::smem_u32(bars + b % ring), (uint32_t)((b / ring) & 1), &abort_s, err_flag, 42);
 }
 
 } // namespace dec

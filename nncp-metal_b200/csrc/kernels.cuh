@@ -189,6 +189,47 @@ __device__ __forceinline__ void vec_load_f32(const float *p, int lane, int D, fl
     }
 }
 
+// v <- norm(v) * g + b for a row over a warp's registers (mode 1 LayerNorm, 2 RMSNorm, 0 nothing); lane 0
+// leaves the statistics in stats[0], stats[1] when wanted
+template <int NC, int W>
+__device__ __forceinline__ void norm_row(float (&v)[NC][W], const float *__restrict__ g, const float *__restrict__ b, int lane, int D,
+                                         int mode, float *stats)
+{
+    if (mode == 0)
+        return;
+    float gv[NC][W], bv[NC][W];
+    vec_load_f32<NC, W>(g, lane, D, gv);
+    vec_load_f32<NC, W>(b, lane, D, bv);
+    float mu = 0.0f;
+    if (mode == 1) {
+        float sum = 0.0f;
+#pragma unroll
+        for (int c = 0; c < NC; c++)
+#pragma unroll
+            for (int e = 0; e < W; e++)
+                sum += v[c][e];
+        mu = warp_sum(sum) / (float)D;
+    }
+    float var = 0.0f;
+#pragma unroll
+    for (int c = 0; c < NC; c++)
+        if (c * 32 * W + lane * W < D)
+#pragma unroll
+            for (int e = 0; e < W; e++)
+                var += (v[c][e] - mu) * (v[c][e] - mu);
+    var = warp_sum(var) / (float)D;
+    const float rstd = 1.0f / sqrtf(var + 1e-5f);
+    if (stats && lane == 0) {
+        stats[0] = mu;
+        stats[1] = rstd;
+    }
+#pragma unroll
+    for (int c = 0; c < NC; c++)
+#pragma unroll
+        for (int e = 0; e < W; e++)
+            v[c][e] = (v[c][e] - mu) * rstd * gv[c][e] + bv[c][e];
+}
+
 // residual_norm_kernel with the row in registers; same arguments and rounding points (s is rounded
 // to the storage type before the statistics), sums taken per lane, then over the warp.
 template <typename T, int NC>
@@ -221,37 +262,7 @@ residual_norm_vec_kernel(const T *__restrict__ a, const T *__restrict__ res, T *
         row_store<T, NC, W>(y + (size_t)r * D, lane, D, v);
         return;
     }
-    float gv[NC][W], bv[NC][W];
-    vec_load_f32<NC, W>(g, lane, D, gv);
-    vec_load_f32<NC, W>(b, lane, D, bv);
-    float mu = 0.0f;
-    if (mode == 1) {
-        float sum = 0.0f;
-#pragma unroll
-        for (int c = 0; c < NC; c++)
-#pragma unroll
-            for (int e = 0; e < W; e++)
-                sum += v[c][e];
-        mu = warp_sum(sum) / (float)D;
-    }
-    float var = 0.0f;
-#pragma unroll
-    for (int c = 0; c < NC; c++)
-        if (c * 32 * W + lane * W < D)
-#pragma unroll
-            for (int e = 0; e < W; e++)
-                var += (v[c][e] - mu) * (v[c][e] - mu);
-    var = warp_sum(var) / (float)D;
-    const float rstd = 1.0f / sqrtf(var + 1e-5f);
-    if (stats && lane == 0) {
-        stats[2 * r] = mu;
-        stats[2 * r + 1] = rstd;
-    }
-#pragma unroll
-    for (int c = 0; c < NC; c++)
-#pragma unroll
-        for (int e = 0; e < W; e++)
-            v[c][e] = (v[c][e] - mu) * rstd * gv[c][e] + bv[c][e];
+    norm_row<NC, W>(v, g, b, lane, D, mode, stats ? stats + 2 * r : nullptr);
     row_store<T, NC, W>(y + (size_t)r * D, lane, D, v);
 }
 
@@ -777,6 +788,28 @@ __device__ __forceinline__ float block_max_256(float v, float *red)
     return s;
 }
 
+// one row of softmax_rows_kernel, in place, by a block of 256 threads
+template <typename T> __device__ __forceinline__ void softmax_row(float *zr, int V, T *d, float scale, float *red)
+{
+    float mx = -INFINITY;
+    for (int i = threadIdx.x; i < V; i += 256)
+        mx = fmaxf(mx, zr[i]);
+    mx = block_max_256(mx, red);
+    float s = 0.0f;
+    for (int i = threadIdx.x; i < V; i += 256) {
+        float e = expf(zr[i] - mx);
+        zr[i] = e;
+        s += e;
+    }
+    s = block_sum_256(s, red);
+    float rs = 1.0f / s;
+    for (int i = threadIdx.x; i < V; i += 256) {
+        const float pv = zr[i] * rs;
+        zr[i] = pv;
+        d[i] = from_f<T>(pv * scale);
+    }
+}
+
 // in-place softmax over the V symbols of each row of fp32 logits (nc_soft_max, nncp.c:1008).
 // The output kernel of the forward pass: besides the probabilities it leaves dz = p * scale, the
 // gradient of the loss with respect to the logits of every symbol but the target (which
@@ -794,25 +827,7 @@ __global__ void __launch_bounds__(256) softmax_rows_kernel(float *__restrict__ z
         return;
     if (r == 0 && threadIdx.x == 0)
         *dz_fixed = 0;
-    float *zr = z + (size_t)r * V;
-    float mx = -INFINITY;
-    for (int i = threadIdx.x; i < V; i += 256)
-        mx = fmaxf(mx, zr[i]);
-    mx = block_max_256(mx, red);
-    float s = 0.0f;
-    for (int i = threadIdx.x; i < V; i += 256) {
-        float e = expf(zr[i] - mx);
-        zr[i] = e;
-        s += e;
-    }
-    s = block_sum_256(s, red);
-    float rs = 1.0f / s;
-    T *d = dz + (size_t)r * V;
-    for (int i = threadIdx.x; i < V; i += 256) {
-        const float pv = zr[i] * rs;
-        zr[i] = pv;
-        d[i] = from_f<T>(pv * scale);
-    }
+    softmax_row(z + (size_t)r * V, V, dz + (size_t)r * V, scale, red);
 }
 
 // The same for rows of up to 16384 logits, V a multiple of 1024: the row stays in registers

@@ -45,6 +45,7 @@ static int coder_depth(int V)
 #include "kernels.cuh"
 #include "gemm_tc2.cuh"
 #include "decoder.cuh"
+#include "step_fp32.cuh"
 
 thread_local char g_nncu_err[512] = "";
 unsigned long long g_nncu_launches = 0;
@@ -137,7 +138,7 @@ struct nncu_model {
     bool use_tc;  // tcgen05 GEMMs
     size_t esz;   // bytes per activation element
     int device;
-    cudaStream_t st;
+    cudaStream_t st, own_st = nullptr; // own_st: made by nncu_own_stream
     cudaStream_t st2;            // weight-gradient GEMMs run here, beside the dX chain
     cudaEvent_t ev_fork, ev_join;
     bool overlap;
@@ -154,6 +155,8 @@ struct nncu_model {
     dec::State *dec_state = nullptr;
     int dec_ring = 0;
     bool dec_open = false;
+    stepf::Layer *step_layers[2] = {nullptr, nullptr}; // one-launch time steps of small fp32 models, per memory twin
+    int step_sp = 0;                                   // streams per cluster (0: the model takes ordinary launches)
     // gradient exchange between ranks (nncu_comm_init): per-layer all-reduces on a third stream,
     // issued as soon as a layer's gradients are complete, so they overlap the rest of backward
     void *comm;
@@ -581,9 +584,60 @@ static int run_graphed(nncu_model *m, int kind, F body)
 
 // ------------------------------------------------------------------ forward
 
+// Streams per cluster of the one-launch time step, 0 where the model is not one it takes: fp32, post-LN,
+// ungated feed-forward, rows that fit the norms' registers, slices of 16 without remainder.  One stream
+// per cluster while the clusters fit the chip together, then two and four (16 streams, one to a cluster:
+// the last cluster waited for the others, 156 us a step instead of 78); beyond that the launches it
+// replaces have rows enough to fill the chip.
+static int step_streams(const nncu_model *m)
+{
+    const nncu_params &p = m->p;
+    const bool kind = !m->bf && (p.ln_flags & NNCU_LN_POST) && !(p.ln_flags & (NNCU_LN_PRE | NNCU_LN_FINAL | NNCU_LN_COEF)) &&
+                      (p.ff_act == NNCU_FF_RELU || p.ff_act == NNCU_FF_GELU);
+    if (!kind || m->D % 16 || m->HD % 16 || m->F % 16 || m->dk % 4 || m->D > stepf::MAXD || m->B > 4 * stepf::MAX_CLUSTERS)
+        return 0;
+    const int sp = m->B <= stepf::MAX_CLUSTERS ? 1 : (m->B <= 2 * stepf::MAX_CLUSTERS ? 2 : 4);
+    return stepf::ring_slots(sp, m->nl, m->D, m->H, m->dk, m->F, m->L, p.d_pos, m->V, 1 << coder_depth(m->V)) ? sp : 0;
+}
+
+// one time step; trees: where the coder's trees of its rows go, NULL if nobody wants them; chained: the
+// kernel before it on the stream is this model's decoder step
+static int step_forward(nncu_model *m, int t, uint16_t *trees, bool chained)
+{
+    const int D = m->D, HD = m->HD, B = m->B, M = m->M;
+    if (t == 0 && M > 0) // the memory rows' keys and values, once per segment
+        for (int l = 0; l < m->nl; l++)
+            NNCU_TRY((mm_nt<float, float>(m, M * B, 2 * HD, D, (const float *)hcat_layer(m, m->cur, l), D, m->lo[l].w_kv,
+                                          at<float>(m->act[l].qkv, HD), 3 * HD, nullptr)));
+    stepf::Args a;
+    a.layers = m->step_layers[m->cur];
+    a.embed = m->W + m->embed;
+    a.w_out = m->W + m->embed_out;
+    a.out_bias = wf(m, m->out_bias);
+    a.ids = m->ids_dev;
+    a.xlast = (float *)m->xlast;
+    a.probs = m->probs;
+    a.dz = (float *)m->dz;
+    a.dz_fixed = m->dz_fixed;
+    a.err_flag = m->err_flag;
+    a.trees = trees;
+    a.nl = m->nl; a.D = D; a.H = m->H; a.dk = m->dk; a.F = m->F; a.T = m->T; a.M = M; a.B = B; a.V = m->V; a.P = m->p.d_pos;
+    a.norm_mode = (m->p.ln_flags & NNCU_LN_RMSNORM) ? 2 : 1;
+    a.act = m->p.ff_act;
+    a.depth = coder_depth(m->V);
+    a.emul = sqrtf((float)D) * m->p.embed_mult;
+    a.br_scale = sqrtf((float)m->dk * (float)D);
+    a.inv_sqrt = 1.0f / sqrtf((float)m->dk);
+    a.scale = 1.0f / ((float)m->T * (float)m->Bt);
+    a.slots = stepf::ring_slots(m->step_sp, m->nl, D, m->H, m->dk, m->F, m->L, a.P, m->V, 1 << a.depth);
+    return stepf::launch(m->st, a, t, m->step_sp, chained);
+}
+
 template <typename AT>
 static int forward_range(nncu_model *m, int t0, int t1)
 {
+    if (t1 - t0 == 1 && m->step_sp)
+        return step_forward(m, t0, nullptr, false);
     const nncu_params &p = m->p;
     const int D = m->D, HD = m->HD, F = m->F, F1 = m->F1, B = m->B, M = m->M, V = m->V;
     const int r0 = t0 * B, nr = (t1 - t0) * B;
@@ -1226,6 +1280,7 @@ int nncu_destroy(nncu_model *m)
     if (m->ev_coder) cudaEventDestroy(m->ev_coder);
     if (m->ev_loss) cudaEventDestroy(m->ev_loss);
     if (m->loss_pin) cudaFreeHost(m->loss_pin);
+    if (m->own_st) cudaStreamDestroy(m->own_st);
     delete m;
     return NNCU_OK;
 }
@@ -1404,6 +1459,8 @@ int nncu_create(const nncu_params *p, nncu_model **out)
                 jobs.push_back(j);
             }
     size_t oJobs = take(sizeof(TransposeJob) * (jobs.size() + 1));
+    m->step_sp = step_streams(m);
+    size_t oStep = take(m->step_sp ? sizeof(stepf::Layer) * 2 * m->nl : 0);
     m->coder_bytes = (size_t)TB * ((size_t)1 << coder_depth(V)) * 2; // a tree per row: 2^ceil(log2 V) entries
     size_t oCoder = take(m->coder_bytes);
 
@@ -1479,6 +1536,28 @@ int nncu_create(const nncu_params *p, nncu_model **out)
     if (!jobs.empty() &&
         cudaMemcpy(m->jobs_dev, jobs.data(), sizeof(TransposeJob) * jobs.size(), cudaMemcpyHostToDevice) != cudaSuccess)
         return fail_cleanup(nncu_fail(NNCU_ERR_CUDA, "job table upload failed"));
+    if (m->step_sp) {
+        std::vector<stepf::Layer> rows((size_t)2 * m->nl);
+        for (int c = 0; c < 2; c++)
+            for (int l = 0; l < m->nl; l++) {
+                const LayerOff &o = m->lo[l];
+                const LayerAct &a = m->act[l];
+                stepf::Layer &y = rows[(size_t)c * m->nl + l];
+                y.w_qkv = m->W + o.w_q; y.w_o = m->W + o.w_o; y.ff1 = m->W + o.ff1; y.ff2 = m->W + o.ff2;
+                y.b_q = wf(m, o.b_q); y.fb1 = wf(m, o.ff_bias1); y.fb2 = wf(m, o.ff_bias2);
+                y.w_r = wf(m, o.w_r); y.b_r = m->W + o.b_r;
+                y.g1 = m->W + o.ln_g1; y.b1 = m->W + o.ln_b1; y.g2 = m->W + o.ln_g2; y.b2 = m->W + o.ln_b2;
+                y.x = (float *)hcat_layer(m, c, l) + (size_t)m->M * m->B * D;
+                y.qkv = (float *)a.qkv; y.o = (float *)a.o; y.s1 = (float *)a.s1; y.y = (float *)a.y;
+                y.hpre = (float *)a.hpre; y.hact = (float *)a.hact; y.s2 = (float *)a.s2;
+                y.lse = a.lse; y.st1 = a.st_1; y.st2 = a.st_2;
+                y.attn_len = p->attn_len[l] ? p->attn_len[l] : m->L;
+            }
+        m->step_layers[0] = (stepf::Layer *)(A + oStep);
+        m->step_layers[1] = m->step_layers[0] + m->nl;
+        if (cudaMemcpy(m->step_layers[0], rows.data(), sizeof(stepf::Layer) * rows.size(), cudaMemcpyHostToDevice) != cudaSuccess)
+            return fail_cleanup(nncu_fail(NNCU_ERR_CUDA, "layer table upload failed"));
+    }
     if ((size_t)8 * 3 * D * 4 > 48 * 1024) {
         cudaFuncSetAttribute(norm_bwd_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * 3 * D * 4);
         cudaFuncSetAttribute(norm_bwd_kernel<bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * 3 * D * 4);
@@ -1530,6 +1609,16 @@ int nncu_set_stream(nncu_model *m, void *cuda_stream)
     CUDA_TRY(cudaStreamSynchronize(m->st));
     m->st = (cudaStream_t)cuda_stream;
     return NNCU_OK;
+}
+
+int nncu_own_stream(nncu_model *m)
+{
+    if (!m)
+        return nncu_fail(NNCU_ERR_INVALID, "null model");
+    CUDA_TRY(cudaSetDevice(m->device));
+    if (!m->own_st)
+        CUDA_TRY(cudaStreamCreateWithFlags(&m->own_st, cudaStreamNonBlocking));
+    return nncu_set_stream(m, m->own_st);
 }
 
 int nncu_reset(nncu_model *m)
@@ -1949,10 +2038,12 @@ static int param_io(nncu_model *m, int index, float *host, size_t numel, float *
     if (m->master_stale && base != m->G)
         return nncu_fail(NNCU_ERR_STATE, "the master weights are sharded over the ranks: nncu_comm_gather_master first");
     CUDA_TRY(cudaStreamSynchronize(m->st));
+    // on the model's stream: it does not wait for the legacy one
     if (to_host)
-        CUDA_TRY(cudaMemcpy(host, base + pi.off, numel * 4, cudaMemcpyDeviceToHost));
+        CUDA_TRY(cudaMemcpyAsync(host, base + pi.off, numel * 4, cudaMemcpyDeviceToHost, m->st));
     else
-        CUDA_TRY(cudaMemcpy(base + pi.off, host, numel * 4, cudaMemcpyHostToDevice));
+        CUDA_TRY(cudaMemcpyAsync(base + pi.off, host, numel * 4, cudaMemcpyHostToDevice, m->st));
+    CUDA_TRY(cudaStreamSynchronize(m->st));
     return NNCU_OK;
 }
 
@@ -2093,9 +2184,9 @@ int nncu_coder_trees(nncu_model *m, int t0, int nt, uint16_t *tree_host)
     CUDA_TRY(cudaSetDevice(m->device));
     int rows = nt * m->B;
     if (pow2)
-        coder_trees_kernel<<<rows, 256, (size_t)2 * m->V * 4, m->st>>>(m->probs + (size_t)t0 * m->B * m->V, m->coder_dev, m->V);
+        coder_trees_kernel<<<rows, tree_threads(P), (size_t)2 * m->V * 4, m->st>>>(m->probs + (size_t)t0 * m->B * m->V, m->coder_dev, m->V);
     else
-        coder_trees_any_kernel<<<rows, 256, (size_t)2 * P * 4, m->st>>>(m->probs + (size_t)t0 * m->B * m->V, m->coder_dev,
+        coder_trees_any_kernel<<<rows, tree_threads(P), (size_t)2 * P * 4, m->st>>>(m->probs + (size_t)t0 * m->B * m->V, m->coder_dev,
                                                                        m->V, P);
     KERNEL_CHECK();
     CUDA_TRY(cudaMemcpyAsync(tree_host, m->coder_dev, sizeof(uint16_t) * (size_t)rows * P, cudaMemcpyDeviceToHost, m->st));
@@ -2183,20 +2274,24 @@ int nncu_decoder_begin(nncu_model *m, const uint8_t *payload_host, size_t len)
 
 // one decode step: the model's one-symbol forward, the prob0 trees of its B rows, and the walk that
 // turns them into symbols (left in the target rows and, for t+1 < seg_len, the next step's input)
-static int decode_step(nncu_model *m, int t, int limit_t, int limit_b)
+static int decode_step(nncu_model *m, int t, int limit_t, int limit_b, bool chained)
 {
     const int B = m->B, V = m->V, nb = coder_depth(V), P = 1 << nb;
     const bool pow2 = P == V;
-    NNCU_TRY(m->bf ? forward_range<bf16>(m, t, t + 1) : forward_range<float>(m, t, t + 1));
-    if (pow2)
-        launch_k(coder_trees_kernel, dim3(B), dim3(256), (size_t)2 * V * 4, m->st,
-                 (const float *)(m->probs + (size_t)t * B * V), m->coder_dev, V);
-    else
-        launch_k(coder_trees_any_kernel, dim3(B), dim3(256), (size_t)2 * P * 4, m->st,
-                 (const float *)(m->probs + (size_t)t * B * V), m->coder_dev, V, P);
-    KERNEL_CHECK();
-    launch_k(pow2 ? dec::decode_step_kernel<false> : dec::decode_step_kernel<true>, dim3(1), dim3(32),
-             dec::smem_bytes(B, P, nb, m->dec_ring), m->st, (const uint16_t *)m->coder_dev,
+    if (m->step_sp) {
+        NNCU_TRY(step_forward(m, t, m->coder_dev, chained));
+    } else {
+        NNCU_TRY(m->bf ? forward_range<bf16>(m, t, t + 1) : forward_range<float>(m, t, t + 1));
+        if (pow2)
+            launch_k(coder_trees_kernel, dim3(B), dim3(tree_threads(P)), (size_t)2 * V * 4, m->st,
+                     (const float *)(m->probs + (size_t)t * B * V), m->coder_dev, V);
+        else
+            launch_k(coder_trees_any_kernel, dim3(B), dim3(tree_threads(P)), (size_t)2 * P * 4, m->st,
+                     (const float *)(m->probs + (size_t)t * B * V), m->coder_dev, V, P);
+        KERNEL_CHECK();
+    }
+    launch_pdl(m->step_sp || nncu_pdl_enabled(), pow2 ? dec::decode_step_kernel<false> : dec::decode_step_kernel<true>, dim3(1), dim3(64),
+               dec::smem_bytes(B, P, nb, m->dec_ring), m->st, (const uint16_t *)m->coder_dev,
              (const uint8_t *)m->dec_payload, m->dec_state, m->tgt_dev + (size_t)t * B,
              t + 1 < m->T ? m->ids_dev + (size_t)(t + 1) * B : (int32_t *)nullptr, t, limit_t, limit_b, B, V, P, nb,
              m->dec_ring, m->err_flag);
@@ -2225,9 +2320,10 @@ int nncu_decode_steps(nncu_model *m, int t0, int nt, const int32_t *ids_t0_host,
         CUDA_TRY(cudaEventRecord(m->ev_ids, m->st));
     }
     bind_xin(m);
-    const bool full = limit_t >= m->T; // every stream active at every step: the shape the graphs hold
+    // every stream active at every step: the shape the graphs hold (a one-launch step is two launches: no graph)
+    const bool full = limit_t >= m->T && !m->step_sp;
     for (int t = t0; t < t0 + nt; t++) {
-        auto body = [&]() { return decode_step(m, t, limit_t, limit_b); };
+        auto body = [&]() { return decode_step(m, t, limit_t, limit_b, t > t0); };
         NNCU_TRY(full ? run_graphed(m, m->step_graphs[(size_t)2 * t + m->cur], body) : body());
         m->steps_done = t + 1;
     }

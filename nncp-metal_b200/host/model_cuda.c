@@ -86,8 +86,16 @@ int nch_bind_cuda(const char *libnncu_path, const nncu_params *p, nch_model_ops 
     x->decoder_begin = dlsym(x->dl, "nncu_decoder_begin");
     x->decode_steps = dlsym(x->dl, "nncu_decode_steps");
     x->decoder_end = dlsym(x->dl, "nncu_decoder_end");
+    int (*own_stream)(nncu_model *) = dlsym(x->dl, "nncu_own_stream");
     if (!create || !x->destroy || !x->reset || !x->set_lr || !x->eval || !x->read_probs || !x->coder_paths ||
         !x->coder_trees || !x->eval_end || !x->eval_gradient || !x->update || create(p, &x->model) != NNCU_OK) {
+        dlclose(x->dl);
+        free(x);
+        return NCH_ERR_MODEL;
+    }
+    /* nobody else queues work behind this model: off the legacy stream its passes are replayed as graphs */
+    if (own_stream && own_stream(x->model) != NNCU_OK) {
+        x->destroy(x->model);
         dlclose(x->dl);
         free(x);
         return NCH_ERR_MODEL;

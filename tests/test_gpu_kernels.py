@@ -95,3 +95,30 @@ def test_gradients_of_a_long_memory_match_the_other_engine(pkg, ln, act, D, n_he
     assert abs(got[0][1] - got[1][1]) < 1e-3 * abs(got[0][1])
     for n in got[0][0]:
         assert rel_err(got[1][0][n], got[0][0][n]) < 2e-2, n
+
+
+@pytest.mark.parametrize("kw", [
+    dict(n_layer=3, d_model=96, n_head=3, d_key=32, d_inner=208, d_pos=20, mem_len=17, seg_len=9, n_streams=1, n_symbols=256),
+    dict(n_layer=2, d_model=256, n_head=8, d_key=32, d_inner=1024, d_pos=32, mem_len=32, seg_len=8, n_streams=16, n_symbols=256),
+    dict(n_layer=2, d_model=512, n_head=4, d_key=64, d_inner=272, d_pos=9, mem_len=5, seg_len=7, n_streams=19, n_symbols=300, ff_act=0),
+    dict(n_layer=2, d_model=64, n_head=1, d_key=16, d_inner=64, d_pos=4, mem_len=0, seg_len=6, n_streams=50, n_symbols=37, use_w_r=0,
+         use_bias=0, query_bias=0),
+    dict(n_layer=1, d_model=48, n_head=12, d_key=4, d_inner=16, d_pos=20, mem_len=40, seg_len=5, n_streams=56, n_symbols=64, attn_len=[11])])
+def test_one_launch_steps_equal_whole_segment_bitwise(pkg, kw):
+    """The one-launch time step of small fp32 models, one to four streams per cluster: probabilities, and
+    through the gradients everything it leaves for the backward pass, bit for bit those of the segment."""
+    p = pkg.abi.make_params(use_bf16=0, init_range=0.3, lr=1e-3, **kw)
+    T, B, V = p.seg_len, p.n_streams, p.n_symbols
+    rng = np.random.default_rng(3)
+    seg, one = pkg.TrfModel(p), pkg.TrfModel(p)
+    seg.reset(); one.reset()
+    for _ in range(3):   # both memory twins
+        ids, tg = rng.integers(0, V, (T, B)).astype(np.int32), rng.integers(0, V, (T, B)).astype(np.int32)
+        a = seg.eval(-1, ids)
+        b = np.concatenate([one.eval(t, ids) for t in range(T)])
+        assert np.array_equal(a, b)
+        for m in (seg, one):
+            m.eval_gradient(tg)
+            m.update()
+        assert seg.weights_hash() == one.weights_hash()
+    seg.close(); one.close()
