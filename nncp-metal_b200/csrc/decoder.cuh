@@ -36,19 +36,21 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_
                  : "memory");
 }
 
-// window bytes a step of `B` streams with `nb` bits per symbol can consume, as a multiple of 16
-__host__ __device__ inline int window_bytes(int B, int nb) { return (2 * B * nb + 15) & ~15; }
+// window bytes a step of `B` streams with `nb` bits per symbol can consume, one to look ahead, as a multiple of 16
+__host__ __device__ inline int window_bytes(int B, int nb) { return (2 * B * nb + 1 + 15) & ~15; }
+// trees of P entries that share a ring slot: small ones come 16 KB at a time
+__host__ __device__ inline int slot_trees(int B, int P) { return P >= 8192 ? 1 : (8192 / P < B ? 8192 / P : B); }
 
 // slots of the ring for trees of P entries (0: the trees do not fit)
 inline int ring_slots(int B, int P, int nb)
 {
     const long avail = (long)MAX_SMEM - window_bytes(B, nb) - 128;
-    long n = avail / ((long)P * 2);
+    long n = avail / ((long)slot_trees(B, P) * P * 2);
     if (P < 8 || n < 2)
         return 0;
     return (int)std::min<long>(n, MAX_RING);
 }
-inline size_t smem_bytes(int B, int P, int nb, int ring) { return (size_t)ring * P * 2 + window_bytes(B, nb) + 128; }
+inline size_t smem_bytes(int B, int P, int nb, int ring) { return (size_t)ring * slot_trees(B, P) * P * 2 + window_bytes(B, nb) + 128; }
 
 // trees: [B][P] prob0 in heap order (entry 0 unused), P = 2^nb >= V.  sym_out[b] and ids_next[b]
 // (when not null) receive the decoded symbol, 0 for the streams past the end of the block: those at
@@ -63,13 +65,15 @@ decode_step_kernel(const uint16_t *__restrict__ trees, const uint8_t *__restrict
     pdl_trigger_late(); // a successor that was launched to overlap this kernel may start on what does not depend on it
     extern __shared__ __align__(128) uint8_t dsm[];
     uint64_t *bars = reinterpret_cast<uint64_t *>(dsm);           // [2][MAX_RING] of 8 bytes: 128
-    uint16_t *slots = reinterpret_cast<uint16_t *>(dsm + 128);    // [ring][P]
-    uint8_t *win = dsm + 128 + (size_t)ring * P * 2;              // payload window
+    const int G = slot_trees(B, P);
+    uint16_t *slots = reinterpret_cast<uint16_t *>(dsm + 128);    // [ring][G][P]
+    uint8_t *win = dsm + 128 + (size_t)ring * G * P * 2;          // payload window
     __shared__ int abort_s;
     __shared__ int issued_s;
     const int tid = threadIdx.x;
     const int n_act = t < limit_t ? B : (t == limit_t ? min(limit_b, B) : 0);
-    const uint32_t slot_bytes = (uint32_t)P * 2u;
+    const uint32_t tree_bytes = (uint32_t)P * 2u;
+    const int n_grp = (n_act + G - 1) / G;
     const unsigned long long pos0 = state->pos, len = state->len;
     uint64_t *done = bars + MAX_RING; // the walker has left a slot
 
@@ -87,32 +91,44 @@ decode_step_kernel(const uint16_t *__restrict__ trees, const uint8_t *__restrict
     __syncthreads();
 
     if (tid == 32) { // the copies, on a warp of their own: the walk does not stop to issue them
-        int b = 0;
-        for (; b < n_act; b++) {
-            const int s = b % ring;
-            if (b >= ring && !tc::mbar_wait(tc::smem_u32(done + s), (uint32_t)((b / ring - 1) & 1), &abort_s, err_flag, 43))
+        int g = 0;
+        for (; g < n_grp; g++) {
+            const int s = g % ring;
+            if (g >= ring && !tc::mbar_wait(tc::smem_u32(done + s), (uint32_t)((g / ring - 1) & 1), &abort_s, err_flag, 43))
                 break;
-            tc::mbar_expect_tx(tc::smem_u32(bars + s), slot_bytes);
-            bulk_load(tc::smem_u32(slots + (size_t)s * P), trees + (size_t)b * P, slot_bytes, tc::smem_u32(bars + s));
+            const uint32_t bytes = (uint32_t)min(G, n_act - g * G) * tree_bytes;
+            tc::mbar_expect_tx(tc::smem_u32(bars + s), bytes);
+            bulk_load(tc::smem_u32(slots + (size_t)s * G * P), trees + (size_t)g * G * P, bytes, tc::smem_u32(bars + s));
         }
-        issued_s = b;
+        issued_s = g;
     }
-    int walked = 0;
+    int walked = 0; // groups whose copy has been waited for
     bool ok = true;
     if (tid == 0) {
-        uint32_t low = state->low, range = state->range, used = 0;
-        const uint32_t left = (uint32_t)min(len - pos0, (unsigned long long)wbytes); // payload bytes in the window
+        uint32_t low = state->low, range = state->range, used = 0, next = win[0];
         const uint32_t half = (uint32_t)P / 2u;
+        int slot = ring - 1, in_slot = G; // the slot in use and the trees of it that have been walked
+        uint32_t phase = 1;
         for (int b = 0; b < B; b++) {
             int c = 0;
             if (b < n_act && ok) {
-                const int s = b % ring;
-                ok = tc::mbar_wait(tc::smem_u32(bars + s), (uint32_t)((b / ring) & 1), &abort_s, err_flag, 41);
+                if (in_slot == G) {
+                    if (b > 0)
+                        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc::smem_u32(done + slot)) : "memory");
+                    in_slot = 0;
+                    if (++slot == ring) {
+                        slot = 0;
+                        phase ^= 1;
+                    }
+                    ok = tc::mbar_wait(tc::smem_u32(bars + slot), phase, &abort_s, err_flag, 41);
+                    walked += ok ? 1 : 0;
+                }
                 if (ok) {
                     // Node k's prob0 is in hand, and its children's (one 32-bit word) are on their way, before the
                     // branch at k is known: what a bit costs is the chain product - compare - select.
                     // (range * prob0) >> 15 is the high word of (range << 8) * (prob0 << 9): range stays below 2^24.
-                    const uint32_t *pairs = reinterpret_cast<const uint32_t *>(slots + (size_t)s * P);
+                    const uint32_t *pairs = reinterpret_cast<const uint32_t *>(slots + ((size_t)slot * G + in_slot) * P);
+                    in_slot++;
                     uint32_t k = 1, p0 = pairs[0] >> 16, kids = pairs[1];
                     auto next_bit = [&]() { // get_bit at node k: the branch taken, low / range / used advanced
                         const uint32_t split = __umulhi(range << 8, p0 << 9);
@@ -122,11 +138,12 @@ decode_step_kernel(const uint16_t *__restrict__ trees, const uint8_t *__restrict
                         kids = pairs[min(k, half - 1)];
                         low = bit ? low - split : low;
                         range = bit ? range - split : split;
-                        while (range < R_LOW) {
-                            range <<= 8;
-                            low <<= 8;
-                            if (used < left)
-                                low += win[used++];
+                        if (range < R_LOW) {
+                            do { // the window is zero past the payload's end; one byte is always in hand
+                                range <<= 8;
+                                low = (low << 8) + next;
+                                next = win[++used];
+                            } while (range < R_LOW);
                         }
                         return bit;
                     };
@@ -147,15 +164,13 @@ decode_step_kernel(const uint16_t *__restrict__ trees, const uint8_t *__restrict
                             next_bit();
                         c = (int)k - V;
                     }
-                    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc::smem_u32(done + s)) : "memory");
-                    walked = b + 1;
                 }
             }
             sym_out[b] = c;
             if (ids_next)
                 ids_next[b] = c;
         }
-        state->pos = pos0 + used;
+        state->pos = min(pos0 + used, len);
         state->low = low;
         state->range = range;
         if (!ok)
@@ -163,8 +178,8 @@ decode_step_kernel(const uint16_t *__restrict__ trees, const uint8_t *__restrict
     }
     __syncthreads();
     if (tid == 0 && !ok) // copies still in flight land in this CTA's shared memory: each gets a bounded chance to finish
-        for (int b = walked; b < issued_s; b++)
-            tc::mbar_wait(tc::smem_u32(bars + b % ring), (uint32_t)((b / ring) & 1), &abort_s, err_flag, 42);
+        for (int g = walked; g < issued_s; g++)
+            tc::mbar_wait(tc::smem_u32(bars + g % ring), (uint32_t)((g / ring) & 1), &abort_s, err_flag, 42);
 }
 
 } // namespace dec

@@ -189,17 +189,12 @@ __device__ __forceinline__ void vec_load_f32(const float *p, int lane, int D, fl
     }
 }
 
-// v <- norm(v) * g + b for a row over a warp's registers (mode 1 LayerNorm, 2 RMSNorm, 0 nothing); lane 0
-// leaves the statistics in stats[0], stats[1] when wanted
+// v <- norm(v) * g + b for a row over a warp's registers (mode 1 LayerNorm, 2 RMSNorm); lane 0 leaves the
+// statistics in stats[0], stats[1] when wanted
 template <int NC, int W>
-__device__ __forceinline__ void norm_row(float (&v)[NC][W], const float *__restrict__ g, const float *__restrict__ b, int lane, int D,
-                                         int mode, float *stats)
+__device__ __forceinline__ void norm_row(float (&v)[NC][W], const float (&gv)[NC][W], const float (&bv)[NC][W], int lane, int D, int mode,
+                                         float *stats)
 {
-    if (mode == 0)
-        return;
-    float gv[NC][W], bv[NC][W];
-    vec_load_f32<NC, W>(g, lane, D, gv);
-    vec_load_f32<NC, W>(b, lane, D, bv);
     float mu = 0.0f;
     if (mode == 1) {
         float sum = 0.0f;
@@ -262,7 +257,10 @@ residual_norm_vec_kernel(const T *__restrict__ a, const T *__restrict__ res, T *
         row_store<T, NC, W>(y + (size_t)r * D, lane, D, v);
         return;
     }
-    norm_row<NC, W>(v, g, b, lane, D, mode, stats ? stats + 2 * r : nullptr);
+    float gv[NC][W], bv[NC][W];
+    vec_load_f32<NC, W>(g, lane, D, gv);
+    vec_load_f32<NC, W>(b, lane, D, bv);
+    norm_row<NC, W>(v, gv, bv, lane, D, mode, stats ? stats + 2 * r : nullptr);
     row_store<T, NC, W>(y + (size_t)r * D, lane, D, v);
 }
 

@@ -155,6 +155,7 @@ struct nncu_model {
     dec::State *dec_state = nullptr;
     int dec_ring = 0;
     bool dec_open = false;
+    CUtensorMap *step_maps = nullptr;
     stepf::Layer *step_layers[2] = {nullptr, nullptr}; // one-launch time steps of small fp32 models, per memory twin
     int step_sp = 0;                                   // streams per cluster (0: the model takes ordinary launches)
     // gradient exchange between ranks (nncu_comm_init): per-layer all-reduces on a third stream,
@@ -594,7 +595,7 @@ static int step_streams(const nncu_model *m)
     const nncu_params &p = m->p;
     const bool kind = !m->bf && (p.ln_flags & NNCU_LN_POST) && !(p.ln_flags & (NNCU_LN_PRE | NNCU_LN_FINAL | NNCU_LN_COEF)) &&
                       (p.ff_act == NNCU_FF_RELU || p.ff_act == NNCU_FF_GELU);
-    if (!kind || m->D % 16 || m->HD % 16 || m->F % 16 || m->dk % 4 || m->D > stepf::MAXD || m->B > 4 * stepf::MAX_CLUSTERS)
+    if (!kind || m->D % 16 || m->HD % 16 || m->F % 16 || m->dk % 4 || m->dk > 128 || m->D > stepf::MAXD || m->B > 4 * stepf::MAX_CLUSTERS)
         return 0;
     const int sp = m->B <= stepf::MAX_CLUSTERS ? 1 : (m->B <= 2 * stepf::MAX_CLUSTERS ? 2 : 4);
     return stepf::ring_slots(sp, m->nl, m->D, m->H, m->dk, m->F, m->L, p.d_pos, m->V, 1 << coder_depth(m->V)) ? sp : 0;
@@ -612,7 +613,7 @@ static int step_forward(nncu_model *m, int t, uint16_t *trees, bool chained)
     stepf::Args a;
     a.layers = m->step_layers[m->cur];
     a.embed = m->W + m->embed;
-    a.w_out = m->W + m->embed_out;
+    a.maps = m->step_maps;
     a.out_bias = wf(m, m->out_bias);
     a.ids = m->ids_dev;
     a.xlast = (float *)m->xlast;
@@ -1460,7 +1461,7 @@ int nncu_create(const nncu_params *p, nncu_model **out)
             }
     size_t oJobs = take(sizeof(TransposeJob) * (jobs.size() + 1));
     m->step_sp = step_streams(m);
-    size_t oStep = take(m->step_sp ? sizeof(stepf::Layer) * 2 * m->nl : 0);
+    size_t oStep = take(m->step_sp ? sizeof(stepf::Layer) * 2 * m->nl : 0), oMaps = take(m->step_sp ? sizeof(CUtensorMap) * (4 * m->nl + 1) : 0);
     m->coder_bytes = (size_t)TB * ((size_t)1 << coder_depth(V)) * 2; // a tree per row: 2^ceil(log2 V) entries
     size_t oCoder = take(m->coder_bytes);
 
@@ -1543,7 +1544,6 @@ int nncu_create(const nncu_params *p, nncu_model **out)
                 const LayerOff &o = m->lo[l];
                 const LayerAct &a = m->act[l];
                 stepf::Layer &y = rows[(size_t)c * m->nl + l];
-                y.w_qkv = m->W + o.w_q; y.w_o = m->W + o.w_o; y.ff1 = m->W + o.ff1; y.ff2 = m->W + o.ff2;
                 y.b_q = wf(m, o.b_q); y.fb1 = wf(m, o.ff_bias1); y.fb2 = wf(m, o.ff_bias2);
                 y.w_r = wf(m, o.w_r); y.b_r = m->W + o.b_r;
                 y.g1 = m->W + o.ln_g1; y.b1 = m->W + o.ln_b1; y.g2 = m->W + o.ln_g2; y.b2 = m->W + o.ln_b2;
@@ -1553,6 +1553,21 @@ int nncu_create(const nncu_params *p, nncu_model **out)
                 y.lse = a.lse; y.st1 = a.st_1; y.st2 = a.st_2;
                 y.attn_len = p->attn_len[l] ? p->attn_len[l] : m->L;
             }
+        std::vector<CUtensorMap> maps((size_t)4 * m->nl + 1);
+        for (int l = 0; l < m->nl; l++) {
+            const LayerOff &o = m->lo[l];
+            int rc = stepf::piece_map(m->W + o.w_q, 3 * HD, D, &maps[4 * l]);
+            rc = rc ? rc : stepf::piece_map(m->W + o.w_o, D, HD, &maps[4 * l + 1]);
+            rc = rc ? rc : stepf::piece_map(m->W + o.ff1, F, D, &maps[4 * l + 2]);
+            rc = rc ? rc : stepf::piece_map(m->W + o.ff2, D, F, &maps[4 * l + 3]);
+            if (rc)
+                return fail_cleanup(rc);
+        }
+        if (int rc = stepf::piece_map(m->W + m->embed_out, V, D, &maps[4 * m->nl]))
+            return fail_cleanup(rc);
+        m->step_maps = (CUtensorMap *)(A + oMaps);
+        if (cudaMemcpy(m->step_maps, maps.data(), sizeof(CUtensorMap) * maps.size(), cudaMemcpyHostToDevice) != cudaSuccess)
+            return fail_cleanup(nncu_fail(NNCU_ERR_CUDA, "tensor map upload failed"));
         m->step_layers[0] = (stepf::Layer *)(A + oStep);
         m->step_layers[1] = m->step_layers[0] + m->nl;
         if (cudaMemcpy(m->step_layers[0], rows.data(), sizeof(stepf::Layer) * rows.size(), cudaMemcpyHostToDevice) != cudaSuccess)
