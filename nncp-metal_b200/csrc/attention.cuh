@@ -23,6 +23,7 @@ struct AttnArgs {
     const void *w_r16; // optional bf16 copy of w_r (same layout), used by the tensor-core kernels
     void *o, *dq, *dkv;
     float *lse, *dwr_part, *dbr_part;
+    int *err_flag; // raised when a bounded wait runs out, may be NULL
     int B, H, dk, T, M, L, P, attn_len, t0, t1, qchunk;
     int smem_pitch; // row pitch of the staged K and table rows (CUDA-core kernels)
     int qp, kvp, dqp, dkvp; // row pitches (elements) of q, kv, dq, dkv; K then V inside a kv row

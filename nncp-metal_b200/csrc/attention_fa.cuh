@@ -23,6 +23,7 @@
 // segments and single queries, which go through different kernels, give the same bits.
 #pragma once
 #include "attention.cuh"
+#include "gemm_tc.cuh"
 
 namespace fa {
 
@@ -597,6 +598,211 @@ __global__ void __launch_bounds__(128) attn_one_kernel(const __grid_constant__ A
         a.lse[((size_t)b * a.H + h) * T + i] = m_run + logf(l);
 }
 
+// The same for head sizes 64 and 128 with tiles that arrive by TMA: 64 rows x 64 columns a copy, 128-byte
+// rows, chunk c of row r at c ^ (r % 8).  The loop above spends most of its instructions on addresses (some 600
+// a block of a warp against 200 of products, on eight warps an SM), and at 128 streams x 8 heads x 576 keys
+// it took 57 us of which HBM needs 23.
+template <int DK> struct OneTmaSmem {
+    static constexpr int NS = DK / 64, TILE = NS * 8192;
+    static constexpr int K = 0, R = 4 * TILE, V = 8 * TILE, S = 12 * TILE, MB = S + 4 * 64 * 4, L4 = MB + 16, BRS = L4 + 16;
+    static size_t bytes(int L) { return (size_t)BRS + (size_t)L * 4 + 1024; }
+};
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap *map, uint32_t bar, int x, int y, int z)
+{
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(dst),
+                 "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(x), "r"(y), "r"(z)
+                 : "memory");
+}
+__device__ __forceinline__ void ldsm4_at(uint32_t (&r)[4], uint32_t at)
+{
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(at));
+}
+__device__ __forceinline__ void ldsm4t_at(uint32_t (&r)[4], uint32_t at)
+{
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(at));
+}
+// byte offset of 16-byte chunk c of row r in a tile
+__device__ __forceinline__ uint32_t tile_at(int r, int c) { return (uint32_t)((c >> 3) * 8192 + r * 128 + (((c & 7) ^ (r & 7)) << 4)); }
+
+template <int DK>
+__global__ void __launch_bounds__(128) attn_one_tma_kernel(const __grid_constant__ AttnArgs a, const __grid_constant__ CUtensorMap map_kv,
+                                                           const __grid_constant__ CUtensorMap map_r, int stage_br)
+{
+    using SM = OneTmaSmem<DK>;
+    constexpr int NS = SM::NS, TILE = SM::TILE, MT = DK / 16, MW = MT / 4; // 16-column slices, and those of one warp
+    extern __shared__ __align__(1024) unsigned char smraw[];
+    __shared__ __align__(8) uint64_t bars[8]; // K and table, V of each warp
+    __shared__ int abort_s, dummy;
+    unsigned char *sm = smraw + ((1024u - (smem_addr(smraw) & 1023u)) & 1023u);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const uint32_t base = smem_addr(sm), Kt = base + SM::K + warp * TILE, Rt = base + SM::R + warp * TILE, Vt = base + SM::V;
+    const uint32_t bar_k = smem_addr(bars + warp), bar_v = smem_addr(bars + 4 + warp);
+    float *sc = reinterpret_cast<float *>(sm + SM::S), *mbs = reinterpret_cast<float *>(sm + SM::MB); // [4][64] scores, [4] maxima
+    float *brs = reinterpret_cast<float *>(sm + SM::BRS);
+    const int b = blockIdx.x / a.H, h = blockIdx.x % a.H, HD = a.H * DK, T = a.T, M = a.M, L = a.L, i = a.t0;
+    const Blocks blk = blocks_of(M, L, a.attn_len, i, i + 1);
+    pdl_trigger();
+    if (threadIdx.x == 0) {
+        abort_s = 0;
+        for (int k = 0; k < 8; k++)
+            tc::mbar_init(smem_addr(bars + k), 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    pdl_wait();
+    int *ef = a.err_flag ? a.err_flag : &dummy;
+    auto fetch_kr = [&](int kb) { // this warp's block of a round
+        if (kb > blk.hi)
+            return;
+        const int j0 = kb * KB, x0 = j0 - i + a.P - M - 1;
+        // rows below the table stand for row 0, and a table in fp32 has to be rounded: such tiles are loaded by hand
+        const bool by_hand = a.w_r && (!a.w_r16 || x0 < 0);
+        if (lane == 0) {
+            const bool r = a.w_r && !by_hand;
+            tc::mbar_expect_tx(bar_k, (uint32_t)(r ? 2 * TILE : TILE));
+#pragma unroll
+            for (int n = 0; n < NS; n++) {
+                tma_load_3d(Kt + n * 8192, &map_kv, bar_k, h * DK + n * 64, b, j0);
+                if (r)
+                    tma_load_3d(Rt + n * 8192, &map_r, bar_k, n * 64, x0, h);
+            }
+        }
+        if (by_hand) {
+            const bf16 *w16 = reinterpret_cast<const bf16 *>(a.w_r16) + (size_t)h * a.P * DK;
+            const float *w32 = a.w_r + (size_t)h * a.P * DK;
+            for (int idx = lane; idx < 64 * (DK / 8); idx += 32) {
+                const int r = idx / (DK / 8), c = idx % (DK / 8), x = min(max(x0 + r, 0), a.P - 1);
+                uint4 v;
+                if (a.w_r16) {
+                    v = *reinterpret_cast<const uint4 *>(w16 + (size_t)x * DK + c * 8);
+                } else {
+                    const float4 u = *reinterpret_cast<const float4 *>(w32 + (size_t)x * DK + c * 8);
+                    const float4 w = *reinterpret_cast<const float4 *>(w32 + (size_t)x * DK + c * 8 + 4);
+                    v = make_uint4(pack2(u.x, u.y), pack2(u.z, u.w), pack2(w.x, w.y), pack2(w.z, w.w));
+                }
+                *reinterpret_cast<uint4 *>(sm + SM::R + warp * TILE + tile_at(r, c)) = v;
+            }
+        }
+    };
+    auto fetch_v = [&](int kb) {
+        if (kb > blk.hi || lane != 0)
+            return;
+        tc::mbar_expect_tx(bar_v, (uint32_t)TILE);
+#pragma unroll
+        for (int n = 0; n < NS; n++)
+            tma_load_3d(Vt + warp * TILE + n * 8192, &map_kv, bar_v, HD + h * DK + n * 64, b, kb * KB);
+    };
+    fetch_kr(blk.lo + warp);
+    fetch_v(blk.lo + warp);
+    if (stage_br) // the head's b_r, scaled
+        for (int r = threadIdx.x; r < L; r += 128)
+            brs[r] = __fmul_rn(a.br_scale, a.b_r[(size_t)h * L + r]);
+    // the query as the second operand: k = 2t, 2t + 1 (+ 8) of every 16-wide slice, the same for all columns
+    uint32_t qf[DK / 16][2];
+    {
+        const bf16 *q = reinterpret_cast<const bf16 *>(a.q) + ((size_t)i * a.B + b) * a.qp + h * DK;
+#pragma unroll
+        for (int ks = 0; ks < DK / 16; ks++) {
+            qf[ks][0] = *reinterpret_cast<const uint32_t *>(q + ks * 16 + 2 * t);
+            qf[ks][1] = *reinterpret_cast<const uint32_t *>(q + ks * 16 + 8 + 2 * t);
+        }
+    }
+    __syncthreads();
+    float o[MW][4], m_run = -INFINITY, l = 0.0f; // l: the part of the sum that lane t of a quad keeps
+#pragma unroll
+    for (int w = 0; w < MW; w++)
+#pragma unroll
+        for (int c = 0; c < 4; c++)
+            o[w][c] = 0.0f;
+    uint32_t phase = 0;
+    for (int kb0 = blk.lo; kb0 <= blk.hi; kb0 += 4, phase ^= 1) {
+        const int kb = kb0 + warp, j0 = kb * KB, nb = min(4, blk.hi - kb0 + 1);
+        if (kb <= blk.hi) {
+            tc::mbar_wait(bar_k, phase, &abort_s, ef, 44); // K and the table rows
+            __syncwarp();
+            float mb = -INFINITY;
+#pragma unroll
+            for (int m = 0; m < 4; m++) {
+                float x[4] = {0.0f, 0.0f, 0.0f, 0.0f}, e[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+                const int r = m * 16 + (lane & 15);
+#pragma unroll
+                for (int ks = 0; ks < DK / 16; ks++) {
+                    uint32_t k4[4];
+                    ldsm4_at(k4, Kt + tile_at(r, ks * 2 + (lane >> 4)));
+                    mma(x, k4, qf[ks][0], qf[ks][1]);
+                    if (a.w_r) {
+                        ldsm4_at(k4, Rt + tile_at(r, ks * 2 + (lane >> 4)));
+                        mma(e, k4, qf[ks][0], qf[ks][1]);
+                    }
+                }
+#pragma unroll
+                for (int c = 0; c < 2; c++) {
+                    const int j = j0 + m * 16 + g + c * 8, d = i + M - j, rr = min(max(j + T - 1 - i, 0), L - 1);
+                    const float br = stage_br ? brs[rr] : __fmul_rn(a.br_scale, __ldg(a.b_r + (size_t)h * L + rr));
+                    const float v = (unsigned)d < (unsigned)a.attn_len ? score_of(x[2 * c], e[2 * c], br, a) : -INFINITY;
+                    mb = fmaxf(mb, v);
+                    if (t == 0)
+                        sc[warp * 64 + m * 16 + g + c * 8] = v;
+                }
+            }
+            mb = fmaxf(mb, __shfl_xor_sync(0xffffffffu, mb, 4));
+            mb = fmaxf(mb, __shfl_xor_sync(0xffffffffu, mb, 8));
+            mb = fmaxf(mb, __shfl_xor_sync(0xffffffffu, mb, 16));
+            if (lane == 0)
+                mbs[warp] = mb;
+            __syncwarp();
+            fetch_kr(kb + 4);
+            tc::mbar_wait(bar_v, phase, &abort_s, ef, 45);
+        }
+        __syncthreads(); // scores, maxima and V of the round are there for everyone
+        for (int s = 0; s < nb; s++) {
+            const float n = fmaxf(m_run, mbs[s]), u = n == -INFINITY ? 0.0f : n, scale = __expf(__fsub_rn(m_run, u));
+            m_run = n;
+            float sum = 0.0f;
+            uint32_t pf[4][2];
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+                const float2 v = *reinterpret_cast<const float2 *>(sc + s * 64 + k * 8 + 2 * t);
+                const float p0 = __expf(__fsub_rn(v.x, u)), p1 = __expf(__fsub_rn(v.y, u));
+                sum = __fadd_rn(sum, __fadd_rn(p0, p1));
+                pf[k >> 1][k & 1] = pack2(p0, p1);
+            }
+            l = __fmaf_rn(l, scale, sum);
+#pragma unroll
+            for (int w = 0; w < MW; w++) {
+                const int m = warp + 4 * w;
+#pragma unroll
+                for (int c = 0; c < 4; c++)
+                    o[w][c] = __fmul_rn(o[w][c], scale);
+#pragma unroll
+                for (int ks = 0; ks < 4; ks++) {
+                    uint32_t v4[4]; // V^T: rows are columns of V, so the 8 x 8 blocks come transposed
+                    ldsm4t_at(v4, Vt + s * TILE + tile_at(ks * 16 + (lane & 7) + (lane >> 4) * 8, m * 2 + ((lane >> 3) & 1)));
+                    mma(o[w], v4, pf[ks][0], pf[ks][1]);
+                }
+            }
+        }
+        __syncthreads(); // the round has been read
+        fetch_v(kb + 4);
+    }
+    l = __fadd_rn(l, __shfl_xor_sync(0xffffffffu, l, 1));
+    l = __fadd_rn(l, __shfl_xor_sync(0xffffffffu, l, 2));
+    const float inv = *static_cast<volatile int *>(&abort_s) ? __int_as_float(0x7fffffff) : __fdiv_rn(1.0f, l); // a wait ran out: no result
+    bf16 *out = reinterpret_cast<bf16 *>(a.o) + ((size_t)i * a.B + b) * HD + h * DK;
+#pragma unroll
+    for (int w = 0; w < MW; w++) {
+        const int m = warp + 4 * w;
+        if (t == 0) {
+            out[m * 16 + g] = __float2bfloat16_rn(__fmul_rn(o[w][0], inv));
+            out[m * 16 + g + 8] = __float2bfloat16_rn(__fmul_rn(o[w][2], inv));
+        }
+    }
+    if (threadIdx.x == 0 && a.lse)
+        a.lse[((size_t)b * a.H + h) * T + i] = m_run + logf(l);
+}
+
 // ---------------- backward ----------------
 //
 // One CTA of eight warps per (stream, head), key blocks in ascending order; per block
@@ -968,19 +1174,50 @@ inline bool fits(int dk, int L)
     }
 }
 
+// tiles of 64 columns x 64 rows of a three-dimensional bf16 tensor whose rows are `mid` or `outer` apart
+inline int tile_map(const void *p, const cuuint64_t (&dims)[3], const cuuint64_t (&strides)[2], bool rows_outer, CUtensorMap *out)
+{
+    tc::EncodeTiledFn fn = tc::encode_fn();
+    if (!fn)
+        return nncu_fail(NNCU_ERR_CUDA, "cuTensorMapEncodeTiled is not available");
+    cuuint32_t box[3] = {64, rows_outer ? 1u : 64u, rows_outer ? 64u : 1u}, estr[3] = {1, 1, 1};
+    CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void *>(p), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? NNCU_OK : nncu_fail(NNCU_ERR_CUDA, "cuTensorMapEncodeTiled failed: %d", (int)r);
+}
+template <int DK> static int forward_one(const AttnArgs &a, cudaStream_t st)
+{
+    if constexpr (DK < 64) {
+        launch_k(attn_one_kernel<DK>, dim3(a.B * a.H), dim3(128), OneSmem<DK>::TOTAL, st, a);
+    } else {
+        CUtensorMap kv, r;
+        const cuuint64_t B = a.B, L = a.L, kvp = a.kvp, H = a.H, P = a.P;
+        NNCU_TRY(tile_map(a.kv, {2 * H * DK, B, L}, {kvp * 2, B * kvp * 2}, true, &kv));
+        r = kv;
+        if (a.w_r16)
+            NNCU_TRY(tile_map(a.w_r16, {DK, P, H}, {DK * 2, P * DK * 2}, false, &r));
+        const size_t most = 227 * 1024 - 128, all = OneTmaSmem<DK>::bytes(a.L);
+        launch_k(attn_one_tma_kernel<DK>, dim3(a.B * a.H), dim3(128), all <= most ? all : OneTmaSmem<DK>::bytes(0), st, a, kv, r,
+                 all <= most ? 1 : 0);
+    }
+    KERNEL_CHECK();
+    return NNCU_OK;
+}
 template <int DK> static int forward_dk(const AttnArgs &a, cudaStream_t st)
 {
-    const size_t smem1 = OneSmem<DK>::TOTAL, smem = FwdSmem<DK>::bytes(a.L);
     static bool attr_done = false;
     if (!attr_done) {
         CUDA_TRY(cudaFuncSetAttribute(attn_fwd_kernel<DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-        CUDA_TRY(cudaFuncSetAttribute(attn_one_kernel<DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+        if constexpr (DK < 64) {
+            CUDA_TRY(cudaFuncSetAttribute(attn_one_kernel<DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+        } else {
+            CUDA_TRY(cudaFuncSetAttribute(attn_one_tma_kernel<DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - 128));
+        }
         attr_done = true;
     }
     if (a.t1 - a.t0 == 1)
-        launch_k(attn_one_kernel<DK>, dim3(a.B * a.H), dim3(128), smem1, st, a);
-    else
-        launch_k(attn_fwd_kernel<DK>, dim3(a.B * a.H, (a.t1 - (a.t0 & ~63) + 63) / 64), dim3(256), smem, st, a);
+        return forward_one<DK>(a, st);
+    launch_k(attn_fwd_kernel<DK>, dim3(a.B * a.H, (a.t1 - (a.t0 & ~63) + 63) / 64), dim3(256), FwdSmem<DK>::bytes(a.L), st, a);
     KERNEL_CHECK();
     return NNCU_OK;
 }
@@ -1022,11 +1259,11 @@ static int backward(const AttnArgs &a, cudaStream_t st)
 template <typename T>
 static int attn_forward_any(const nncu_attn_shape *s, const void *q, const void *kv, const float *w_r,
                             const float *b_r, void *out, float *lse, cudaStream_t st,
-                            const AttnPitch *pt = nullptr, const void *w_r16 = nullptr)
+                            const AttnPitch *pt = nullptr, const void *w_r16 = nullptr, int *err_flag = nullptr)
 {
     if (sizeof(T) == 2) {
         AttnArgs a = attn_args(s, pt);
-        a.q = q; a.kv = kv; a.w_r = w_r; a.b_r = b_r; a.o = out; a.lse = lse;
+        a.q = q; a.kv = kv; a.w_r = w_r; a.b_r = b_r; a.o = out; a.lse = lse; a.err_flag = err_flag;
         a.w_r16 = w_r ? w_r16 : nullptr;
         if (fa::supported(a) && fa::fits(a.dk, a.L))
             return fa::forward(a, st);

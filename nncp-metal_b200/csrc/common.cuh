@@ -36,28 +36,25 @@ int nncu_fail(int code, const char *fmt, ...);
 // predecessor has completed and its writes are visible.  Rules for a kernel launched this way:
 // every thread executes pdl_wait() before its first global-memory access and before any early
 // return, so that the kernel cannot complete before its predecessor has.  Both calls are no-ops in
-// a kernel launched the ordinary way.  Off unless NNCU_PDL=1: on the c2 train step (graph replay,
-// kernels of 3-20 us) it measured within 1 % of ordinary launches.  pdl_trigger() (successor
-// starts as soon as all CTAs of this kernel are resident) is compiled in only with
-// -DNNCU_PDL_TRIGGER: it measured 4 % slower, the resident successors taking SM resources from
-// the side stream's kernels.
+// a kernel launched the ordinary way.  On in the one-symbol steps of a decoder, a single chain of short
+// kernels (128 streams, 12 layers of 512: 80.4 -> 76.2 ms a segment of 64 steps; pdl_trigger() lets the
+// successor start as soon as all CTAs of a kernel are resident); off in whole-segment passes unless
+// NNCU_PDL=1: there a side stream's kernels fill the gaps, and the resident successors take SM resources
+// from them (train steps of the bf16 models between 4 % faster and 2 % slower).
 __device__ __forceinline__ void pdl_wait()
 {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
-// the same signal, given late in a kernel (its successor's launch then overlaps only the tail)
-__device__ __forceinline__ void pdl_trigger_late()
-{
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
 __device__ __forceinline__ void pdl_trigger()
 {
-#ifdef NNCU_PDL_TRIGGER
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-#endif
 }
+// set while the launches of a one-symbol step are queued by this thread
+extern thread_local bool g_nncu_step_chain;
 inline bool nncu_pdl_enabled()
 {
+    if (g_nncu_step_chain)
+        return true;
     static int on = -1;
     if (on < 0) {
         const char *e = getenv("NNCU_PDL");

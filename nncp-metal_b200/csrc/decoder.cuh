@@ -62,7 +62,7 @@ decode_step_kernel(const uint16_t *__restrict__ trees, const uint8_t *__restrict
                    int B, int V, int P, int nb, int ring, int *err_flag)
 {
     pdl_wait();
-    pdl_trigger_late(); // a successor that was launched to overlap this kernel may start on what does not depend on it
+    pdl_trigger(); // a successor that was launched to overlap this kernel may start on what does not depend on it
     extern __shared__ __align__(128) uint8_t dsm[];
     uint64_t *bars = reinterpret_cast<uint64_t *>(dsm);           // [2][MAX_RING] of 8 bytes: 128
     const int G = slot_trees(B, P);

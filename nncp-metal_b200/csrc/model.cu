@@ -50,6 +50,7 @@ static int coder_depth(int V)
 thread_local char g_nncu_err[512] = "";
 unsigned long long g_nncu_launches = 0;
 GemmProfiler *g_nncu_prof = nullptr;
+thread_local bool g_nncu_step_chain = false;
 
 int nncu_fail(int code, const char *fmt, ...)
 {
@@ -681,7 +682,7 @@ static int forward_range(nncu_model *m, int t0, int t1)
         const AttnPitch pt = {3 * HD, 3 * HD, 3 * HD, 3 * HD};
         NNCU_TRY(attn_forward_any<AT>(&s, at<AT>(a.qkv, (size_t)M * B * 3 * HD), at<AT>(a.qkv, HD),
                                       wf(m, o.w_r), m->W + o.b_r, a.o, a.lse, m->st, &pt,
-                                      (m->bf && o.w_r != NONE) ? m->Wb + o.w_r : nullptr));
+                                      (m->bf && o.w_r != NONE) ? m->Wb + o.w_r : nullptr, m->err_flag));
         // output projection, residual, post-LN (nncp.c:865-920)
         if (o.alpha != NONE) { // LN_COEF: the projection is kept as it is for the backward pass, tmp = alpha * it
             AT *ao = at<AT>(a.ao, (size_t)r0 * D);
@@ -2291,6 +2292,10 @@ int nncu_decoder_begin(nncu_model *m, const uint8_t *payload_host, size_t len)
 // turns them into symbols (left in the target rows and, for t+1 < seg_len, the next step's input)
 static int decode_step(nncu_model *m, int t, int limit_t, int limit_b, bool chained)
 {
+    struct Chain { // the launches of a step are one chain on one stream: each may set itself up under the one before
+        Chain() { g_nncu_step_chain = true; }
+        ~Chain() { g_nncu_step_chain = false; }
+    } chain;
     const int B = m->B, V = m->V, nb = coder_depth(V), P = 1 << nb;
     const bool pow2 = P == V;
     if (m->step_sp) {
@@ -2305,8 +2310,8 @@ static int decode_step(nncu_model *m, int t, int limit_t, int limit_b, bool chai
                      (const float *)(m->probs + (size_t)t * B * V), m->coder_dev, V, P);
         KERNEL_CHECK();
     }
-    launch_pdl(m->step_sp || nncu_pdl_enabled(), pow2 ? dec::decode_step_kernel<false> : dec::decode_step_kernel<true>, dim3(1), dim3(64),
-               dec::smem_bytes(B, P, nb, m->dec_ring), m->st, (const uint16_t *)m->coder_dev,
+    launch_k(pow2 ? dec::decode_step_kernel<false> : dec::decode_step_kernel<true>, dim3(1), dim3(64),
+             dec::smem_bytes(B, P, nb, m->dec_ring), m->st, (const uint16_t *)m->coder_dev,
              (const uint8_t *)m->dec_payload, m->dec_state, m->tgt_dev + (size_t)t * B,
              t + 1 < m->T ? m->ids_dev + (size_t)(t + 1) * B : (int32_t *)nullptr, t, limit_t, limit_b, B, V, P, nb,
              m->dec_ring, m->err_flag);

@@ -210,7 +210,7 @@ __global__ void __launch_bounds__(256, 1) step_kernel(const __grid_constant__ Ar
         issue();
     cluster_wait();
     pdl_wait();
-    pdl_trigger_late();
+    pdl_trigger();
     if (blockIdx.x == 0 && tid == 0)
         *a.dz_fixed = 0;
     int cslot = 0;
