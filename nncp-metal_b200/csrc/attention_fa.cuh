@@ -632,7 +632,7 @@ __global__ void __launch_bounds__(128) attn_one_tma_kernel(const __grid_constant
 {
     using SM = OneTmaSmem<DK>;
     constexpr int NS = SM::NS, TILE = SM::TILE, MT = DK / 16, MW = MT / 4; // 16-column slices, and those of one warp
-    extern __shared__ __align__(1024) unsigned char smraw[];
+    extern __shared__ __align__(16) unsigned char smraw[];
     __shared__ __align__(8) uint64_t bars[8]; // K and table, V of each warp
     __shared__ int abort_s, dummy;
     unsigned char *sm = smraw + ((1024u - (smem_addr(smraw) & 1023u)) & 1023u);
@@ -1196,7 +1196,7 @@ template <int DK> static int forward_one(const AttnArgs &a, cudaStream_t st)
         r = kv;
         if (a.w_r16)
             NNCU_TRY(tile_map(a.w_r16, {DK, P, H}, {DK * 2, P * DK * 2}, false, &r));
-        const size_t most = 227 * 1024 - 128, all = OneTmaSmem<DK>::bytes(a.L);
+        const size_t most = 226 * 1024, all = OneTmaSmem<DK>::bytes(a.L);
         launch_k(attn_one_tma_kernel<DK>, dim3(a.B * a.H), dim3(128), all <= most ? all : OneTmaSmem<DK>::bytes(0), st, a, kv, r,
                  all <= most ? 1 : 0);
     }
@@ -1211,7 +1211,7 @@ template <int DK> static int forward_dk(const AttnArgs &a, cudaStream_t st)
         if constexpr (DK < 64) {
             CUDA_TRY(cudaFuncSetAttribute(attn_one_kernel<DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
         } else {
-            CUDA_TRY(cudaFuncSetAttribute(attn_one_tma_kernel<DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - 128));
+            CUDA_TRY(cudaFuncSetAttribute(attn_one_tma_kernel<DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
         }
         attr_done = true;
     }
