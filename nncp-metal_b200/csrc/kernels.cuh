@@ -703,56 +703,79 @@ act_bwd_kernel(const T *__restrict__ hpre, const T *__restrict__ dhact, T *__res
     }
 }
 
-// Two columns per thread (4-byte accesses), ACT_BWD_ROWS rows per block (short serial chains:
-// the kernel is bound by the latency of its per-element math, not by bytes); element
-// arithmetic as in act_bwd_kernel.  F even; grid (ceil(F/256), ceil(rows/ACT_BWD_ROWS)).
+// W = 2 or 4 columns per thread, ACT_BWD_ROWS rows per block; element arithmetic as in act_bwd_kernel.
+// Bound by its instructions (some 20 an element) and, before that, by latency: all of a thread's loads go
+// out before the first is used.  F a multiple of W; grid (ceil(F / (128 W)), ceil(rows/ACT_BWD_ROWS)).
+template <int W>
 __global__ void __launch_bounds__(128)
 act_bwd_vec_kernel(const bf16 *__restrict__ hpre, const bf16 *__restrict__ dhact, bf16 *__restrict__ dhpre,
                    float *__restrict__ part, int rows, int F, int F1, int act)
 {
     pdl_trigger();
     pdl_wait();
-    const int i = (blockIdx.x * 128 + threadIdx.x) * 2;
+    constexpr int N = W / 2; // words of two columns
+    struct alignas(4 * N) Pack {
+        __nv_bfloat162 v[N];
+    };
+    const int i = (blockIdx.x * 128 + threadIdx.x) * W;
     if (i >= F)
         return;
-    const int r0 = blockIdx.y * ACT_BWD_ROWS, r1 = min(rows, r0 + ACT_BWD_ROWS);
-    float s0[2] = {0.0f, 0.0f}, s1[2] = {0.0f, 0.0f};
+    const int r0 = blockIdx.y * ACT_BWD_ROWS, n = min(rows - r0, ACT_BWD_ROWS);
+    const bool gated = !(act == NNCU_FF_RELU || act == NNCU_FF_GELU);
+    Pack pa[ACT_BWD_ROWS], pd[ACT_BWD_ROWS], pg[ACT_BWD_ROWS];
+#pragma unroll
+    for (int rr = 0; rr < ACT_BWD_ROWS; rr++)
+        if (rr < n) {
+            const size_t r = r0 + rr;
+            pa[rr] = *reinterpret_cast<const Pack *>(hpre + r * F1 + i);
+            pd[rr] = *reinterpret_cast<const Pack *>(dhact + r * F + i);
+            if (gated)
+                pg[rr] = *reinterpret_cast<const Pack *>(hpre + r * F1 + F + i);
+        }
+    float s0[W], s1[W];
+#pragma unroll
+    for (int j = 0; j < W; j++)
+        s0[j] = s1[j] = 0.0f;
 #pragma unroll
     for (int rr = 0; rr < ACT_BWD_ROWS; rr++) {
-        const int r = r0 + rr;
-        if (r >= r1)
+        if (rr >= n)
             break;
-        const __nv_bfloat162 a2 = *reinterpret_cast<const __nv_bfloat162 *>(hpre + (size_t)r * F1 + i);
-        const __nv_bfloat162 d2 = *reinterpret_cast<const __nv_bfloat162 *>(dhact + (size_t)r * F + i);
-        const float a[2] = {__low2float(a2), __high2float(a2)}, d[2] = {__low2float(d2), __high2float(d2)};
-        bf16 o0[2], o1[2];
-        if (act == NNCU_FF_RELU || act == NNCU_FF_GELU) {
+        const size_t r = r0 + rr;
+        Pack o0, o1;
 #pragma unroll
-            for (int j = 0; j < 2; j++) {
-                o0[j] = from_f<bf16>(act == NNCU_FF_RELU ? (a[j] > 0.0f ? d[j] : 0.0f) : d[j] * gelu_grad_hw(a[j]));
-                s0[j] += to_f(o0[j]);
-            }
-        } else {
-            const __nv_bfloat162 g2 = *reinterpret_cast<const __nv_bfloat162 *>(hpre + (size_t)r * F1 + F + i);
-            const float gate[2] = {__low2float(g2), __high2float(g2)};
+        for (int k = 0; k < N; k++) {
+            const float a[2] = {__low2float(pa[rr].v[k]), __high2float(pa[rr].v[k])}, d[2] = {__low2float(pd[rr].v[k]), __high2float(pd[rr].v[k])};
+            bf16 x[2], y[2];
+            if (!gated) {
 #pragma unroll
-            for (int j = 0; j < 2; j++) {
-                o0[j] = from_f<bf16>(d[j] * gate[j] * gate_grad_hw(a[j], act));
-                o1[j] = from_f<bf16>(d[j] * gate_hw(a[j], act));
-                s0[j] += to_f(o0[j]);
-                s1[j] += to_f(o1[j]);
+                for (int j = 0; j < 2; j++) {
+                    x[j] = from_f<bf16>(act == NNCU_FF_RELU ? (a[j] > 0.0f ? d[j] : 0.0f) : d[j] * gelu_grad_hw(a[j]));
+                    s0[2 * k + j] += to_f(x[j]);
+                }
+            } else {
+                const float gate[2] = {__low2float(pg[rr].v[k]), __high2float(pg[rr].v[k])};
+#pragma unroll
+                for (int j = 0; j < 2; j++) {
+                    x[j] = from_f<bf16>(d[j] * gate[j] * gate_grad_hw(a[j], act));
+                    y[j] = from_f<bf16>(d[j] * gate_hw(a[j], act));
+                    s0[2 * k + j] += to_f(x[j]);
+                    s1[2 * k + j] += to_f(y[j]);
+                }
+                o1.v[k] = __halves2bfloat162(y[0], y[1]);
             }
-            *reinterpret_cast<__nv_bfloat162 *>(dhpre + (size_t)r * F1 + F + i) = __halves2bfloat162(o1[0], o1[1]);
+            o0.v[k] = __halves2bfloat162(x[0], x[1]);
         }
-        *reinterpret_cast<__nv_bfloat162 *>(dhpre + (size_t)r * F1 + i) = __halves2bfloat162(o0[0], o0[1]);
+        *reinterpret_cast<Pack *>(dhpre + r * F1 + i) = o0;
+        if (gated)
+            *reinterpret_cast<Pack *>(dhpre + r * F1 + F + i) = o1;
     }
     if (part) {
         float *row = part + (size_t)blockIdx.y * F1;
-        row[i] = s0[0];
-        row[i + 1] = s0[1];
-        if (F1 > F) {
-            row[F + i] = s1[0];
-            row[F + i + 1] = s1[1];
+#pragma unroll
+        for (int j = 0; j < W; j++) {
+            row[i + j] = s0[j];
+            if (gated)
+                row[F + i + j] = s1[j];
         }
     }
 }

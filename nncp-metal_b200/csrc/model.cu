@@ -963,14 +963,16 @@ static int backward(nncu_model *m)
         NNCU_TRY(mm_tn(m, D, F, TB, dt2, D, atc<AT>(a.hact, 0), F, gf(m, o.ff2)));
         NNCU_TRY(mm_nn(m, TB, F, D, dt2, D, o.ff2, dh, F, (const AT *)nullptr));
         float *apart = o.ff_bias1 != NONE ? part_slot(m) : nullptr;
-        const bool act_vec = sizeof(AT) == 2 && F % 2 == 0;
         const int act_rows = ACT_BWD_ROWS;
-        if (act_vec)
-            launch_k(act_bwd_vec_kernel, dim3(ceil_div(F, 256), ceil_div(TB, act_rows)), dim3(128), 0, m->st,
-                     (const bf16 *)atc<AT>(a.hpre, 0), (const bf16 *)dh, (bf16 *)dhp, apart, TB, F, F1, p.ff_act);
-        else
+        if (sizeof(AT) == 2 && F % 2 == 0) {
+            // four columns a thread where the rows allow it and the blocks still are two per SM
+            const bool wide = F % 4 == 0 && (long)ceil_div(F, 512) * ceil_div(TB, act_rows) >= 2 * 148;
+            launch_k(wide ? act_bwd_vec_kernel<4> : act_bwd_vec_kernel<2>, dim3(ceil_div(F, wide ? 512 : 256), ceil_div(TB, act_rows)), dim3(128), 0,
+                     m->st, (const bf16 *)atc<AT>(a.hpre, 0), (const bf16 *)dh, (bf16 *)dhp, apart, TB, F, F1, p.ff_act);
+        } else {
             launch_k(act_bwd_kernel<AT>, dim3(ceil_div(F, 128), ceil_div(TB, act_rows)), dim3(128), 0, m->st,
                      atc<AT>(a.hpre, 0), (const AT *)dh, dhp, apart, TB, F, F1, p.ff_act);
+        }
         KERNEL_CHECK();
         if (apart)
             NNCU_TRY(reduce_cols(m, apart, ceil_div(TB, act_rows), F1, F1, gf(m, o.ff_bias1), 0));
