@@ -36,8 +36,8 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_
                  : "memory");
 }
 
-// window bytes a step of `B` streams with `nb` bits per symbol can consume, one to look ahead, as a multiple of 16
-__host__ __device__ inline int window_bytes(int B, int nb) { return (2 * B * nb + 1 + 15) & ~15; }
+// window bytes a step of `B` streams with `nb` bits per symbol can consume, twelve to look ahead, as a multiple of 16
+__host__ __device__ inline int window_bytes(int B, int nb) { return (2 * B * nb + 12 + 15) & ~15; }
 // trees of P entries that share a ring slot: small ones come 16 KB at a time
 __host__ __device__ inline int slot_trees(int B, int P) { return P >= 8192 ? 1 : (8192 / P < B ? 8192 / P : B); }
 
@@ -105,8 +105,29 @@ decode_step_kernel(const uint16_t *__restrict__ trees, const uint8_t *__restrict
     int walked = 0; // groups whose copy has been waited for
     bool ok = true;
     if (tid == 0) {
-        uint32_t low = state->low, range = state->range, used = 0, next = win[0];
-        const uint32_t half = (uint32_t)P / 2u;
+        // What a bit costs is a chain of dependent instructions on one thread, so nothing in it branches: a node's
+        // prob0 is in hand, and its children's (one 32-bit word) are on their way, before the branch at it is
+        // known; (range * prob0) >> 15 is the high word of (range << 8) * (prob0 << 9), range staying below
+        // 2^24; renormalisation shifts by 0, 8 or 16 (two bytes always suffice: range is at least 1) and draws
+        // on the next eight payload bytes in two registers, topped up after every second bit if need be.
+        uint32_t low = state->low, range = state->range, used = 0, hi, lo, drawn; // drawn: bits taken from hi : lo
+        const uint32_t *words = reinterpret_cast<const uint32_t *>(win);
+        auto top_up = [&]() { // the eight window bytes from `used` on (zero past the payload's end)
+            const uint32_t *w = words + (used >> 2);
+            const uint32_t w0 = __byte_perm(w[0], 0, 0x0123), w1 = __byte_perm(w[1], 0, 0x0123), w2 = __byte_perm(w[2], 0, 0x0123);
+            const uint32_t sh = (used & 3) * 8;
+            hi = __funnelshift_l(w1, w0, sh);
+            lo = __funnelshift_l(w2, w1, sh);
+            drawn = 0;
+        };
+        const uint32_t last = (uint32_t)P / 2u - 1; // word of the last pair: below the tree's leaves there is nothing to load
+        top_up();
+        auto check = [&]() {
+            if (drawn > 32) {
+                used += drawn >> 3;
+                top_up();
+            }
+        };
         int slot = ring - 1, in_slot = G; // the slot in use and the trees of it that have been walked
         uint32_t phase = 1;
         for (int b = 0; b < B; b++) {
@@ -124,44 +145,56 @@ decode_step_kernel(const uint16_t *__restrict__ trees, const uint8_t *__restrict
                     walked += ok ? 1 : 0;
                 }
                 if (ok) {
-                    // Node k's prob0 is in hand, and its children's (one 32-bit word) are on their way, before the
-                    // branch at k is known: what a bit costs is the chain product - compare - select.
-                    // (range * prob0) >> 15 is the high word of (range << 8) * (prob0 << 9): range stays below 2^24.
                     const uint32_t *pairs = reinterpret_cast<const uint32_t *>(slots + ((size_t)slot * G + in_slot) * P);
                     in_slot++;
-                    uint32_t k = 1, p0 = pairs[0] >> 16, kids = pairs[1];
-                    auto next_bit = [&]() { // get_bit at node k: the branch taken, low / range / used advanced
-                        const uint32_t split = __umulhi(range << 8, p0 << 9);
+                    uint32_t k = 1, p9 = (pairs[0] >> 16) << 9, kids = pairs[1];
+                    auto next_bit = [&]() { // get_bit at node k: the branch taken, the decoder's state advanced
+                        const uint32_t split = __umulhi(range << 8, p9);
                         const bool bit = low >= split;
                         k = 2 * k + (bit ? 1u : 0u);
-                        p0 = bit ? kids >> 16 : kids & 0xffffu;
-                        kids = pairs[min(k, half - 1)];
+                        const uint32_t p1 = (kids >> 16) << 9, p0 = (kids & 0xffffu) << 9;
+                        p9 = bit ? p1 : p0;
+                        kids = pairs[min(k, last)];
                         low = bit ? low - split : low;
                         range = bit ? range - split : split;
-                        if (range < R_LOW) {
-                            do { // the window is zero past the payload's end; one byte is always in hand
-                                range <<= 8;
-                                low = (low << 8) + next;
-                                next = win[++used];
-                            } while (range < R_LOW);
-                        }
+                        const uint32_t s = range < R_LOW ? (range < 0x100u ? 16u : 8u) : 0u;
+                        range <<= s;
+                        low = __funnelshift_l(hi, low, s);
+                        hi = __funnelshift_l(lo, hi, s);
+                        lo <<= s;
+                        drawn += s;
                         return bit;
                     };
-                    if constexpr (ANY) {
-                        int lo = 0, n = V;
-                        for (int lvl = 0; lvl < nb && n > 1; lvl++) {
+                    if constexpr (ANY) { // every node above the last level is split, one of the last if it has two symbols
+                        int first = 0, n = V;
+                        auto down = [&](bool bit) {
                             const int h = n >> 1;
-                            if (next_bit()) {
-                                lo += h;
-                                n -= h;
-                            } else {
-                                n = h;
-                            }
+                            first = bit ? first + h : first;
+                            n = bit ? n - h : h;
+                        };
+                        int lvl = 1;
+                        for (; lvl + 1 < nb; lvl += 2) {
+                            down(next_bit());
+                            down(next_bit());
+                            check();
                         }
-                        c = lo;
+                        if (lvl < nb)
+                            down(next_bit());
+                        if (n > 1)
+                            down(next_bit());
+                        check();
+                        c = first;
                     } else {
-                        for (int lvl = 0; lvl < nb; lvl++)
+                        int lvl = 0;
+                        for (; lvl + 1 < nb; lvl += 2) {
                             next_bit();
+                            next_bit();
+                            check();
+                        }
+                        if (lvl < nb) {
+                            next_bit();
+                            check();
+                        }
                         c = (int)k - V;
                     }
                 }
@@ -170,6 +203,7 @@ decode_step_kernel(const uint16_t *__restrict__ trees, const uint8_t *__restrict
             if (ids_next)
                 ids_next[b] = c;
         }
+        used += drawn >> 3;
         state->pos = min(pos0 + used, len);
         state->low = low;
         state->range = range;
