@@ -206,7 +206,8 @@ struct nncu_model {
     int n_jobs, n_job_tiles;
     uint16_t *coder_dev;
     size_t coder_bytes;
-    // host staging (pinned)
+    // host staging (pinned), one allocation
+    char *pin = nullptr;
     int32_t *ids_pin, *tgt_pin, *sym_pin; // pinned staging of ids, targets, coder symbols
     uint16_t *coder_pin;                  // pinned landing area of nncu_coder_paths_begin
     float *loss_pin;
@@ -1139,7 +1140,7 @@ static int refresh_shadows(nncu_model *m)
 
 // ------------------------------------------------------------------ parameter table
 
-static uint64_t splitmix64(uint64_t x)
+__host__ __device__ static inline uint64_t splitmix64(uint64_t x)
 {
     x += 0x9E3779B97F4A7C15ull;
     x = (x ^ (x >> 30)) * 0xBF58476D1CE4E5B9ull;
@@ -1155,29 +1156,43 @@ static uint64_t name_hash(const char *s)
     }
     return h;
 }
-static inline float u01(uint64_t key, uint64_t idx, uint32_t k)
+__device__ static inline float u01(uint64_t key, uint64_t idx, uint32_t k)
 {
     uint64_t r = splitmix64(key ^ splitmix64(idx * 16 + k));
     return (float)(r >> 40) * (1.0f / 16777216.0f);
 }
 // Counter-based initial values: element i of parameter `name` depends only on
 // (seed, name, i).  Integer hashing plus exactly-rounded float adds/multiplies,
-// so encoder and decoder hosts produce the same bits (trf_init draws from
+// so every host and the device produce the same bits (trf_init draws from
 // nc_tensor_set_rnd_unif in creation order, nncp.c:263-266, whose generator is
-// not part of the reference tree).
-static void init_values(float *dst, size_t n, const char *name, uint32_t seed, int kind, float scale)
+// not part of the reference tree).  On the device: one host thread took 5 ms for the
+// 2.2 M parameters of a level-6 model, and the upload as much again.
+__global__ void init_values_kernel(float *__restrict__ dst, size_t n, uint64_t key, int kind, float scale)
 {
-    uint64_t key = splitmix64(name_hash(name) ^ ((uint64_t)seed << 32));
-    for (size_t i = 0; i < n; i++) {
-        if (kind == NNCU_INIT_NORMAL) {
-            float s = 0.0f;
-            for (uint32_t k = 0; k < 12; k++)
-                s += u01(key, i, k);
-            dst[i] = (s - 6.0f) * scale;
-        } else {
-            dst[i] = (2.0f * u01(key, i, 0) - 1.0f) * scale;
-        }
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n)
+        return;
+    if (kind == NNCU_INIT_NORMAL) {
+        float s = 0.0f;
+        for (uint32_t k = 0; k < 12; k++)
+            s = __fadd_rn(s, u01(key, i, k));
+        dst[i] = __fmul_rn(__fsub_rn(s, 6.0f), scale);
+    } else {
+        dst[i] = __fmul_rn(__fsub_rn(__fmul_rn(2.0f, u01(key, i, 0)), 1.0f), scale);
     }
+}
+__global__ void fill_kernel(float *__restrict__ dst, size_t n, float v)
+{
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n)
+        dst[i] = v;
+}
+static int init_values(float *dst_dev, size_t n, const char *name, uint32_t seed, int kind, float scale, cudaStream_t st)
+{
+    const uint64_t key = splitmix64(name_hash(name) ^ ((uint64_t)seed << 32));
+    init_values_kernel<<<ceil_div((long long)n, 256), 256, 0, st>>>(dst_dev, n, key, kind, scale);
+    KERNEL_CHECK();
+    return NNCU_OK;
 }
 
 static size_t add_param(nncu_model *m, const char *base, int idx, size_t numel, int rows = 0, int cols = 0,
@@ -1274,16 +1289,12 @@ int nncu_destroy(nncu_model *m)
     if (m->ev_fork) cudaEventDestroy(m->ev_fork);
     if (m->ev_join) cudaEventDestroy(m->ev_join);
     if (m->arena) cudaFree(m->arena);
-    if (m->ids_pin) cudaFreeHost(m->ids_pin);
-    if (m->tgt_pin) cudaFreeHost(m->tgt_pin);
-    if (m->sym_pin) cudaFreeHost(m->sym_pin);
-    if (m->coder_pin) cudaFreeHost(m->coder_pin);
+    if (m->pin) cudaFreeHost(m->pin);
     if (m->ev_ids) cudaEventDestroy(m->ev_ids);
     if (m->ev_tgt) cudaEventDestroy(m->ev_tgt);
     if (m->ev_sym) cudaEventDestroy(m->ev_sym);
     if (m->ev_coder) cudaEventDestroy(m->ev_coder);
     if (m->ev_loss) cudaEventDestroy(m->ev_loss);
-    if (m->loss_pin) cudaFreeHost(m->loss_pin);
     if (m->own_st) cudaStreamDestroy(m->own_st);
     delete m;
     return NNCU_OK;
@@ -1311,11 +1322,11 @@ int nncu_create(const nncu_params *p, nncu_model **out)
     if (dev < 0)
         CUDA_TRY(cudaGetDevice(&dev));
     CUDA_TRY(cudaSetDevice(dev));
-    cudaDeviceProp prop;
-    CUDA_TRY(cudaGetDeviceProperties(&prop, dev));
-    if (prop.major != 10)
-        return nncu_fail(NNCU_ERR_CUDA, "device %d is sm_%d%d; this library is built for sm_100a only",
-                         dev, prop.major, prop.minor);
+    int major = 0, minor = 0; // two attributes: the whole property table takes the driver a millisecond
+    CUDA_TRY(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev));
+    CUDA_TRY(cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, dev));
+    if (major != 10)
+        return nncu_fail(NNCU_ERR_CUDA, "device %d is sm_%d%d; this library is built for sm_100a only", dev, major, minor);
 
     nncu_model *m = new nncu_model();
     m->p = *p;
@@ -1525,12 +1536,17 @@ int nncu_create(const nncu_params *p, nncu_model **out)
         const char *e = getenv("NNCU_NO_OVERLAP");
         m->overlap = !(e && e[0] == '1');
     }
-    if (cudaMallocHost(&m->ids_pin, sizeof(int32_t) * TB) != cudaSuccess ||
-        cudaMallocHost(&m->tgt_pin, sizeof(int32_t) * TB) != cudaSuccess ||
-        cudaMallocHost(&m->sym_pin, sizeof(int32_t) * TB) != cudaSuccess ||
-        cudaMallocHost(&m->coder_pin, sizeof(uint16_t) * TB * 16) != cudaSuccess ||
-        cudaMallocHost(&m->loss_pin, 64) != cudaSuccess)
-        return fail_cleanup(nncu_fail(NNCU_ERR_NOMEM, "pinned host allocation failed"));
+    {
+        // one pinned allocation for all staging areas: each costs the driver half a millisecond
+        const size_t rows = (sizeof(int32_t) * TB + 63) & ~(size_t)63, paths = (sizeof(uint16_t) * TB * 16 + 63) & ~(size_t)63;
+        if (cudaMallocHost(&m->pin, 3 * rows + paths + 64) != cudaSuccess)
+            return fail_cleanup(nncu_fail(NNCU_ERR_NOMEM, "pinned host allocation failed"));
+        m->ids_pin = (int32_t *)m->pin;
+        m->tgt_pin = (int32_t *)(m->pin + rows);
+        m->sym_pin = (int32_t *)(m->pin + 2 * rows);
+        m->coder_pin = (uint16_t *)(m->pin + 3 * rows);
+        m->loss_pin = (float *)(m->pin + 3 * rows + paths);
+    }
     if (cudaEventCreateWithFlags(&m->ev_ids, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&m->ev_tgt, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&m->ev_sym, cudaEventDisableTiming) != cudaSuccess ||
@@ -1592,25 +1608,25 @@ int nncu_create(const nncu_params *p, nncu_model **out)
         }
     }
 
-    // ---- initial values (trf_init, nncp.c:341-497), computed on the host
+    // ---- initial values (trf_init, nncp.c:341-497); what is not named stays zero
+    int rc = NNCU_OK;
     {
-        std::vector<float> host(m->n_floats, 0.0f);
-        float a0 = p->init_kind == NNCU_INIT_NORMAL ? p->init_range : p->init_range / sqrtf((float)D);
+        const float a0 = p->init_kind == NNCU_INIT_NORMAL ? p->init_range : p->init_range / sqrtf((float)D);
         for (const ParamInfo &pi : m->pinfo) {
-            float *dst = host.data() + pi.off;
+            float *dst = m->W + pi.off;
+            if (rc != NNCU_OK)
+                break;
             if (!strncmp(pi.name, "ln_g", 4)) {
-                for (size_t k = 0; k < pi.numel; k++)
-                    dst[k] = 1.0f;
+                fill_kernel<<<ceil_div((long long)pi.numel, 256), 256, 0, m->st>>>(dst, pi.numel, 1.0f);
             } else if (!strncmp(pi.name, "w_", 2) || !strncmp(pi.name, "ff1", 3) || !strncmp(pi.name, "embed", 5)) {
-                init_values(dst, pi.numel, pi.name, p->seed, p->init_kind, a0);
+                rc = init_values(dst, pi.numel, pi.name, p->seed, p->init_kind, a0, m->st);
             } else if (!strncmp(pi.name, "ff2", 3)) {
-                init_values(dst, pi.numel, pi.name, p->seed, p->init_kind, a0 * sqrtf((float)D / (float)F));
+                rc = init_values(dst, pi.numel, pi.name, p->seed, p->init_kind, a0 * sqrtf((float)D / (float)F), m->st);
             }
         }
-        if (cudaMemcpy(m->W, host.data(), m->n_floats * 4, cudaMemcpyHostToDevice) != cudaSuccess)
-            return fail_cleanup(nncu_fail(NNCU_ERR_CUDA, "weight upload failed"));
     }
-    int rc = refresh_shadows(m);
+    if (rc == NNCU_OK)
+        rc = refresh_shadows(m);
     if (rc == NNCU_OK && cudaStreamSynchronize(m->st) != cudaSuccess)
         rc = nncu_fail(NNCU_ERR_CUDA, "initialisation kernels failed: %s", cudaGetErrorString(cudaGetLastError()));
     if (rc != NNCU_OK)
