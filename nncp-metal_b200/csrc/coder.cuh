@@ -93,22 +93,32 @@ coder_paths_fast_kernel(const float *__restrict__ probs, const int32_t *__restri
             p0s[d] = v;
     };
     const float4 *pr = reinterpret_cast<const float4 *>(probs + (size_t)row * V);
+    // The path's nodes of up to 128 leaves, and so their left children, lie in the 128 leaves that one warp
+    // reads in one step: every other step only sums (looking at every node cost three
+    // times the 20 us that 2048 rows of 16384 take to read).
+    const int mine = (s >> 7) - w; // 8 j for the step of this warp that has the symbol's leaf
 #pragma unroll
     for (int j = 0; j < 16; j++) {
         if (j < nv4) {
             const unsigned g = (unsigned)(j * 256 + tid);
             const float4 q = pr[g];
-            keep((unsigned)V + 4u * g, q.x); // a leaf that is a left child
-            keep((unsigned)V + 4u * g + 2u, q.z);
             const float a = __fadd_rn(q.x, q.y), b = __fadd_rn(q.z, q.w);
-            keep((unsigned)(V >> 1) + 2u * g, a);
             float v = __fadd_rn(a, b);
-            keep((unsigned)(V >> 2) + g, v);
+            if (mine == 8 * j) {
+                keep((unsigned)V + 4u * g, q.x); // a leaf that is a left child
+                keep((unsigned)V + 4u * g + 2u, q.z);
+                keep((unsigned)(V >> 1) + 2u * g, a);
+                keep((unsigned)(V >> 2) + g, v);
 #pragma unroll
-            for (int q2 = 1; q2 <= 5; q2++) {
-                v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, 1 << (q2 - 1)));
-                if ((lane & ((1 << q2) - 1)) == 0)
-                    keep((unsigned)(V >> (2 + q2)) + (g >> q2), v);
+                for (int q2 = 1; q2 <= 5; q2++) {
+                    v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, 1 << (q2 - 1)));
+                    if (q2 < 5 && (lane & ((1 << q2) - 1)) == 0)
+                        keep((unsigned)(V >> (2 + q2)) + (g >> q2), v);
+                }
+            } else {
+#pragma unroll
+                for (int q2 = 1; q2 <= 5; q2++)
+                    v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, 1 << (q2 - 1)));
             }
             if (lane == 0)
                 heap[NW + j * 8 + w] = v; // depth log2(NW): node NW + (g >> 5)
@@ -116,6 +126,8 @@ coder_paths_fast_kernel(const float *__restrict__ probs, const int32_t *__restri
     }
     __syncthreads();
     if (w == 0) {
+        if (lane == 0)
+            p0s[L - 8] = heap[2 * (leafK >> 8)]; // the left of the path's two nodes of 128 leaves
         for (int n = NW >> 1; n >= 1; n >>= 1) {
             for (int k = n + lane; k < 2 * n; k += 32) {
                 const float v = __fadd_rn(heap[2 * k], heap[2 * k + 1]);

@@ -500,8 +500,10 @@ static int norm_bwd(nncu_model *m, const AT *dy, const AT *x, size_t g_off, size
     float *part = part_slot(m);
     const float *g = m->W + g_off;
     const int ws = dxsum ? 1 : 0;
-    // eight warps a block, one row each, until the blocks are two per SM; then more rows per warp
-    const int rpb = 8 * std::max(1, ceil_div(rows, 8 * 2 * 148));
+    // eight warps a block, one row each, until the blocks fill the chip once; then more rows per warp.  Blocks
+    // of the widest rows have an SM to themselves (their sums alone are 96 registers a thread), others share it
+    const int per_sm = norm_in_registers<AT>(m->D, 4) && !norm_in_registers<AT>(m->D, 3) ? 1 : 2;
+    const int rpb = 8 * std::max(1, ceil_div(rows, 8 * per_sm * 148));
     const int blocks = ceil_div(rows, rpb);
     if (norm_in_registers<AT>(m->D, 4))
         with_chunks<AT>(m->D, [&](auto nc) {
@@ -1072,13 +1074,13 @@ static int backward(nncu_model *m)
         CUDA_TRY(cudaMemsetAsync(m->first_dev, 0x7f, sizeof(int) * (size_t)V, m->st3));
         launch_k(first_rows_kernel, dim3(ceil_div(rows, 256)), dim3(256), 0, m->st3, (const int32_t *)m->ids_all, rows, V, m->first_dev);
         KERNEL_CHECK();
-        launch_k(embed_grad_kernel<AT>, dim3(rows), dim3(128), 0, m->st3, (const int32_t *)m->ids_all, (const AT *)m->dx_all,
+        launch_k(embed_grad_kernel<AT>, dim3(rows, ceil_div(D, 256)), dim3(128), 0, m->st3, (const int32_t *)m->ids_all, (const AT *)m->dx_all,
                  gf(m, m->embed), (const int *)m->first_dev, rows, D, emul, V);
         KERNEL_CHECK();
         NNCU_TRY(opt_range(m, m->embed, m->embed_out, false));
     } else {
         CUDA_TRY(cudaMemsetAsync(gf(m, m->embed), 0, sizeof(float) * (size_t)V * D, m->st));
-        launch_k(embed_grad_kernel<AT>, dim3(TB), dim3(128), 0, m->st, (const int32_t *)m->ids_dev, (const AT *)dx, gf(m, m->embed),
+        launch_k(embed_grad_kernel<AT>, dim3(TB, ceil_div(D, 256)), dim3(128), 0, m->st, (const int32_t *)m->ids_dev, (const AT *)dx, gf(m, m->embed),
                  (const int *)m->first_dev, TB, D, emul, V);
         KERNEL_CHECK();
         NNCU_TRY(flush_reductions(m));
