@@ -54,9 +54,15 @@ constexpr int MAX_CLUSTERS = 14;             // clusters that are on the chip to
 constexpr int KC = 256, SLOT = 8 * KC;       // columns of a weight piece, floats of a ring slot
 constexpr int MAX_SLOTS = 4;                 // ring slots per warp
 
+// columns of an N-wide output per CTA, whole groups of eight
+__host__ __device__ inline int per_cta(int N) { return ((N + CLUSTER - 1) / CLUSTER + 7) & ~7; }
+
+// weight pieces of a warp for N output columns, at most
+__host__ __device__ inline int pieces_of(int N, int K) { return (per_cta(N) / 8 + 7) / 8 * ((K + KC - 1) / KC); }
+
 // shared memory, in floats
 struct Plan {
-    int ring, layers, prods, x, qkv, ob, tmp, y, ha, lg, S, kv, pair, ks, total;
+    int ring, layers, prods, list, cap, x, qkv, ob, tmp, y, ha, lg, S, kv, pair, ks, total;
 };
 __host__ __device__ inline Plan plan_of(int SP, int nl, int D, int H, int dk, int F, int L, int P, int V, int tree, int slots)
 {
@@ -67,6 +73,8 @@ __host__ __device__ inline Plan plan_of(int SP, int nl, int D, int H, int dk, in
     p.ks = dk + 4;
     p.ring = take(8 * slots * SLOT); // first: its slots are 1024-byte aligned
     p.prods = take((4 * nl + 1) * 4);
+    p.cap = nl * (pieces_of(3 * HD, D) + pieces_of(D, HD) + pieces_of(F, D) + pieces_of(D, F)) + pieces_of(V, D);
+    p.list = take(8 * p.cap);
     p.layers = take(nl * (int)(sizeof(Layer) / 4));
     p.x = take(SP * D);
     p.qkv = take(SP * 3 * HD);
@@ -118,9 +126,6 @@ __device__ __forceinline__ void await(uint32_t bar, uint32_t parity, volatile in
 struct Product {
     int K, n0, groups, turn;
 };
-// columns of an N-wide output per CTA, whole groups of eight
-__device__ __forceinline__ int per_cta(int N) { return ((N + CLUSTER - 1) / CLUSTER + 7) & ~7; }
-
 template <int SP>
 __global__ void __launch_bounds__(256, 1) step_kernel(const __grid_constant__ Args a, int t)
 {
@@ -174,35 +179,35 @@ __global__ void __launch_bounds__(256, 1) step_kernel(const __grid_constant__ Ar
     __syncthreads();
 
     // This warp's stream of weight pieces: the groups of eight columns are dealt round robin over the warps
-    // through all products, a group's pieces follow one another.  The state of what is issued next:
-    int ap = 0, ag = warp, ak = 0, aslot = 0, ahead = 0; // product, group, first column, slot; pieces issued and not read yet
-    auto settle = [&]() {
-        while (ap < np && ag >= prods[ap].groups) {
-            ap++;
-            if (ap < np)
-                ag = (warp - prods[ap].turn) & 7;
-        }
-    };
-    settle();
+    // through all products, a group's pieces follow one another.  An entry of the list is (product, row / 8, piece).
+    uint32_t *list = reinterpret_cast<uint32_t *>(sm + pl.list) + warp * pl.cap;
+    int n_list = 0;
+    for (int i = 0; i < np; i++) {
+        const Product p = prods[i];
+        const int pieces = (p.K + KC - 1) / KC;
+        for (int g = (warp - p.turn) & 7; g < p.groups; g += 8)
+            for (int k = 0; k < pieces; k++, n_list++)
+                if (lane == 0)
+                    list[n_list] = (uint32_t)(i | ((p.n0 >> 3) + g) << 8 | k << 22);
+    }
+    __syncwarp();
+    int at_list = 0, aslot = 0, ahead = 0; // entries issued, slot of the next; pieces issued and not read yet
+    uint32_t next = n_list ? list[0] : 0;
     auto issue = [&]() {
-        if (ap >= np)
+        if (at_list >= n_list)
             return;
-        const Product p = prods[ap];
         if (lane == 0) {
             tc::mbar_expect_tx(rbar + 8 * aslot, SLOT * 4);
             asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(
                              ring0 + aslot * SLOT * 4),
-                         "l"(reinterpret_cast<uint64_t>(a.maps + ap)), "r"(rbar + 8 * aslot), "r"(0), "r"(p.n0 + ag * 8), "r"(ak >> 5)
+                         "l"(reinterpret_cast<uint64_t>(a.maps + (next & 255u))), "r"(rbar + 8 * aslot), "r"(0), "r"((next >> 8 & 0x3fffu) * 8),
+                         "r"((next >> 22) * (KC / 32))
                          : "memory");
         }
         ahead++;
         aslot = aslot + 1 == slots ? 0 : aslot + 1;
-        ak += KC;
-        if (ak >= p.K) {
-            ak = 0;
-            ag += 8;
-            settle();
-        }
+        if (++at_list < n_list)
+            next = list[at_list];
     };
     // The weights may be read ahead of the kernel before: a launch that overlaps it is only made behind a
     // decoder step of the same call, which writes none.
@@ -286,7 +291,7 @@ __global__ void __launch_bounds__(256, 1) step_kernel(const __grid_constant__ Ar
                 acc[r] = __fadd_rn(acc[r], __shfl_xor_sync(0xffffffffu, acc[r], 16));
             }
             f(n, bv, acc);
-            while (ahead < slots && ap < np)
+            while (ahead < slots && at_list < n_list)
                 issue();
         }
     };
@@ -340,6 +345,9 @@ __global__ void __launch_bounds__(256, 1) step_kernel(const __grid_constant__ Ar
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     stage(0);
+    // attention: 2^alog warps a pair; this warp's first pair
+    const int alog = npair <= 1 ? 3 : (npair == 2 ? 2 : (npair <= 4 ? 1 : 0)), aw = 1 << alog, w = warp & (aw - 1);
+    const int ar0 = (rank + (warp >> alog) * CLUSTER) / H, ah0 = rank + (warp >> alog) * CLUSTER - ar0 * H;
 
     // embedding rows (rows past the last stream stay zero)
     for (int i = tid; i < SP * D; i += 256) {
@@ -376,9 +384,8 @@ __global__ void __launch_bounds__(256, 1) step_kernel(const __grid_constant__ Ar
         __syncthreads();
         // Attention, aw warps a pair (attn_row's operations): the two dot products of 32 keys are two tasks, the
         // first warp takes the softmax, 32 output columns are a warp's.
-        const int aw = npair <= 1 ? 8 : (npair == 2 ? 4 : (npair <= 4 ? 2 : 1)), w = warp % aw;
-        for (int p0 = 0; p0 < npair; p0 += 8 / aw) {
-            const int p = p0 + warp / aw, pair = rank + p * CLUSTER, r = pair / H, h = pair - r * H, b = b0 + r;
+        for (int p0 = 0; p0 < npair; p0 += 8 >> alog) {
+            const int p = p0 + (warp >> alog), pair = rank + p * CLUSTER, r = p0 ? pair / H : ar0, h = p0 ? pair - r * H : ah0, b = b0 + r;
             const bool on = p < npair;
             float *Ks = sm + pl.kv + p * pl.pair, *Vs = Ks + L * pl.ks, *Rs = Vs + L * dk, *br = Rs + P * pl.ks, *ps = br + ((L + 3) & ~3),
                   *pz = ps + ((L + 3) & ~3), *os = pz + ((L + 3) & ~3);
@@ -428,14 +435,14 @@ __global__ void __launch_bounds__(256, 1) step_kernel(const __grid_constant__ Ar
                     const int e = e0 + lane, n4 = min(8, (dk - e0) / 4);
                     if (e < dk) {
                         float acc = 0.0f;
-#pragma unroll 8
+#pragma unroll 16
                         for (int j = jlo; j < jhi; j++)
                             acc = fmaf(ps[j], Vs[j * dk + e], acc);
                         os[e] = fmaf(ps[jhi], vf[e], acc);
                     }
                     __syncwarp();
                     for (int i = lane; i < n4 * CLUSTER; i += 32) {
-                        const int c = i / n4, at = e0 + (i - c * n4) * 4;
+                        const int c = n4 == 8 ? i >> 3 : i / n4, at = e0 + (i - c * n4) * 4;
                         const float4 v = *reinterpret_cast<const float4 *>(os + at);
                         send4(tc::smem_u32(ob + r * HD + h * dk + at), bar0 + 8 * OB, c, v);
                         if (c == 0)
