@@ -421,21 +421,6 @@ __global__ void __launch_bounds__(256) attn_bwd_kernel(AttnArgs a)
     }
 }
 
-// table[h][x] (+)= sum over streams b (ascending) of part[b][h][x]
-__global__ void reduce_streams_kernel(const float *__restrict__ part, int B, size_t per_stream,
-                                      float *__restrict__ out, int accumulate)
-{
-    pdl_trigger();
-    pdl_wait();
-    size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= per_stream)
-        return;
-    float s = 0.0f;
-    for (int b = 0; b < B; b++)
-        s += part[(size_t)b * per_stream + i];
-    out[i] = accumulate ? out[i] + s : s;
-}
-
 static int attn_check_shape(const nncu_attn_shape *s)
 {
     if (!s || s->n_streams < 1 || s->n_head < 1 || s->d_key < 1 || s->seg_len < 1 ||

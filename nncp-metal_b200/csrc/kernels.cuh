@@ -409,44 +409,10 @@ __global__ void splitk_reduce_kernel(const float *__restrict__ ws, int ksplit, s
     }
 }
 
-// Column reduction of partial sums, fixed order: out_k[c] = sum_p part[p*stride + off_k + c].
-// blockIdx.y selects the output k (up to 3); a block owns 32 columns, its 8 warps each sum
-// a contiguous range of parts, and the 8 range sums are added in range order.
-struct ReduceOut {
-    float *out[3];
-    int off[3];
-};
-__global__ void __launch_bounds__(256)
-reduce_cols_kernel(const float *__restrict__ part, int n_parts, int stride, int n, ReduceOut ro)
-{
-    pdl_trigger();
-    pdl_wait();
-    __shared__ float sm[8][33];
-    const int c = blockIdx.x * 32 + (threadIdx.x & 31), grp = threadIdx.x >> 5;
-    const int k = blockIdx.y;
-    const int per = (n_parts + 7) / 8;
-    float s = 0.0f;
-    if (c < n) {
-        const float *src = part + ro.off[k] + c;
-        const int p1 = min(n_parts, (grp + 1) * per);
-        for (int p = grp * per; p < p1; p++)
-            s += src[(size_t)p * stride];
-    }
-    sm[grp][threadIdx.x & 31] = s;
-    __syncthreads();
-    if (grp == 0 && c < n) {
-        float t = 0.0f;
-#pragma unroll
-        for (int w = 0; w < 8; w++)
-            t += sm[w][threadIdx.x];
-        ro.out[k][c] = t;
-    }
-}
-
 // Every column / stream reduction of one layer's backward pass in one launch.  Job kinds:
 //   0  out[c] = sum over parts p of part[p*stride + off + c], the parts dealt to 8 groups of
-//      consecutive parts whose sums are added in group order (reduce_cols_kernel's association)
-//   1  out[i] (+)= sum over parts (streams) in order of part[p*stride + i]   (reduce_streams_kernel)
+//      consecutive parts whose sums are added in group order
+//   1  out[i] (+)= sum over parts (streams) in order of part[p*stride + i]
 // blk0 is the job's first block; a block finds its job by a short scan (the table is a kernel
 // argument, so the launch can sit in a captured graph).
 struct ReduceJob {
@@ -473,6 +439,7 @@ __global__ void __launch_bounds__(256) reduce_jobs_kernel(const __grid_constant_
         const int i = blk * 256 + threadIdx.x;
         if (i < jb.n) {
             float s = 0.0f;
+#pragma unroll 8 // eight parts' loads in flight
             for (int p = 0; p < jb.n_parts; p++)
                 s += jb.part[(size_t)p * jb.stride + i];
             jb.out[i] = jb.accumulate ? jb.out[i] + s : s;
@@ -485,6 +452,7 @@ __global__ void __launch_bounds__(256) reduce_jobs_kernel(const __grid_constant_
     if (c < jb.n) {
         const float *src = jb.part + jb.off + c;
         const int p1 = min(jb.n_parts, (grp + 1) * per);
+#pragma unroll 8
         for (int p = grp * per; p < p1; p++)
             s += src[(size_t)p * jb.stride];
     }

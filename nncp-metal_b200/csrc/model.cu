@@ -2312,10 +2312,7 @@ int nncu_decoder_begin(nncu_model *m, const uint8_t *payload_host, size_t len)
 // turns them into symbols (left in the target rows and, for t+1 < seg_len, the next step's input)
 static int decode_step(nncu_model *m, int t, int limit_t, int limit_b, bool chained)
 {
-    struct Chain { // the launches of a step are one chain on one stream: each may set itself up under the one before
-        Chain() { g_nncu_step_chain = true; }
-        ~Chain() { g_nncu_step_chain = false; }
-    } chain;
+    ChainScope chain; // the launches of a step are one chain on one stream: each may set itself up under the one before
     const int B = m->B, V = m->V, nb = coder_depth(V), P = 1 << nb;
     const bool pow2 = P == V;
     if (m->step_sp) {
@@ -2445,6 +2442,7 @@ int nncu_attention_forward(const nncu_attn_shape *s, const void *q, const void *
     if (!q || !kv || !b_r || !out)
         return nncu_fail(NNCU_ERR_INVALID, "null tensor");
     cudaStream_t st = (cudaStream_t)cuda_stream;
+    ChainScope chain;
     return s->dtype_bf16 ? attn_forward_any<bf16>(s, q, kv, w_r, b_r, out, lse, st)
                          : attn_forward_any<float>(s, q, kv, w_r, b_r, out, lse, st);
 }
@@ -2456,29 +2454,42 @@ int nncu_attention_backward(const nncu_attn_shape *s, const void *q, const void 
     NNCU_TRY(attn_check_shape(s));
     if (!q || !kv || !b_r || !out || !lse || !dout || !dq || !dkv)
         return nncu_fail(NNCU_ERR_INVALID, "null tensor");
+    ChainScope chain; // every kernel of the op waits for its predecessor before it touches memory
     cudaStream_t st = (cudaStream_t)cuda_stream;
     return s->dtype_bf16
                ? attn_backward_any<bf16>(s, q, kv, w_r, b_r, out, lse, dout, dq, dkv, dwr_part, dbr_part, st)
                : attn_backward_any<float>(s, q, kv, w_r, b_r, out, lse, dout, dq, dkv, dwr_part, dbr_part, st);
 }
 
+// both tables' sums over the streams, in stream order, by one launch
+static int reduce_tables(const nncu_attn_shape *s, const float *dwr_part, const float *dbr_part, float *dw_r, float *db_r, int accumulate,
+                         cudaStream_t st)
+{
+    ReduceJobs jobs;
+    memset(&jobs, 0, sizeof(jobs));
+    int blocks = 0;
+    auto add = [&](const float *part, float *out, size_t n) {
+        if (!part || !out)
+            return;
+        ReduceJob &j = jobs.job[jobs.n_jobs++];
+        j.part = part; j.out = out; j.n_parts = s->n_streams; j.stride = j.n = (int)n; j.kind = 1; j.accumulate = accumulate; j.blk0 = blocks;
+        blocks += ceil_div((long long)n, 256);
+    };
+    add(dbr_part, db_r, (size_t)s->n_head * (s->mem_len + s->seg_len));
+    add(dwr_part, dw_r, (size_t)s->n_head * s->d_pos * s->d_key);
+    if (!blocks)
+        return NNCU_OK;
+    launch_k(reduce_jobs_kernel, dim3(blocks), dim3(256), 0, st, jobs);
+    KERNEL_CHECK();
+    return NNCU_OK;
+}
+
 int nncu_attention_reduce_tables(const nncu_attn_shape *s, const float *dwr_part, const float *dbr_part,
                                  float *dw_r, float *db_r, int accumulate, void *cuda_stream)
 {
     NNCU_TRY(attn_check_shape(s));
-    cudaStream_t st = (cudaStream_t)cuda_stream;
-    const int L = s->mem_len + s->seg_len;
-    if (dbr_part && db_r) {
-        size_t n = (size_t)s->n_head * L;
-        launch_k(reduce_streams_kernel, dim3(ceil_div(n, 256)), dim3(256), 0, st, dbr_part, s->n_streams, n, db_r, accumulate);
-        KERNEL_CHECK();
-    }
-    if (dwr_part && dw_r) {
-        size_t n = (size_t)s->n_head * s->d_pos * s->d_key;
-        launch_k(reduce_streams_kernel, dim3(ceil_div(n, 256)), dim3(256), 0, st, dwr_part, s->n_streams, n, dw_r, accumulate);
-        KERNEL_CHECK();
-    }
-    return NNCU_OK;
+    ChainScope chain;
+    return reduce_tables(s, dwr_part, dbr_part, dw_r, db_r, accumulate, (cudaStream_t)cuda_stream);
 }
 
 // ---- attention backward with its scratch inside the library image
@@ -2520,19 +2531,12 @@ int nncu_attention_backward_noalloc(const nncu_attn_shape *s, const void *q, con
     }
     float *dwr_part = w_r ? g_noalloc_ptr[dev] : nullptr;
     float *dbr_part = g_noalloc_ptr[dev] + n_wr;
+    ChainScope chain;
     cudaStream_t st = (cudaStream_t)cuda_stream;
     NNCU_TRY(s->dtype_bf16
                  ? attn_backward_any<bf16>(s, q, kv, w_r, b_r, out, lse, dout, dq, dkv, dwr_part, dbr_part, st)
                  : attn_backward_any<float>(s, q, kv, w_r, b_r, out, lse, dout, dq, dkv, dwr_part, dbr_part, st));
-    const size_t nb = (size_t)s->n_head * L;
-    launch_k(reduce_streams_kernel, dim3(ceil_div(nb, 256)), dim3(256), 0, st, dbr_part, s->n_streams, nb, db_r, 0);
-    KERNEL_CHECK();
-    if (w_r) {
-        const size_t nw = (size_t)s->n_head * s->d_pos * s->d_key;
-        launch_k(reduce_streams_kernel, dim3(ceil_div(nw, 256)), dim3(256), 0, st, dwr_part, s->n_streams, nw, dw_r, 0);
-        KERNEL_CHECK();
-    }
-    return NNCU_OK;
+    return reduce_tables(s, dwr_part, dbr_part, dw_r, db_r, 0, st);
 }
 
 // ---- dense contraction test hooks
