@@ -283,8 +283,7 @@ __global__ void __launch_bounds__(256, DK <= 64 ? 2 : 1) attn_fwd_kernel(const _
     // of this tile: [half][row A, row B][8] maxima, then [row A, row B][32] sums of half 0
     float *mx = reinterpret_cast<float *>(sm + SM::MX) + qt * 6 * 32, *sums = mx + 32;
     uint4 *pfs = reinterpret_cast<uint4 *>(sm + SM::PF) + qt * 4 * 32; // A fragments of the tile's probabilities, [16-key step][lane]
-    pdl_trigger();
-    pdl_wait();
+    pdl_wait(); // no early trigger: successors resident beside these CTAs cost more than their launch (33 % of the op alone)
 
     const bf16 *q = reinterpret_cast<const bf16 *>(a.q) + ((size_t)i0 * a.B + b) * a.qp + h * DK;
     const bf16 *kv = reinterpret_cast<const bf16 *>(a.kv) + (size_t)b * a.kvp + h * DK;
@@ -855,8 +854,7 @@ __global__ void __launch_bounds__(256, DK <= 64 ? 2 : 1) attn_bwd_kernel(const _
     // skew scratch: the warps of key half 0 use their tile's rows of PS (written after both warps of the tile
     // have read their scratch), the others an area of their own
     float *es = hf == 0 ? reinterpret_cast<float *>(PS + qt * 16 * LPS) : reinterpret_cast<float *>(sm + SM::ES) + qt * 16 * ESC;
-    pdl_trigger();
-    pdl_wait();
+    pdl_wait(); // no early trigger: successors resident beside these CTAs cost more than their launch (33 % of the op alone)
 
     const bf16 *kv = reinterpret_cast<const bf16 *>(a.kv) + (size_t)b * a.kvp + h * DK;
     const bf16 *dout = reinterpret_cast<const bf16 *>(a.dout) + (size_t)b * HD + h * DK;

@@ -427,7 +427,6 @@ struct ReduceJobs {
 };
 __global__ void __launch_bounds__(256) reduce_jobs_kernel(const __grid_constant__ ReduceJobs jobs)
 {
-    pdl_trigger();
     pdl_wait();
     __shared__ float sm[8][33];
     int j = 0;
