@@ -22,8 +22,6 @@
 // eight) that meet at the end.  A block in which a row sees nothing changes no bit.  So whole
 // segments and single queries, which go through different kernels, give the same bits.
 #pragma once
-#include <type_traits>
-
 #include "attention.cuh"
 #include "gemm_tc.cuh"
 
@@ -602,12 +600,10 @@ __global__ void __launch_bounds__(128) attn_one_kernel(const __grid_constant__ A
 // The same for head sizes 64 and 128 with tiles that arrive by TMA: 64 rows x 64 columns a copy, 128-byte
 // rows, chunk c of row r at c ^ (r % 8).  The loop above spends most of its instructions on addresses (some 600
 // a block of a warp against 200 of products, on eight warps an SM), and at 128 streams x 8 heads x 576 keys
-// it took 57 us of which HBM needs 23.  W warps, W key blocks a round: three where they need no more rounds
-// than four do, since 72 KB of tiles let three CTAs share an SM (the nine blocks of 576 keys: 3 + 3 + 3
-// instead of 4 + 4 + 1).
-template <int DK, int W> struct OneTmaSmem {
+// it took 57 us of which HBM needs 23.
+template <int DK> struct OneTmaSmem {
     static constexpr int NS = DK / 64, TILE = NS * 8192;
-    static constexpr int K = 0, R = W * TILE, V = 2 * W * TILE, S = 3 * W * TILE, MB = S + W * 64 * 4, BRS = MB + 16;
+    static constexpr int K = 0, R = 4 * TILE, V = 8 * TILE, S = 12 * TILE, MB = S + 4 * 64 * 4, L4 = MB + 16, BRS = L4 + 16;
     static size_t bytes(int L) { return (size_t)BRS + (size_t)L * 4 + 1024; }
 };
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap *map, uint32_t bar, int x, int y, int z)
@@ -629,27 +625,27 @@ __device__ __forceinline__ void ldsm4t_at(uint32_t (&r)[4], uint32_t at)
 // byte offset of 16-byte chunk c of row r in a tile
 __device__ __forceinline__ uint32_t tile_at(int r, int c) { return (uint32_t)((c >> 3) * 8192 + r * 128 + (((c & 7) ^ (r & 7)) << 4)); }
 
-template <int DK, int W>
-__global__ void __launch_bounds__(32 * W) attn_one_tma_kernel(const __grid_constant__ AttnArgs a, const __grid_constant__ CUtensorMap map_kv,
+template <int DK>
+__global__ void __launch_bounds__(128) attn_one_tma_kernel(const __grid_constant__ AttnArgs a, const __grid_constant__ CUtensorMap map_kv,
                                                            const __grid_constant__ CUtensorMap map_r, int stage_br)
 {
-    using SM = OneTmaSmem<DK, W>;
-    constexpr int NS = SM::NS, TILE = SM::TILE, MT = DK / 16, MW = (MT + W - 1) / W; // 16-column slices, and those of one warp
+    using SM = OneTmaSmem<DK>;
+    constexpr int NS = SM::NS, TILE = SM::TILE, MT = DK / 16, MW = MT / 4; // 16-column slices, and those of one warp
     extern __shared__ __align__(16) unsigned char smraw[];
-    __shared__ __align__(8) uint64_t bars[2 * W]; // K and table, V of each warp
+    __shared__ __align__(8) uint64_t bars[8]; // K and table, V of each warp
     __shared__ int abort_s, dummy;
     unsigned char *sm = smraw + ((1024u - (smem_addr(smraw) & 1023u)) & 1023u);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const uint32_t base = smem_addr(sm), Kt = base + SM::K + warp * TILE, Rt = base + SM::R + warp * TILE, Vt = base + SM::V;
-    const uint32_t bar_k = smem_addr(bars + warp), bar_v = smem_addr(bars + W + warp);
-    float *sc = reinterpret_cast<float *>(sm + SM::S), *mbs = reinterpret_cast<float *>(sm + SM::MB); // [W][64] scores, [W] maxima
+    const uint32_t bar_k = smem_addr(bars + warp), bar_v = smem_addr(bars + 4 + warp);
+    float *sc = reinterpret_cast<float *>(sm + SM::S), *mbs = reinterpret_cast<float *>(sm + SM::MB); // [4][64] scores, [4] maxima
     float *brs = reinterpret_cast<float *>(sm + SM::BRS);
     const int b = blockIdx.x / a.H, h = blockIdx.x % a.H, HD = a.H * DK, T = a.T, M = a.M, L = a.L, i = a.t0;
     const Blocks blk = blocks_of(M, L, a.attn_len, i, i + 1);
     pdl_trigger();
     if (threadIdx.x == 0) {
         abort_s = 0;
-        for (int k = 0; k < 2 * W; k++)
+        for (int k = 0; k < 8; k++)
             tc::mbar_init(smem_addr(bars + k), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -700,7 +696,7 @@ __global__ void __launch_bounds__(32 * W) attn_one_tma_kernel(const __grid_const
     fetch_kr(blk.lo + warp);
     fetch_v(blk.lo + warp);
     if (stage_br) // the head's b_r, scaled
-        for (int r = threadIdx.x; r < L; r += 32 * W)
+        for (int r = threadIdx.x; r < L; r += 128)
             brs[r] = __fmul_rn(a.br_scale, a.b_r[(size_t)h * L + r]);
     // the query as the second operand: k = 2t, 2t + 1 (+ 8) of every 16-wide slice, the same for all columns
     uint32_t qf[DK / 16][2];
@@ -720,8 +716,8 @@ __global__ void __launch_bounds__(32 * W) attn_one_tma_kernel(const __grid_const
         for (int c = 0; c < 4; c++)
             o[w][c] = 0.0f;
     uint32_t phase = 0;
-    for (int kb0 = blk.lo; kb0 <= blk.hi; kb0 += W, phase ^= 1) {
-        const int kb = kb0 + warp, j0 = kb * KB, nb = min(W, blk.hi - kb0 + 1);
+    for (int kb0 = blk.lo; kb0 <= blk.hi; kb0 += 4, phase ^= 1) {
+        const int kb = kb0 + warp, j0 = kb * KB, nb = min(4, blk.hi - kb0 + 1);
         if (kb <= blk.hi) {
             tc::mbar_wait(bar_k, phase, &abort_s, ef, 44); // K and the table rows
             __syncwarp();
@@ -756,7 +752,7 @@ __global__ void __launch_bounds__(32 * W) attn_one_tma_kernel(const __grid_const
             if (lane == 0)
                 mbs[warp] = mb;
             __syncwarp();
-            fetch_kr(kb + W);
+            fetch_kr(kb + 4);
             tc::mbar_wait(bar_v, phase, &abort_s, ef, 45);
         }
         __syncthreads(); // scores, maxima and V of the round are there for everyone
@@ -775,9 +771,7 @@ __global__ void __launch_bounds__(32 * W) attn_one_tma_kernel(const __grid_const
             l = __fmaf_rn(l, scale, sum);
 #pragma unroll
             for (int w = 0; w < MW; w++) {
-                const int m = warp + W * w;
-                if (MT % W != 0 && m >= MT)
-                    break;
+                const int m = warp + 4 * w;
 #pragma unroll
                 for (int c = 0; c < 4; c++)
                     o[w][c] = __fmul_rn(o[w][c], scale);
@@ -790,7 +784,7 @@ __global__ void __launch_bounds__(32 * W) attn_one_tma_kernel(const __grid_const
             }
         }
         __syncthreads(); // the round has been read
-        fetch_v(kb + W);
+        fetch_v(kb + 4);
     }
     l = __fadd_rn(l, __shfl_xor_sync(0xffffffffu, l, 1));
     l = __fadd_rn(l, __shfl_xor_sync(0xffffffffu, l, 2));
@@ -798,8 +792,8 @@ __global__ void __launch_bounds__(32 * W) attn_one_tma_kernel(const __grid_const
     bf16 *out = reinterpret_cast<bf16 *>(a.o) + ((size_t)i * a.B + b) * HD + h * DK;
 #pragma unroll
     for (int w = 0; w < MW; w++) {
-        const int m = warp + W * w;
-        if (t == 0 && (MT % W == 0 || m < MT)) {
+        const int m = warp + 4 * w;
+        if (t == 0) {
             out[m * 16 + g] = __float2bfloat16_rn(__fmul_rn(o[w][0], inv));
             out[m * 16 + g + 8] = __float2bfloat16_rn(__fmul_rn(o[w][2], inv));
         }
@@ -1200,18 +1194,9 @@ template <int DK> static int forward_one(const AttnArgs &a, cudaStream_t st)
         r = kv;
         if (a.w_r16)
             NNCU_TRY(tile_map(a.w_r16, {DK, P, H}, {DK * 2, P * DK * 2}, false, &r));
-        const Blocks blk = blocks_of(a.M, a.L, a.attn_len, a.t0, a.t1);
-        const int n = blk.hi - blk.lo + 1;
-        auto go = [&](auto w) {
-            constexpr int W = decltype(w)::value;
-            const size_t most = 226 * 1024, all = OneTmaSmem<DK, W>::bytes(a.L);
-            launch_k(attn_one_tma_kernel<DK, W>, dim3(a.B * a.H), dim3(32 * W), all <= most ? all : OneTmaSmem<DK, W>::bytes(0), st, a, kv, r,
-                     all <= most ? 1 : 0);
-        };
-        if ((n + 2) / 3 == (n + 3) / 4)
-            go(std::integral_constant<int, 3>());
-        else
-            go(std::integral_constant<int, 4>());
+        const size_t most = 226 * 1024, all = OneTmaSmem<DK>::bytes(a.L);
+        launch_k(attn_one_tma_kernel<DK>, dim3(a.B * a.H), dim3(128), all <= most ? all : OneTmaSmem<DK>::bytes(0), st, a, kv, r,
+                 all <= most ? 1 : 0);
     }
     KERNEL_CHECK();
     return NNCU_OK;
@@ -1224,8 +1209,7 @@ template <int DK> static int forward_dk(const AttnArgs &a, cudaStream_t st)
         if constexpr (DK < 64) {
             CUDA_TRY(cudaFuncSetAttribute(attn_one_kernel<DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
         } else {
-            CUDA_TRY(cudaFuncSetAttribute(attn_one_tma_kernel<DK, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
-            CUDA_TRY(cudaFuncSetAttribute(attn_one_tma_kernel<DK, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
+            CUDA_TRY(cudaFuncSetAttribute(attn_one_tma_kernel<DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
         }
         attr_done = true;
     }
