@@ -1010,8 +1010,8 @@ __global__ void first_rows_kernel(const int32_t *__restrict__ ids, int rows, int
 }
 
 // blockIdx.y selects 256 columns, two of them a thread's.  A frequent symbol's sum is a chain of rows, bound
-// by how many of their loads are in flight (32) and by the list; four columns a thread and 16 rows,
-// one column range after the other, took 52 us for 2048 rows of 1024.
+// by how many of their loads are in flight and by the list; four columns a thread, one range of 512 columns
+// after the other, took 52 us for 2048 rows of 1024.
 template <typename T>
 __global__ void __launch_bounds__(128)
 embed_grad_kernel(const int32_t *__restrict__ ids, const T *__restrict__ dx, float *__restrict__ g,
@@ -1019,7 +1019,7 @@ embed_grad_kernel(const int32_t *__restrict__ ids, const T *__restrict__ dx, flo
 {
     pdl_trigger();
     pdl_wait();
-    constexpr int SPAN = 2048, FLIGHT = 32; // rows listed per pass, rows loaded together
+    constexpr int SPAN = 2048, FLIGHT = 16; // rows listed per pass, rows loaded together
     __shared__ int list[SPAN];
     __shared__ int wcnt[2][4]; // per-warp hit counts of a chunk, double-buffered by chunk parity
     const int r0 = blockIdx.x, c0 = blockIdx.y * 256 + threadIdx.x;
@@ -1070,12 +1070,11 @@ embed_grad_kernel(const int32_t *__restrict__ ids, const T *__restrict__ dx, flo
         for (int k0 = 0; k0 < n; k0 += FLIGHT) {
             float x[FLIGHT][2];
 #pragma unroll
-            for (int u = 0; u < FLIGHT; u++)
-                if (k0 + u < n) {
-                    const T *src = dx + (size_t)list[k0 + u] * D + c0;
-                    x[u][0] = in0 ? to_f(src[0]) : 0.0f;
-                    x[u][1] = in1 ? to_f(src[128]) : 0.0f;
-                }
+            for (int u = 0; u < FLIGHT; u++) {
+                const T *src = dx + (size_t)list[min(k0 + u, n - 1)] * D + c0;
+                x[u][0] = in0 ? to_f(src[0]) : 0.0f;
+                x[u][1] = in1 ? to_f(src[128]) : 0.0f;
+            }
 #pragma unroll
             for (int u = 0; u < FLIGHT; u++)
                 if (k0 + u < n) {
