@@ -109,7 +109,10 @@ decode_step_kernel(const uint16_t *__restrict__ trees, const uint8_t *__restrict
         // prob0 is in hand, and its children's (one 32-bit word) are on their way, before the branch at it is
         // known; (range * prob0) >> 15 is the high word of (range << 8) * (prob0 << 9), range staying below
         // 2^24; renormalisation shifts by 0, 8 or 16 (two bytes always suffice: range is at least 1) and draws
-        // on the next eight payload bytes in two registers, topped up after every second bit if need be.
+        // on the next eight payload bytes in two registers.  A branch costs some 15 cycles of this chain (50 a
+        // bit without any, 76 with two every second bit), so four bits go between two looks at the payload;
+        // that is enough unless they draw more than the 32 bits that are certain to be there, and then they are
+        // walked again two at a time.
         uint32_t low = state->low, range = state->range, used = 0, hi, lo, drawn; // drawn: bits taken from hi : lo
         const uint32_t *words = reinterpret_cast<const uint32_t *>(win);
         auto top_up = [&]() { // the eight window bytes from `used` on (zero past the payload's end)
@@ -130,6 +133,7 @@ decode_step_kernel(const uint16_t *__restrict__ trees, const uint8_t *__restrict
         };
         int slot = ring - 1, in_slot = G; // the slot in use and the trees of it that have been walked
         uint32_t phase = 1;
+        bool ready = false; // the next slot's copy was seen complete before the present slot's last tree
         for (int b = 0; b < B; b++) {
             int c = 0;
             if (b < n_act && ok) {
@@ -141,12 +145,20 @@ decode_step_kernel(const uint16_t *__restrict__ trees, const uint8_t *__restrict
                         slot = 0;
                         phase ^= 1;
                     }
-                    ok = tc::mbar_wait(tc::smem_u32(bars + slot), phase, &abort_s, err_flag, 41);
+                    ok = ready || tc::mbar_wait(tc::smem_u32(bars + slot), phase, &abort_s, err_flag, 41);
                     walked += ok ? 1 : 0;
                 }
                 if (ok) {
                     const uint32_t *pairs = reinterpret_cast<const uint32_t *>(slots + ((size_t)slot * G + in_slot) * P);
-                    in_slot++;
+                    if (++in_slot == G) { // asked here, needed behind the walk
+                        const bool wrap = slot + 1 == ring;
+                        uint32_t done_next;
+                        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                                     : "=r"(done_next)
+                                     : "r"(tc::smem_u32(bars + (wrap ? 0 : slot + 1))), "r"(phase ^ (wrap ? 1u : 0u))
+                                     : "memory");
+                        ready = done_next != 0;
+                    }
                     uint32_t k = 1, p9 = (pairs[0] >> 16) << 9, kids = pairs[1];
                     auto next_bit = [&]() { // get_bit at node k: the branch taken, the decoder's state advanced
                         const uint32_t split = __umulhi(range << 8, p9);
@@ -165,6 +177,24 @@ decode_step_kernel(const uint16_t *__restrict__ trees, const uint8_t *__restrict
                         drawn += s;
                         return bit;
                     };
+                    auto four = [&](auto step) {
+                        const uint32_t low0 = low, range0 = range, hi0 = hi, lo0 = lo, drawn0 = drawn, k0 = k, p0 = p9, kids0 = kids;
+                        step(next_bit(), 0);
+                        step(next_bit(), 1);
+                        step(next_bit(), 2);
+                        step(next_bit(), 3);
+                        if (drawn > 32) {
+                            if (drawn > 64) { // not seen in practice: four symbols' worth of improbable branches
+                                low = low0; range = range0; hi = hi0; lo = lo0; drawn = drawn0; k = k0; p9 = p0; kids = kids0;
+                                step(next_bit(), 0);
+                                step(next_bit(), 1);
+                                check();
+                                step(next_bit(), 2);
+                                step(next_bit(), 3);
+                            }
+                            check();
+                        }
+                    };
                     if constexpr (ANY) { // every node above the last level is split, one of the last if it has two symbols
                         int first = 0, n = V;
                         auto down = [&](bool bit) {
@@ -172,24 +202,36 @@ decode_step_kernel(const uint16_t *__restrict__ trees, const uint8_t *__restrict
                             first = bit ? first + h : first;
                             n = bit ? n - h : h;
                         };
-                        int lvl = 1;
-                        for (; lvl + 1 < nb; lvl += 2) {
-                            down(next_bit());
+                        int lvl = 1, first0 = 0, n0 = V;
+                        for (; lvl + 3 < nb; lvl += 4) {
+                            first0 = first;
+                            n0 = n;
+                            four([&](bool bit, int i) {
+                                if (i == 0) { // also where the four are walked again
+                                    first = first0;
+                                    n = n0;
+                                }
+                                down(bit);
+                            });
+                        }
+                        for (; lvl < nb; lvl++) {
                             down(next_bit());
                             check();
                         }
-                        if (lvl < nb)
+                        if (n > 1) {
                             down(next_bit());
-                        if (n > 1)
-                            down(next_bit());
-                        check();
+                            check();
+                        }
                         c = first;
                     } else {
                         int lvl = 0;
-                        for (; lvl + 1 < nb; lvl += 2) {
+                        for (; lvl + 3 < nb; lvl += 4)
+                            four([](bool, int) {});
+                        if (lvl + 1 < nb) {
                             next_bit();
                             next_bit();
                             check();
+                            lvl += 2;
                         }
                         if (lvl < nb) {
                             next_bit();

@@ -122,3 +122,34 @@ def test_one_launch_steps_equal_whole_segment_bitwise(pkg, kw):
             m.update()
         assert seg.weights_hash() == one.weights_hash()
     seg.close(); one.close()
+
+
+@pytest.mark.parametrize("V", [16, 256, 300, 16384])
+def test_decoder_walk_of_improbable_branches(pkg, V):
+    """Trees of nearly certain branches and payloads that keep taking the others (two payload bytes a bit), over the
+    end of the payload: the device's symbols against the host's walk of the same trees."""
+    p = pkg.abi.make_params(n_layer=1, d_model=64, n_head=2, d_key=32, d_inner=64, d_pos=8, mem_len=8, seg_len=4, n_streams=7,
+                            n_symbols=V, init_range=0.05)
+    T, B, L = 4, 7, pkg.host.library()
+    rng = np.random.default_rng(V)
+    bias = np.zeros(V, np.float32)
+    bias[rng.integers(0, V, max(2, V // 8))] = 25.0
+    for payload in (b"\xff" * 900, b"\x00" * 900, b"\x00\xff\xfe" * 300, bytes(rng.integers(0, 2, 900, dtype=np.uint8) * 255), b"\xff" * 40):
+        dev, ref = pkg.TrfModel(p), pkg.TrfModel(p)
+        for m in (dev, ref):
+            m.set_param("out_bias", bias)
+            m.reset()
+        dev.decoder_begin(payload)
+        got = dev.decode_steps(0, T, np.zeros(B, np.int32))
+        buf = C.create_string_buffer(payload, len(payload))
+        hd, ids, want = L.nch_dec_new(buf, len(payload)), np.zeros((T, B), np.int32), np.zeros((T, B), np.int32)
+        for t in range(T):
+            ids[t] = want[t - 1] if t else 0
+            ref.eval(t, ids, read=False)
+            trees = np.ascontiguousarray(ref.coder_trees(t, 1))
+            for b in range(B):
+                want[t, b] = L.nch_read_sym_tree(hd, trees[b].ctypes.data_as(C.c_void_p), V)
+        L.nch_dec_free(hd)
+        assert np.array_equal(got, want)
+        dev.decoder_end()
+        dev.close(); ref.close()
