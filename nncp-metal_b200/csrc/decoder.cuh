@@ -15,6 +15,8 @@
 // sends n >> 1 left): the walk then carries the node's range beside its heap index and ends when
 // one symbol is left (template argument ANY); a tree row has P = 2^ceil(log2 V) entries.
 #pragma once
+#include <type_traits>
+
 #include "common.cuh"
 #include "gemm_tc.cuh"
 
@@ -55,7 +57,7 @@ inline size_t smem_bytes(int B, int P, int nb, int ring) { return (size_t)ring *
 // trees: [B][P] prob0 in heap order (entry 0 unused), P = 2^nb >= V.  sym_out[b] and ids_next[b]
 // (when not null) receive the decoded symbol, 0 for the streams past the end of the block: those at
 // step `t` are b >= limit_b when t == limit_t, and all of them when t > limit_t.
-template <bool ANY>
+template <bool ANY, int NB>
 __global__ void __launch_bounds__(64)
 decode_step_kernel(const uint16_t *__restrict__ trees, const uint8_t *__restrict__ payload, State *state,
                    int32_t *__restrict__ sym_out, int32_t *__restrict__ ids_next, int t, int limit_t, int limit_b,
@@ -109,10 +111,10 @@ decode_step_kernel(const uint16_t *__restrict__ trees, const uint8_t *__restrict
         // prob0 is in hand, and its children's (one 32-bit word) are on their way, before the branch at it is
         // known; (range * prob0) >> 15 is the high word of (range << 8) * (prob0 << 9), range staying below
         // 2^24; renormalisation shifts by 0, 8 or 16 (two bytes always suffice: range is at least 1) and draws
-        // on the next eight payload bytes in two registers.  A branch costs some 15 cycles of this chain (50 a
-        // bit without any, 76 with two every second bit), so four bits go between two looks at the payload;
-        // that is enough unless they draw more than the 32 bits that are certain to be there, and then they are
-        // walked again two at a time.
+        // on the next eight payload bytes in two registers.  A branch costs some 15 cycles of this chain (53 a bit
+        // without any, 76 with two every second bit), so up to eight bits go between two looks at the
+        // payload: enough unless they draw more than the 32 bits that are certain to be there, and then they are
+        // walked again one at a time.
         uint32_t low = state->low, range = state->range, used = 0, hi, lo, drawn; // drawn: bits taken from hi : lo
         const uint32_t *words = reinterpret_cast<const uint32_t *>(win);
         auto top_up = [&]() { // the eight window bytes from `used` on (zero past the payload's end)
@@ -134,116 +136,113 @@ decode_step_kernel(const uint16_t *__restrict__ trees, const uint8_t *__restrict
         int slot = ring - 1, in_slot = G; // the slot in use and the trees of it that have been walked
         uint32_t phase = 1;
         bool ready = false; // the next slot's copy was seen complete before the present slot's last tree
-        for (int b = 0; b < B; b++) {
-            int c = 0;
-            if (b < n_act && ok) {
-                if (in_slot == G) {
-                    if (b > 0)
-                        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc::smem_u32(done + slot)) : "memory");
-                    in_slot = 0;
-                    if (++slot == ring) {
-                        slot = 0;
-                        phase ^= 1;
-                    }
-                    ok = ready || tc::mbar_wait(tc::smem_u32(bars + slot), phase, &abort_s, err_flag, 41);
-                    walked += ok ? 1 : 0;
+        int32_t *const next_in = ids_next ? ids_next : sym_out;
+        int b = 0;
+        for (; b < n_act; b++) {
+            if (in_slot == G) {
+                if (b > 0)
+                    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc::smem_u32(done + slot)) : "memory");
+                in_slot = 0;
+                slot = slot + 1 == ring ? 0 : slot + 1;
+                phase ^= slot == 0 ? 1u : 0u;
+                if (!ready && !tc::mbar_wait(tc::smem_u32(bars + slot), phase, &abort_s, err_flag, 41)) {
+                    ok = false;
+                    break;
                 }
-                if (ok) {
-                    const uint32_t *pairs = reinterpret_cast<const uint32_t *>(slots + ((size_t)slot * G + in_slot) * P);
-                    if (++in_slot == G) { // asked here, needed behind the walk
-                        const bool wrap = slot + 1 == ring;
-                        uint32_t done_next;
-                        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                                     : "=r"(done_next)
-                                     : "r"(tc::smem_u32(bars + (wrap ? 0 : slot + 1))), "r"(phase ^ (wrap ? 1u : 0u))
-                                     : "memory");
-                        ready = done_next != 0;
-                    }
-                    uint32_t k = 1, p9 = (pairs[0] >> 16) << 9, kids = pairs[1];
-                    auto next_bit = [&]() { // get_bit at node k: the branch taken, the decoder's state advanced
-                        const uint32_t split = __umulhi(range << 8, p9);
-                        const bool bit = low >= split;
-                        k = 2 * k + (bit ? 1u : 0u);
-                        const uint32_t p1 = (kids >> 16) << 9, p0 = (kids & 0xffffu) << 9;
-                        p9 = bit ? p1 : p0;
-                        kids = pairs[min(k, last)];
-                        low = bit ? low - split : low;
-                        range = bit ? range - split : split;
-                        const uint32_t s = range < R_LOW ? (range < 0x100u ? 16u : 8u) : 0u;
-                        range <<= s;
-                        low = __funnelshift_l(hi, low, s);
-                        hi = __funnelshift_l(lo, hi, s);
-                        lo <<= s;
-                        drawn += s;
-                        return bit;
-                    };
-                    auto four = [&](auto step) {
-                        const uint32_t low0 = low, range0 = range, hi0 = hi, lo0 = lo, drawn0 = drawn, k0 = k, p0 = p9, kids0 = kids;
-                        step(next_bit(), 0);
-                        step(next_bit(), 1);
-                        step(next_bit(), 2);
-                        step(next_bit(), 3);
-                        if (drawn > 32) {
-                            if (drawn > 64) { // not seen in practice: four symbols' worth of improbable branches
-                                low = low0; range = range0; hi = hi0; lo = lo0; drawn = drawn0; k = k0; p9 = p0; kids = kids0;
-                                step(next_bit(), 0);
-                                step(next_bit(), 1);
-                                check();
-                                step(next_bit(), 2);
-                                step(next_bit(), 3);
-                            }
-                            check();
-                        }
-                    };
-                    if constexpr (ANY) { // every node above the last level is split, one of the last if it has two symbols
-                        int first = 0, n = V;
-                        auto down = [&](bool bit) {
-                            const int h = n >> 1;
-                            first = bit ? first + h : first;
-                            n = bit ? n - h : h;
-                        };
-                        int lvl = 1, first0 = 0, n0 = V;
-                        for (; lvl + 3 < nb; lvl += 4) {
-                            first0 = first;
-                            n0 = n;
-                            four([&](bool bit, int i) {
-                                if (i == 0) { // also where the four are walked again
-                                    first = first0;
-                                    n = n0;
-                                }
-                                down(bit);
-                            });
-                        }
-                        for (; lvl < nb; lvl++) {
-                            down(next_bit());
-                            check();
-                        }
-                        if (n > 1) {
-                            down(next_bit());
-                            check();
-                        }
-                        c = first;
-                    } else {
-                        int lvl = 0;
-                        for (; lvl + 3 < nb; lvl += 4)
-                            four([](bool, int) {});
-                        if (lvl + 1 < nb) {
-                            next_bit();
-                            next_bit();
-                            check();
-                            lvl += 2;
-                        }
-                        if (lvl < nb) {
-                            next_bit();
-                            check();
-                        }
-                        c = (int)k - V;
-                    }
-                }
+                walked++;
             }
+            const uint32_t *pairs = reinterpret_cast<const uint32_t *>(slots + ((size_t)slot * G + in_slot) * P);
+            if (++in_slot == G) { // asked here, needed behind the walk
+                const bool wrap = slot + 1 == ring;
+                uint32_t done_next;
+                asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                             : "=r"(done_next)
+                             : "r"(tc::smem_u32(bars + (wrap ? 0 : slot + 1))), "r"(phase ^ (wrap ? 1u : 0u))
+                             : "memory");
+                ready = done_next != 0;
+            }
+            uint32_t k = 1, p9 = (pairs[0] >> 16) << 9, kids = pairs[1];
+            auto next_bit = [&]() { // get_bit at node k: the branch taken, the decoder's state advanced
+                const uint32_t split = __umulhi(range << 8, p9);
+                const bool bit = low >= split;
+                k = 2 * k + (bit ? 1u : 0u);
+                const uint32_t p1 = (kids >> 16) << 9, p0 = (kids & 0xffffu) << 9;
+                p9 = bit ? p1 : p0;
+                kids = pairs[min(k, last)];
+                low = bit ? low - split : low;
+                range = bit ? range - split : split;
+                const uint32_t s = range < R_LOW ? (range < 0x100u ? 16u : 8u) : 0u;
+                range <<= s;
+                low = __funnelshift_l(hi, low, s);
+                hi = __funnelshift_l(lo, hi, s);
+                lo <<= s;
+                drawn += s;
+                return bit;
+            };
+            auto run = [&](auto count, auto step) { // `count` bits, step(bit, index); an index 0 starts over
+                constexpr int N = decltype(count)::value;
+                const uint32_t low0 = low, range0 = range, hi0 = hi, lo0 = lo, drawn0 = drawn, k0 = k, p0 = p9, kids0 = kids;
+#pragma unroll
+                for (int i = 0; i < N; i++)
+                    step(next_bit(), i);
+                if (drawn > 32) {
+                    if (drawn > 64) { // a run of improbable branches
+                        low = low0; range = range0; hi = hi0; lo = lo0; drawn = drawn0; k = k0; p9 = p0; kids = kids0;
+#pragma unroll 1
+                        for (int i = 0; i < N; i++) {
+                            step(next_bit(), i);
+                            check();
+                        }
+                    }
+                    check();
+                }
+            };
+            int c;
+            if constexpr (ANY) { // every node above the last level is split, one of the last if it has two symbols
+                int first = 0, n = V, first0 = 0, n0 = V;
+                auto down = [&](bool bit) {
+                    const int h = n >> 1;
+                    first = bit ? first + h : first;
+                    n = bit ? n - h : h;
+                };
+                int lvl = 1;
+                for (; lvl + 3 < nb; lvl += 4) {
+                    first0 = first;
+                    n0 = n;
+                    run(std::integral_constant<int, 4>(), [&](bool bit, int i) {
+                        if (i == 0) {
+                            first = first0;
+                            n = n0;
+                        }
+                        down(bit);
+                    });
+                }
+                for (; lvl < nb; lvl++) {
+                    down(next_bit());
+                    check();
+                }
+                if (n > 1) {
+                    down(next_bit());
+                    check();
+                }
+                c = first;
+            } else {
+                auto nothing = [](bool, int) {};
+                constexpr int HALF = (NB + 1) / 2; // up to eight bits at once, else two halves
+                if constexpr (NB <= 8) {
+                    run(std::integral_constant<int, NB>(), nothing);
+                } else {
+                    run(std::integral_constant<int, HALF>(), nothing);
+                    run(std::integral_constant<int, NB - HALF>(), nothing);
+                }
+                c = (int)k - V;
+            }
+            next_in[b] = c;
             sym_out[b] = c;
-            if (ids_next)
-                ids_next[b] = c;
+        }
+        for (; b < B; b++) { // past the end of the block
+            next_in[b] = 0;
+            sym_out[b] = 0;
         }
         used += drawn >> 3;
         state->pos = min(pos0 + used, len);
@@ -256,6 +255,28 @@ decode_step_kernel(const uint16_t *__restrict__ trees, const uint8_t *__restrict
     if (tid == 0 && !ok) // copies still in flight land in this CTA's shared memory: each gets a bounded chance to finish
         for (int g = walked; g < issued_s; g++)
             tc::mbar_wait(tc::smem_u32(bars + g % ring), (uint32_t)((g / ring) & 1), &abort_s, err_flag, 42);
+}
+
+typedef void (*StepKernel)(const uint16_t *, const uint8_t *, State *, int32_t *, int32_t *, int, int, int, int, int, int, int, int, int *);
+// the kernel for trees of depth nb
+inline StepKernel step_kernel_of(bool pow2, int nb)
+{
+    if (!pow2)
+        return decode_step_kernel<true, 0>;
+    switch (nb) {
+    case 3: return decode_step_kernel<false, 3>;
+    case 4: return decode_step_kernel<false, 4>;
+    case 5: return decode_step_kernel<false, 5>;
+    case 6: return decode_step_kernel<false, 6>;
+    case 7: return decode_step_kernel<false, 7>;
+    case 8: return decode_step_kernel<false, 8>;
+    case 9: return decode_step_kernel<false, 9>;
+    case 10: return decode_step_kernel<false, 10>;
+    case 11: return decode_step_kernel<false, 11>;
+    case 12: return decode_step_kernel<false, 12>;
+    case 13: return decode_step_kernel<false, 13>;
+    default: return decode_step_kernel<false, 14>; // the tree kernels' shared memory ends here
+    }
 }
 
 } // namespace dec

@@ -2299,7 +2299,7 @@ int nncu_decoder_begin(nncu_model *m, const uint8_t *payload_host, size_t len)
     s0.range = dec::R_TOP;
     CUDA_TRY(cudaMemcpyAsync(m->dec_state, &s0, sizeof(s0), cudaMemcpyHostToDevice, m->st));
     CUDA_TRY(cudaStreamSynchronize(m->st));
-    CUDA_TRY(cudaFuncSetAttribute(pow2 ? dec::decode_step_kernel<false> : dec::decode_step_kernel<true>,
+    CUDA_TRY(cudaFuncSetAttribute(dec::step_kernel_of(pow2, nb),
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dec::smem_bytes(m->B, P, nb, ring)));
     m->dec_ring = ring;
     m->dec_open = true;
@@ -2327,7 +2327,7 @@ static int decode_step(nncu_model *m, int t, int limit_t, int limit_b, bool chai
                      (const float *)(m->probs + (size_t)t * B * V), m->coder_dev, V, P);
         KERNEL_CHECK();
     }
-    launch_k(pow2 ? dec::decode_step_kernel<false> : dec::decode_step_kernel<true>, dim3(1), dim3(64),
+    launch_k(dec::step_kernel_of(pow2, nb), dim3(1), dim3(64),
              dec::smem_bytes(B, P, nb, m->dec_ring), m->st, (const uint16_t *)m->coder_dev,
              (const uint8_t *)m->dec_payload, m->dec_state, m->tgt_dev + (size_t)t * B,
              t + 1 < m->T ? m->ids_dev + (size_t)(t + 1) * B : (int32_t *)nullptr, t, limit_t, limit_b, B, V, P, nb,
