@@ -9,7 +9,7 @@
 // can run ahead is the data movement: a second warp fills a ring of shared-memory slots with the next
 // streams' trees by bulk copies (2 V bytes each, completion on an mbarrier) while the current one is
 // walked, and the payload bytes the step can consume at most (two per bit) are staged in shared memory
-// up front.  128 streams of 14 bits: 156 us with one load of prob0 behind every decision.
+// up front.  128 streams of 14 bits: 156 us with one load of prob0 behind every decision, 95 now.
 //
 // An alphabet that is not a power of two has the uneven tree of write_sym (a node of n symbols
 // sends n >> 1 left): the walk then carries the node's range beside its heap index and ends when

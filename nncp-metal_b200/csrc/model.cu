@@ -1,7 +1,8 @@
 // model.cu -- the Transformer-XL train step behind the C ABI of include/nncu.h.
 //
 // Host-side orchestration only; every number is produced by the kernels in
-// gemm_simt.cuh, gemm_tc.cuh, attention.cuh, attention_fa.cuh, kernels.cuh and coder.cuh.
+// gemm_simt.cuh, gemm_tc.cuh, gemm_tc2.cuh, attention.cuh, attention_fa.cuh, kernels.cuh, coder.cuh,
+// decoder.cuh and step_fp32.cuh.
 //
 //   forward_range    trf_eval            nncp.c:581-1029
 //   backward         trf_eval_gradient   nncp.c:1099-1193 (hand-derived adjoint)
