@@ -187,8 +187,11 @@ struct nncu_model {
     void *xlast, *xf, *pool[4], *dz, *dh, *dhp, *dof, *dqkv, *tA, *tB;
     float *st_f, *probs, *dwr_part, *dbr_part, *part, *logp, *loss_dev;
     size_t part_floats = 0; // floats per region of `part`
-    float *skw = nullptr;   // split-K workspace [SPLITK][TB][D] (models with n_symbols >= SPLITK_MIN_K)
-    size_t skw_floats = 0;
+    // Split-K workspaces: skw for products on the main stream (the output head's dX), skw_side for weight
+    // gradients, which run on the side stream beside them.  Two regions, because nothing orders the head's
+    // dX, queued on the main stream, behind the head's weight gradient, queued on the side stream before it.
+    float *skw = nullptr, *skw_side = nullptr;
+    size_t skw_floats = 0, skw_side_floats = 0;
     int part_idx = 0;       // regions handed out since the last join
     ReduceJobs rjobs;       // column / stream reductions queued since the last flush (one launch per layer)
     int rjob_blocks = 0;
@@ -378,14 +381,14 @@ static int mm_tn(nncu_model *m, int Nout, int Kin, int R, const bf16 *dY, long l
         // over the idle pairs; the parts are added in order.  1536 x 512 x 73728: 176 us with one CTA per
         // 128 x 64 tile, 12 tiles of 256 x 256 on 74 pairs in six parts 78.
         const int tiles = tc2::tile_count(Nout, Kin, 256, x), parts = tiles ? tc2::PAIRS / tiles : 1;
-        if (R >= 8192 && parts >= 2 && Nout % 256 == 0 && Kin % 4 == 0 && m->skw) {
+        if (R >= 8192 && parts >= 2 && Nout % 256 == 0 && Kin % 4 == 0) {
             x.ksplit = std::min(parts, 8);
             const size_t n = (size_t)Nout * Kin;
-            if (n * x.ksplit <= m->skw_floats) {
-                NNCU_TRY((tc2::launch<256, float, true, true>(st, Nout, Kin, R, dY, ldy, X, ldx, m->skw, Kin, nullptr, nullptr, m->err_flag,
+            if (n * x.ksplit <= m->skw_side_floats) {
+                NNCU_TRY((tc2::launch<256, float, true, true>(st, Nout, Kin, R, dY, ldy, X, ldx, m->skw_side, Kin, nullptr, nullptr, m->err_flag,
                                                               1 << 30, x)));
-                launch_k(splitk_reduce_kernel<float>, dim3((unsigned)ceil_div((long long)(n / 4), 256)), dim3(256), 0, st, m->skw, x.ksplit, n,
-                         Gout);
+                launch_k(splitk_reduce_kernel<float>, dim3((unsigned)ceil_div((long long)(n / 4), 256)), dim3(256), 0, st, m->skw_side, x.ksplit,
+                         n, Gout);
                 KERNEL_CHECK();
                 return NNCU_OK;
             }
@@ -1458,9 +1461,11 @@ int nncu_create(const nncu_params *p, nncu_model **out)
     part_floats = std::max(part_floats, (size_t)ceil_div(TB, ACT_BWD_ROWS) * F1);
     size_t oPart = take(part_floats * 4 * PART_SLOTS);
     m->part_floats = part_floats;
-    // split-K workspace: the output head's dX (SPLITK parts) and the projections' weight gradients (up to 8)
+    // split-K workspaces: the output head's dX (SPLITK parts) and, for contractions of 8192 rows and more, the
+    // weight gradients (up to 8 parts of the projection's; the others split where their parts fit)
     const size_t skw_floats = !m->use_tc ? 0 : std::max(V >= SPLITK_MIN_K ? (size_t)SPLITK * TB * D : 0, LB >= 8192 ? (size_t)8 * 3 * HD * D : 0);
-    size_t oSkw = take(skw_floats * 4 + 256);
+    const size_t skw_side_floats = LB >= 8192 ? skw_floats : 0;
+    size_t oSkw = take(skw_floats * 4 + 256), oSkwSide = take(skw_side_floats * 4 + 256);
     size_t oLogp = take((size_t)TB * 4), oLoss = take(256);
     size_t oIds = take((size_t)TB * 4), oTgt = take((size_t)TB * 4), oErr = take(256), oHash = take(256);
     size_t oTgtFixed = take((size_t)TB * 4), oFirst = take((size_t)V * 4), oSym = take((size_t)TB * 4);
@@ -1508,6 +1513,8 @@ int nncu_create(const nncu_params *p, nncu_model **out)
     m->dwr_part = (float *)(A + oWr); m->dbr_part = (float *)(A + oBr); m->part = (float *)(A + oPart);
     m->skw = skw_floats ? (float *)(A + oSkw) : nullptr;
     m->skw_floats = skw_floats;
+    m->skw_side = skw_side_floats ? (float *)(A + oSkwSide) : nullptr;
+    m->skw_side_floats = skw_side_floats;
     m->logp = (float *)(A + oLogp); m->loss_dev = (float *)(A + oLoss);
     m->hyper_dev = m->loss_dev + 8;
     m->ids_dev = (int32_t *)(A + oIds); m->tgt_dev = (int32_t *)(A + oTgt);
