@@ -798,6 +798,46 @@ template <typename T> __device__ __forceinline__ void softmax_row(float *zr, int
     }
 }
 
+// Rows whose sum softmax_rows_reg_kernel takes, in an order of its own: whoever computes such a row alone
+// keeps to that order, so that a symbol step has the bits of the whole segment.
+__host__ __device__ inline bool softmax_by_fours(int V) { return V % 1024 == 0 && V <= 16384; }
+
+// one row as softmax_rows_reg_kernel computes it (four neighbouring logits at a time), in place
+template <typename T> __device__ __forceinline__ void softmax_row_by_fours(float *zr, int V, T *d, float scale, float *red)
+{
+    float4 *z4 = reinterpret_cast<float4 *>(zr);
+    float mx = -INFINITY;
+    for (int i = threadIdx.x; i < V / 4; i += 256) {
+        const float4 v = z4[i];
+        mx = fmaxf(mx, fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w)));
+    }
+    mx = block_max_256(mx, red);
+    float s = 0.0f;
+    for (int i = threadIdx.x; i < V / 4; i += 256) {
+        float4 v = z4[i];
+        v.x = expf(v.x - mx);
+        v.y = expf(v.y - mx);
+        v.z = expf(v.z - mx);
+        v.w = expf(v.w - mx);
+        z4[i] = v;
+        s += (v.x + v.y) + (v.z + v.w);
+    }
+    s = block_sum_256(s, red);
+    const float rs = 1.0f / s;
+    for (int i = threadIdx.x; i < V / 4; i += 256) {
+        float4 v = z4[i];
+        v.x *= rs;
+        v.y *= rs;
+        v.z *= rs;
+        v.w *= rs;
+        z4[i] = v;
+        d[4 * i] = from_f<T>(v.x * scale);
+        d[4 * i + 1] = from_f<T>(v.y * scale);
+        d[4 * i + 2] = from_f<T>(v.z * scale);
+        d[4 * i + 3] = from_f<T>(v.w * scale);
+    }
+}
+
 // in-place softmax over the V symbols of each row of fp32 logits (nc_soft_max, nncp.c:1008).
 // The output kernel of the forward pass: besides the probabilities it leaves dz = p * scale, the
 // gradient of the loss with respect to the logits of every symbol but the target (which

@@ -755,7 +755,7 @@ static int forward_range(nncu_model *m, int t0, int t1)
     // the output kernel: probabilities for the coder, and p / (T * B) for the backward pass
     AT *dzr = reinterpret_cast<AT *>(m->dz) + (size_t)r0 * V;
     const float sc = 1.0f / ((float)m->T * (float)m->Bt);
-    if (V % 1024 == 0 && V <= 16384)
+    if (softmax_by_fours(V))
         launch_k(softmax_rows_reg_kernel<AT>, dim3(nr), dim3(256), 0, m->st, pr, nr, V, dzr, sc, m->dz_fixed);
     else
         launch_k(softmax_rows_kernel<AT>, dim3(nr), dim3(256), 0, m->st, pr, nr, V, dzr, sc, m->dz_fixed);

@@ -523,7 +523,12 @@ __global__ void __launch_bounds__(256, 1) step_kernel(const __grid_constant__ Ar
     if (rank < nb) {
         await(bar0 + 8 * LG, 0, &abort_s, a.err_flag);
         const size_t pr = (size_t)(row0 + rank) * V;
-        softmax_row(lg, V, a.dz + pr, a.scale, red);
+        if (softmax_by_fours(V)) {
+            softmax_row_by_fours(lg, V, a.dz + pr, a.scale, red);
+            __syncthreads(); // the copy below reads it column by column
+        } else {
+            softmax_row(lg, V, a.dz + pr, a.scale, red);
+        }
         for (int i = tid; i < V; i += 256)
             a.probs[pr + i] = lg[i];
         __syncthreads();

@@ -1,0 +1,74 @@
+"""Shapes at which paths that share or outgrow a resource meet: workspaces of two streams, associations of
+two kernels for one row, CTAs without a share of the work."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from conftest import rel_err
+
+pytestmark = pytest.mark.gpu
+
+
+def test_split_head_gradients_beside_each_other(pkg, monkeypatch):
+    """8192 symbols, d_model 256, 128 streams x 64: the head's weight gradient (side stream) and its dX (main
+    stream) are both split over the contraction.  The gradients are the other engine's, the same every time,
+    and those of a model without a side stream bit for bit."""
+    kw = dict(n_layer=1, d_model=256, n_head=4, d_key=64, d_inner=256, d_pos=80, mem_len=16, seg_len=64, n_streams=128,
+              n_symbols=8192, use_bf16=1, init_range=0.05)
+    rng = np.random.default_rng(5)
+    ids, tg = (rng.integers(0, 8192, (64, 128)).astype(np.int32) for _ in range(2))
+    got = []
+    for backend, no_overlap, times in ((2, "0", 6), (2, "1", 1), (1, "0", 1)):
+        monkeypatch.setenv("NNCU_NO_OVERLAP", no_overlap)
+        m = pkg.TrfModel(pkg.abi.make_params(gemm_backend=backend, **kw))
+        m.reset()
+        for _ in range(times):
+            m.eval(-1, ids, read=False)
+            m.eval_gradient(tg)
+            got.append({n: m.get_grad(n) for n in m.info})
+        m.close()
+    first, other = got[0], got[-1]
+    for g in got[1:-1]:
+        for n in first:
+            assert np.array_equal(g[n], first[n]), n
+    for n in first:  # bf16 operands of both engines, fp32 sums: as in the other comparisons of engines
+        assert rel_err(first[n], other[n]) < 2e-2, n
+
+
+@pytest.mark.parametrize("V,D", [(1024, 64), (3072, 96), (4096, 32)])
+def test_one_launch_steps_of_wide_alphabets_equal_whole_segment_bitwise(pkg, V, D):
+    """fp32 models whose alphabet is a multiple of 1024: whole segments take the softmax that keeps a row in
+    registers, and the one-launch step the same sums in the same order; so the symbols coded from a whole
+    segment's probabilities come back."""
+    p = pkg.abi.make_params(n_layer=2, d_model=D, n_head=2, d_key=16, d_inner=128, d_pos=12, mem_len=9, seg_len=6, n_streams=3,
+                            n_symbols=V, use_bf16=0, init_range=0.5)
+    T, B, L = 6, 3, pkg.host.library()
+    rng = np.random.default_rng(V)
+    seg, one = pkg.TrfModel(p), pkg.TrfModel(p)
+    seg.reset(); one.reset()
+    ids, tg = (rng.integers(0, V, (T, B)).astype(np.int32) for _ in range(2))
+    ids[1:] = tg[:-1]
+    a = seg.eval(-1, ids)
+    b = np.concatenate([one.eval(t, ids) for t in range(T)])
+    assert np.array_equal(a, b)
+    for m in (seg, one):
+        m.eval_gradient(tg)
+        m.update()
+    assert seg.weights_hash() == one.weights_hash()
+    one.eval_end()
+    # the next segment: coded from whole-segment probabilities, decoded step by step
+    ids[0] = tg[-1]
+    tg = rng.integers(0, V, (T, B)).astype(np.int32)
+    ids[1:] = tg[:-1]
+    seg.eval(-1, ids, read=False)
+    paths = seg.coder_paths(0, T, tg)
+    enc, data = L.nch_enc_new(), C.c_void_p()
+    L.nch_write_sym_paths_any(enc, paths.ctypes.data_as(C.c_void_p), V, tg.ctypes.data_as(C.c_void_p), T * B)
+    n = L.nch_enc_finish(enc, C.byref(data))
+    payload = C.string_at(data.value, n)
+    L.nch_enc_free(enc)
+    one.decoder_begin(payload)
+    assert np.array_equal(one.decode_steps(0, T, np.ascontiguousarray(ids[0])), tg)
+    one.decoder_end()
+    seg.close(); one.close()
