@@ -15,7 +15,8 @@
 //     both ends of the launch.
 //   - Norms are computed by every CTA for itself: cheaper than another exchange.
 // Buffers need no second copy: whoever writes a buffer again has, through the exchanges between,
-// heard from every CTA of the cluster since it last read it.
+// heard from every CTA of the cluster since it last read it.  That takes a share for every CTA in two
+// of the products (step_deal.h); models too narrow for it pay a cluster-wide barrier behind each norm.
 //
 // Same bits as the launches it replaces: a dot product is the four chains of gemm_simt.cuh, one thread
 // each; attention, norm, softmax and tree rows are the device functions of those kernels.  Every value
@@ -28,6 +29,7 @@
 #include "gemm_simt.cuh"
 #include "gemm_tc.cuh"
 #include "kernels.cuh"
+#include "step_deal.h"
 
 namespace stepf {
 
@@ -48,14 +50,10 @@ struct Args {
     float emul, br_scale, inv_sqrt, scale;
 };
 
-constexpr int CLUSTER = 8;                   // CTAs that share a group of streams
 constexpr int MAXD = 512;                    // row length that the norms' registers hold
 constexpr int MAX_CLUSTERS = 14;             // clusters that are on the chip together (fifteen were, of 16)
 constexpr int KC = 256, SLOT = 8 * KC;       // columns of a weight piece, floats of a ring slot
 constexpr int MAX_SLOTS = 4;                 // ring slots per warp
-
-// columns of an N-wide output per CTA, whole groups of eight
-__host__ __device__ inline int per_cta(int N) { return ((N + CLUSTER - 1) / CLUSTER + 7) & ~7; }
 
 // weight pieces of a warp for N output columns, at most
 __host__ __device__ inline int pieces_of(int N, int K) { return (per_cta(N) / 8 + 7) / 8 * ((K + KC - 1) / KC); }
@@ -149,6 +147,7 @@ __global__ void __launch_bounds__(256, 1) step_kernel(const __grid_constant__ Ar
     const uint32_t bar0 = tc::smem_u32(bars), rbar = bar0 + 8 * (6 + warp * MAX_SLOTS), ring0 = tc::smem_u32(ring);
     const int npair = (nb * H + CLUSTER - 1 - rank) / CLUSTER; // (stream, head) pairs of this CTA: rank, rank + CLUSTER, ...
     const int V4 = (V + 3) & ~3;
+    const bool ordered = exchanges_order_reuse(HD, F);
     auto expect = [&](int bar) { // bytes that an exchange brings to this CTA
         return (uint32_t)(bar == QKV ? npair * 3 * dk * 4 : bar == OB ? nb * HD * 4 : bar == HA ? nb * F * 4 : bar == LG ? (rank < nb ? V4 * 4 : 0) : nb * D * 4);
     };
@@ -165,11 +164,11 @@ __global__ void __launch_bounds__(256, 1) step_kernel(const __grid_constant__ Ar
     if (tid == 32) {
         int turn = 0;
         for (int i = 0; i < np; i++) {
-            const int j = i & 3, N = i == np - 1 ? V : (j == 0 ? 3 * HD : (j == 2 ? F : D)), per = per_cta(N);
+            const int j = i & 3, N = i == np - 1 ? V : (j == 0 ? 3 * HD : (j == 2 ? F : D));
             Product p;
             p.K = i == np - 1 ? D : (j == 1 ? HD : (j == 3 ? F : D));
-            p.n0 = min(N, rank * per);
-            p.groups = (min(N, p.n0 + per) - p.n0 + 7) >> 3;
+            p.n0 = deal_from(N, rank);
+            p.groups = (deal_from(N, rank + 1) - p.n0 + 7) >> 3;
             p.turn = turn;
             turn = (turn + p.groups) & 7;
             prods[i] = p;
@@ -482,6 +481,10 @@ __global__ void __launch_bounds__(256, 1) step_kernel(const __grid_constant__ Ar
                 row_store<float, 4, 4>(out + r * D, lane, D, v);
             }
             __syncthreads();
+            if (!ordered) {
+                cluster_arrive();
+                cluster_wait();
+            }
         };
         landed(OB, l);
         product(4 * l + 1, ob, nullptr, 0, [&](int n, float4, const float(&acc)[SP]) { to_all(tmp, D, T1, n, gather(acc), D); });

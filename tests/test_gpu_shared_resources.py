@@ -72,3 +72,22 @@ def test_one_launch_steps_of_wide_alphabets_equal_whole_segment_bitwise(pkg, V, 
     assert np.array_equal(one.decode_steps(0, T, np.ascontiguousarray(ids[0])), tg)
     one.decoder_end()
     seg.close(); one.close()
+
+
+@pytest.mark.parametrize("D,H,dk,F,B", [(16, 1, 16, 16, 3), (48, 12, 4, 16, 40), (112, 7, 16, 112, 5), (64, 1, 16, 64, 9), (96, 3, 32, 208, 1),
+                                        (64, 4, 16, 48, 17)])
+def test_one_launch_steps_of_narrow_models_equal_whole_segment_bitwise(pkg, D, H, dk, F, B):
+    """Products too narrow to give every CTA of a cluster a share, and ones that only just do."""
+    p = pkg.abi.make_params(n_layer=3, d_model=D, n_head=H, d_key=dk, d_inner=F, d_pos=14, mem_len=9, seg_len=6, n_streams=B, n_symbols=72,
+                            use_bf16=0, init_range=0.4, lr=1e-3)
+    rng = np.random.default_rng(D + F)
+    seg, one = pkg.TrfModel(p), pkg.TrfModel(p)
+    seg.reset(); one.reset()
+    for _ in range(4):
+        ids, tg = (rng.integers(0, 72, (6, B)).astype(np.int32) for _ in range(2))
+        assert np.array_equal(seg.eval(-1, ids), np.concatenate([one.eval(t, ids) for t in range(6)]))
+        for m in (seg, one):
+            m.eval_gradient(tg)
+            m.update()
+        assert seg.weights_hash() == one.weights_hash()
+    seg.close(); one.close()
