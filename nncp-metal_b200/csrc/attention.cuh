@@ -493,7 +493,8 @@ static int attn_forward_t(const nncu_attn_shape *s, const void *q, const void *k
     a.smem_pitch = fwd_pitch<T>(a, w_r != nullptr, smem);
     if (smem > 227 * 1024)
         return nncu_fail(NNCU_ERR_RANGE, "attention forward: %zu bytes of shared memory needed", smem);
-    CUDA_TRY(cudaFuncSetAttribute(attn_fwd_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    static DeviceOnce once;
+    NNCU_TRY(smem_limit(once, attn_fwd_kernel<T>, SMEM_MOST));
     launch_k(attn_fwd_kernel<T>, dim3(a.B * a.H, chunks), dim3(256), smem, st, a);
     KERNEL_CHECK();
     return NNCU_OK;
@@ -515,7 +516,8 @@ static int attn_backward_t(const nncu_attn_shape *s, const void *q, const void *
     if (smem > 227 * 1024)
         return nncu_fail(NNCU_ERR_RANGE, "attention backward: %zu bytes of shared memory needed", smem);
     auto kernel = a.dk % 4 == 0 ? attn_bwd_kernel<T, 4> : attn_bwd_kernel<T, 1>;
-    CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    static DeviceOnce once[2];
+    NNCU_TRY(smem_limit(once[a.dk % 4 == 0 ? 0 : 1], kernel, SMEM_MOST));
     launch_k(kernel, dim3(a.B * a.H), dim3(256), smem, st, a);
     KERNEL_CHECK();
     return NNCU_OK;

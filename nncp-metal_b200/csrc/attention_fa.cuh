@@ -1185,7 +1185,9 @@ inline int tile_map(const void *p, const cuuint64_t (&dims)[3], const cuuint64_t
 }
 template <int DK> static int forward_one(const AttnArgs &a, cudaStream_t st)
 {
+    static DeviceOnce once;
     if constexpr (DK < 64) {
+        NNCU_TRY(smem_limit(once, attn_one_kernel<DK>, OneSmem<DK>::TOTAL));
         launch_k(attn_one_kernel<DK>, dim3(a.B * a.H), dim3(128), OneSmem<DK>::TOTAL, st, a);
     } else {
         CUtensorMap kv, r;
@@ -1194,6 +1196,7 @@ template <int DK> static int forward_one(const AttnArgs &a, cudaStream_t st)
         r = kv;
         if (a.w_r16)
             NNCU_TRY(tile_map(a.w_r16, {DK, P, H}, {DK * 2, P * DK * 2}, false, &r));
+        NNCU_TRY(smem_limit(once, attn_one_tma_kernel<DK>, 226 * 1024)); // its barriers are static
         const size_t most = 226 * 1024, all = OneTmaSmem<DK>::bytes(a.L);
         launch_k(attn_one_tma_kernel<DK>, dim3(a.B * a.H), dim3(128), all <= most ? all : OneTmaSmem<DK>::bytes(0), st, a, kv, r,
                  all <= most ? 1 : 0);
@@ -1203,29 +1206,18 @@ template <int DK> static int forward_one(const AttnArgs &a, cudaStream_t st)
 }
 template <int DK> static int forward_dk(const AttnArgs &a, cudaStream_t st)
 {
-    static bool attr_done = false;
-    if (!attr_done) {
-        CUDA_TRY(cudaFuncSetAttribute(attn_fwd_kernel<DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-        if constexpr (DK < 64) {
-            CUDA_TRY(cudaFuncSetAttribute(attn_one_kernel<DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-        } else {
-            CUDA_TRY(cudaFuncSetAttribute(attn_one_tma_kernel<DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
-        }
-        attr_done = true;
-    }
     if (a.t1 - a.t0 == 1)
         return forward_one<DK>(a, st);
+    static DeviceOnce once;
+    NNCU_TRY(smem_limit(once, attn_fwd_kernel<DK>, SMEM_MOST));
     launch_k(attn_fwd_kernel<DK>, dim3(a.B * a.H, (a.t1 - (a.t0 & ~63) + 63) / 64), dim3(256), FwdSmem<DK>::bytes(a.L), st, a);
     KERNEL_CHECK();
     return NNCU_OK;
 }
 template <int DK> static int backward_dk(const AttnArgs &a, cudaStream_t st)
 {
-    static bool attr_done = false;
-    if (!attr_done) {
-        CUDA_TRY(cudaFuncSetAttribute(attn_bwd_kernel<DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-        attr_done = true;
-    }
+    static DeviceOnce once;
+    NNCU_TRY(smem_limit(once, attn_bwd_kernel<DK>, SMEM_MOST));
     launch_k(attn_bwd_kernel<DK>, dim3(a.B * a.H), dim3(256), BwdSmem<DK>::bytes(a.L), st, a);
     KERNEL_CHECK();
     return NNCU_OK;

@@ -149,6 +149,8 @@ coder_paths_fast_kernel(const float *__restrict__ probs, const int32_t *__restri
     }
 }
 
+constexpr int CODER_SMEM = 200 * 1024; // the tree kernels' shared memory ends here
+
 // Threads of a tree block: a row's tree is a division a node and two passes of log2 P barriers, bound by
 // the divisions for large alphabets (16384 symbols, 128 rows on 128 SMs: 42 us with 256 threads) and by
 // the barriers for small ones.

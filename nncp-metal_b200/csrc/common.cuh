@@ -6,6 +6,7 @@
 #include <stdio.h>
 #include <stdlib.h>
 
+#include "device_once.h"
 #include "nncu.h"
 
 typedef __nv_bfloat16 bf16;
@@ -29,6 +30,20 @@ int nncu_fail(int code, const char *fmt, ...);
         if (rc_ != NNCU_OK)  \
             return rc_;      \
     } while (0)
+
+constexpr int SMEM_MOST = 227 * 1024; // shared memory a block can have
+
+// Lets a kernel take up to `bytes` of dynamic shared memory on the current device; `once` is the kernel's own.
+// The limit is the most that any shape asks for, so models of different shapes do not lower one another's.
+template <typename K> static int smem_limit(DeviceOnce &once, K kernel, int bytes)
+{
+    int dev = -1;
+    CUDA_TRY(cudaGetDevice(&dev));
+    return once.run(dev, [&]() -> int {
+        CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+        return NNCU_OK;
+    });
+}
 
 // Programmatic dependent launch.  A kernel started through launch_k may begin while the kernel
 // before it on the stream is still draining: its CTAs become resident, run whatever comes before

@@ -231,12 +231,8 @@ static int launch(cudaStream_t st, int M, int N, int K, const TA *A, long lda, c
                   const float *bias, const TC *addsrc, int bias_n)
 {
     constexpr size_t smem = smem_bytes<BM, BN, MODE != GEMM_TN, MODE == GEMM_NT>();
-    static bool attr_done = false;
-    if (!attr_done) {
-        CUDA_TRY(cudaFuncSetAttribute(gemm_simt_kernel<BM, BN, TM, TN, MODE, TA, TB, TC>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        attr_done = true;
-    }
+    static DeviceOnce once;
+    NNCU_TRY(smem_limit(once, gemm_simt_kernel<BM, BN, TM, TN, MODE, TA, TB, TC>, (int)smem));
     const int vec_a = (reinterpret_cast<uintptr_t>(A) & 15) == 0 && lda % 4 == 0;
     const int vec_b = (reinterpret_cast<uintptr_t>(B) & 15) == 0 && ldb % 4 == 0;
     launch_k(gemm_simt_kernel<BM, BN, TM, TN, MODE, TA, TB, TC>, dim3(ceil_div(N, BN), ceil_div(M, BM)), dim3(256), smem, st,

@@ -709,12 +709,8 @@ static int launch(cudaStream_t st, int M, int N, int K, const bf16 *A, long lda,
     const int staged = ((reinterpret_cast<uintptr_t>(C) & 15) == 0 && (ldc * sizeof(TC)) % 16 == 0) ? 1 : 0;
     if (staged)
         NNCU_TRY(make_tmap(C, (long)M * ksplit, N, ldc, 32, &mc, 128 / (int)sizeof(TC), (int)sizeof(TC)));
-    static bool attr_done = false;
-    if (!attr_done) {
-        CUDA_TRY(cudaFuncSetAttribute(gemm_tc_kernel<BN, TC, AMN, BMN>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, SL::TOTAL));
-        attr_done = true;
-    }
+    static DeviceOnce once;
+    NNCU_TRY(smem_limit(once, gemm_tc_kernel<BN, TC, AMN, BMN>, SL::TOTAL));
     dim3 grid(ceil_div(N, BN), ceil_div(M, BM), ksplit);
     GemmProfiler *pr = g_nncu_prof;
     const bool timed = pr && pr->n < GemmProfiler::MAX_EV;

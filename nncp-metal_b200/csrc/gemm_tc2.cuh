@@ -476,11 +476,8 @@ static int launch(cudaStream_t st, int M, int N, int K, const bf16 *A, long lda,
     mc2 = mc;
     if (x.C2)
         NNCU_TRY(tc::make_tmap(x.C2, M, N, ldc, 32, &mc2, 128 / (int)sizeof(TC), (int)sizeof(TC)));
-    static bool attr_done = false;
-    if (!attr_done) {
-        CUDA_TRY(cudaFuncSetAttribute(gemm_pair_kernel<BN, TC, AMN, BMN>, cudaFuncAttributeMaxDynamicSharedMemorySize, SL::TOTAL));
-        attr_done = true;
-    }
+    static DeviceOnce once;
+    NNCU_TRY(smem_limit(once, gemm_pair_kernel<BN, TC, AMN, BMN>, SL::TOTAL));
     Shape sh;
     sh.M = M; sh.N = N; sh.K = K;
     sh.hole_m = x.hole_m; sh.hole_n = x.hole_n; sh.skip_m = x.skip_m; sh.skip_k = x.skip_k;

@@ -1602,20 +1602,16 @@ int nncu_create(const nncu_params *p, nncu_model **out)
         if (cudaMemcpy(m->step_layers[0], rows.data(), sizeof(stepf::Layer) * rows.size(), cudaMemcpyHostToDevice) != cudaSuccess)
             return fail_cleanup(nncu_fail(NNCU_ERR_CUDA, "layer table upload failed"));
     }
-    if ((size_t)8 * 3 * D * 4 > 48 * 1024) {
-        cudaFuncSetAttribute(norm_bwd_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * 3 * D * 4);
-        cudaFuncSetAttribute(norm_bwd_kernel<bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * 3 * D * 4);
-    }
-    if ((size_t)2 * V * 4 > 48 * 1024 && (size_t)2 * V * 4 <= 200 * 1024) {
-        cudaFuncSetAttribute(coder_paths_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * V * 4);
-        cudaFuncSetAttribute(coder_trees_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * V * 4);
-    }
     {
-        const size_t heap_bytes = ((size_t)2 << coder_depth(V)) * 4; // the any-alphabet kernels: 2 * 2^ceil(log2 V) floats
-        if (heap_bytes > 48 * 1024 && heap_bytes <= 200 * 1024) {
-            cudaFuncSetAttribute(coder_paths_any_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)heap_bytes);
-            cudaFuncSetAttribute(coder_trees_any_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)heap_bytes);
-        }
+        static DeviceOnce norm_f, norm_b, paths, trees, paths_any, trees_any;
+        int rc = smem_limit(norm_f, norm_bwd_kernel<float>, SMEM_MOST);
+        rc = rc ? rc : smem_limit(norm_b, norm_bwd_kernel<bf16>, SMEM_MOST);
+        rc = rc ? rc : smem_limit(paths, coder_paths_kernel, CODER_SMEM);
+        rc = rc ? rc : smem_limit(trees, coder_trees_kernel, CODER_SMEM);
+        rc = rc ? rc : smem_limit(paths_any, coder_paths_any_kernel, CODER_SMEM);
+        rc = rc ? rc : smem_limit(trees_any, coder_trees_any_kernel, CODER_SMEM);
+        if (rc != NNCU_OK)
+            return fail_cleanup(rc);
     }
 
     // ---- initial values (trf_init, nncp.c:341-497); what is not named stays zero
@@ -2154,7 +2150,7 @@ static int coder_paths_enqueue(nncu_model *m, int t0, int nt, const int32_t *sym
     const int nb = coder_depth(m->V), P = 1 << nb;
     if (m->V < 2)
         return nncu_fail(NNCU_ERR_INVALID, "coder-ready output needs at least two symbols");
-    if ((size_t)2 * P * 4 > 200 * 1024)
+    if ((size_t)2 * P * 4 > CODER_SMEM)
         return nncu_fail(NNCU_ERR_RANGE, "n_symbols %d is beyond the limit of the coder kernels (16384; 25600 for a power of two)", m->V);
     CUDA_TRY(cudaSetDevice(m->device));
     int rows = nt * m->B;
@@ -2223,7 +2219,7 @@ int nncu_coder_trees(nncu_model *m, int t0, int nt, uint16_t *tree_host)
     const int P = 1 << coder_depth(m->V);
     if (m->V < 2)
         return nncu_fail(NNCU_ERR_INVALID, "coder-ready output needs at least two symbols");
-    if ((size_t)2 * P * 4 > 200 * 1024)
+    if ((size_t)2 * P * 4 > CODER_SMEM)
         return nncu_fail(NNCU_ERR_RANGE, "n_symbols %d is beyond the limit of the coder kernels (16384; 25600 for a power of two)", m->V);
     CUDA_TRY(cudaSetDevice(m->device));
     int rows = nt * m->B;
@@ -2272,7 +2268,7 @@ int nncu_decoder_begin(nncu_model *m, const uint8_t *payload_host, size_t len)
     const bool pow2 = coder_bits(m->V) >= 1;
     const int nb = coder_depth(m->V), P = 1 << nb; // a tree row has P entries (P = V for a power of two)
     const int ring = dec::ring_slots(m->B, P, nb);
-    if (ring < 2 || (size_t)2 * P * 4 > 200 * 1024)
+    if (ring < 2 || (size_t)2 * P * 4 > CODER_SMEM)
         return nncu_fail(NNCU_ERR_RANGE, "n_symbols %d with %d streams does not fit the decoder's shared memory", m->V, m->B);
     CUDA_TRY(cudaSetDevice(m->device));
     CUDA_TRY(cudaStreamSynchronize(m->st));
@@ -2307,8 +2303,8 @@ int nncu_decoder_begin(nncu_model *m, const uint8_t *payload_host, size_t len)
     s0.range = dec::R_TOP;
     CUDA_TRY(cudaMemcpyAsync(m->dec_state, &s0, sizeof(s0), cudaMemcpyHostToDevice, m->st));
     CUDA_TRY(cudaStreamSynchronize(m->st));
-    CUDA_TRY(cudaFuncSetAttribute(dec::step_kernel_of(pow2, nb),
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dec::smem_bytes(m->B, P, nb, ring)));
+    static DeviceOnce once[16]; // per tree depth, 15: any alphabet
+    NNCU_TRY(smem_limit(once[pow2 ? nb : 15], dec::step_kernel_of(pow2, nb), dec::MAX_SMEM));
     m->dec_ring = ring;
     m->dec_open = true;
     if (m->step_graphs.empty())

@@ -54,6 +54,7 @@ constexpr int MAXD = 512;                    // row length that the norms' regis
 constexpr int MAX_CLUSTERS = 14;             // clusters that are on the chip together (fifteen were, of 16)
 constexpr int KC = 256, SLOT = 8 * KC;       // columns of a weight piece, floats of a ring slot
 constexpr int MAX_SLOTS = 4;                 // ring slots per warp
+constexpr int MAX_SMEM = 220 * 1024;         // of the plan
 
 // weight pieces of a warp for N output columns, at most
 __host__ __device__ inline int pieces_of(int N, int K) { return (per_cta(N) / 8 + 7) / 8 * ((K + KC - 1) / KC); }
@@ -573,7 +574,7 @@ inline int piece_map(const float *W, int N, int K, CUtensorMap *out)
 inline int ring_slots(int sp, int nl, int D, int H, int dk, int F, int L, int P, int V, int tree)
 {
     for (int s = MAX_SLOTS; s >= 2; s--)
-        if ((size_t)plan_of(sp, nl, D, H, dk, F, L, P, V, tree, s).total * 4 <= 220 * 1024)
+        if (plan_of(sp, nl, D, H, dk, F, L, P, V, tree, s).total * 4 <= MAX_SMEM)
             return s;
     return 0;
 }
@@ -581,7 +582,8 @@ inline int ring_slots(int sp, int nl, int D, int H, int dk, int F, int L, int P,
 template <int SP> static int launch_sp(cudaStream_t st, const Args &a, int t, bool chained)
 {
     const Plan pl = plan_of(SP, a.nl, a.D, a.H, a.dk, a.F, a.M + a.T, a.P, a.V, 1 << a.depth, a.slots);
-    CUDA_TRY(cudaFuncSetAttribute(step_kernel<SP>, cudaFuncAttributeMaxDynamicSharedMemorySize, pl.total * 4));
+    static DeviceOnce once;
+    NNCU_TRY(smem_limit(once, step_kernel<SP>, MAX_SMEM));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(CLUSTER * ceil_div(a.B, SP)));
     cfg.blockDim = dim3(256);

@@ -91,3 +91,45 @@ def test_one_launch_steps_of_narrow_models_equal_whole_segment_bitwise(pkg, D, H
             m.update()
         assert seg.weights_hash() == one.weights_hash()
     seg.close(); one.close()
+
+
+def test_models_of_other_shapes_leave_a_models_launches_alone(pkg):
+    """Shared-memory limits are the kernels', not the models': a smaller model made later, on the same
+    device, must not lower them.  Coder trees, two open decoders, one-launch steps."""
+    def model(V, B, F=64):
+        m = pkg.TrfModel(pkg.abi.make_params(n_layer=1, d_model=64, n_head=2, d_key=32, d_inner=F, d_pos=8, mem_len=8, seg_len=4,
+                                             n_streams=B, n_symbols=V, use_bf16=0, init_range=0.05))
+        m.reset()
+        return m
+
+    big, small = model(16384, 2), model(8192, 2)
+    ids = np.zeros((4, 2), np.int32)
+    big.eval(-1, ids, read=False)
+    big.coder_trees(0, 1)
+    big.close(); small.close()
+    big, small = model(4096, 50, 512), model(4096, 2)
+    big.decoder_begin(b"\x55" * 9000)
+    small.decoder_begin(b"\x55" * 900)
+    for m, B in ((big, 50), (small, 2), (big, 50)):
+        m.decode_steps(0, 2, np.zeros(B, np.int32))
+        m.eval_end()
+    big.close(); small.close()
+
+
+def test_two_devices_of_one_process(pkg):
+    """fp32 and bf16 models on a second device after the first."""
+    torch = pytest.importorskip("torch")
+    if torch.cuda.device_count() < 2:
+        pytest.skip("needs two devices")
+    kw = dict(n_layer=1, d_model=64, n_head=2, d_key=32, d_inner=64, d_pos=8, mem_len=8, seg_len=4, n_streams=2, n_symbols=256)
+    ids = np.zeros((4, 2), np.int32)
+    for bf16 in (0, 1):
+        probs = []
+        for device in (0, 1):
+            m = pkg.TrfModel(pkg.abi.make_params(use_bf16=bf16, device=device, **kw))
+            m.reset()
+            probs.append(m.eval(-1, ids))
+            m.eval_gradient(ids)
+            m.synchronize()
+            m.close()
+        assert np.array_equal(*probs)
