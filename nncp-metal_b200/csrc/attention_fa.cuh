@@ -683,6 +683,7 @@ __global__ void __launch_bounds__(128) attn_one_tma_kernel(const __grid_constant
                 }
                 *reinterpret_cast<uint4 *>(sm + SM::R + warp * TILE + tile_at(r, c)) = v;
             }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); // a later round's tile may come by TMA to the same place
         }
     };
     auto fetch_v = [&](int kb) {

@@ -133,3 +133,20 @@ def test_two_devices_of_one_process(pkg):
             m.synchronize()
             m.close()
         assert np.array_equal(*probs)
+
+
+@pytest.mark.parametrize("dk", [64, 128])
+def test_query_kernel_table_tiles_by_hand_and_by_copy(pkg, dk):
+    """A table that ends inside the left pad: the one-query kernel writes a warp's first tiles of it by
+    ordinary stores and has the later ones copied to the same place; every step is the segment's, bit for bit."""
+    p = pkg.abi.make_params(n_layer=2, d_model=2 * dk, n_head=2, d_key=dk, d_inner=128, d_pos=200, mem_len=500, seg_len=8, n_streams=5,
+                            n_symbols=256, use_bf16=1, init_range=0.3)
+    rng = np.random.default_rng(dk)
+    seg, one = pkg.TrfModel(p), pkg.TrfModel(p)
+    seg.reset(); one.reset()
+    for _ in range(2):
+        ids = rng.integers(0, 256, (8, 5)).astype(np.int32)
+        assert np.array_equal(seg.eval(-1, ids), np.concatenate([one.eval(t, ids) for t in range(8)]))
+        for m in (seg, one):
+            m.memory_shift()
+    seg.close(); one.close()
