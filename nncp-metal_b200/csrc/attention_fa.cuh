@@ -652,13 +652,14 @@ __global__ void __launch_bounds__(128) attn_one_tma_kernel(const __grid_constant
     __syncthreads();
     pdl_wait();
     int *ef = a.err_flag ? a.err_flag : &dummy;
+    bool ok = true; // this lane's waits: after one that ran out it issues no copy and waits no more
     auto fetch_kr = [&](int kb) { // this warp's block of a round
         if (kb > blk.hi)
             return;
         const int j0 = kb * KB, x0 = j0 - i + a.P - M - 1;
         // rows below the table stand for row 0, and a table in fp32 has to be rounded: such tiles are loaded by hand
         const bool by_hand = a.w_r && (!a.w_r16 || x0 < 0);
-        if (lane == 0) {
+        if (lane == 0 && ok) {
             const bool r = a.w_r && !by_hand;
             tc::mbar_expect_tx(bar_k, (uint32_t)(r ? 2 * TILE : TILE));
 #pragma unroll
@@ -687,7 +688,7 @@ __global__ void __launch_bounds__(128) attn_one_tma_kernel(const __grid_constant
         }
     };
     auto fetch_v = [&](int kb) {
-        if (kb > blk.hi || lane != 0)
+        if (kb > blk.hi || lane != 0 || !ok)
             return;
         tc::mbar_expect_tx(bar_v, (uint32_t)TILE);
 #pragma unroll
@@ -720,7 +721,7 @@ __global__ void __launch_bounds__(128) attn_one_tma_kernel(const __grid_constant
     for (int kb0 = blk.lo; kb0 <= blk.hi; kb0 += 4, phase ^= 1) {
         const int kb = kb0 + warp, j0 = kb * KB, nb = min(4, blk.hi - kb0 + 1);
         if (kb <= blk.hi) {
-            tc::mbar_wait(bar_k, phase, &abort_s, ef, 44); // K and the table rows
+            ok = ok && tc::mbar_wait(bar_k, phase, &abort_s, ef, 44); // K and the table rows
             __syncwarp();
             float mb = -INFINITY;
 #pragma unroll
@@ -754,7 +755,7 @@ __global__ void __launch_bounds__(128) attn_one_tma_kernel(const __grid_constant
                 mbs[warp] = mb;
             __syncwarp();
             fetch_kr(kb + 4);
-            tc::mbar_wait(bar_v, phase, &abort_s, ef, 45);
+            ok = ok && tc::mbar_wait(bar_v, phase, &abort_s, ef, 45);
         }
         __syncthreads(); // scores, maxima and V of the round are there for everyone
         for (int s = 0; s < nb; s++) {
@@ -787,6 +788,13 @@ __global__ void __launch_bounds__(128) attn_one_tma_kernel(const __grid_constant
         __syncthreads(); // the round has been read
         fetch_v(kb + 4);
     }
+    if (lane == 0 && !ok) { // copies still in flight land in this CTA's shared memory: both phases get a bounded chance to finish
+        for (uint32_t parity = 0; parity < 2; parity++) {
+            tc::mbar_wait(bar_k, parity, &abort_s, ef, 44);
+            tc::mbar_wait(bar_v, parity, &abort_s, ef, 45);
+        }
+    }
+    __syncwarp();
     l = __fadd_rn(l, __shfl_xor_sync(0xffffffffu, l, 1));
     l = __fadd_rn(l, __shfl_xor_sync(0xffffffffu, l, 2));
     const float inv = *static_cast<volatile int *>(&abort_s) ? __int_as_float(0x7fffffff) : __fdiv_rn(1.0f, l); // a wait ran out: no result
