@@ -284,7 +284,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             return stg0 + (blk++ & 1) * 4096;
         };
         unsigned char *stg = stg0;
-        for (int idx = blockIdx.x / 2; ok && idx < units; idx += stride, ti++) {
+        // a warp whose wait ran out goes on to the end without working: the barriers of its half count on it
+        for (int idx = blockIdx.x / 2; idx < units; idx += stride, ti++) {
             const Unit u = unit_at(idx, sh, nt, hm, hn);
             const int row0 = u.tm * 256 + (int)rank * 128 + quarter * 32, row = row0 + lane, n0 = u.tn * BN + half * (BN / 2);
             if (bias) { // this half's columns, by the four warps that use them
@@ -293,6 +294,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                     bias_s[half * (BN / 2) + i] = n0 + i < min(sh.N, sh.bias_n) ? __ldg(bias + n0 + i) : 0.0f;
                 asm volatile("bar.sync %0, 128;" ::"r"(1 + half) : "memory");
             }
+            if (!ok)
+                continue;
             // even sums into registers
             uint32_t e[NCH][32];
             const bool has_even = u.kb0 + (u.kb0 & 1) < u.kb1, has_odd = u.kb0 + ((u.kb0 ^ 1) & 1) < u.kb1;
@@ -300,7 +303,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                 ok = mbar_wait(accf0, (uint32_t)(ti & 1), abort_s, err_flag, 55);
             ok = __all_sync(0xffffffffu, ok);
             if (!ok)
-                break;
+                continue;
             fence_after_sync();
 #pragma unroll
             for (int c = 0; c < NCH; c++) {
@@ -321,7 +324,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             }
             ok = __all_sync(0xffffffffu, ok);
             if (!ok)
-                break;
+                continue;
             fence_after_sync();
 #pragma unroll
             for (int c = 0; c < NCH; c++)
