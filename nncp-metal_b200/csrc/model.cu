@@ -1193,6 +1193,12 @@ __global__ void fill_kernel(float *__restrict__ dst, size_t n, float v)
     if (i < n)
         dst[i] = v;
 }
+static int fill(float *dst_dev, size_t n, float v, cudaStream_t st)
+{
+    fill_kernel<<<ceil_div((long long)n, 256), 256, 0, st>>>(dst_dev, n, v);
+    KERNEL_CHECK();
+    return NNCU_OK;
+}
 static int init_values(float *dst_dev, size_t n, const char *name, uint32_t seed, int kind, float scale, cudaStream_t st)
 {
     const uint64_t key = splitmix64(name_hash(name) ^ ((uint64_t)seed << 32));
@@ -1623,7 +1629,7 @@ int nncu_create(const nncu_params *p, nncu_model **out)
             if (rc != NNCU_OK)
                 break;
             if (!strncmp(pi.name, "ln_g", 4)) {
-                fill_kernel<<<ceil_div((long long)pi.numel, 256), 256, 0, m->st>>>(dst, pi.numel, 1.0f);
+                rc = fill(dst, pi.numel, 1.0f, m->st);
             } else if (!strncmp(pi.name, "w_", 2) || !strncmp(pi.name, "ff1", 3) || !strncmp(pi.name, "embed", 5)) {
                 rc = init_values(dst, pi.numel, pi.name, p->seed, p->init_kind, a0, m->st);
             } else if (!strncmp(pi.name, "ff2", 3)) {

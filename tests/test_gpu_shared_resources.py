@@ -150,3 +150,15 @@ def test_query_kernel_table_tiles_by_hand_and_by_copy(pkg, dk):
         for m in (seg, one):
             m.memory_shift()
     seg.close(); one.close()
+
+
+def test_launches_of_a_models_creation_are_counted(pkg):
+    """Every launch is checked and counted: one for each parameter whose initial values are not zero."""
+    prof = pkg.abi.Profile()
+    lib = pkg.library()
+    lib.nncu_profile_begin(0)
+    m = pkg.TrfModel(pkg.abi.make_params(n_layer=2, d_model=64, n_head=2, d_key=32, d_inner=64, d_pos=8, mem_len=8, seg_len=4, n_streams=2,
+                                         n_symbols=64, use_bf16=0))
+    lib.nncu_profile_end(C.byref(prof))
+    assert prof.launches == sum(n.startswith(("ln_g", "w_", "ff1", "ff2", "embed")) for n in m.info)
+    m.close()
