@@ -418,7 +418,7 @@ typedef struct nncu_profile {
     uint64_t launches;      /* kernels launched by this library since nncu_profile_begin */
     uint64_t gemm_launches; /* timed tcgen05 GEMM launches */
     double gemm_ms;         /* sum of their device durations */
-    double gemm_flops;      /* sum of 2*M*N*K over them */
+    double gemm_flops;      /* sum of 2*M*N*K over them, less what a launch leaves out */
 } nncu_profile;
 int nncu_profile_begin(int time_gemms);
 int nncu_profile_end(nncu_profile *out);

@@ -494,7 +494,9 @@ static int launch(cudaStream_t st, int M, int N, int K, const bf16 *A, long lda,
              addsrc, ldc, err_flag);
     if (timed) {
         cudaEventRecord(pr->ev[2 * pr->n + 1], st);
-        pr->flops[pr->n++] = 2.0 * M * N * K;
+        // what is left out is no work: the hole's tiles, and the terms that whole row tiles skip
+        const double hole = (double)(x.hole_m / 256 * 256) * (x.hole_n / BN * BN), skipped = (double)(x.skip_m / 256 * 256) * (x.skip_k / BK * BK);
+        pr->flops[pr->n++] = 2.0 * (((double)M * N - hole) * K - skipped * N);
     }
     KERNEL_CHECK();
     return NNCU_OK;

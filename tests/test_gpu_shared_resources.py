@@ -162,3 +162,24 @@ def test_launches_of_a_models_creation_are_counted(pkg):
     lib.nncu_profile_end(C.byref(prof))
     assert prof.launches == sum(n.startswith(("ln_g", "w_", "ff1", "ff2", "embed")) for n in m.info)
     m.close()
+
+
+def test_profiled_work_leaves_out_what_is_not_computed(pkg):
+    """A long memory: the memory rows' queries are neither projected nor part of the weight gradient."""
+    D, F, T, M, B, V = 512, 1024, 64, 512, 32, 1024
+    lib, prof = pkg.library(), pkg.abi.Profile()
+    m = pkg.TrfModel(pkg.abi.make_params(n_layer=1, d_model=D, n_head=8, d_key=64, d_inner=F, d_pos=M + T, mem_len=M, seg_len=T, n_streams=B,
+                                         n_symbols=V, use_bf16=1, init_range=0.05))
+    m.reset()
+    ids = np.zeros((T, B), np.int32)
+    work = []
+    for step in (lambda: m.eval(-1, ids, read=False), lambda: m.eval_gradient(ids)):
+        lib.nncu_profile_begin(1)
+        step()
+        lib.nncu_profile_end(C.byref(prof))
+        work.append(prof.gemm_flops)
+    m.close()
+    rows, dense = T * B, 2 * T * B * D * (D + 2 * F + V)   # output projection, feed-forward, head
+    project = 2 * (M * B * 2 * D + rows * 3 * D) * D
+    assert work[0] == dense + project
+    assert work[1] == 2 * dense + project + 2 * rows * 3 * D * D
