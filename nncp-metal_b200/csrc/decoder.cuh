@@ -29,7 +29,7 @@ struct State {
 };
 
 constexpr uint32_t R_LOW = (0xffu << 8) + 1u, R_TOP = 0xffu << 16;
-constexpr int MAX_RING = 8, MAX_SMEM = 200 * 1024;
+constexpr int MAX_RING = 8, MAX_SMEM = 200 * 1024 + 16; // 16: the window's bytes to look ahead
 
 __device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar)
 {
@@ -40,19 +40,27 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_
 
 // window bytes a step of `B` streams with `nb` bits per symbol can consume, twelve to look ahead, as a multiple of 16
 __host__ __device__ inline int window_bytes(int B, int nb) { return (2 * B * nb + 12 + 15) & ~15; }
-// trees of P entries that share a ring slot: small ones come 16 KB at a time
-__host__ __device__ inline int slot_trees(int B, int P) { return P >= 8192 ? 1 : (8192 / P < B ? 8192 / P : B); }
+// shared memory left for the ring
+__host__ __device__ inline int ring_bytes(int B, int nb) { return MAX_SMEM - window_bytes(B, nb) - 128; }
+// trees of P entries that share a ring slot: small ones come 16 KB at a time, fewer where a step of very many
+// streams leaves no room for two such slots
+__host__ __device__ inline int slot_trees(int B, int P, int nb)
+{
+    int n = P >= 8192 ? 1 : (8192 / P < B ? 8192 / P : B);
+    while (n > 1 && 2 * n * P * 2 > ring_bytes(B, nb))
+        n >>= 1;
+    return n;
+}
 
 // slots of the ring for trees of P entries (0: the trees do not fit)
 inline int ring_slots(int B, int P, int nb)
 {
-    const long avail = (long)MAX_SMEM - window_bytes(B, nb) - 128;
-    long n = avail / ((long)slot_trees(B, P) * P * 2);
+    const int n = ring_bytes(B, nb) / (slot_trees(B, P, nb) * P * 2);
     if (P < 8 || n < 2)
         return 0;
-    return (int)std::min<long>(n, MAX_RING);
+    return std::min(n, MAX_RING);
 }
-inline size_t smem_bytes(int B, int P, int nb, int ring) { return (size_t)ring * slot_trees(B, P) * P * 2 + window_bytes(B, nb) + 128; }
+inline size_t smem_bytes(int B, int P, int nb, int ring) { return (size_t)ring * slot_trees(B, P, nb) * P * 2 + window_bytes(B, nb) + 128; }
 
 // trees: [B][P] prob0 in heap order (entry 0 unused), P = 2^nb >= V.  sym_out[b] and ids_next[b]
 // (when not null) receive the decoded symbol, 0 for the streams past the end of the block: those at
@@ -67,7 +75,7 @@ decode_step_kernel(const uint16_t *__restrict__ trees, const uint8_t *__restrict
     pdl_trigger(); // a successor that was launched to overlap this kernel may start on what does not depend on it
     extern __shared__ __align__(128) uint8_t dsm[];
     uint64_t *bars = reinterpret_cast<uint64_t *>(dsm);           // [2][MAX_RING] of 8 bytes: 128
-    const int G = slot_trees(B, P);
+    const int G = slot_trees(B, P, nb);
     uint16_t *slots = reinterpret_cast<uint16_t *>(dsm + 128);    // [ring][G][P]
     uint8_t *win = dsm + 128 + (size_t)ring * G * P * 2;          // payload window
     __shared__ int abort_s;

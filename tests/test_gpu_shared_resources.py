@@ -183,3 +183,28 @@ def test_profiled_work_leaves_out_what_is_not_computed(pkg):
     project = 2 * (M * B * 2 * D + rows * 3 * D) * D
     assert work[0] == dense + project
     assert work[1] == 2 * dense + project + 2 * rows * 3 * D * D
+
+
+@pytest.mark.parametrize("B,V", [(11500, 256), (12690, 256), (10900, 300)])
+def test_decoder_of_very_many_streams(pkg, B, V):
+    """The payload window of so many streams leaves room for a few trees only: they still go through the
+    ring, and the symbols are those of the host's walk of the same trees."""
+    p = pkg.abi.make_params(n_layer=1, d_model=16, n_head=1, d_key=16, d_inner=16, d_pos=2, mem_len=0, seg_len=2, n_streams=B, n_symbols=V,
+                            use_bf16=0, init_range=0.5)
+    L = pkg.host.library()
+    payload = np.random.default_rng(B).integers(0, 256, 20000, dtype=np.uint8).tobytes()
+    dev, ref = pkg.TrfModel(p), pkg.TrfModel(p)
+    dev.reset(); ref.reset()
+    dev.decoder_begin(payload)
+    got = dev.decode_steps(0, 2, np.zeros(B, np.int32))
+    buf = C.create_string_buffer(payload, len(payload))
+    hd, ids, want = L.nch_dec_new(buf, len(payload)), np.zeros((2, B), np.int32), np.zeros((2, B), np.int32)
+    for t in range(2):
+        ids[t] = want[t - 1] if t else 0
+        ref.eval(t, ids, read=False)
+        trees = np.ascontiguousarray(ref.coder_trees(t, 1))
+        for b in range(B):
+            want[t, b] = L.nch_read_sym_tree(hd, trees[b].ctypes.data_as(C.c_void_p), V)
+    L.nch_dec_free(hd)
+    assert np.array_equal(got, want)
+    dev.close(); ref.close()
