@@ -78,11 +78,14 @@ __device__ __forceinline__ void quad_transpose(uint32_t (&v)[4], int t)
     if (o2) { v[0] = a; v[1] = b; } else { v[2] = a; v[3] = b; }
 }
 
+inline __host__ __device__ bool aligned_to(const void *p, int bytes) { return (reinterpret_cast<uintptr_t>(p) & (bytes - 1)) == 0; }
+
 // One row of a warp tile out as bf16: lane t of the quad holds columns nt * 8 + 2t, + 1 of the N / 8
-// column groups in x[nt][c], x[nt][c + 1].  Rows of 32 columns and more leave in 16-byte pieces.
-template <int NT> __device__ __forceinline__ void store_row(bf16 *dst, const float (&x)[NT][4], int c, int t, bool act)
+// column groups in x[nt][c], x[nt][c + 1].  Rows of 32 columns and more leave in 16-byte pieces where the
+// destination is aligned to them (WIDE).
+template <bool WIDE, int NT> __device__ __forceinline__ void store_row(bf16 *dst, const float (&x)[NT][4], int c, int t, bool act)
 {
-    if constexpr (NT % 4 == 0) {
+    if constexpr (WIDE && NT % 4 == 0) {
 #pragma unroll
         for (int n4 = 0; n4 < NT; n4 += 4) {
             uint32_t v[4];
@@ -112,8 +115,32 @@ __device__ __forceinline__ void load_rows(bf16 *dst, const bf16 *src, size_t pit
         cp16(dst + r * LD + c, ok ? src + (size_t)r * pitch + c : src, ok);
     }
 }
+// sixteen zero bytes, by words where the destination is not aligned to them
+template <bool WIDE> __device__ __forceinline__ void zero16(void *p)
+{
+    if constexpr (WIDE) {
+        *reinterpret_cast<uint4 *>(p) = make_uint4(0u, 0u, 0u, 0u);
+    } else {
+#pragma unroll
+        for (int w = 0; w < 4; w++)
+            reinterpret_cast<uint32_t *>(p)[w] = 0u;
+    }
+}
+// eight consecutive fp32 table entries as bf16; one at a time where they are not aligned to 16 bytes
+// (WIDE: they are known to be)
+template <bool WIDE> __device__ __forceinline__ void table_piece(bf16 *dst, const float *p)
+{
+    if (WIDE || aligned_to(p, 16)) {
+        const float4 u = *reinterpret_cast<const float4 *>(p), v = *reinterpret_cast<const float4 *>(p + 4);
+        *reinterpret_cast<uint4 *>(dst) = make_uint4(pack2(u.x, u.y), pack2(u.z, u.w), pack2(v.x, v.y), pack2(v.z, v.w));
+    } else {
+#pragma unroll 1
+        for (int e = 0; e < 8; e++)
+            dst[e] = __float2bfloat16_rn(p[e]);
+    }
+}
 // rows x0 .. x0 + rows - 1 of one head's position table, clamped to [0, P)
-template <int DK>
+template <int DK, bool WIDE>
 __device__ __forceinline__ void load_table(bf16 *dst, const AttnArgs &a, int h, int x0, int rows, int tid, int nthr)
 {
     constexpr int LD = DK + 8, CPR = DK / 8;
@@ -125,9 +152,7 @@ __device__ __forceinline__ void load_table(bf16 *dst, const AttnArgs &a, int h, 
         if (a.w_r16) {
             cp16(dst + r * LD + c, w16 + (size_t)x * DK + c, true);
         } else {
-            const float4 u = *reinterpret_cast<const float4 *>(w32 + (size_t)x * DK + c);
-            const float4 v = *reinterpret_cast<const float4 *>(w32 + (size_t)x * DK + c + 4);
-            *reinterpret_cast<uint4 *>(dst + r * LD + c) = make_uint4(pack2(u.x, u.y), pack2(u.z, u.w), pack2(v.x, v.y), pack2(v.z, v.w));
+            table_piece<WIDE>(dst + r * LD + c, w32 + (size_t)x * DK + c);
         }
     }
 }
@@ -263,7 +288,7 @@ template <int DK> struct FwdSmem {
     static size_t bytes(int L) { return (size_t)BRS + br_bytes(L); }
 };
 
-template <int DK>
+template <int DK, bool WIDE> // WIDE: out takes 16-byte stores, an fp32 table 16-byte loads
 __global__ void __launch_bounds__(256, DK <= 64 ? 2 : 1) attn_fwd_kernel(const __grid_constant__ AttnArgs a)
 {
     using SM = FwdSmem<DK>;
@@ -287,7 +312,7 @@ __global__ void __launch_bounds__(256, DK <= 64 ? 2 : 1) attn_fwd_kernel(const _
     const bf16 *kv = reinterpret_cast<const bf16 *>(a.kv) + (size_t)b * a.kvp + h * DK;
     auto fetch_r = [&](int gr) { // table group gr: window rows 0-63 of block gr, 64-127 of block gr - 1
         if (a.w_r)
-            load_table<DK>(Rs + (gr % 3) * 64 * LD, a, h, gr * KB - i0 + a.P - M - 64, 64, threadIdx.x, 256);
+            load_table<DK, WIDE>(Rs + (gr % 3) * 64 * LD, a, h, gr * KB - i0 + a.P - M - 64, 64, threadIdx.x, 256);
     };
     auto fetch = [&](int kb) {
         const int j0 = kb * KB;
@@ -430,8 +455,8 @@ __global__ void __launch_bounds__(256, DK <= 64 ? 2 : 1) attn_fwd_kernel(const _
             o[n][3] = __fmul_rn(o[n][3], rB);
         }
         bf16 *out = reinterpret_cast<bf16 *>(a.o) + ((size_t)iA * a.B + b) * HD + h * DK + hf * (DK / 2) * (NCH - 1);
-        store_row<NTC>(out, o, 0, t, okA);
-        store_row<NTC>(out + (size_t)8 * a.B * HD, o, 2, t, okB);
+        store_row<WIDE>(out, o, 0, t, okA);
+        store_row<WIDE>(out + (size_t)8 * a.B * HD, o, 2, t, okB);
     }
     if (hf == 0 && t == 0 && a.lse) {
         float *lse = a.lse + ((size_t)b * a.H + h) * T;
@@ -478,7 +503,7 @@ __global__ void __launch_bounds__(128) attn_one_kernel(const __grid_constant__ A
             return;
         load_rows<DK>(Ks, kv + (size_t)j0 * a.B * a.kvp, (size_t)a.B * a.kvp, 64, lane, 32, [&](int r) { return j0 + r < L; });
         if (a.w_r)
-            load_table<DK>(Rs, a, h, j0 - i + a.P - M - 1, 64, lane, 32);
+            load_table<DK, false>(Rs, a, h, j0 - i + a.P - M - 1, 64, lane, 32);
     };
     auto fetch_v = [&](int kb) {
         const int j0 = kb * KB;
@@ -674,15 +699,11 @@ __global__ void __launch_bounds__(128) attn_one_tma_kernel(const __grid_constant
             const float *w32 = a.w_r + (size_t)h * a.P * DK;
             for (int idx = lane; idx < 64 * (DK / 8); idx += 32) {
                 const int r = idx / (DK / 8), c = idx % (DK / 8), x = min(max(x0 + r, 0), a.P - 1);
-                uint4 v;
-                if (a.w_r16) {
-                    v = *reinterpret_cast<const uint4 *>(w16 + (size_t)x * DK + c * 8);
-                } else {
-                    const float4 u = *reinterpret_cast<const float4 *>(w32 + (size_t)x * DK + c * 8);
-                    const float4 w = *reinterpret_cast<const float4 *>(w32 + (size_t)x * DK + c * 8 + 4);
-                    v = make_uint4(pack2(u.x, u.y), pack2(u.z, u.w), pack2(w.x, w.y), pack2(w.z, w.w));
-                }
-                *reinterpret_cast<uint4 *>(sm + SM::R + warp * TILE + tile_at(r, c)) = v;
+                bf16 *dst = reinterpret_cast<bf16 *>(sm + SM::R + warp * TILE + tile_at(r, c));
+                if (a.w_r16)
+                    *reinterpret_cast<uint4 *>(dst) = *reinterpret_cast<const uint4 *>(w16 + (size_t)x * DK + c * 8);
+                else
+                    table_piece<false>(dst, w32 + (size_t)x * DK + c * 8);
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); // a later round's tile may come by TMA to the same place
         }
@@ -836,7 +857,7 @@ template <int DK> struct BwdSmem {
     static size_t bytes(int L) { return (size_t)BRS + br_bytes(L); }
 };
 
-template <int DK>
+template <int DK, bool WIDE> // WIDE: dq, dkv and the table's partials take 16-byte stores, an fp32 table 16-byte loads
 __global__ void __launch_bounds__(256, DK <= 64 ? 2 : 1) attn_bwd_kernel(const __grid_constant__ AttnArgs a)
 {
     using SM = BwdSmem<DK>;
@@ -877,7 +898,7 @@ __global__ void __launch_bounds__(256, DK <= 64 ? 2 : 1) attn_bwd_kernel(const _
     // table group gr (window rows 0-63 of block gr, 64-127 of block gr - 1) into its slot of the two
     auto fetch_r = [&](int gr) {
         if (a.w_r)
-            load_table<DK>(Rs + (gr & 1) * 64 * LD, a, h, window0(gr), 64, threadIdx.x, 256);
+            load_table<DK, WIDE>(Rs + (gr & 1) * 64 * LD, a, h, window0(gr), 64, threadIdx.x, 256);
     };
     load_rows<DK>(Qs, reinterpret_cast<const bf16 *>(a.q) + (size_t)b * a.qp + h * DK, (size_t)a.B * a.qp, 64, threadIdx.x, 256,
                   [&](int r) { return r < T; });
@@ -915,8 +936,8 @@ __global__ void __launch_bounds__(256, DK <= 64 ? 2 : 1) attn_bwd_kernel(const _
         for (int idx = threadIdx.x; idx < 64 * (DK / 8); idx += 256) {
             const int j = kb * KB + idx / (DK / 8), c = (idx % (DK / 8)) * 8;
             if (j < L) {
-                *reinterpret_cast<uint4 *>(dkv + (size_t)j * a.B * a.dkvp + c) = make_uint4(0u, 0u, 0u, 0u);
-                *reinterpret_cast<uint4 *>(dkv + (size_t)j * a.B * a.dkvp + HD + c) = make_uint4(0u, 0u, 0u, 0u);
+                zero16<WIDE>(dkv + (size_t)j * a.B * a.dkvp + c);
+                zero16<WIDE>(dkv + (size_t)j * a.B * a.dkvp + HD + c);
             }
         }
     }
@@ -925,7 +946,7 @@ __global__ void __launch_bounds__(256, DK <= 64 ? 2 : 1) attn_bwd_kernel(const _
         for (int idx = threadIdx.x; idx < P * DK / 4; idx += 256) {
             const int x = idx / (DK / 4);
             if (x < x_lo || x > x_hi)
-                reinterpret_cast<float4 *>(dwr)[idx] = make_float4(0.f, 0.f, 0.f, 0.f);
+                zero16<WIDE>(reinterpret_cast<float4 *>(dwr) + idx);
         }
     if (dbr)
         for (int r = threadIdx.x; r < L; r += 256)
@@ -1098,9 +1119,9 @@ __global__ void __launch_bounds__(256, DK <= 64 ? 2 : 1) attn_bwd_kernel(const _
                 }
                 const int jA = j0 + qt * 16 + g, jB = jA + 8;
                 bf16 *dst = dkv + (which ? 0 : HD) + hf * (DK / 2) * (NCH - 1) + (size_t)(jA < L ? jA : 0) * a.B * a.dkvp;
-                store_row<NTC>(dst, acc, 0, t, jA < L);
+                store_row<WIDE>(dst, acc, 0, t, jA < L);
                 dst += (size_t)(jB < L ? 8 : 0) * a.B * a.dkvp;
-                store_row<NTC>(dst, acc, 2, t, jB < L);
+                store_row<WIDE>(dst, acc, 2, t, jB < L);
             }
         }
         // dR and the column sums of one table group: the lower one (window columns 0-63) belongs to the warps of
@@ -1139,9 +1160,9 @@ __global__ void __launch_bounds__(256, DK <= 64 ? 2 : 1) attn_bwd_kernel(const _
             for (int c = 0; c < 4; c++)
                 dq[n][c] = __fadd_rn(dq[n][c], dqr[n][c]);
         bf16 *dst = reinterpret_cast<bf16 *>(a.dq) + ((size_t)(iA < T ? iA : 0) * a.B + b) * a.dqp + h * DK + hf * (DK / 2) * (NCH - 1);
-        store_row<NTC>(dst, dq, 0, t, iA < T);
+        store_row<WIDE>(dst, dq, 0, t, iA < T);
         dst += (size_t)(iB < T ? 8 : 0) * a.B * a.dqp;
-        store_row<NTC>(dst, dq, 2, t, iB < T);
+        store_row<WIDE>(dst, dq, 2, t, iB < T);
     }
     if (dwr && x_lo <= 0) // table row 0: the warps' shares, in warp order (the loop's last barrier is behind them)
         for (int d = threadIdx.x; d < DK; d += 256) {
@@ -1156,18 +1177,18 @@ __global__ void __launch_bounds__(256, DK <= 64 ? 2 : 1) attn_bwd_kernel(const _
 
 // ---------------- host side ----------------
 
-// head sizes and operand placements the kernels take (16-byte loads and stores everywhere)
+// head sizes and operand placements the kernels take: 16-byte copies of the bf16 operands, stores of two
+// elements at least; the fp32 table and `out` as an input may lie anywhere
 inline bool head_size(int dk) { return dk == 16 || dk == 32 || dk == 64 || dk == 128; }
-inline bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 inline bool supported(const AttnArgs &a)
 {
-    return head_size(a.dk) && a.qp % 8 == 0 && a.kvp % 8 == 0 && aligned16(a.q) && aligned16(a.kv) && aligned16(a.o) &&
-           aligned16(a.w_r) && aligned16(a.w_r16);
+    return head_size(a.dk) && a.qp % 8 == 0 && a.kvp % 8 == 0 && aligned_to(a.q, 16) && aligned_to(a.kv, 16) && aligned_to(a.o, 4) &&
+           aligned_to(a.w_r16, 16);
 }
 inline bool supported_bwd(const AttnArgs &a)
 {
-    return supported(a) && a.T <= 64 && a.t0 == 0 && a.t1 == a.T && a.dqp % 8 == 0 && a.dkvp % 8 == 0 && aligned16(a.dq) &&
-           aligned16(a.dkv) && aligned16(a.dout) && aligned16(a.out) && aligned16(a.dwr_part) && a.lse;
+    return supported(a) && a.T <= 64 && a.t0 == 0 && a.t1 == a.T && a.dqp % 8 == 0 && a.dkvp % 8 == 0 && aligned_to(a.dq, 4) &&
+           aligned_to(a.dkv, 4) && aligned_to(a.dout, 16) && aligned_to(a.dwr_part, 8) && a.lse;
 }
 // shared memory both kernels of a shape need
 inline bool fits(int dk, int L)
@@ -1217,17 +1238,21 @@ template <int DK> static int forward_dk(const AttnArgs &a, cudaStream_t st)
 {
     if (a.t1 - a.t0 == 1)
         return forward_one<DK>(a, st);
-    static DeviceOnce once;
-    NNCU_TRY(smem_limit(once, attn_fwd_kernel<DK>, SMEM_MOST));
-    launch_k(attn_fwd_kernel<DK>, dim3(a.B * a.H, (a.t1 - (a.t0 & ~63) + 63) / 64), dim3(256), FwdSmem<DK>::bytes(a.L), st, a);
+    static DeviceOnce once[2];
+    const bool wide = aligned_to(a.o, 16) && aligned_to(a.w_r, 16);
+    auto kernel = wide ? attn_fwd_kernel<DK, true> : attn_fwd_kernel<DK, false>;
+    NNCU_TRY(smem_limit(once[wide], kernel, SMEM_MOST));
+    launch_k(kernel, dim3(a.B * a.H, (a.t1 - (a.t0 & ~63) + 63) / 64), dim3(256), FwdSmem<DK>::bytes(a.L), st, a);
     KERNEL_CHECK();
     return NNCU_OK;
 }
 template <int DK> static int backward_dk(const AttnArgs &a, cudaStream_t st)
 {
-    static DeviceOnce once;
-    NNCU_TRY(smem_limit(once, attn_bwd_kernel<DK>, SMEM_MOST));
-    launch_k(attn_bwd_kernel<DK>, dim3(a.B * a.H), dim3(256), BwdSmem<DK>::bytes(a.L), st, a);
+    static DeviceOnce once[2];
+    const bool wide = aligned_to(a.dq, 16) && aligned_to(a.dkv, 16) && aligned_to(a.dwr_part, 16) && aligned_to(a.w_r, 16);
+    auto kernel = wide ? attn_bwd_kernel<DK, true> : attn_bwd_kernel<DK, false>;
+    NNCU_TRY(smem_limit(once[wide], kernel, SMEM_MOST));
+    launch_k(kernel, dim3(a.B * a.H), dim3(256), BwdSmem<DK>::bytes(a.L), st, a);
     KERNEL_CHECK();
     return NNCU_OK;
 }

@@ -208,3 +208,46 @@ def test_decoder_of_very_many_streams(pkg, B, V):
     L.nch_dec_free(hd)
     assert np.array_equal(got, want)
     dev.close(); ref.close()
+
+
+@pytest.mark.parametrize("dk,T,M,alen", [(16, 20, 300, 0), (32, 64, 500, 90), (64, 64, 836, 0), (64, 64, 600, 130), (128, 33, 500, 200)])
+def test_attention_of_operands_inside_larger_buffers(pkg, dk, T, M, alen):
+    """An fp32 table, results and partials that start between 16-byte boundaries, as views of larger buffers do, with
+    more keys than the CUDA-core kernels hold: the bits of the aligned call, segments and single queries."""
+    torch = pytest.importorskip("torch")
+    lib = pkg.library()
+    B, H, L, P = 2, 3, T + M, T + M - 5
+    g = torch.Generator(device="cuda").manual_seed(dk + M)
+    q, dout = (torch.randn(T * B, H * dk, generator=g, device="cuda").bfloat16() for _ in range(2))
+    kv = torch.randn(L * B, 2 * H * dk, generator=g, device="cuda").bfloat16()
+    w_r, b_r = 0.1 * torch.randn(H, P, dk, generator=g, device="cuda"), 0.1 * torch.randn(H, L, generator=g, device="cuda")
+
+    def place(t, by):   # the same values, `by` elements into a buffer
+        room = torch.full((t.numel() + 16,), float("nan"), device="cuda", dtype=t.dtype)
+        view = room[by:by + t.numel()].view(t.shape)
+        view.copy_(t)
+        return view
+
+    got = []
+    for off in (0, 1):
+        table = place(w_r, off)
+        out, one, dq, dkv = (place(torch.full_like(t, float("nan")), 2 * off) for t in (q, q, q, kv))
+        lse = torch.zeros(B * H, T, device="cuda")
+        part, dbr = place(torch.full((B, H, P, dk), float("nan"), device="cuda"), 2 * off), torch.zeros(B, H, L, device="cuda")
+
+        def shape(t0, t1):
+            return C.byref(pkg.abi.AttnShape(B, H, dk, T, M, P, alen, t0, t1, float(np.sqrt(dk * 512.0)), 1))
+
+        calls = [lib.nncu_attention_forward(shape(0, T), q.data_ptr(), kv.data_ptr(), table.data_ptr(), b_r.data_ptr(), out.data_ptr(),
+                                            lse.data_ptr(), None)]
+        calls += [lib.nncu_attention_forward(shape(t, t + 1), q.data_ptr(), kv.data_ptr(), table.data_ptr(), b_r.data_ptr(), one.data_ptr(),
+                                             None, None) for t in range(T)]
+        calls += [lib.nncu_attention_backward(shape(0, T), q.data_ptr(), kv.data_ptr(), table.data_ptr(), b_r.data_ptr(), out.data_ptr(),
+                                              lse.data_ptr(), dout.data_ptr(), dq.data_ptr(), dkv.data_ptr(), part.data_ptr(), dbr.data_ptr(),
+                                              None)]
+        assert not any(calls), lib.nncu_last_error()
+        torch.cuda.synchronize()
+        got.append((out, one, lse, dq, dkv, part, dbr))
+    for a, b in zip(*got):
+        assert torch.equal(a, b) and not a.isnan().any()
+    assert torch.equal(got[0][0], got[0][1])
