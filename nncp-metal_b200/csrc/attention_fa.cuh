@@ -479,7 +479,7 @@ __global__ void __launch_bounds__(256, DK <= 64 ? 2 : 1) attn_fwd_kernel(const _
 // the same bits either way round.
 template <int DK> struct OneSmem {
     static constexpr int LD = DK + 8, TILE = 64 * LD * 2;
-    static constexpr int K = 0, R = 4 * TILE, V = 8 * TILE, S = 12 * TILE, MB = S + 4 * 64 * 4, L4 = MB + 16, TOTAL = L4 + 16;
+    static constexpr int K = 0, R = 4 * TILE, V = 8 * TILE, S = 12 * TILE, MB = S + 4 * 64 * 4, TOTAL = MB + 16;
 };
 
 template <int DK>
@@ -628,7 +628,7 @@ __global__ void __launch_bounds__(128) attn_one_kernel(const __grid_constant__ A
 // it took 57 us of which HBM needs 23; this loop takes 39.
 template <int DK> struct OneTmaSmem {
     static constexpr int NS = DK / 64, TILE = NS * 8192;
-    static constexpr int K = 0, R = 4 * TILE, V = 8 * TILE, S = 12 * TILE, MB = S + 4 * 64 * 4, L4 = MB + 16, BRS = L4 + 16;
+    static constexpr int K = 0, R = 4 * TILE, V = 8 * TILE, S = 12 * TILE, MB = S + 4 * 64 * 4, BRS = MB + 16;
     static size_t bytes(int L) { return (size_t)BRS + (size_t)L * 4 + 1024; }
 };
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap *map, uint32_t bar, int x, int y, int z)

@@ -84,8 +84,8 @@ inline bool nncu_pdl_enabled()
     return on != 0;
 }
 template <typename... KArgs, typename... Args>
-static cudaError_t launch_pdl(bool early, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
-                              Args &&...args)
+static cudaError_t launch_k(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                            Args &&...args)
 {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
@@ -96,14 +96,8 @@ static cudaError_t launch_pdl(bool early, void (*kernel)(KArgs...), dim3 grid, d
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = early ? 1 : 0;
+    cfg.numAttrs = nncu_pdl_enabled() ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
-}
-template <typename... KArgs, typename... Args>
-static cudaError_t launch_k(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
-                            Args &&...args)
-{
-    return launch_pdl(nncu_pdl_enabled(), kernel, grid, block, smem, st, static_cast<KArgs>(args)...);
 }
 
 // every kernel launch in the library is followed by exactly one KERNEL_CHECK

@@ -2,9 +2,9 @@
 // epilogue under the next tile's mainloop.
 //
 // Two CTAs of a cluster share a 256 x BN tile (tcgen05.mma cta_group::2, M = 256): each loads its own
-// 128 rows of A and half of the B rows by TMA, so a pair reads 24 KB (BN = 256: 32 KB) of shared
-// memory per 16-wide step and SM for twice the products of a single-CTA 128 x BN tile; below
-// that the single-CTA kernel is bound by shared-memory reads (128 x 128: 64 cycles of reads for 32
+// 128 rows of A and half of the B rows by TMA, so an SM reads 32 KB of shared
+// memory per 64-wide k-block for the products of a single-CTA 128 x BN tile, which reads 48 KB; below
+// that width the single-CTA kernel is bound by shared-memory reads (128 x 128: 64 cycles of reads for 32
 // of products).  One pair per two SMs walks the tiles in order.
 //
 // Same bits as gemm_tc.cuh: an output is (chain of the even 64-wide k-blocks) + (chain of the odd
@@ -36,6 +36,7 @@ using tc::smem_u32;
 using tc::tmem_ld32;
 using tc::tmem_ld_wait;
 
+constexpr int BN = 256; // columns of a tile
 constexpr uint32_t LEADER = 0xFEFFFFFFu; // clears the CTA bit of a shared::cluster address: the leader's copy
 
 __device__ __forceinline__ uint32_t cta_rank()
@@ -113,9 +114,9 @@ struct Shape {
     int act; // activation whose value goes to a second output (-1: none)
 };
 
-template <int BN> struct Smem {
+struct Smem {
     static constexpr int A_BYTES = 128 * BK * 2, B_BYTES = BN / 2 * BK * 2, STAGE = A_BYTES + B_BYTES;
-    static constexpr int STAGES = BN == 256 ? 5 : 6;
+    static constexpr int STAGES = 5;
     static constexpr int C = STAGES * STAGE;       // two 32-row x 128-byte blocks for each epilogue warp
     static constexpr int BIAS = C + 8 * 8192;      // BN floats
     static constexpr int BAR = BIAS + BN * 4;      // full, empty [STAGES]; acc_full, acc_empty [2]; TMEM slot; abort flag
@@ -151,13 +152,13 @@ __device__ __forceinline__ void tile_at(int idx, int nt, int hm, int hn, int &tm
     }
 }
 
-template <int BN, typename TC, bool AMN, bool BMN>
+template <typename TC, bool AMN, bool BMN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(384, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                  const __grid_constant__ CUtensorMap map_c, const __grid_constant__ CUtensorMap map_c2,
                  const __grid_constant__ Shape sh, const float *__restrict__ bias, const TC *addsrc, long ldc, int *err_flag)
 {
-    using SL = Smem<BN>;
+    using SL = Smem;
     constexpr int ST = SL::STAGES;
     extern __shared__ unsigned char smraw_[];
     unsigned char *sm = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smraw_) + 1023) & ~(uintptr_t)1023);
@@ -453,17 +454,17 @@ struct Extra {
     void *C2 = nullptr;
 };
 constexpr int PAIRS = 74; // CTA pairs the chip holds (148 SMs)
-static int tile_count(int M, int N, int BN, const Extra &x)
+static int tile_count(int M, int N, const Extra &x)
 {
     const int hm = x.hole_m / 256, hn = x.hole_n / BN, mt = ceil_div(M, 256), nt = ceil_div(N, BN);
     return hm * (nt - hn) + (mt - hm) * nt;
 }
 
-template <int BN, typename TC, bool AMN, bool BMN>
+template <typename TC, bool AMN, bool BMN>
 static int launch(cudaStream_t st, int M, int N, int K, const bf16 *A, long lda, const bf16 *B, long ldb, TC *C, long ldc,
                   const float *bias, const TC *addsrc, int *err_flag, int bias_n, const Extra &x)
 {
-    using SL = Smem<BN>;
+    using SL = Smem;
     if (x.ksplit > 1 && (M % 256 || bias || addsrc || x.C2))
         return nncu_fail(NNCU_ERR_INVALID, "split-K needs whole row tiles and a bare product");
     CUtensorMap ma, mb, mc, mc2;
@@ -480,17 +481,17 @@ static int launch(cudaStream_t st, int M, int N, int K, const bf16 *A, long lda,
     if (x.C2)
         NNCU_TRY(tc::make_tmap(x.C2, M, N, ldc, 32, &mc2, 128 / (int)sizeof(TC), (int)sizeof(TC)));
     static DeviceOnce once;
-    NNCU_TRY(smem_limit(once, gemm_pair_kernel<BN, TC, AMN, BMN>, SL::TOTAL));
+    NNCU_TRY(smem_limit(once, gemm_pair_kernel<TC, AMN, BMN>, SL::TOTAL));
     Shape sh;
     sh.M = M; sh.N = N; sh.K = K;
     sh.hole_m = x.hole_m; sh.hole_n = x.hole_n; sh.skip_m = x.skip_m; sh.skip_k = x.skip_k;
     sh.ksplit = x.ksplit; sh.bias_n = bias_n; sh.act = x.C2 ? x.act : -1;
-    const int units = tile_count(M, N, BN, x) * x.ksplit;
+    const int units = tile_count(M, N, x) * x.ksplit;
     GemmProfiler *pr = g_nncu_prof;
     const bool timed = pr && pr->n < GemmProfiler::MAX_EV;
     if (timed)
         cudaEventRecord(pr->ev[2 * pr->n], st);
-    launch_k(gemm_pair_kernel<BN, TC, AMN, BMN>, dim3(2 * std::min(units, PAIRS)), dim3(384), SL::TOTAL, st, ma, mb, mc, mc2, sh, bias,
+    launch_k(gemm_pair_kernel<TC, AMN, BMN>, dim3(2 * std::min(units, PAIRS)), dim3(384), SL::TOTAL, st, ma, mb, mc, mc2, sh, bias,
              addsrc, ldc, err_flag);
     if (timed) {
         cudaEventRecord(pr->ev[2 * pr->n + 1], st);
@@ -503,7 +504,7 @@ static int launch(cudaStream_t st, int M, int N, int K, const bf16 *A, long lda,
 }
 
 // Whether the pair kernel (256-wide tiles) is the better one for an output.  Times of both kernels in us as
-// fitted to launches of 256..73728 rows (ncu, cold): a pair launch costs 9 and each round of tiles over
+// fitted to launches of 256..73728 rows (ncu, cold): a pair launch costs 8 and each round of tiles over
 // the 74 pairs 0.34 per 64-wide k-block plus 1 (the epilogue of the last is exposed, the others mostly
 // run under the next mainloop); the single-CTA kernel 1 plus, per round of CTAs, 4.4 + 0.13 per k-block
 // (64-wide tiles, one per SM) or 4.4 + 0.46 (128-wide, two per SM).  So the pair kernel takes outputs
@@ -513,10 +514,10 @@ template <typename TC> static bool pair_better(int M, int N, int K, const void *
 {
     if ((reinterpret_cast<uintptr_t>(C) & 15) || (ldc * sizeof(TC)) % 16 || (reinterpret_cast<uintptr_t>(addsrc) & 15))
         return false;
-    const double kb = ceil_div(K, BK), rounds = ceil_div(tile_count(M, N, 256, x), PAIRS);
+    const double kb = ceil_div(K, BK), rounds = ceil_div(tile_count(M, N, x), PAIRS);
     const double pair = 8.0 + rounds * (0.34 * kb + 1.0);
     const long mt = ceil_div(M, 128), c64 = mt * ceil_div(N, 64), c128 = mt * ceil_div(N, 128);
-    const bool wide = c128 >= 200 || N <= 64; // what tc::gemm takes
+    const bool wide = c128 >= 200 || N <= 64; // what tc::gemm takes, its 256-wide tiles (bf16 outputs of 200 and more) counted as 128-wide
     const double one = wide ? 1.0 + std::max(1.0, c128 / 296.0) * (4.4 + 0.46 * kb) : 1.0 + std::max(1.0, c64 / 148.0) * (4.4 + 0.13 * kb);
     return pair < one;
 }
@@ -536,7 +537,7 @@ static int gemm(cudaStream_t st, int M, int N, int K, const bf16 *A, long lda, c
     if (pair_better<TC>(M, N, K, C, ldc, addsrc, x)) {
         if (did_act)
             *did_act = x.C2 != nullptr;
-        return launch<256, TC, AMN, BMN>(st, M, N, K, A, lda, B, ldb, C, ldc, bias, addsrc, err_flag, bias_n, x);
+        return launch<TC, AMN, BMN>(st, M, N, K, A, lda, B, ldb, C, ldc, bias, addsrc, err_flag, bias_n, x);
     }
     return tc::gemm<TC, AMN, BMN>(st, M, N, K, A, lda, B, ldb, C, ldc, bias, addsrc, err_flag, bias_n);
 }

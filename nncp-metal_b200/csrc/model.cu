@@ -380,12 +380,12 @@ static int mm_tn(nncu_model *m, int Nout, int Kin, int R, const bf16 *dY, long l
         // A long contraction into few tiles (the projection's weight gradient over all memory rows) is split
         // over the idle pairs; the parts are added in order.  1536 x 512 x 73728: 176 us with one CTA per
         // 128 x 64 tile, 12 tiles of 256 x 256 on 74 pairs in six parts 78.
-        const int tiles = tc2::tile_count(Nout, Kin, 256, x), parts = tiles ? tc2::PAIRS / tiles : 1;
+        const int tiles = tc2::tile_count(Nout, Kin, x), parts = tiles ? tc2::PAIRS / tiles : 1;
         if (R >= 8192 && parts >= 2 && Nout % 256 == 0 && Kin % 4 == 0) {
             x.ksplit = std::min(parts, 8);
             const size_t n = (size_t)Nout * Kin;
             if (n * x.ksplit <= m->skw_side_floats) {
-                NNCU_TRY((tc2::launch<256, float, true, true>(st, Nout, Kin, R, dY, ldy, X, ldx, m->skw_side, Kin, nullptr, nullptr, m->err_flag,
+                NNCU_TRY((tc2::launch<float, true, true>(st, Nout, Kin, R, dY, ldy, X, ldx, m->skw_side, Kin, nullptr, nullptr, m->err_flag,
                                                               1 << 30, x)));
                 launch_k(splitk_reduce_kernel<float>, dim3((unsigned)ceil_div((long long)(n / 4), 256)), dim3(256), 0, st, m->skw_side, x.ksplit,
                          n, Gout);
@@ -459,7 +459,7 @@ static int colsum(nncu_model *m, const AT *A, long lda, int R, int N, float *out
     return reduce_cols(m, part, chunks, N, N, out, 0);
 }
 
-// Rows whose length is a multiple of 16 bytes and that fit a warp's registers (16 KB of them over the
+// Rows whose length is a multiple of 16 bytes and that fit a warp's registers (4 KB over the
 // lanes: up to 2048 bf16 or 1024 fp32 elements) go through the one-pass kernels; f(NC) launches the one
 // for NC 512-byte chunks.
 template <typename AT> static bool norm_in_registers(int D, int max_chunks)
@@ -596,7 +596,7 @@ static int run_graphed(nncu_model *m, int kind, F body)
 // Streams per cluster of the one-launch time step, 0 where the model is not one it takes: fp32, post-LN,
 // ungated feed-forward, rows that fit the norms' registers, slices of 16 without remainder.  One stream
 // per cluster while the clusters fit the chip together, then two and four (16 streams, one to a cluster:
-// the last cluster waited for the others, 156 us a step instead of 78); beyond that the launches it
+// the last cluster waited for the others and a step took twice as long as with two); beyond that the launches it
 // replaces have rows enough to fill the chip.
 static int step_streams(const nncu_model *m)
 {

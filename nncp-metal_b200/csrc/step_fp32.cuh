@@ -1,7 +1,7 @@
 // step_fp32.cuh -- the forward pass of one time step of a small fp32 model in one launch.
 //
 // A decoder runs the model one symbol per stream at a time: for the fp32 models of the lower levels
-// (2-4 layers, d_model 64-512, up to 64 streams) that was 37 launches of 3-5 us for 2 MFLOP a stream,
+// (fp32, post-LN, d_model up to 512 and like d_inner a multiple of 16, up to 56 streams) that was 37 launches of 3-5 us for 2 MFLOP a stream,
 // 128 us a step (16 streams, 4 layers of 256; 62 us now, the serial decoder's 10 us included).  Streams do not meet in the forward pass, so a cluster of eight CTAs takes SP of them
 // through the whole network by itself.  What bounds a step then is a chain: five exchanges of
 // activations a layer (projection, attention, output projection, feed-forward up and down) with short
@@ -117,7 +117,7 @@ __device__ __forceinline__ void await(uint32_t bar, uint32_t parity, volatile in
                      : "memory");
     if (!ok) {
         *abort_s = 1;
-        atomicExch(err_flag, 51);
+        atomicExch(err_flag, 61);
     }
 }
 
