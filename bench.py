@@ -13,8 +13,8 @@ streams are sharded across ranks and gradients are summed by NCCL all-reduces in
 `e2e`     the same steps through the host-buffer plugin calls: ids from pinned host memory
           every step, the coder-ready prob0 paths and the loss read back every step (encoder order:
           the next segment's forward pass is queued before the host waits for this segment's results).
-`roofline` the tcgen05 GEMM kernel: sum of 2*M*N*K over its launches / sum of their CUDA-event
-          durations, against the measured bf16 peak.
+`roofline` the tcgen05 GEMM kernels: sum of 2*M*N*K over their launches, less what a launch leaves out,
+          / sum of their CUDA-event durations, against the measured bf16 peak.
 `attention` the isolated attention op of BASELINE config[1] (forward, and forward + backward)
           through nncu_attention_forward / _backward: TFLOP/s and the fraction of its
           min(tensor, HBM) roofline.
@@ -783,12 +783,12 @@ def main():
         if pr.gemm_launches:
             ach = pr.gemm_flops / (pr.gemm_ms * 1e-3) / 1e12
             traffic = profile_traffic("gemm_tc_kernel_c2_dram_traffic.md") if (args.config == "c2" and world == 1) else None
-            roof = {"bound": "tensor", "kernel": "gemm_tc_kernel (tcgen05 bf16 GEMM, all operand arrangements)",
+            roof = {"bound": "tensor", "kernel": "gemm_tc_kernel and gemm_pair_kernel (tcgen05 bf16 GEMM, all operand arrangements)",
                     "achieved": ach, "peak": peak_tf, "unit": "TFLOP/s", "frac": ach / peak_tf,
                     "peak_source": f"{which} bf16_tflops_sustained",
                     "traffic": traffic,
                     "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum per launch, from the committed "
-                                      "profile summary of this kernel on this workload (not re-measured by this run)",
+                                      "profile summary of these kernels on this workload (not re-measured by this run)",
                     "launches_per_step": pr.gemm_launches / min(K, 3),
                     "share_of_step": (pr.gemm_ms / min(K, 3)) / (ms / K)}
     attn = None
