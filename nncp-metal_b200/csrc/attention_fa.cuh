@@ -4,7 +4,7 @@
 // Same math as attention.cuh (nncp.c:722-800 and its adjoint).  Per (stream, head) the
 // contractions are 64 queries x 64-key blocks x head size, a few hundred warp-level products; what
 // bounds the op is the chain load -> scores -> softmax -> product, not the tensor rate (measured
-// 544 TFLOP/s for mma.sync on this part, of which the op needs a quarter).  A warp's products need
+// 555 TFLOP/s for mma.sync on this part, of which the op needs a quarter).  A warp's products need
 // no hand-off through tensor memory and barriers, two CTAs share an SM, and the relative shift is a
 // 3 KB round trip through shared memory private to the warp.  The tcgen05 kernels these replace
 // spent 47 k cycles per 128-key block of a stream pair (64 streams x 16 heads, 320 keys: backward
