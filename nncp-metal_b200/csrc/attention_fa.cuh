@@ -650,7 +650,7 @@ __device__ __forceinline__ void ldsm4t_at(uint32_t (&r)[4], uint32_t at)
 // byte offset of 16-byte chunk c of row r in a tile
 __device__ __forceinline__ uint32_t tile_at(int r, int c) { return (uint32_t)((c >> 3) * 8192 + r * 128 + (((c & 7) ^ (r & 7)) << 4)); }
 
-template <int DK>
+template <int DK, bool WIDE> // WIDE: an fp32 table takes 16-byte loads
 __global__ void __launch_bounds__(128) attn_one_tma_kernel(const __grid_constant__ AttnArgs a, const __grid_constant__ CUtensorMap map_kv,
                                                            const __grid_constant__ CUtensorMap map_r, int stage_br)
 {
@@ -699,11 +699,19 @@ __global__ void __launch_bounds__(128) attn_one_tma_kernel(const __grid_constant
             const float *w32 = a.w_r + (size_t)h * a.P * DK;
             for (int idx = lane; idx < 64 * (DK / 8); idx += 32) {
                 const int r = idx / (DK / 8), c = idx % (DK / 8), x = min(max(x0 + r, 0), a.P - 1);
-                bf16 *dst = reinterpret_cast<bf16 *>(sm + SM::R + warp * TILE + tile_at(r, c));
-                if (a.w_r16)
-                    *reinterpret_cast<uint4 *>(dst) = *reinterpret_cast<const uint4 *>(w16 + (size_t)x * DK + c * 8);
-                else
-                    table_piece<false>(dst, w32 + (size_t)x * DK + c * 8);
+                if constexpr (WIDE) {
+                    uint4 v;
+                    if (a.w_r16) {
+                        v = *reinterpret_cast<const uint4 *>(w16 + (size_t)x * DK + c * 8);
+                    } else {
+                        const float4 u = *reinterpret_cast<const float4 *>(w32 + (size_t)x * DK + c * 8);
+                        const float4 w = *reinterpret_cast<const float4 *>(w32 + (size_t)x * DK + c * 8 + 4);
+                        v = make_uint4(pack2(u.x, u.y), pack2(u.z, u.w), pack2(w.x, w.y), pack2(w.z, w.w));
+                    }
+                    *reinterpret_cast<uint4 *>(sm + SM::R + warp * TILE + tile_at(r, c)) = v;
+                } else {
+                    table_piece<false>(reinterpret_cast<bf16 *>(sm + SM::R + warp * TILE + tile_at(r, c)), w32 + (size_t)x * DK + c * 8);
+                }
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); // a later round's tile may come by TMA to the same place
         }
@@ -1215,9 +1223,9 @@ inline int tile_map(const void *p, const cuuint64_t (&dims)[3], const cuuint64_t
 }
 template <int DK> static int forward_one(const AttnArgs &a, cudaStream_t st)
 {
-    static DeviceOnce once;
+    static DeviceOnce once[2];
     if constexpr (DK < 64) {
-        NNCU_TRY(smem_limit(once, attn_one_kernel<DK>, OneSmem<DK>::TOTAL));
+        NNCU_TRY(smem_limit(once[0], attn_one_kernel<DK>, OneSmem<DK>::TOTAL));
         launch_k(attn_one_kernel<DK>, dim3(a.B * a.H), dim3(128), OneSmem<DK>::TOTAL, st, a);
     } else {
         CUtensorMap kv, r;
@@ -1226,9 +1234,11 @@ template <int DK> static int forward_one(const AttnArgs &a, cudaStream_t st)
         r = kv;
         if (a.w_r16)
             NNCU_TRY(tile_map(a.w_r16, {DK, P, H}, {DK * 2, P * DK * 2}, false, &r));
-        NNCU_TRY(smem_limit(once, attn_one_tma_kernel<DK>, 226 * 1024)); // its barriers are static
+        const bool wide = a.w_r16 || aligned_to(a.w_r, 16);
+        auto kernel = wide ? attn_one_tma_kernel<DK, true> : attn_one_tma_kernel<DK, false>;
+        NNCU_TRY(smem_limit(once[wide], kernel, 226 * 1024)); // its barriers are static
         const size_t most = 226 * 1024, all = OneTmaSmem<DK>::bytes(a.L);
-        launch_k(attn_one_tma_kernel<DK>, dim3(a.B * a.H), dim3(128), all <= most ? all : OneTmaSmem<DK>::bytes(0), st, a, kv, r,
+        launch_k(kernel, dim3(a.B * a.H), dim3(128), all <= most ? all : OneTmaSmem<DK>::bytes(0), st, a, kv, r,
                  all <= most ? 1 : 0);
     }
     KERNEL_CHECK();
