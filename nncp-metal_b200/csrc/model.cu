@@ -1609,12 +1609,13 @@ int nncu_create(const nncu_params *p, nncu_model **out)
             return fail_cleanup(nncu_fail(NNCU_ERR_CUDA, "layer table upload failed"));
     }
     {
-        static DeviceOnce norm_f, norm_b, paths, trees, paths_any, trees_any;
+        static DeviceOnce norm_f, norm_b, paths, trees, paths_any, paths_any_wide, trees_any;
         int rc = smem_limit(norm_f, norm_bwd_kernel<float>, SMEM_MOST);
         rc = rc ? rc : smem_limit(norm_b, norm_bwd_kernel<bf16>, SMEM_MOST);
         rc = rc ? rc : smem_limit(paths, coder_paths_kernel, CODER_SMEM);
         rc = rc ? rc : smem_limit(trees, coder_trees_kernel, CODER_SMEM);
         rc = rc ? rc : smem_limit(paths_any, coder_paths_any_kernel, CODER_SMEM);
+        rc = rc ? rc : smem_limit(paths_any_wide, coder_paths_any_fast_kernel<5>, 16384 * 4); // the others' rows need no more than the default
         rc = rc ? rc : smem_limit(trees_any, coder_trees_any_kernel, CODER_SMEM);
         if (rc != NNCU_OK)
             return fail_cleanup(rc);
@@ -2170,7 +2171,9 @@ static int coder_paths_enqueue(nncu_model *m, int t0, int nt, const int32_t *sym
     cudaStream_t st = side_fork(m);
     CUDA_TRY(cudaMemcpyAsync(m->sym_dev, m->sym_pin, sizeof(int32_t) * rows, cudaMemcpyHostToDevice, st));
     CUDA_TRY(cudaEventRecord(m->ev_sym, st));
-    if (!pow2)
+    if (const PathsAnyKernel fast = pow2 ? nullptr : paths_any_fast(nb))
+        fast<<<rows, 256, (size_t)m->V * 4, st>>>(m->probs + (size_t)t0 * m->B * m->V, m->sym_dev, m->coder_dev, m->V);
+    else if (!pow2)
         coder_paths_any_kernel<<<rows, 256, (size_t)2 * P * 4, st>>>(m->probs + (size_t)t0 * m->B * m->V, m->sym_dev,
                                                                     m->coder_dev, m->V, P, nb);
     else if (m->V >= 1024 && m->V <= 16384)

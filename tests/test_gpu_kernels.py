@@ -153,3 +153,21 @@ def test_decoder_walk_of_improbable_branches(pkg, V):
         assert np.array_equal(got, want)
         dev.decoder_end()
         dev.close(); ref.close()
+
+
+@pytest.mark.parametrize("V", [257, 511, 514, 1027, 2050, 4099, 8191, 9208, 16383])
+def test_coder_paths_of_any_alphabet_by_subtrees(pkg, oracle, V):
+    """Every depth that the kernel of 256 subtrees takes (9 to 14), least and most two-symbol nodes, rows on and off
+    16-byte boundaries: the integers of write_sym, equal."""
+    m = pkg.TrfModel(pkg.abi.make_params(n_layer=1, d_model=64, n_head=2, d_key=32, d_inner=128, d_pos=16, mem_len=8, seg_len=8,
+                                         n_streams=3, n_symbols=V, init_range=0.5))
+    rng = np.random.default_rng(V)
+    ids, syms = (rng.integers(0, V, (8, 3)).astype(np.int32) for _ in range(2))
+    syms[0], syms[1] = [0, V - 1, V // 2], [V // 2 - 1, V // 256, V // 256 + 1]
+    probs, paths = m.eval(-1, ids), m.coder_paths(0, 8, syms)
+    for t in range(8):
+        for b in range(3):
+            want = oracle.sym_path(probs[t, b], syms[t, b])
+            got = paths[t * 3 + b]
+            assert np.array_equal(got[:len(want)], want) and not got[len(want):].any(), (t, b)
+    m.close()
