@@ -840,6 +840,182 @@ __global__ void __launch_bounds__(128) attn_one_tma_kernel(const __grid_constant
         a.lse[((size_t)b * a.H + h) * T + i] = m_run + logf(l);
 }
 
+// Many streams and heads: a warp of its own for every (stream, head), a CTA each, up to nine on an SM.  The four warps
+// of the kernel above meet twice a round and its CTAs take turns at loading and at computing; here nothing
+// meets, K and the table rows of the next block are on their way as soon as the scores are taken and V as soon as
+// its products are, and 128 streams x 8 heads are one wave.  128 x 8 pairs of 576
+// keys: 26.4 us, the kernel above 40.6, HBM 23.  Same association.
+template <int DK> struct OneWarpSmem {
+    static constexpr int NS = DK / 64, TILE = NS * 8192, K = 0, R = TILE, V = 2 * TILE, S = 3 * TILE, TOTAL = S + 64 * 4 + 1024;
+};
+template <int DK>
+__global__ void __launch_bounds__(32) attn_one_warp_kernel(const __grid_constant__ AttnArgs a, const __grid_constant__ CUtensorMap map_kv,
+                                                           const __grid_constant__ CUtensorMap map_r)
+{
+    using SM = OneWarpSmem<DK>;
+    constexpr int NS = SM::NS, TILE = SM::TILE, MT = DK / 16; // 16-column slices
+    extern __shared__ __align__(16) unsigned char smraw[];
+    __shared__ __align__(8) uint64_t bars[2]; // K and table, V
+    __shared__ int abort_s, dummy;
+    unsigned char *sm = smraw + ((1024u - (smem_addr(smraw) & 1023u)) & 1023u);
+    const int lane = threadIdx.x, g = lane >> 2, t = lane & 3;
+    const uint32_t base = smem_addr(sm), Kt = base + SM::K, Rt = base + SM::R, Vt = base + SM::V;
+    const uint32_t bar_k = smem_addr(bars), bar_v = smem_addr(bars + 1);
+    float *sc = reinterpret_cast<float *>(sm + SM::S);
+    const int b = blockIdx.x / a.H, h = blockIdx.x % a.H, HD = a.H * DK, T = a.T, M = a.M, L = a.L, i = a.t0;
+    const Blocks blk = blocks_of(M, L, a.attn_len, i, i + 1);
+    pdl_trigger();
+    if (lane == 0) {
+        abort_s = 0;
+        tc::mbar_init(bar_k, 1);
+        tc::mbar_init(bar_v, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncwarp();
+    pdl_wait();
+    int *ef = a.err_flag ? a.err_flag : &dummy;
+    bool ok = true; // this lane's waits: after one that ran out it issues no copy and waits no more
+    float br[4][2]; // of the block that is being fetched
+    auto fetch_kr = [&](int kb) {
+        if (kb > blk.hi)
+            return;
+        const int j0 = kb * KB, x0 = j0 - i + a.P - M - 1;
+        // rows below the table stand for row 0: such tiles are loaded by hand
+        const bool by_hand = a.w_r && x0 < 0;
+        if (lane == 0 && ok) {
+            const bool r = a.w_r && !by_hand;
+            tc::mbar_expect_tx(bar_k, (uint32_t)(r ? 2 * TILE : TILE));
+#pragma unroll
+            for (int n = 0; n < NS; n++) {
+                tma_load_3d(Kt + n * 8192, &map_kv, bar_k, h * DK + n * 64, b, j0);
+                if (r)
+                    tma_load_3d(Rt + n * 8192, &map_r, bar_k, n * 64, x0, h);
+            }
+        }
+        if (by_hand) {
+            const bf16 *w16 = reinterpret_cast<const bf16 *>(a.w_r16) + (size_t)h * a.P * DK;
+            for (int idx = lane; idx < 64 * (DK / 8); idx += 32) {
+                const int r = idx / (DK / 8), c = idx % (DK / 8), x = min(max(x0 + r, 0), a.P - 1);
+                *reinterpret_cast<uint4 *>(sm + SM::R + tile_at(r, c)) = *reinterpret_cast<const uint4 *>(w16 + (size_t)x * DK + c * 8);
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); // a later block's tile may come by TMA to the same place
+        }
+#pragma unroll
+        for (int m = 0; m < 4; m++)
+#pragma unroll
+            for (int c = 0; c < 2; c++)
+                br[m][c] = __ldg(a.b_r + (size_t)h * L + min(max(j0 + m * 16 + g + c * 8 + T - 1 - i, 0), L - 1));
+    };
+    auto fetch_v = [&](int kb) {
+        if (kb > blk.hi || lane != 0 || !ok)
+            return;
+        tc::mbar_expect_tx(bar_v, (uint32_t)TILE);
+#pragma unroll
+        for (int n = 0; n < NS; n++)
+            tma_load_3d(Vt + n * 8192, &map_kv, bar_v, HD + h * DK + n * 64, b, kb * KB);
+    };
+    fetch_kr(blk.lo);
+    fetch_v(blk.lo);
+    // the query as the second operand: k = 2t, 2t + 1 (+ 8) of every 16-wide slice, the same for all columns
+    uint32_t qf[DK / 16][2];
+    {
+        const bf16 *q = reinterpret_cast<const bf16 *>(a.q) + ((size_t)i * a.B + b) * a.qp + h * DK;
+#pragma unroll
+        for (int ks = 0; ks < DK / 16; ks++) {
+            qf[ks][0] = *reinterpret_cast<const uint32_t *>(q + ks * 16 + 2 * t);
+            qf[ks][1] = *reinterpret_cast<const uint32_t *>(q + ks * 16 + 8 + 2 * t);
+        }
+    }
+    float o[MT][4], m_run = -INFINITY, l = 0.0f; // l: the part of the sum that lane t of a quad keeps
+#pragma unroll
+    for (int m = 0; m < MT; m++)
+#pragma unroll
+        for (int c = 0; c < 4; c++)
+            o[m][c] = 0.0f;
+    uint32_t phase = 0;
+    for (int kb = blk.lo; kb <= blk.hi; kb++, phase ^= 1) {
+        const int j0 = kb * KB;
+        ok = ok && tc::mbar_wait(bar_k, phase, &abort_s, ef, 46); // K and the table rows
+        __syncwarp();
+        float mb = -INFINITY;
+#pragma unroll
+        for (int m = 0; m < 4; m++) {
+            float x[4] = {0.0f, 0.0f, 0.0f, 0.0f}, e[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            const int r = m * 16 + (lane & 15);
+#pragma unroll
+            for (int ks = 0; ks < DK / 16; ks++) {
+                uint32_t k4[4];
+                ldsm4_at(k4, Kt + tile_at(r, ks * 2 + (lane >> 4)));
+                mma(x, k4, qf[ks][0], qf[ks][1]);
+                if (a.w_r) {
+                    ldsm4_at(k4, Rt + tile_at(r, ks * 2 + (lane >> 4)));
+                    mma(e, k4, qf[ks][0], qf[ks][1]);
+                }
+            }
+#pragma unroll
+            for (int c = 0; c < 2; c++) {
+                const int j = j0 + m * 16 + g + c * 8, d = i + M - j;
+                const float v = (unsigned)d < (unsigned)a.attn_len ? score_of(x[2 * c], e[2 * c], __fmul_rn(a.br_scale, br[m][c]), a) : -INFINITY;
+                mb = fmaxf(mb, v);
+                if (t == 0)
+                    sc[m * 16 + g + c * 8] = v;
+            }
+        }
+        mb = fmaxf(mb, __shfl_xor_sync(0xffffffffu, mb, 4));
+        mb = fmaxf(mb, __shfl_xor_sync(0xffffffffu, mb, 8));
+        mb = fmaxf(mb, __shfl_xor_sync(0xffffffffu, mb, 16));
+        __syncwarp(); // the scores are there, K and the table rows have been read
+        fetch_kr(kb + 1);
+        const float n = fmaxf(m_run, mb), u = n == -INFINITY ? 0.0f : n, scale = __expf(__fsub_rn(m_run, u));
+        m_run = n;
+        float sum = 0.0f;
+        uint32_t pf[4][2];
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            const float2 v = *reinterpret_cast<const float2 *>(sc + k * 8 + 2 * t);
+            const float p0 = __expf(__fsub_rn(v.x, u)), p1 = __expf(__fsub_rn(v.y, u));
+            sum = __fadd_rn(sum, __fadd_rn(p0, p1));
+            pf[k >> 1][k & 1] = pack2(p0, p1);
+        }
+        l = __fmaf_rn(l, scale, sum);
+        ok = ok && tc::mbar_wait(bar_v, phase, &abort_s, ef, 47);
+        __syncwarp();
+#pragma unroll
+        for (int m = 0; m < MT; m++) {
+#pragma unroll
+            for (int c = 0; c < 4; c++)
+                o[m][c] = __fmul_rn(o[m][c], scale);
+#pragma unroll
+            for (int ks = 0; ks < 4; ks++) {
+                uint32_t v4[4]; // V^T: rows are columns of V, so the 8 x 8 blocks come transposed
+                ldsm4t_at(v4, Vt + tile_at(ks * 16 + (lane & 7) + (lane >> 4) * 8, m * 2 + ((lane >> 3) & 1)));
+                mma(o[m], v4, pf[ks][0], pf[ks][1]);
+            }
+        }
+        __syncwarp(); // V and the scores have been read
+        fetch_v(kb + 1);
+    }
+    if (lane == 0 && !ok) { // copies still in flight land in this CTA's shared memory: both phases get a bounded chance to finish
+        for (uint32_t parity = 0; parity < 2; parity++) {
+            tc::mbar_wait(bar_k, parity, &abort_s, ef, 46);
+            tc::mbar_wait(bar_v, parity, &abort_s, ef, 47);
+        }
+    }
+    __syncwarp();
+    l = __fadd_rn(l, __shfl_xor_sync(0xffffffffu, l, 1));
+    l = __fadd_rn(l, __shfl_xor_sync(0xffffffffu, l, 2));
+    const float inv = *static_cast<volatile int *>(&abort_s) ? __int_as_float(0x7fffffff) : __fdiv_rn(1.0f, l); // a wait ran out: no result
+    bf16 *out = reinterpret_cast<bf16 *>(a.o) + ((size_t)i * a.B + b) * HD + h * DK;
+#pragma unroll
+    for (int m = 0; m < MT; m++)
+        if (t == 0) {
+            out[m * 16 + g] = __float2bfloat16_rn(__fmul_rn(o[m][0], inv));
+            out[m * 16 + g + 8] = __float2bfloat16_rn(__fmul_rn(o[m][2], inv));
+        }
+    if (lane == 0 && a.lse)
+        a.lse[((size_t)b * a.H + h) * T + i] = m_run + logf(l);
+}
+
 // ---------------- backward ----------------
 //
 // One CTA of eight warps per (stream, head), key blocks in ascending order; per block
@@ -1221,6 +1397,10 @@ inline int tile_map(const void *p, const cuuint64_t (&dims)[3], const cuuint64_t
                     CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? NNCU_OK : nncu_fail(NNCU_ERR_CUDA, "cuTensorMapEncodeTiled failed: %d", (int)r);
 }
+// (stream, head) pairs from which a warp each is better than four: the warps have to fill the chip.  Steps of four
+// layers over 528 keys, with four warps and with one: head size 64, 256 pairs 177 / 203 us, 384 225 / 221, 768 294 / 270;
+// head size 128, 128 pairs 184 / 210 us, 256 252 / 244, 512 377 / 300.
+template <int DK> constexpr int one_warp_pairs() { return DK == 64 ? 384 : 256; }
 template <int DK> static int forward_one(const AttnArgs &a, cudaStream_t st)
 {
     static DeviceOnce once[2];
@@ -1234,6 +1414,13 @@ template <int DK> static int forward_one(const AttnArgs &a, cudaStream_t st)
         r = kv;
         if (a.w_r16)
             NNCU_TRY(tile_map(a.w_r16, {DK, P, H}, {DK * 2, P * DK * 2}, false, &r));
+        if (a.B * a.H >= one_warp_pairs<DK>() && (!a.w_r || a.w_r16)) {
+            static DeviceOnce once_warp;
+            NNCU_TRY(smem_limit(once_warp, attn_one_warp_kernel<DK>, OneWarpSmem<DK>::TOTAL));
+            launch_k(attn_one_warp_kernel<DK>, dim3(a.B * a.H), dim3(32), OneWarpSmem<DK>::TOTAL, st, a, kv, r);
+            KERNEL_CHECK();
+            return NNCU_OK;
+        }
         const bool wide = a.w_r16 || aligned_to(a.w_r, 16);
         auto kernel = wide ? attn_one_tma_kernel<DK, true> : attn_one_tma_kernel<DK, false>;
         NNCU_TRY(smem_limit(once[wide], kernel, 226 * 1024)); // its barriers are static

@@ -171,3 +171,27 @@ def test_coder_paths_of_any_alphabet_by_subtrees(pkg, oracle, V):
             got = paths[t * 3 + b]
             assert np.array_equal(got[:len(want)], want) and not got[len(want):].any(), (t, b)
     m.close()
+
+
+@pytest.mark.parametrize("kw", [
+    dict(d_model=256, n_head=4, d_key=64, d_pos=150, mem_len=130, seg_len=20, n_streams=130),                        # three key blocks
+    dict(d_model=256, n_head=4, d_key=64, d_pos=40, mem_len=130, seg_len=20, n_streams=130),                         # copies of table row 0
+    dict(d_model=256, n_head=2, d_key=128, d_pos=90, mem_len=64, seg_len=26, n_streams=256),
+    dict(d_model=256, n_head=2, d_key=128, d_pos=220, mem_len=200, seg_len=20, n_streams=256, attn_len=[70, 1]),     # windows
+    dict(d_model=128, n_head=2, d_key=64, d_pos=5, mem_len=0, seg_len=5, n_streams=256, use_w_r=0)])                 # one key, no table
+def test_one_query_by_a_warp_equals_whole_segment_bitwise(pkg, kw):
+    """Time steps of many streams: a warp for every (stream, head), against the segment kernel, bit for bit."""
+    p = pkg.abi.make_params(n_layer=2, d_inner=256, n_symbols=64, use_bf16=1, init_range=0.3, lr=1e-3, **kw)
+    T, B, V = p.seg_len, p.n_streams, p.n_symbols
+    rng = np.random.default_rng(5)
+    seg, one = pkg.TrfModel(p), pkg.TrfModel(p)
+    seg.reset(); one.reset()
+    for _ in range(3):
+        ids, tg = rng.integers(0, V, (T, B)).astype(np.int32), rng.integers(0, V, (T, B)).astype(np.int32)
+        a = seg.eval(-1, ids)
+        assert np.array_equal(a, np.concatenate([one.eval(t, ids) for t in range(T)]))
+        for m in (seg, one):
+            m.eval_gradient(tg)
+            m.update()
+        assert seg.weights_hash() == one.weights_hash()
+    seg.close(); one.close()
