@@ -275,7 +275,7 @@ template <int BN, typename TC, bool AMN, bool BMN>
 __global__ void __launch_bounds__(256, SmemLayout<BN>::CTAS_PER_SM)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                const __grid_constant__ CUtensorMap map_c, int staged, TC *C, long ldc, const float *__restrict__ bias, const TC *addsrc, int M, int N,
-               int K, int *err_flag, int bias_n)
+               int K, int *err_flag, int bias_n, int weights_ahead)
 {
     using SL = SmemLayout<BN>;
     extern __shared__ unsigned char smraw_[];
@@ -319,6 +319,26 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     fence_before_sync();
     __syncthreads();
     fence_after_sync();
+    constexpr bool DUAL = (SL::STAGES % 2) == 0;
+    constexpr int KSTEP = DUAL ? 2 : 1;
+    auto load_b = [&](uint32_t dst, uint32_t fb, int kx) {
+        if (BMN) {
+#pragma unroll
+            for (int nb = 0; nb < BN / 64; nb++)
+                tma_load_2d(dst + SL::A_BYTES + nb * 8192, &map_b, fb, n0 + nb * 64, kx);
+        } else {
+            tma_load_2d(dst + SL::A_BYTES, &map_b, fb, kx, n0);
+        }
+    };
+    // B is weights, which no kernel of this chain writes (embed_kernel, the first of a pass, lets its successors start only
+    // when what came before the pass is complete): the ring's first blocks of it are fetched before the wait.  Decoding
+    // with 128 streams, 12 layers of 512, where the keys and values of a step push the weights out of L2: 50.1 ->
+    // 48.9 ms a segment.
+    if (weights_ahead && !TC_MODE(1) && lane == 0 && (warp == 0 || (DUAL && warp == 7)))
+        for (int kb = warp == 0 ? 0 : 1; kb < min(nkb, SL::STAGES); kb += KSTEP) {
+            mbar_expect_tx(smem_u32(full + kb), SL::STAGE_BYTES);
+            load_b(smem_u32(sm) + kb * SL::STAGE_BYTES, smem_u32(full + kb), (kb_first + kb) * BK);
+        }
     // everything above (barriers, tensor-map prefetch, TMEM allocation) may overlap the tail of the
     // kernel before this one on the stream; from here on its results are read
     pdl_wait();
@@ -336,8 +356,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     // owns its own stages (even / odd k-blocks).  With an odd ring the pairs would share stages, and
     // a thread two rounds ahead of its partner would mistake the parity of a barrier that has not
     // completed once for a completion: there one thread loads and one issues, as before.
-    constexpr bool DUAL = (SL::STAGES % 2) == 0;
-    constexpr int KSTEP = DUAL ? 2 : 1;
     if (warp == 0 || (DUAL && warp == 7)) {
         if (lane == 0) {
             // warp 0 fills the stages of the even k-blocks, warp 7 those of the odd ones (a k-block
@@ -355,7 +373,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 if (TC_MODE(1)) {
                     mbar_expect_tx(fb, 0);
                 } else {
-                    mbar_expect_tx(fb, SL::STAGE_BYTES);
+                    const bool ahead = weights_ahead && kb < SL::STAGES;
+                    if (!ahead)
+                        mbar_expect_tx(fb, SL::STAGE_BYTES);
                     if (AMN) {
 #pragma unroll
                         for (int mb = 0; mb < BM / 64; mb++)
@@ -363,13 +383,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     } else {
                         tma_load_2d(dst, &map_a, fb, kx, m0);
                     }
-                    if (BMN) {
-#pragma unroll
-                        for (int nb = 0; nb < BN / 64; nb++)
-                            tma_load_2d(dst + SL::A_BYTES + nb * 8192, &map_b, fb, n0 + nb * 64, kx);
-                    } else {
-                        tma_load_2d(dst + SL::A_BYTES, &map_b, fb, kx, n0);
-                    }
+                    if (!ahead)
+                        load_b(dst, fb, kx);
                 }
                 s += KSTEP;
                 if (s >= SL::STAGES)
@@ -690,7 +705,7 @@ static bool usable(const void *A, long lda, const void *B, long ldb, int K)
 template <int BN, typename TC, bool AMN, bool BMN>
 static int launch(cudaStream_t st, int M, int N, int K, const bf16 *A, long lda, const bf16 *B,
                   long ldb, TC *C, long ldc, const float *bias, const TC *addsrc, int *err_flag, int bias_n,
-                  int ksplit = 1)
+                  int ksplit = 1, bool weights = false)
 {
     using SL = SmemLayout<BN>;
     if (ksplit > 1 && (M % BM != 0 || bias || addsrc))
@@ -728,11 +743,11 @@ static int launch(cudaStream_t st, int M, int N, int K, const bf16 *A, long lda,
 
 // A: [M][K] (lda) or, AMN, [K][M]; B: [N][K] (ldb) or, BMN, [K][N].  C bf16 or fp32; addsrc
 // (may be NULL, may alias C) is added to the product.  err_flag: device int raised when a
-// bounded wait expires.
+// bounded wait expires.  weights: B is one of the model's matrices.
 template <typename TC, bool AMN, bool BMN>
 static int gemm(cudaStream_t st, int M, int N, int K, const bf16 *A, long lda, const bf16 *B,
                 long ldb, TC *C, long ldc, const float *bias, const TC *addsrc, int *err_flag,
-                int bias_n = 1 << 30)
+                int bias_n = 1 << 30, bool weights = false)
 {
     if (M <= 0 || N <= 0)
         return NNCU_OK;
@@ -758,10 +773,10 @@ static int gemm(cudaStream_t st, int M, int N, int K, const bf16 *A, long lda, c
         f32_wide = (e && e[0] == '1') ? 1 : 0;
     }
     if (mt * ceil_div(N, 256) >= min_tiles && (sizeof(TC) == 2 || f32_wide))
-        return launch<256, TC, AMN, BMN>(st, M, N, K, A, lda, B, ldb, C, ldc, bias, addsrc, err_flag, bias_n);
+        return launch<256, TC, AMN, BMN>(st, M, N, K, A, lda, B, ldb, C, ldc, bias, addsrc, err_flag, bias_n, 1, weights);
     if (mt * ceil_div(N, 128) >= min_tiles || N <= 64)
-        return launch<128, TC, AMN, BMN>(st, M, N, K, A, lda, B, ldb, C, ldc, bias, addsrc, err_flag, bias_n);
-    return launch<64, TC, AMN, BMN>(st, M, N, K, A, lda, B, ldb, C, ldc, bias, addsrc, err_flag, bias_n);
+        return launch<128, TC, AMN, BMN>(st, M, N, K, A, lda, B, ldb, C, ldc, bias, addsrc, err_flag, bias_n, 1, weights);
+    return launch<64, TC, AMN, BMN>(st, M, N, K, A, lda, B, ldb, C, ldc, bias, addsrc, err_flag, bias_n, 1, weights);
 }
 
 // Long contractions with few output tiles (the output head's dX: K = n_symbols): `ksplit` CTAs

@@ -14,8 +14,8 @@ template <typename T>
 __global__ void embed_kernel(const int32_t *__restrict__ ids, const float *__restrict__ embed,
                              T *__restrict__ x, int rows, int D, float mult, int V)
 {
-    pdl_trigger();
     pdl_wait();
+    pdl_trigger(); // behind the wait: the GEMM that follows reads weights before its own, and an update may precede this kernel
     int r = blockIdx.x;
     if (r >= rows)
         return;

@@ -271,8 +271,11 @@ static int mm_nt_impl(nncu_model *m, int M, int N, int K, const bf16 *A, long ld
                       TC *C, long ldc, const float *bias, int bias_n, const tc2::Extra &x, bool *did_act)
 {
     const bf16 *Wt = m->Wb + w_off;
-    if (m->use_tc && tc::usable(A, lda, Wt, K, K))
-        return tc2::gemm<TC, false, false>(m->st, M, N, K, A, lda, Wt, K, C, ldc, bias, nullptr, m->err_flag, bias_n, x, did_act);
+    if (m->use_tc && tc::usable(A, lda, Wt, K, K)) {
+        tc2::Extra xw = x;
+        xw.weights = true;
+        return tc2::gemm<TC, false, false>(m->st, M, N, K, A, lda, Wt, K, C, ldc, bias, nullptr, m->err_flag, bias_n, xw, did_act);
+    }
     return gemm_simt<bf16, bf16, TC>(m->st, GEMM_NT, M, N, K, A, lda, Wt, K, C, ldc, bias, (const TC *)nullptr, bias_n);
 }
 template <typename AT, typename TC>
@@ -318,8 +321,10 @@ static int mm_nn(nncu_model *m, int M, int Kin, int Nout, const bf16 *dY, long l
             KERNEL_CHECK();
             return NNCU_OK;
         }
+        tc2::Extra xw;
+        xw.weights = true;
         return tc2::gemm<bf16, false, true>(m->st, M, Kin, Nout, dY, ldy, m->Wb + w_off, Kin, C, ldc, nullptr,
-                                           addsrc, m->err_flag);
+                                           addsrc, m->err_flag, 1 << 30, xw);
     }
     const bf16 *WT = m->WbT + w_off; // [Kin][Nout]
     if (m->use_tc && tc::usable(dY, ldy, WT, Nout, Nout))
