@@ -195,3 +195,26 @@ def test_one_query_by_a_warp_equals_whole_segment_bitwise(pkg, kw):
             m.update()
         assert seg.weights_hash() == one.weights_hash()
     seg.close(); one.close()
+
+
+@pytest.mark.parametrize("mode,M,N,K", [(0, 2048, 1024, 1024), (0, 2000, 1000, 72), (1, 1930, 1032, 136), (2, 2056, 1000, 1096), (0, 18900, 72, 520),
+                                        (0, 2041, 1016, 8)])
+@pytest.mark.parametrize("c_f32", [0, 1])
+def test_one_round_gemm_vs_fp32(pkg, mode, M, N, K, c_f32):
+    """Outputs of 75 to 148 tiles of 128 x 128, one to an SM: ragged edges, one k-block to more than the ring holds, and
+    the rows of a launch that takes narrower tiles."""
+    lib = pkg.library()
+    g = torch.Generator(device="cuda").manual_seed(M + N + K + mode)
+    a = torch.randn((K, M) if mode == 2 else (M, K), generator=g, device="cuda").bfloat16()
+    b = torch.randn((N, K) if mode == 0 else (K, N), generator=g, device="cuda").bfloat16()
+    ref = (a.float().T if mode == 2 else a.float()) @ (b.float().T if mode == 0 else b.float())
+    c = torch.full((M, N), float("nan"), device="cuda", dtype=torch.float32 if c_f32 else torch.bfloat16)
+    assert lib.nncu_gemm_bf16(pkg.abi.GEMM_TCGEN05, mode, M, N, K, a.data_ptr(), a.shape[1], b.data_ptr(), b.shape[1],
+                              c.data_ptr(), N, c_f32, None) == 0, lib.nncu_last_error()
+    assert (c.float() - ref).abs().max().item() < (5e-5 if c_f32 else 5e-3) * ref.abs().max().item()
+    if mode == 0:
+        part = torch.zeros(40, N, device="cuda", dtype=c.dtype)
+        off = M - 40
+        assert lib.nncu_gemm_bf16(pkg.abi.GEMM_TCGEN05, 0, 40, N, K, a[off:].data_ptr(), K, b.data_ptr(), K,
+                                  part.data_ptr(), N, c_f32, None) == 0, lib.nncu_last_error()
+        assert torch.equal(part, c[off:])
