@@ -726,14 +726,14 @@ static int launch(cudaStream_t st, int M, int N, int K, const bf16 *A, long lda,
     if (staged)
         NNCU_TRY(make_tmap(C, (long)M * ksplit, N, ldc, 32, &mc, 128 / (int)sizeof(TC), (int)sizeof(TC)));
     static DeviceOnce once;
-    NNCU_TRY(smem_limit(once, gemm_tc_kernel<BN, TC, AMN, BMN>, SL::TOTAL));
+    NNCU_TRY(smem_limit(once, gemm_tc_kernel<BN, TC, AMN, BMN, DEEP>, SL::TOTAL));
     dim3 grid(ceil_div(N, BN), ceil_div(M, BM), ksplit);
     GemmProfiler *pr = g_nncu_prof;
     const bool timed = pr && pr->n < GemmProfiler::MAX_EV;
     if (timed)
         cudaEventRecord(pr->ev[2 * pr->n], st);
-    launch_k(gemm_tc_kernel<BN, TC, AMN, BMN>, dim3(grid), dim3(256), SL::TOTAL, st, ma, mb, mc, staged, C, ldc, bias, addsrc,
-             M, N, K, err_flag, bias_n);
+    launch_k(gemm_tc_kernel<BN, TC, AMN, BMN, DEEP>, dim3(grid), dim3(256), SL::TOTAL, st, ma, mb, mc, staged, C, ldc, bias, addsrc,
+             M, N, K, err_flag, bias_n, weights ? 1 : 0);
     if (timed) {
         cudaEventRecord(pr->ev[2 * pr->n + 1], st);
         pr->flops[pr->n++] = 2.0 * M * N * K;
