@@ -254,9 +254,31 @@ template <int W, typename T> __device__ __forceinline__ void store_w(T *p, const
         p[w] = from_f<T>(v[w]);
 }
 
-// One CTA per (stream, head): the whole problem sits in shared memory and what bounds it is the rate
-// of shared-memory reads, so every inner loop reads W = 4 elements per access (head sizes that are
-// a multiple of four; W = 1 otherwise) and each gradient row is a register tile of W columns.
+// A cluster of 1 to 8 CTAs per (stream, head).  The whole problem sits in the shared memory of each: a CTA takes
+// every C-th group of eight query rows, writes their P and dS into all of the cluster's copies, and after the
+// cluster's barrier every C-th part of the results; association and bits do not depend on C.  What bounds a CTA
+// is the rate of shared-memory reads, so every inner loop reads W = 4 elements per access (head sizes that are
+// a multiple of four; W = 1 otherwise) and each gradient row is a register tile of W columns.  One CTA per
+// (stream, head) left the chip to 16 CTAs (4 streams x 4 heads of 32, 32 queries over 64 keys: 29 us a launch; a step of two
+// such layers 208 -> 192 us with four) or to 128 of eight warps (16 x 8 heads: 27 us; a step of four layers 772 -> 739 us
+// with two, and eight queries a CTA in the forward kernel).
+__device__ __forceinline__ uint32_t cluster_rank()
+{
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+// the address of `p` in the shared memory of CTA `rank` of the cluster
+__device__ __forceinline__ uint32_t peer_addr(const void *p, uint32_t rank)
+{
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void peer_store(uint32_t at, float v)
+{
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(at), "f"(v) : "memory");
+}
 template <typename T, int W>
 __global__ void __launch_bounds__(256) attn_bwd_kernel(AttnArgs a)
 {
@@ -276,8 +298,12 @@ __global__ void __launch_bounds__(256) attn_bwd_kernel(AttnArgs a)
     float *Dr = dS + (size_t)Tn * (L + 1);              // [T]: D_i, later the row's sum over the left pad
     const int ls = L + 1;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int C = gridDim.y, rank = C > 1 ? (int)cluster_rank() : 0; // the cluster lies along y
     const int b = blockIdx.x / a.H, h = blockIdx.x % a.H;
     const int HD = a.H * dk;
+    const int tid = rank * blockDim.x + threadIdx.x, nthr = C * blockDim.x; // of the cluster
+    if (C > 1) // the others are there before anything is written to them
+        asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");
     pdl_trigger();
     pdl_wait();
 
@@ -292,8 +318,10 @@ __global__ void __launch_bounds__(256) attn_bwd_kernel(AttnArgs a)
     if (a.w_r)
         stage_rows(Rs, ks, a.w_r + (size_t)h * P * dk, (size_t)dk, P, dk);
     __syncthreads();
+    if (C > 1)
+        asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
     // P and dS, zero where the pair is masked
-    for (int i = warp; i < Tn; i += 8) {
+    for (int i = rank * 8 + warp; i < Tn; i += 8 * C) {
         // D_i = dO_i . O_i  (= sum_j P_ij dP_ij)
         float D = 0.0f;
         for (int e = lane; e < dk; e += 32)
@@ -311,23 +339,33 @@ __global__ void __launch_bounds__(256) attn_bwd_kernel(AttnArgs a)
                 p = expf(score_ij<T>(i, j, Tn, L, P, dk, a.inv_sqrt, a.br_scale, qf, Ks, a.w_r ? Rs : nullptr, ks, a.b_r + (size_t)h * L) - lse);
                 d = p * (dot_q<T>(dof, Vs + (size_t)j * vs, dk) - D) * a.inv_sqrt;
             }
-            Pm[(size_t)i * ls + j] = p;
-            dS[(size_t)i * ls + j] = d;
+            if (C == 1) {
+                Pm[(size_t)i * ls + j] = p;
+                dS[(size_t)i * ls + j] = d;
+            } else {
+                for (int c = 0; c < C; c++) {
+                    peer_store(peer_addr(Pm + (size_t)i * ls + j, c), p);
+                    peer_store(peer_addr(dS + (size_t)i * ls + j, c), d);
+                }
+            }
             if (j <= jpad)
                 pad += d;
         }
         pad = warp_sum(pad);
-        if (lane == 0)
-            Dr[i] = pad;
+        if (lane < C)
+            peer_store(peer_addr(Dr + i, lane), pad);
     }
-    __syncthreads();
+    if (C > 1)
+        asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+    else
+        __syncthreads();
     const int nw = dk / W; // column groups
     const bool vec = (reinterpret_cast<uintptr_t>(a.dkv) & (4 * sizeof(T) - 1)) == 0 && (reinterpret_cast<uintptr_t>(a.dq) & (4 * sizeof(T) - 1)) == 0 &&
                      a.dkvp % 4 == 0 && a.dqp % 4 == 0;
     // dV[j] = sum_i P_ij dO_i ; dK[j] = sum_i dS_ij q_i     (i ascending), two keys per thread
     T *dkv = reinterpret_cast<T *>(a.dkv) + (size_t)b * a.dkvp + h * dk;
     const int half = (L + 1) / 2;
-    for (int idx = threadIdx.x; idx < half * nw; idx += blockDim.x) {
+    for (int idx = tid; idx < half * nw; idx += nthr) {
         const int j0 = idx / nw, e = (idx - j0 * nw) * W, j1 = j0 + half < L ? j0 + half : j0;
         float av[2][W] = {}, ak[2][W] = {};
 #pragma unroll 4
@@ -356,7 +394,7 @@ __global__ void __launch_bounds__(256) attn_bwd_kernel(AttnArgs a)
     }
     // dQ[i] = sum_j dS_ij (k_j + w_r[pi(i,j)])               (j ascending)
     T *dq = reinterpret_cast<T *>(a.dq) + (size_t)b * a.dqp + h * dk;
-    for (int idx = threadIdx.x; idx < Tn * nw; idx += blockDim.x) {
+    for (int idx = tid; idx < Tn * nw; idx += nthr) {
         const int i = idx / nw, e = (idx - i * nw) * W;
         int jlo, jhi;
         key_range(a, i, jlo, jhi);
@@ -385,7 +423,7 @@ __global__ void __launch_bounds__(256) attn_bwd_kernel(AttnArgs a)
     // row 0 the whole left pad
     if (a.w_r && a.dwr_part) {
         float *dst = a.dwr_part + ((size_t)b * a.H + h) * P * dk;
-        for (int idx = threadIdx.x; idx < P * nw; idx += blockDim.x) {
+        for (int idx = tid; idx < P * nw; idx += nthr) {
             const int p = idx / nw, e = (idx - p * nw) * W, j0 = p + L - P - (Tn - 1);
             float acc[W] = {};
 #pragma unroll 4
@@ -408,7 +446,7 @@ __global__ void __launch_bounds__(256) attn_bwd_kernel(AttnArgs a)
     }
     if (a.dbr_part) {
         float *dst = a.dbr_part + ((size_t)b * a.H + h) * L;
-        for (int r = threadIdx.x; r < L; r += blockDim.x) {
+        for (int r = tid; r < L; r += nthr) {
             float acc = 0.0f;
 #pragma unroll 4
             for (int i = 0; i < Tn; i++) {
@@ -485,10 +523,11 @@ static int attn_forward_t(const nncu_attn_shape *s, const void *q, const void *k
     AttnArgs a = attn_args(s, pt);
     a.q = q; a.kv = kv; a.w_r = w_r; a.b_r = b_r; a.o = out; a.lse = lse;
     const int nq = a.t1 - a.t0;
-    // enough CTAs to fill the GPU, but at least 8 queries (one per warp) per CTA
-    int chunks = max(1, min(ceil_div(nq, 8), ceil_div(2 * 148, a.B * a.H)));
-    a.qchunk = ceil_div(nq, chunks);
-    chunks = ceil_div(nq, a.qchunk);
+    // Eight queries (one per warp) a CTA while four CTAs per SM take them all, else whole rounds of eight for two per
+    // SM (32 queries of 16 x 8 heads went in chunks of 11, two rounds of the warps)
+    const long heads = (long)a.B * a.H;
+    a.qchunk = heads * ceil_div(nq, 8) <= 4 * 148 ? 8 : (ceil_div(nq, max(1, ceil_div(2 * 148, heads))) + 7) & ~7;
+    const int chunks = ceil_div(nq, a.qchunk);
     size_t smem = 0;
     a.smem_pitch = fwd_pitch<T>(a, w_r != nullptr, smem);
     if (smem > 227 * 1024)
@@ -518,7 +557,24 @@ static int attn_backward_t(const nncu_attn_shape *s, const void *q, const void *
     auto kernel = a.dk % 4 == 0 ? attn_bwd_kernel<T, 4> : attn_bwd_kernel<T, 1>;
     static DeviceOnce once[2];
     NNCU_TRY(smem_limit(once[a.dk % 4 == 0 ? 0 : 1], kernel, SMEM_MOST));
-    launch_k(kernel, dim3(a.B * a.H), dim3(256), smem, st, a);
+    // as many CTAs per (stream, head) as two to an SM hold, each with a query row for every warp
+    int C = 1;
+    while (C < 8 && 2 * C * a.B * a.H <= 2 * 148 && 2 * C * 8 <= a.T)
+        C *= 2;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(a.B * a.H, C);
+    cfg.blockDim = dim3(256);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = attr[0].val.clusterDim.z = 1;
+    attr[0].val.clusterDim.y = C;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = nncu_pdl_enabled() ? 2 : 1;
+    CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, a));
     KERNEL_CHECK();
     return NNCU_OK;
 }

@@ -218,3 +218,11 @@ def test_one_round_gemm_vs_fp32(pkg, mode, M, N, K, c_f32):
         assert lib.nncu_gemm_bf16(pkg.abi.GEMM_TCGEN05, 0, 40, N, K, a[off:].data_ptr(), K, b.data_ptr(), K,
                                   part.data_ptr(), N, c_f32, None) == 0, lib.nncu_last_error()
         assert torch.equal(part, c[off:])
+
+
+@pytest.mark.parametrize("B,H,dk,T,M,P,alen", [(1, 1, 16, 64, 20, 84, 0), (2, 2, 32, 40, 30, 50, 0), (3, 2, 8, 16, 40, 56, 21), (1, 3, 6, 15, 9, 20, 0),
+                                               (75, 2, 8, 16, 5, 21, 0), (37, 2, 16, 33, 8, 41, 0), (1, 2, 32, 32, 1, 33, 2)])
+def test_fp32_attention_by_clusters(pkg, oracle, B, H, dk, T, M, P, alen):
+    """One to eight CTAs per (stream, head): as many as the shape gives, rows and results that do not divide evenly.  (Of a window of
+    one key the gradients of queries and keys are rounding only: dS = P (dP - D) is zero.)"""
+    _attn_case(pkg, oracle, B, H, dk, T, M, P, alen, False, 9)
