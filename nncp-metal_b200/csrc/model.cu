@@ -133,6 +133,10 @@ struct TransposeJob {
 
 constexpr int SPLITK = 4, SPLITK_MIN_K = 8192; // split-K of the output head's dX GEMM
 
+// Buffers of the backward pass that the side stream reads exist twice, a layer's gradients of the residual stream
+// three times: the main stream goes on with layer l - 1 while the side stream is still at layer l, and waits for it
+// only before layer l - 2 (side_release).
+constexpr int POOL = 4, POOLS = 3 * POOL;
 struct nncu_model {
     nncu_params p;
     int D, H, dk, HD, F, F1, T, B, M, L, V, TB, LB, Bt, nl;
@@ -142,7 +146,7 @@ struct nncu_model {
     int device;
     cudaStream_t st, own_st = nullptr; // own_st: made by nncu_own_stream
     cudaStream_t st2;            // weight-gradient GEMMs run here, beside the dX chain
-    cudaEvent_t ev_fork, ev_join;
+    cudaEvent_t ev_fork, ev_join, ev_side[2]; // ev_side: the side stream is done with a layer's operands (by layer parity)
     bool overlap;
     // CUDA graphs of the whole-segment forward and of the backward pass, one per memory twin
     struct StepGraph {
@@ -184,22 +188,22 @@ struct nncu_model {
     char *hcat[2];
     int cur;
     std::vector<LayerAct> act;
-    void *xlast, *xf, *pool[4], *dz, *dh, *dhp, *dof, *dqkv, *tA, *tB;
-    float *st_f, *probs, *dwr_part, *dbr_part, *part, *logp, *loss_dev;
+    void *xlast, *xf, *pool[POOLS], *dz, *dh, *dhp[2], *dof, *dqkv[2], *tA, *tB;
+    float *st_f, *probs, *dwr_part[2], *dbr_part[2], *part, *logp, *loss_dev;
     size_t part_floats = 0; // floats per region of `part`
     // Split-K workspaces: skw for products on the main stream (the output head's dX), skw_side for weight
     // gradients, which run on the side stream beside them.  Two regions, because nothing orders the head's
     // dX, queued on the main stream, behind the head's weight gradient, queued on the side stream before it.
     float *skw = nullptr, *skw_side = nullptr;
     size_t skw_floats = 0, skw_side_floats = 0;
-    int part_idx = 0;       // regions handed out since the last join
+    int part_idx = 0, part_half = 0; // regions handed out in this layer, of which half
     ReduceJobs rjobs;       // column / stream reductions queued since the last flush (one launch per layer)
     int rjob_blocks = 0;
     bool fuse_update = false; // this backward pass applies the optimizer to each bucket as it completes
     float *hyper_dev = nullptr; // {lr, bias correction} of the fused optimizer step
     int32_t *ids_dev, *tgt_dev;
-    void *dt_ff = nullptr, *dt_at = nullptr; // LN_COEF: alpha * d(residual sum) of the two sub-layers, [TB][D]
-    float *alpha_part = nullptr;             // LN_COEF: per-row shares of d alpha, [2][TB]
+    void *dt_ff[2] = {}, *dt_at[2] = {}; // LN_COEF: alpha * d(residual sum) of the two sub-layers, [TB][D]
+    float *alpha_part[2] = {};           // LN_COEF: per-row shares of d alpha, [2][TB]
     int32_t *sym_dev;   // [TB] symbols whose coder paths are wanted (nncu_coder_paths*)
     int32_t *tgt_fixed; // the targets whose entries of dz carry the (p - 1) correction
     int *dz_fixed;      // device flag: dz has been corrected since the last forward pass
@@ -348,20 +352,31 @@ static cudaStream_t side_fork(nncu_model *m)
 }
 static void side_join(nncu_model *m)
 {
-    m->part_idx = 0;
     if (!m->overlap || g_nncu_prof)
         return;
     cudaEventRecord(m->ev_join, m->st2);
     cudaStreamWaitEvent(m->st, m->ev_join, 0);
 }
+// The end of a layer's backward pass: the side stream's work on it is marked, and the main stream waits for the
+// layer before (l + 1), whose buffers layer l - 1 takes.  With a join at every layer the main stream stood still for
+// the projection's weight gradient and two reductions, up to 20 us of a layer
+// (12 layers of 512, 2048 rows: 2543 -> 2489 us; 2 layers of 128: 205 -> 194).
+static void side_release(nncu_model *m, int l)
+{
+    if (!m->overlap || g_nncu_prof)
+        return;
+    cudaEventRecord(m->ev_side[l & 1], m->st2);
+    if (l + 1 < m->nl)
+        cudaStreamWaitEvent(m->st, m->ev_side[(l + 1) & 1], 0);
+}
 // Partial column sums go to one of PART_SLOTS scratch regions, so that the kernel that reduces
 // them can run on the side stream while the main stream's next kernel fills another region.
-// At most nine regions are taken between two joins (output bias, final norm, four norms, the
-// activation, two bias sums); a join makes all of them free again.
+// At most nine regions are taken in a layer (output bias and final norm before the first, four norms, the
+// activation, two bias sums); the layers take the two halves in turn.
 constexpr int PART_SLOTS = 10;
 static float *part_slot(nncu_model *m)
 {
-    float *p = m->part + (size_t)(m->part_idx % PART_SLOTS) * m->part_floats;
+    float *p = m->part + (size_t)((m->part_half * PART_SLOTS) + m->part_idx % PART_SLOTS) * m->part_floats;
     m->part_idx++;
     return p;
 }
@@ -882,16 +897,18 @@ static int bucket_layers(nncu_model *m)
 
 // ------------------------------------------------------------------ backward
 
+// a buffer of the set of layer l that is none of `used`
 template <typename AT>
-static AT *pick(nncu_model *m, std::initializer_list<const void *> used)
+static AT *pick(nncu_model *m, int l, std::initializer_list<const void *> used)
 {
-    for (int i = 0; i < 4; i++) {
+    for (int i = 0; i < POOL; i++) {
+        void *p = m->pool[l % 3 * POOL + i];
         bool taken = false;
         for (const void *u : used)
-            if (u == m->pool[i])
+            if (u == p)
                 taken = true;
         if (!taken)
-            return reinterpret_cast<AT *>(m->pool[i]);
+            return reinterpret_cast<AT *>(p);
     }
     return nullptr;
 }
@@ -904,11 +921,7 @@ static int backward(nncu_model *m)
     const int TB = m->TB, LB = m->LB;
     const bool pre = p.ln_flags & NNCU_LN_PRE, post = p.ln_flags & NNCU_LN_POST;
     AT *dz = reinterpret_cast<AT *>(m->dz);
-    AT *dh = reinterpret_cast<AT *>(m->dh), *dhp = reinterpret_cast<AT *>(m->dhp);
-    AT *dof = reinterpret_cast<AT *>(m->dof);
-    // [L*B][dq | dk | dv]; the dq columns of the memory rows are never written and stay zero
-    AT *dqkv = reinterpret_cast<AT *>(m->dqkv);
-    AT *dq = dqkv + (size_t)M * B * 3 * HD, *dkv = dqkv + HD;
+    AT *dh = reinterpret_cast<AT *>(m->dh), *dof = reinterpret_cast<AT *>(m->dof);
     const AttnPitch pt = {3 * HD, 3 * HD, 3 * HD, 3 * HD};
 
     // loss and d logits (nncp.c:1170-1175)
@@ -930,13 +943,15 @@ static int backward(nncu_model *m)
     // the norm that produces it takes them along
     auto bias2_of = [&](int l) { return l >= 0 && m->lo[l].ff_bias2 != NONE && m->lo[l].alpha == NONE ? gf(m, m->lo[l].ff_bias2) : nullptr; };
     bool bias2_done = false;
+    m->part_half = (m->nl - 1) & 1; // the last layer's: their reductions are its flush
+    m->part_idx = 0;
     if (m->out_bias != NONE)
         NNCU_TRY(colsum<AT>(m, dz, V, TB, V, gf(m, m->out_bias)));
     NNCU_TRY(mm_tn(m, V, D, TB, dz, V, xf, D, gf(m, m->embed_out)));
-    AT *dx = pick<AT>(m, {});
+    AT *dx = pick<AT>(m, m->nl, {});
     NNCU_TRY(mm_nn(m, TB, D, V, dz, V, m->embed_out, dx, D, (const AT *)nullptr));
     if (p.ln_flags & NNCU_LN_FINAL) {
-        AT *t = pick<AT>(m, {dx});
+        AT *t = pick<AT>(m, m->nl, {dx});
         NNCU_TRY(norm_bwd<AT>(m, dx, atc<AT>(m->xlast, 0), m->ln_g, m->ln_b, m->st_f, nullptr, t, TB,
                               pre ? bias2_of(m->nl - 1) : nullptr));
         bias2_done = pre;
@@ -952,11 +967,20 @@ static int backward(nncu_model *m)
         const LayerOff &o = m->lo[l];
         LayerAct &a = m->act[l];
         const AT *hc = reinterpret_cast<const AT *>(hcat_layer(m, m->cur, l));
+        const int half = l & 1;
+        if (l < m->nl - 1) {
+            m->part_half = half;
+            m->part_idx = 0;
+        }
+        AT *dhp = reinterpret_cast<AT *>(m->dhp[half]);
+        // [L*B][dq | dk | dv]; the dq columns of the memory rows are never written and stay zero
+        AT *dqkv = reinterpret_cast<AT *>(m->dqkv[half]), *dq = dqkv + (size_t)M * B * 3 * HD, *dkv = dqkv + HD;
+        float *dwr_part = m->dwr_part[half], *dbr_part = m->dbr_part[half], *alpha_part = m->alpha_part[half];
         // ---- feed-forward block
         AT *ds2 = dx;
         const bool coef = o.alpha != NONE;
         if (post) {
-            ds2 = pick<AT>(m, {dx});
+            ds2 = pick<AT>(m, l, {dx});
             NNCU_TRY(norm_bwd<AT>(m, dx, atc<AT>(a.s2, 0), o.ln_g2, o.ln_b2, a.st_2, nullptr, ds2, TB, bias2_of(l)));
         } else if (o.ff_bias2 != NONE && !coef && !bias2_done) {
             NNCU_TRY(colsum<AT>(m, ds2, D, TB, D, gf(m, o.ff_bias2)));
@@ -965,9 +989,9 @@ static int backward(nncu_model *m)
         // layer's join), the residual keeps ds2; the rows' shares of d alpha wait for the layer's reduction launch
         AT *dt2 = ds2;
         if (coef) {
-            dt2 = reinterpret_cast<AT *>(m->dt_ff);
+            dt2 = reinterpret_cast<AT *>(m->dt_ff[half]);
             launch_k(scale_dot_kernel<AT>, dim3(TB), dim3(128), 0, m->st, (const AT *)ds2, atc<AT>(a.aff, 0),
-                     (const float *)(m->W + o.alpha), dt2, m->alpha_part, TB, D);
+                     (const float *)(m->W + o.alpha), dt2, alpha_part, TB, D);
             KERNEL_CHECK();
             if (o.ff_bias2 != NONE)
                 NNCU_TRY(colsum<AT>(m, dt2, D, TB, D, gf(m, o.ff_bias2)));
@@ -990,9 +1014,9 @@ static int backward(nncu_model *m)
             NNCU_TRY(reduce_cols(m, apart, ceil_div(TB, act_rows), F1, F1, gf(m, o.ff_bias1), 0));
         const AT *u = pre ? atc<AT>(a.u, 0) : atc<AT>(a.y, 0);
         NNCU_TRY(mm_tn(m, F1, D, TB, dhp, F1, u, D, gf(m, o.ff1)));
-        AT *dy = pick<AT>(m, {ds2});
+        AT *dy = pick<AT>(m, l, {ds2});
         if (pre) {
-            AT *du = pick<AT>(m, {ds2, dy});
+            AT *du = pick<AT>(m, l, {ds2, dy});
             NNCU_TRY(mm_nn(m, TB, D, F1, dhp, F1, o.ff1, du, D, (const AT *)nullptr));
             NNCU_TRY(norm_bwd<AT>(m, du, atc<AT>(a.y, 0), o.ln_g2, o.ln_b2, a.st_pre2, ds2, dy, TB));
         } else {
@@ -1001,31 +1025,31 @@ static int backward(nncu_model *m)
         // ---- attention block
         AT *ds1 = dy;
         if (post) {
-            ds1 = pick<AT>(m, {dy, ds2});
+            ds1 = pick<AT>(m, l, {dy, ds2});
             NNCU_TRY(norm_bwd<AT>(m, dy, atc<AT>(a.s1, 0), o.ln_g1, o.ln_b1, a.st_1, nullptr, ds1, TB));
         }
         AT *dt1 = ds1;
         if (coef) {
-            dt1 = reinterpret_cast<AT *>(m->dt_at);
+            dt1 = reinterpret_cast<AT *>(m->dt_at[half]);
             launch_k(scale_dot_kernel<AT>, dim3(TB), dim3(128), 0, m->st, (const AT *)ds1, atc<AT>(a.ao, 0),
-                     (const float *)(m->W + o.alpha), dt1, m->alpha_part + TB, TB, D);
+                     (const float *)(m->W + o.alpha), dt1, alpha_part + TB, TB, D);
             KERNEL_CHECK();
             // d alpha = sum over the rows of both sub-layers, one ordered job
-            NNCU_TRY(queue_reduction(m, 1, m->alpha_part, 2 * TB, 1, 1, 0, gf(m, o.alpha), 0));
+            NNCU_TRY(queue_reduction(m, 1, alpha_part, 2 * TB, 1, 1, 0, gf(m, o.alpha), 0));
         }
         NNCU_TRY(mm_tn(m, D, HD, TB, dt1, D, atc<AT>(a.o, 0), HD, gf(m, o.w_o)));
         NNCU_TRY(mm_nn(m, TB, HD, D, dt1, D, o.w_o, dof, HD, (const AT *)nullptr));
         nncu_attn_shape s = attn_shape(m, l, 0, m->T);
         NNCU_TRY(attn_backward_any<AT>(&s, at<AT>(a.qkv, (size_t)M * B * 3 * HD), at<AT>(a.qkv, HD), wf(m, o.w_r),
-                                       m->W + o.b_r, a.o, a.lse, dof, dq, dkv, m->dwr_part, m->dbr_part, m->st,
+                                       m->W + o.b_r, a.o, a.lse, dof, dq, dkv, dwr_part, dbr_part, m->st,
                                        &pt, (m->bf && o.w_r != NONE) ? m->Wb + o.w_r : nullptr));
         {
-            // the partials are next written after the join at the layer's end
+            // the partials are next written two layers on
             size_t nb = (size_t)m->H * m->L;
-            NNCU_TRY(queue_reduction(m, 1, m->dbr_part, B, (int)nb, (int)nb, 0, gf(m, o.b_r), p.tied_b_r ? 1 : 0));
+            NNCU_TRY(queue_reduction(m, 1, dbr_part, B, (int)nb, (int)nb, 0, gf(m, o.b_r), p.tied_b_r ? 1 : 0));
             if (o.w_r != NONE) {
                 size_t nw = (size_t)m->H * p.d_pos * m->dk;
-                NNCU_TRY(queue_reduction(m, 1, m->dwr_part, B, (int)nw, (int)nw, 0, gf(m, o.w_r), p.tied_w_r ? 1 : 0));
+                NNCU_TRY(queue_reduction(m, 1, dwr_part, B, (int)nw, (int)nw, 0, gf(m, o.w_r), p.tied_w_r ? 1 : 0));
             }
         }
         // d[w_q ; w_kv] = [dq | dk | dv]^T [memory ; segment] in one contraction over all L*B rows
@@ -1033,9 +1057,9 @@ static int backward(nncu_model *m)
         if (o.b_q != NONE)
             NNCU_TRY(colsum<AT>(m, dq, 3 * HD, TB, HD, gf(m, o.b_q)));
         // d(attention input) = [dq | dk | dv](segment rows) [w_q ; w_kv]; the memory rows get no gradient
-        AT *dxn = pick<AT>(m, {ds1, ds2}); // ds1, ds2 are still read by weight-gradient GEMMs
+        AT *dxn = pick<AT>(m, l, {ds1, ds2}); // ds1, ds2 are still read by weight-gradient GEMMs
         if (pre) {
-            AT *dx1 = pick<AT>(m, {ds1, ds2, dxn});
+            AT *dx1 = pick<AT>(m, l, {ds1, ds2, dxn});
             NNCU_TRY(mm_nn(m, TB, D, 3 * HD, dq, 3 * HD, o.w_q, dx1, D, (const AT *)nullptr));
             NNCU_TRY(norm_bwd<AT>(m, dx1, atc<AT>(a.xin, 0), o.ln_g1, o.ln_b1, a.st_pre1, ds1, dxn, TB,
                                   bias2_of(l - 1)));
@@ -1044,7 +1068,10 @@ static int backward(nncu_model *m)
             NNCU_TRY(mm_nn(m, TB, D, 3 * HD, dq, 3 * HD, o.w_q, dxn, D, (const AT *)ds1));
         }
         NNCU_TRY(flush_reductions(m));
-        side_join(m); // this layer's weight gradients are done before dhp, dqkv, ds1, ds2 are rewritten
+        if (m->comm || m->fuse_update)
+            side_join(m); // the layer's gradients are exchanged next, or its weights updated
+        else
+            side_release(m, l);
         const int G = bucket_layers(m);
         if (G > 1) {
             // several layers per exchange: their slots are contiguous, and the group is complete when its
@@ -1088,6 +1115,8 @@ static int backward(nncu_model *m)
         KERNEL_CHECK();
         NNCU_TRY(opt_range(m, m->embed, m->embed_out, false));
     } else {
+        if (m->nl == 1) // first_rows_kernel; with more layers the main stream has waited for the last one's side work
+            side_join(m);
         CUDA_TRY(cudaMemsetAsync(gf(m, m->embed), 0, sizeof(float) * (size_t)V * D, m->st));
         launch_k(embed_grad_kernel<AT>, dim3(TB, ceil_div(D, 256)), dim3(128), 0, m->st, (const int32_t *)m->ids_dev, (const AT *)dx, gf(m, m->embed),
                  (const int *)m->first_dev, TB, D, emul, V);
@@ -1305,6 +1334,8 @@ int nncu_destroy(nncu_model *m)
     if (m->st2) { cudaStreamSynchronize(m->st2); cudaStreamDestroy(m->st2); }
     if (m->ev_fork) cudaEventDestroy(m->ev_fork);
     if (m->ev_join) cudaEventDestroy(m->ev_join);
+    for (cudaEvent_t ev : m->ev_side)
+        if (ev) cudaEventDestroy(ev);
     if (m->arena) cudaFree(m->arena);
     if (m->pin) cudaFreeHost(m->pin);
     if (m->ev_ids) cudaEventDestroy(m->ev_ids);
@@ -1350,7 +1381,7 @@ int nncu_create(const nncu_params *p, nncu_model **out)
     m->device = dev;
     m->st = 0;
     m->st2 = nullptr;
-    m->ev_fork = m->ev_join = nullptr;
+    m->ev_fork = m->ev_join = m->ev_side[0] = m->ev_side[1] = nullptr;
     m->overlap = false;
     memset(m->graphs, 0, sizeof(m->graphs));
     m->comm = nullptr;
@@ -1454,23 +1485,31 @@ int nncu_create(const nncu_params *p, nncu_model **out)
         x.ao = coef ? take((size_t)TB * D * e) : NONE;
         x.aff = coef ? take((size_t)TB * D * e) : NONE;
     }
-    size_t oDtFf = coef ? take((size_t)TB * D * e) : 0, oDtAt = coef ? take((size_t)TB * D * e) : 0;
-    size_t oAlphaPart = coef ? take((size_t)2 * TB * 4) : 0;
+    size_t oDt[4] = {}, oAlphaPart[2] = {};
+    for (int i = 0; coef && i < 2; i++) {
+        oDt[i] = take((size_t)TB * D * e);
+        oDt[2 + i] = take((size_t)TB * D * e);
+        oAlphaPart[i] = take((size_t)2 * TB * 4);
+    }
     size_t oXlast = take((size_t)TB * D * e), oXf = take((size_t)TB * D * e), oStf = take((size_t)TB * 8);
     size_t oProbs = take((size_t)TB * V * 4);
-    size_t oPool[4];
-    for (int i = 0; i < 4; i++)
+    size_t oPool[POOLS];
+    for (int i = 0; i < POOLS; i++)
         oPool[i] = take((size_t)TB * D * e);
-    size_t oDz = take((size_t)TB * V * e), oDh = take((size_t)TB * F * e), oDhp = take((size_t)TB * F1 * e);
+    auto slot = [](size_t bytes) { return (bytes + 255) & ~(size_t)255; }; // one of two copies
+    const size_t n_dhp = slot((size_t)TB * F1 * e);
+    size_t oDz = take((size_t)TB * V * e), oDh = take((size_t)TB * F * e), oDhp = take(2 * n_dhp);
     size_t oDof = take((size_t)TB * HD * e);
-    size_t oDqkv = take((size_t)LB * 3 * HD * e);
+    const size_t n_dqkv = slot((size_t)LB * 3 * HD * e);
+    size_t oDqkv = take(2 * n_dqkv);
     size_t max_n = (size_t)std::max(std::max(V, F1), std::max(3 * HD, D));
     size_t max_k = (size_t)std::max(std::max(F, D), HD);
     size_t oTA = m->use_tc ? take(max_n * LB * 2) : 0, oTB = m->use_tc ? take(max_k * LB * 2) : 0;
-    size_t oWr = take((size_t)m->B * m->H * p->d_pos * m->dk * 4), oBr = take((size_t)m->B * m->H * m->L * 4);
-    size_t part_floats = std::max((size_t)ceil_div(LB, 32) * max_n, (size_t)ceil_div(TB, 8) * 3 * D);
+    const size_t n_wr = slot((size_t)m->B * m->H * p->d_pos * m->dk * 4), n_br = slot((size_t)m->B * m->H * m->L * 4);
+    size_t oWr = take(2 * n_wr), oBr = take(2 * n_br);
+    size_t part_floats = std::max((size_t)ceil_div(TB, 64) * std::max(V, std::max(D, HD)), (size_t)ceil_div(TB, 8) * 3 * D);
     part_floats = std::max(part_floats, (size_t)ceil_div(TB, ACT_BWD_ROWS) * F1);
-    size_t oPart = take(part_floats * 4 * PART_SLOTS);
+    size_t oPart = take(part_floats * 4 * 2 * PART_SLOTS);
     m->part_floats = part_floats;
     // split-K workspaces: the output head's dX (SPLITK parts) and, for contractions of 8192 rows and more, the
     // weight gradients (up to 8 parts of the projection's; the others split where their parts fit)
@@ -1517,11 +1556,17 @@ int nncu_create(const nncu_params *p, nncu_model **out)
     m->hcat[0] = A + oH0; m->hcat[1] = A + oH1;
     m->act.resize(m->nl);
     m->xlast = A + oXlast; m->xf = A + oXf; m->st_f = (float *)(A + oStf); m->probs = (float *)(A + oProbs);
-    for (int i = 0; i < 4; i++)
+    for (int i = 0; i < POOLS; i++)
         m->pool[i] = A + oPool[i];
-    m->dz = A + oDz; m->dh = A + oDh; m->dhp = A + oDhp; m->dof = A + oDof; m->dqkv = A + oDqkv;
+    m->dz = A + oDz; m->dh = A + oDh; m->dof = A + oDof;
+    for (int i = 0; i < 2; i++) {
+        m->dhp[i] = A + oDhp + i * n_dhp;
+        m->dqkv[i] = A + oDqkv + i * n_dqkv;
+        m->dwr_part[i] = (float *)(A + oWr + i * n_wr);
+        m->dbr_part[i] = (float *)(A + oBr + i * n_br);
+    }
     m->tA = m->use_tc ? A + oTA : nullptr; m->tB = m->use_tc ? A + oTB : nullptr;
-    m->dwr_part = (float *)(A + oWr); m->dbr_part = (float *)(A + oBr); m->part = (float *)(A + oPart);
+    m->part = (float *)(A + oPart);
     m->skw = skw_floats ? (float *)(A + oSkw) : nullptr;
     m->skw_floats = skw_floats;
     m->skw_side = skw_side_floats ? (float *)(A + oSkwSide) : nullptr;
@@ -1548,12 +1593,17 @@ int nncu_create(const nncu_params *p, nncu_model **out)
         a.ao = coef ? A + x.ao : nullptr; a.aff = coef ? A + x.aff : nullptr;
     }
     if (coef) {
-        m->dt_ff = A + oDtFf; m->dt_at = A + oDtAt;
-        m->alpha_part = (float *)(A + oAlphaPart);
+        for (int i = 0; i < 2; i++) {
+            m->dt_ff[i] = A + oDt[i];
+            m->dt_at[i] = A + oDt[2 + i];
+            m->alpha_part[i] = (float *)(A + oAlphaPart[i]);
+        }
     }
     if (cudaStreamCreateWithFlags(&m->st2, cudaStreamNonBlocking) == cudaSuccess &&
         cudaEventCreateWithFlags(&m->ev_fork, cudaEventDisableTiming) == cudaSuccess &&
-        cudaEventCreateWithFlags(&m->ev_join, cudaEventDisableTiming) == cudaSuccess) {
+        cudaEventCreateWithFlags(&m->ev_join, cudaEventDisableTiming) == cudaSuccess &&
+        cudaEventCreateWithFlags(&m->ev_side[0], cudaEventDisableTiming) == cudaSuccess &&
+        cudaEventCreateWithFlags(&m->ev_side[1], cudaEventDisableTiming) == cudaSuccess) {
         const char *e = getenv("NNCU_NO_OVERLAP");
         m->overlap = !(e && e[0] == '1');
     }

@@ -226,3 +226,34 @@ def test_fp32_attention_by_clusters(pkg, oracle, B, H, dk, T, M, P, alen):
     """One to eight CTAs per (stream, head): as many as the shape gives, rows and results that do not divide evenly.  (Of a window of
     one key the gradients of queries and keys are rounding only: dS = P (dP - D) is zero.)"""
     _attn_case(pkg, oracle, B, H, dk, T, M, P, alen, False, 9)
+
+
+@pytest.mark.parametrize("kw", [dict(n_layer=1), dict(n_layer=2), dict(n_layer=3), dict(n_layer=5, ln_flags=2 | 4 | 16, ff_act=2),
+                                dict(n_layer=3, use_bf16=0), dict(n_layer=4, use_bf16=0, tied_w_r=1, tied_b_r=1)])
+def test_gradients_with_and_without_the_side_stream_are_the_same_bits(pkg, monkeypatch, kw):
+    """Weight gradients and reductions run up to two layers behind the main stream, from buffers that layers take in
+    turn: every gradient of several steps and models, against one stream."""
+    base = dict(d_model=256, n_head=4, d_key=64, d_inner=512, d_pos=48, mem_len=16, seg_len=32, n_streams=4, n_symbols=512,
+                use_bf16=1, lr=1e-3, init_range=0.03)
+    p = pkg.abi.make_params(**dict(base, **kw))
+    rng = np.random.default_rng(2)
+    steps = [tuple(rng.integers(0, 512, (32, 4)).astype(np.int32) for _ in range(2)) for _ in range(3)]
+
+    def run():
+        m, got = pkg.TrfModel(p), []
+        m.reset()
+        for ids, tg in steps:
+            m.eval(-1, ids, read=False)
+            m.eval_gradient(tg)
+            got.append({n: m.get_grad(n) for n in m.info})
+            m.update()
+        m.close()
+        return got
+
+    monkeypatch.setenv("NNCU_NO_OVERLAP", "1")
+    want = run()
+    monkeypatch.delenv("NNCU_NO_OVERLAP")
+    for _ in range(6):
+        for a, b in zip(want, run()):
+            for n in a:
+                assert np.array_equal(a[n], b[n]), n
