@@ -534,7 +534,7 @@ static int attn_forward_t(const nncu_attn_shape *s, const void *q, const void *k
         return nncu_fail(NNCU_ERR_RANGE, "attention forward: %zu bytes of shared memory needed", smem);
     static DeviceOnce once;
     NNCU_TRY(smem_limit(once, attn_fwd_kernel<T>, SMEM_MOST));
-    launch_k(attn_fwd_kernel<T>, dim3(a.B * a.H, chunks), dim3(256), smem, st, a);
+    launch_kind(EDGE_ATTN, attn_fwd_kernel<T>, dim3(a.B * a.H, chunks), dim3(256), smem, st, a);
     KERNEL_CHECK();
     return NNCU_OK;
 }
@@ -573,7 +573,7 @@ static int attn_backward_t(const nncu_attn_shape *s, const void *q, const void *
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = nncu_pdl_enabled() ? 2 : 1;
+    cfg.numAttrs = (g_nncu_edges & EDGE_ATTN) ? 2 : 1;
     CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, a));
     KERNEL_CHECK();
     return NNCU_OK;

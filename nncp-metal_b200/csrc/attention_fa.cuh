@@ -1406,7 +1406,7 @@ template <int DK> static int forward_one(const AttnArgs &a, cudaStream_t st)
     static DeviceOnce once[2];
     if constexpr (DK < 64) {
         NNCU_TRY(smem_limit(once[0], attn_one_kernel<DK>, OneSmem<DK>::TOTAL));
-        launch_k(attn_one_kernel<DK>, dim3(a.B * a.H), dim3(128), OneSmem<DK>::TOTAL, st, a);
+        launch_kind(EDGE_ATTN, attn_one_kernel<DK>, dim3(a.B * a.H), dim3(128), OneSmem<DK>::TOTAL, st, a);
     } else {
         CUtensorMap kv, r;
         const cuuint64_t B = a.B, L = a.L, kvp = a.kvp, H = a.H, P = a.P;
@@ -1417,7 +1417,7 @@ template <int DK> static int forward_one(const AttnArgs &a, cudaStream_t st)
         if (a.B * a.H >= one_warp_pairs<DK>() && (!a.w_r || a.w_r16)) {
             static DeviceOnce once_warp;
             NNCU_TRY(smem_limit(once_warp, attn_one_warp_kernel<DK>, OneWarpSmem<DK>::TOTAL));
-            launch_k(attn_one_warp_kernel<DK>, dim3(a.B * a.H), dim3(32), OneWarpSmem<DK>::TOTAL, st, a, kv, r);
+            launch_kind(EDGE_ATTN, attn_one_warp_kernel<DK>, dim3(a.B * a.H), dim3(32), OneWarpSmem<DK>::TOTAL, st, a, kv, r);
             KERNEL_CHECK();
             return NNCU_OK;
         }
@@ -1425,7 +1425,7 @@ template <int DK> static int forward_one(const AttnArgs &a, cudaStream_t st)
         auto kernel = wide ? attn_one_tma_kernel<DK, true> : attn_one_tma_kernel<DK, false>;
         NNCU_TRY(smem_limit(once[wide], kernel, 226 * 1024)); // its barriers are static
         const size_t most = 226 * 1024, all = OneTmaSmem<DK>::bytes(a.L);
-        launch_k(kernel, dim3(a.B * a.H), dim3(128), all <= most ? all : OneTmaSmem<DK>::bytes(0), st, a, kv, r,
+        launch_kind(EDGE_ATTN, kernel, dim3(a.B * a.H), dim3(128), all <= most ? all : OneTmaSmem<DK>::bytes(0), st, a, kv, r,
                  all <= most ? 1 : 0);
     }
     KERNEL_CHECK();
@@ -1439,7 +1439,7 @@ template <int DK> static int forward_dk(const AttnArgs &a, cudaStream_t st)
     const bool wide = aligned_to(a.o, 16) && aligned_to(a.w_r, 16);
     auto kernel = wide ? attn_fwd_kernel<DK, true> : attn_fwd_kernel<DK, false>;
     NNCU_TRY(smem_limit(once[wide], kernel, SMEM_MOST));
-    launch_k(kernel, dim3(a.B * a.H, (a.t1 - (a.t0 & ~63) + 63) / 64), dim3(256), FwdSmem<DK>::bytes(a.L), st, a);
+    launch_kind(EDGE_ATTN, kernel, dim3(a.B * a.H, (a.t1 - (a.t0 & ~63) + 63) / 64), dim3(256), FwdSmem<DK>::bytes(a.L), st, a);
     KERNEL_CHECK();
     return NNCU_OK;
 }
@@ -1449,7 +1449,7 @@ template <int DK> static int backward_dk(const AttnArgs &a, cudaStream_t st)
     const bool wide = aligned_to(a.dq, 16) && aligned_to(a.dkv, 16) && aligned_to(a.dwr_part, 16) && aligned_to(a.w_r, 16);
     auto kernel = wide ? attn_bwd_kernel<DK, true> : attn_bwd_kernel<DK, false>;
     NNCU_TRY(smem_limit(once[wide], kernel, SMEM_MOST));
-    launch_k(kernel, dim3(a.B * a.H), dim3(256), BwdSmem<DK>::bytes(a.L), st, a);
+    launch_kind(EDGE_ATTN, kernel, dim3(a.B * a.H), dim3(256), BwdSmem<DK>::bytes(a.L), st, a);
     KERNEL_CHECK();
     return NNCU_OK;
 }

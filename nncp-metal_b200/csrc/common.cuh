@@ -51,12 +51,18 @@ template <typename K> static int smem_limit(DeviceOnce &once, K kernel, int byte
 // predecessor has completed and its writes are visible.  Rules for a kernel launched this way:
 // every thread executes pdl_wait() before its first global-memory access and before any early
 // return, so that the kernel cannot complete before its predecessor has.  Both calls are no-ops in
-// a kernel launched the ordinary way.  On in the one-symbol steps of a decoder, a single chain of short
-// kernels (128 streams, 12 layers of 512: 80.4 -> 76.2 ms a segment of 64 steps; pdl_trigger() lets the
-// successor start as soon as all CTAs of a kernel are resident), and in the isolated attention op
-// (forward, backward and reduction of 16 x 8 heads 36.4 -> 28.0 us); off in whole-segment passes unless
-// NNCU_PDL=1: there a side stream's kernels fill the gaps, and the resident successors take SM resources
-// from them (train steps of the bf16 models between 4 % faster and 2 % slower).
+// a kernel launched the ordinary way.
+//
+// Which launches get such an edge (g_nncu_edges):
+//   all      the one-symbol steps of a decoder, a single chain of short kernels (128 streams, 12 layers of 512: 80.4 ->
+//            76.2 ms a segment of 64 steps; pdl_trigger() lets the successor start as soon as all CTAs of a kernel
+//            are resident), and the isolated attention op (16 x 8 heads 36.4 -> 28.0 us)
+//   GEMMs    whole-segment passes of bf16 models: a tensor-core GEMM sets up barriers, tensor memory and tensor maps
+//            before it needs its operands, a microsecond that passes under its predecessor (6 layers of 512, 1024
+//            rows: 790 -> 756 us; 12 layers, 2048 rows: 2489 -> 2345; 8 layers, 650 rows: 1307 -> 1216).  Edges on the
+//            short kernels beside them take SM resources from the side stream's (1 to 2 % slower with them)
+//   others   whole-segment passes of fp32 models, whose GEMMs have nothing to set up (4 layers of 256, 512 rows:
+//            737 -> 699 us, with edges on the GEMMs too 759), but for the attention kernels
 __device__ __forceinline__ void pdl_wait()
 {
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -65,27 +71,20 @@ __device__ __forceinline__ void pdl_trigger()
 {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
-// set while the launches of a chain are queued by this thread
-extern thread_local bool g_nncu_step_chain;
-struct ChainScope {
-    const bool before = g_nncu_step_chain;
-    ChainScope() { g_nncu_step_chain = true; }
-    ~ChainScope() { g_nncu_step_chain = before; }
+enum { EDGE_GEMM = 1, EDGE_OTHER = 2, EDGE_ATTN = 4 };
+// the kinds of launches of this thread that get an edge
+extern thread_local int g_nncu_edges;
+struct EdgeScope {
+    const int before = g_nncu_edges;
+    explicit EdgeScope(int kinds) { g_nncu_edges |= kinds; }
+    ~EdgeScope() { g_nncu_edges = before; }
 };
-inline bool nncu_pdl_enabled()
-{
-    if (g_nncu_step_chain)
-        return true;
-    static int on = -1;
-    if (on < 0) {
-        const char *e = getenv("NNCU_PDL");
-        on = (e && e[0] == '1') ? 1 : 0;
-    }
-    return on != 0;
-}
+struct ChainScope : EdgeScope {
+    ChainScope() : EdgeScope(EDGE_GEMM | EDGE_OTHER | EDGE_ATTN) {}
+};
 template <typename... KArgs, typename... Args>
-static cudaError_t launch_k(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
-                            Args &&...args)
+static cudaError_t launch_kind(int kind, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                               Args &&...args)
 {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
@@ -96,8 +95,13 @@ static cudaError_t launch_k(void (*kernel)(KArgs...), dim3 grid, dim3 block, siz
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = nncu_pdl_enabled() ? 1 : 0;
+    cfg.numAttrs = (g_nncu_edges & kind) ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+template <typename... KArgs, typename... Args>
+static cudaError_t launch_k(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args &&...args)
+{
+    return launch_kind(EDGE_OTHER, kernel, grid, block, smem, st, static_cast<Args &&>(args)...);
 }
 
 // every kernel launch in the library is followed by exactly one KERNEL_CHECK

@@ -235,7 +235,7 @@ static int launch(cudaStream_t st, int M, int N, int K, const TA *A, long lda, c
     NNCU_TRY(smem_limit(once, gemm_simt_kernel<BM, BN, TM, TN, MODE, TA, TB, TC>, (int)smem));
     const int vec_a = (reinterpret_cast<uintptr_t>(A) & 15) == 0 && lda % 4 == 0;
     const int vec_b = (reinterpret_cast<uintptr_t>(B) & 15) == 0 && ldb % 4 == 0;
-    launch_k(gemm_simt_kernel<BM, BN, TM, TN, MODE, TA, TB, TC>, dim3(ceil_div(N, BN), ceil_div(M, BM)), dim3(256), smem, st,
+    launch_kind(EDGE_GEMM, gemm_simt_kernel<BM, BN, TM, TN, MODE, TA, TB, TC>, dim3(ceil_div(N, BN), ceil_div(M, BM)), dim3(256), smem, st,
              M, N, K, A, lda, B, ldb, C, ldc, bias, addsrc, bias_n, vec_a, vec_b);
     KERNEL_CHECK();
     return NNCU_OK;

@@ -732,7 +732,7 @@ static int launch(cudaStream_t st, int M, int N, int K, const bf16 *A, long lda,
     const bool timed = pr && pr->n < GemmProfiler::MAX_EV;
     if (timed)
         cudaEventRecord(pr->ev[2 * pr->n], st);
-    launch_k(gemm_tc_kernel<BN, TC, AMN, BMN, DEEP>, dim3(grid), dim3(256), SL::TOTAL, st, ma, mb, mc, staged, C, ldc, bias, addsrc,
+    launch_kind(EDGE_GEMM, gemm_tc_kernel<BN, TC, AMN, BMN, DEEP>, dim3(grid), dim3(256), SL::TOTAL, st, ma, mb, mc, staged, C, ldc, bias, addsrc,
              M, N, K, err_flag, bias_n, weights ? 1 : 0);
     if (timed) {
         cudaEventRecord(pr->ev[2 * pr->n + 1], st);

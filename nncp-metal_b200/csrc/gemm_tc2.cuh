@@ -492,7 +492,7 @@ static int launch(cudaStream_t st, int M, int N, int K, const bf16 *A, long lda,
     const bool timed = pr && pr->n < GemmProfiler::MAX_EV;
     if (timed)
         cudaEventRecord(pr->ev[2 * pr->n], st);
-    launch_k(gemm_pair_kernel<TC, AMN, BMN>, dim3(2 * std::min(units, PAIRS)), dim3(384), SL::TOTAL, st, ma, mb, mc, mc2, sh, bias,
+    launch_kind(EDGE_GEMM, gemm_pair_kernel<TC, AMN, BMN>, dim3(2 * std::min(units, PAIRS)), dim3(384), SL::TOTAL, st, ma, mb, mc, mc2, sh, bias,
              addsrc, ldc, err_flag);
     if (timed) {
         cudaEventRecord(pr->ev[2 * pr->n + 1], st);

@@ -51,7 +51,7 @@ static int coder_depth(int V)
 thread_local char g_nncu_err[512] = "";
 unsigned long long g_nncu_launches = 0;
 GemmProfiler *g_nncu_prof = nullptr;
-thread_local bool g_nncu_step_chain = false;
+thread_local int g_nncu_edges = 0;
 
 int nncu_fail(int code, const char *fmt, ...)
 {
@@ -1752,6 +1752,9 @@ static void bind_xin(nncu_model *m)
         m->act[l].xin = hcat_layer(m, m->cur, l) + (size_t)m->M * m->B * m->D * m->esz;
 }
 
+// programmatic edges of a whole-segment pass (common.cuh)
+static int pass_edges(const nncu_model *m) { return m->bf ? EDGE_GEMM : EDGE_OTHER; }
+
 static int eval_common(nncu_model *m, int output_index)
 {
     if (output_index >= m->T)
@@ -1763,6 +1766,7 @@ static int eval_common(nncu_model *m, int output_index)
         CUDA_TRY(cudaStreamWaitEvent(m->st, m->ev_coder, 0));
     int t0 = output_index < 0 ? 0 : output_index, t1 = output_index < 0 ? m->T : output_index + 1;
     auto body = [&]() { return m->bf ? forward_range<bf16>(m, t0, t1) : forward_range<float>(m, t0, t1); };
+    EdgeScope edges(output_index < 0 ? pass_edges(m) : 0);
     int rc = output_index < 0 ? run_graphed(m, GRAPH_FWD, body) : body();
     if (rc != NNCU_OK)
         return rc;
@@ -1873,6 +1877,7 @@ static int gradient_common(nncu_model *m, bool fused = false)
         const float hyper[2] = {m->lr, m->p.bias_correction ? 1.0f / (1.0f - powf(m->p.beta2, (float)m->step)) : 1.0f};
         CUDA_TRY(cudaMemcpyAsync(m->hyper_dev, hyper, sizeof(hyper), cudaMemcpyHostToDevice, m->st));
     }
+    EdgeScope edges(pass_edges(m));
     m->fuse_update = fused;
     m->shard_update = fused && m->comm && m->comm_ranks > 1 && shard_enabled();
     m->sparse_embed = fused && m->comm && m->comm_ranks > 1 && (m->shard_update || sparse_embed_enabled());
