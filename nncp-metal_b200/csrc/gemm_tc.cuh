@@ -744,11 +744,12 @@ static int launch(cudaStream_t st, int M, int N, int K, const bf16 *A, long lda,
 
 // A: [M][K] (lda) or, AMN, [K][M]; B: [N][K] (ldb) or, BMN, [K][N].  C bf16 or fp32; addsrc
 // (may be NULL, may alias C) is added to the product.  err_flag: device int raised when a
-// bounded wait expires.  weights: B is one of the model's matrices.
+// bounded wait expires.  weights: B is one of the model's matrices.  aside: other launches
+// of this model run at the same time.
 template <typename TC, bool AMN, bool BMN>
 static int gemm(cudaStream_t st, int M, int N, int K, const bf16 *A, long lda, const bf16 *B,
                 long ldb, TC *C, long ldc, const float *bias, const TC *addsrc, int *err_flag,
-                int bias_n = 1 << 30, bool weights = false)
+                int bias_n = 1 << 30, bool weights = false, bool aside = false)
 {
     if (M <= 0 || N <= 0)
         return NNCU_OK;
@@ -779,7 +780,9 @@ static int gemm(cudaStream_t st, int M, int N, int K, const bf16 *A, long lda, c
         return launch<128, TC, AMN, BMN>(st, M, N, K, A, lda, B, ldb, C, ldc, bias, addsrc, err_flag, bias_n, 1, weights);
     // Where 64-wide tiles are more than one round and 128-wide ones fit the chip at once, these read a third less from L2
     // (2048 x 1024, K 1024 to 6144, a hundred such launches in a step of 20 layers: 10760 -> 10320 us a step)
-    if (mt * ceil_div(N, 64) > 148 && mt * ceil_div(N, 128) <= 148)
+    // Launches beside a pass's own chain (weight gradients) take them whatever they are: half the SMs for about the same time
+    // leaves more to the chain (12 layers of 512, 2048 rows: 2345 -> 2271 us; 6 layers, 1024 rows: 756 -> 733)
+    if ((aside ? N > 64 : mt * ceil_div(N, 64) > 148) && mt * ceil_div(N, 128) <= 148)
         return launch<128, TC, AMN, BMN, true>(st, M, N, K, A, lda, B, ldb, C, ldc, bias, addsrc, err_flag, bias_n, 1, weights);
     return launch<64, TC, AMN, BMN>(st, M, N, K, A, lda, B, ldb, C, ldc, bias, addsrc, err_flag, bias_n, 1, weights);
 }

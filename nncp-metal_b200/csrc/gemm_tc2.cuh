@@ -452,6 +452,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 struct Extra {
     int hole_m = 0, hole_n = 0, skip_m = 0, skip_k = 0, ksplit = 1, act = -1;
     void *C2 = nullptr;
+    bool aside = false;   // runs beside the pass's own chain of launches (tc::gemm)
     bool weights = false; // B is one of the model's matrices (tc::gemm)
 };
 constexpr int PAIRS = 74; // CTA pairs the chip holds (148 SMs)
@@ -540,7 +541,7 @@ static int gemm(cudaStream_t st, int M, int N, int K, const bf16 *A, long lda, c
             *did_act = x.C2 != nullptr;
         return launch<TC, AMN, BMN>(st, M, N, K, A, lda, B, ldb, C, ldc, bias, addsrc, err_flag, bias_n, x);
     }
-    return tc::gemm<TC, AMN, BMN>(st, M, N, K, A, lda, B, ldb, C, ldc, bias, addsrc, err_flag, bias_n, x.weights);
+    return tc::gemm<TC, AMN, BMN>(st, M, N, K, A, lda, B, ldb, C, ldc, bias, addsrc, err_flag, bias_n, x.weights, x.aside);
 }
 
 } // namespace tc2

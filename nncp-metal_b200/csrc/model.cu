@@ -395,6 +395,7 @@ static int mm_tn(nncu_model *m, int Nout, int Kin, int R, const bf16 *dY, long l
         // dY is [R][Nout] = [k][m], X is [R][Kin] = [k][n]: both MN-major, read in place
         cudaStream_t st = side_fork(m);
         tc2::Extra x;
+        x.aside = st != m->st;
         x.skip_m = skip_n;
         x.skip_k = skip_r;
         // A long contraction into few tiles (the projection's weight gradient over all memory rows) is split
