@@ -1386,13 +1386,14 @@ inline bool fits(int dk, int L)
     }
 }
 
-// tiles of 64 columns x 64 rows of a three-dimensional bf16 tensor whose rows are `mid` or `outer` apart
-inline int tile_map(const void *p, const cuuint64_t (&dims)[3], const cuuint64_t (&strides)[2], bool rows_outer, CUtensorMap *out)
+// tiles of 64 columns x `rows` of a three-dimensional bf16 tensor whose rows are `mid` or `outer` apart
+inline int tile_map(const void *p, const cuuint64_t (&dims)[3], const cuuint64_t (&strides)[2], bool rows_outer, CUtensorMap *out,
+                    cuuint32_t rows = 64)
 {
     tc::EncodeTiledFn fn = tc::encode_fn();
     if (!fn)
         return nncu_fail(NNCU_ERR_CUDA, "cuTensorMapEncodeTiled is not available");
-    cuuint32_t box[3] = {64, rows_outer ? 1u : 64u, rows_outer ? 64u : 1u}, estr[3] = {1, 1, 1};
+    cuuint32_t box[3] = {64, rows_outer ? 1u : rows, rows_outer ? rows : 1u}, estr[3] = {1, 1, 1};
     CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void *>(p), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                     CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? NNCU_OK : nncu_fail(NNCU_ERR_CUDA, "cuTensorMapEncodeTiled failed: %d", (int)r);
@@ -1474,6 +1475,11 @@ static int backward(const AttnArgs &a, cudaStream_t st)
 
 } // namespace fa
 
+namespace fab { // attention_bwd.cuh
+static bool takes(const AttnArgs &a);
+static int backward(const AttnArgs &a, cudaStream_t st);
+} // namespace fab
+
 // ---- dispatch: bf16 goes to the tensor-core kernels when the shape allows, everything else to the
 // CUDA-core kernels of attention.cuh.  The choice depends on the shape only, never on the query
 // range, so one-symbol steps and whole segments take the same arithmetic.
@@ -1496,15 +1502,16 @@ template <typename T>
 static int attn_backward_any(const nncu_attn_shape *s, const void *q, const void *kv, const float *w_r,
                              const float *b_r, const void *out, const float *lse, const void *dout,
                              void *dq, void *dkv, float *dwr_part, float *dbr_part, cudaStream_t st,
-                             const AttnPitch *pt = nullptr, const void *w_r16 = nullptr)
+                             const AttnPitch *pt = nullptr, const void *w_r16 = nullptr, int *err_flag = nullptr)
 {
     if (sizeof(T) == 2) {
         AttnArgs a = attn_args(s, pt);
         a.w_r16 = w_r ? w_r16 : nullptr;
+        a.err_flag = err_flag;
         a.q = q; a.kv = kv; a.w_r = w_r; a.b_r = b_r; a.out = out; a.lse = const_cast<float *>(lse);
         a.dout = dout; a.dq = dq; a.dkv = dkv; a.dwr_part = dwr_part; a.dbr_part = dbr_part;
         if (fa::supported_bwd(a) && fa::fits(a.dk, a.L))
-            return fa::backward(a, st);
+            return fab::takes(a) ? fab::backward(a, st) : fa::backward(a, st);
     }
     return attn_backward_t<T>(s, q, kv, w_r, b_r, out, lse, dout, dq, dkv, dwr_part, dbr_part, st, pt);
 }

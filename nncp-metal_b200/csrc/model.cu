@@ -30,6 +30,7 @@
 #include <vector>
 
 #include "attention_fa.cuh"
+#include "attention_bwd.cuh"
 #include "coder.cuh"
 
 // ceil(log2 V): the depth of the coder's tree for any alphabet (its heap has 1 << depth slots per row)
@@ -1043,7 +1044,7 @@ static int backward(nncu_model *m)
         nncu_attn_shape s = attn_shape(m, l, 0, m->T);
         NNCU_TRY(attn_backward_any<AT>(&s, at<AT>(a.qkv, (size_t)M * B * 3 * HD), at<AT>(a.qkv, HD), wf(m, o.w_r),
                                        m->W + o.b_r, a.o, a.lse, dof, dq, dkv, dwr_part, dbr_part, m->st,
-                                       &pt, (m->bf && o.w_r != NONE) ? m->Wb + o.w_r : nullptr));
+                                       &pt, (m->bf && o.w_r != NONE) ? m->Wb + o.w_r : nullptr, m->err_flag));
         {
             // the partials are next written two layers on
             size_t nb = (size_t)m->H * m->L;

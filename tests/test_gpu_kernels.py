@@ -257,3 +257,12 @@ def test_gradients_with_and_without_the_side_stream_are_the_same_bits(pkg, monke
         for a, b in zip(want, run()):
             for n in a:
                 assert np.array_equal(a[n], b[n]), n
+
+
+@pytest.mark.parametrize("B,H,dk,T,M,P,alen", [(1, 1, 64, 64, 64, 128, 0), (2, 1, 64, 64, 65, 100, 0), (3, 2, 64, 1, 127, 128, 0), (40, 4, 64, 33, 160, 193, 0),
+                                               (1, 2, 64, 63, 400, 30, 90), (2, 2, 128, 64, 192, 256, 0), (1, 1, 128, 17, 112, 60, 0),
+                                               (75, 2, 128, 16, 130, 146, 0), (1, 2, 128, 64, 500, 564, 70)])
+def test_attention_adjoint_on_128_key_blocks_bf16(pkg, oracle, B, H, dk, T, M, P, alen):
+    """The persistent kernel of head sizes 64 and 128: whole and ragged key blocks, one query, more (stream, head) pairs
+    than CTAs, tables that end inside the left pad, windows that leave whole blocks out."""
+    _attn_case(pkg, oracle, B, H, dk, T, M, P, alen, True, 11)
