@@ -495,7 +495,6 @@ __global__ void __launch_bounds__(128) attn_one_kernel(const __grid_constant__ A
     const int b = blockIdx.x / a.H, h = blockIdx.x % a.H, HD = a.H * DK, T = a.T, M = a.M, L = a.L, i = a.t0;
     const Blocks blk = blocks_of(M, L, a.attn_len, i, i + 1);
     pdl_trigger();
-    pdl_wait();
     const bf16 *kv = reinterpret_cast<const bf16 *>(a.kv) + (size_t)b * a.kvp + h * DK;
     auto fetch_kr = [&](int kb) { // this warp's block of a round
         const int j0 = kb * KB;
@@ -511,10 +510,15 @@ __global__ void __launch_bounds__(128) attn_one_kernel(const __grid_constant__ A
             load_rows<DK>(Vall + warp * 64 * LD, kv + HD + (size_t)j0 * a.B * a.kvp, (size_t)a.B * a.kvp, 64, lane, 32,
                           [&](int r) { return j0 + r < L; });
     };
+    const bool early = a.ahead && blk.lo + warp < blk.hi; // the last block holds this step's own key, which the predecessor writes
+    if (!early)
+        pdl_wait();
     fetch_kr(blk.lo + warp);
     cp_commit();
     fetch_v(blk.lo + warp);
     cp_commit();
+    if (early)
+        pdl_wait();
     // the query as the second operand: k = 2t, 2t + 1 (+ 8) of every 16-wide slice, the same for all columns
     uint32_t qf[DK / 16][2];
     {
@@ -675,7 +679,6 @@ __global__ void __launch_bounds__(128) attn_one_tma_kernel(const __grid_constant
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
-    pdl_wait();
     int *ef = a.err_flag ? a.err_flag : &dummy;
     bool ok = true; // this lane's waits: after one that ran out it issues no copy and waits no more
     auto fetch_kr = [&](int kb) { // this warp's block of a round
@@ -724,11 +727,23 @@ __global__ void __launch_bounds__(128) attn_one_tma_kernel(const __grid_constant
         for (int n = 0; n < NS; n++)
             tma_load_3d(Vt + warp * TILE + n * 8192, &map_kv, bar_v, HD + h * DK + n * 64, b, kb * KB);
     };
-    fetch_kr(blk.lo + warp);
-    fetch_v(blk.lo + warp);
+    // the last block holds this step's own key, which the predecessor writes
+    const bool early = a.ahead && blk.lo + warp < blk.hi;
+    if (!a.ahead)
+        pdl_wait();
+    if (early) {
+        fetch_kr(blk.lo + warp);
+        fetch_v(blk.lo + warp);
+    }
     if (stage_br) // the head's b_r, scaled
         for (int r = threadIdx.x; r < L; r += 128)
             brs[r] = __fmul_rn(a.br_scale, a.b_r[(size_t)h * L + r]);
+    if (a.ahead)
+        pdl_wait();
+    if (!early) {
+        fetch_kr(blk.lo + warp);
+        fetch_v(blk.lo + warp);
+    }
     // the query as the second operand: k = 2t, 2t + 1 (+ 8) of every 16-wide slice, the same for all columns
     uint32_t qf[DK / 16][2];
     {
@@ -872,7 +887,6 @@ __global__ void __launch_bounds__(32) attn_one_warp_kernel(const __grid_constant
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncwarp();
-    pdl_wait();
     int *ef = a.err_flag ? a.err_flag : &dummy;
     bool ok = true; // this lane's waits: after one that ran out it issues no copy and waits no more
     float br[4][2]; // of the block that is being fetched
@@ -914,8 +928,13 @@ __global__ void __launch_bounds__(32) attn_one_warp_kernel(const __grid_constant
         for (int n = 0; n < NS; n++)
             tma_load_3d(Vt + n * 8192, &map_kv, bar_v, HD + h * DK + n * 64, b, kb * KB);
     };
+    const bool early = a.ahead && blk.lo < blk.hi; // the last block holds this step's own key, which the predecessor writes
+    if (!early)
+        pdl_wait();
     fetch_kr(blk.lo);
     fetch_v(blk.lo);
+    if (early)
+        pdl_wait();
     // the query as the second operand: k = 2t, 2t + 1 (+ 8) of every 16-wide slice, the same for all columns
     uint32_t qf[DK / 16][2];
     {
@@ -1486,11 +1505,11 @@ static int backward(const AttnArgs &a, cudaStream_t st);
 template <typename T>
 static int attn_forward_any(const nncu_attn_shape *s, const void *q, const void *kv, const float *w_r,
                             const float *b_r, void *out, float *lse, cudaStream_t st,
-                            const AttnPitch *pt = nullptr, const void *w_r16 = nullptr, int *err_flag = nullptr)
+                            const AttnPitch *pt = nullptr, const void *w_r16 = nullptr, int *err_flag = nullptr, bool ahead = false)
 {
     if (sizeof(T) == 2) {
         AttnArgs a = attn_args(s, pt);
-        a.q = q; a.kv = kv; a.w_r = w_r; a.b_r = b_r; a.o = out; a.lse = lse; a.err_flag = err_flag;
+        a.q = q; a.kv = kv; a.w_r = w_r; a.b_r = b_r; a.o = out; a.lse = lse; a.err_flag = err_flag; a.ahead = ahead ? 1 : 0;
         a.w_r16 = w_r ? w_r16 : nullptr;
         if (fa::supported(a) && fa::fits(a.dk, a.L))
             return fa::forward(a, st);

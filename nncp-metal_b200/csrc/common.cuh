@@ -49,8 +49,10 @@ template <typename K> static int smem_limit(DeviceOnce &once, K kernel, int byte
 // before it on the stream is still draining: its CTAs become resident, run whatever comes before
 // pdl_wait() (barrier set-up, TMEM allocation, index arithmetic) and block there until the
 // predecessor has completed and its writes are visible.  Rules for a kernel launched this way:
-// every thread executes pdl_wait() before its first global-memory access and before any early
-// return, so that the kernel cannot complete before its predecessor has.  Both calls are no-ops in
+// every thread executes pdl_wait() before its first access to memory that a kernel of the same pass or step
+// touches and before any early return, so that the kernel cannot complete before its predecessor has.  (What
+// stands since before the pass may be read earlier -- parameters, keys of other steps, the decoder's state -- because the
+// pass's first kernel triggers only behind its own wait.)  Both calls are no-ops in
 // a kernel launched the ordinary way.
 //
 // Which launches get such an edge (g_nncu_edges):

@@ -71,8 +71,6 @@ decode_step_kernel(const uint16_t *__restrict__ trees, const uint8_t *__restrict
                    int32_t *__restrict__ sym_out, int32_t *__restrict__ ids_next, int t, int limit_t, int limit_b,
                    int B, int V, int P, int nb, int ring, int *err_flag)
 {
-    pdl_wait();
-    pdl_trigger(); // a successor that was launched to overlap this kernel may start on what does not depend on it
     extern __shared__ __align__(128) uint8_t dsm[];
     uint64_t *bars = reinterpret_cast<uint64_t *>(dsm);           // [2][MAX_RING] of 8 bytes: 128
     const int G = slot_trees(B, P, nb);
@@ -96,8 +94,22 @@ decode_step_kernel(const uint16_t *__restrict__ trees, const uint8_t *__restrict
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     const int wbytes = window_bytes(B, nb);
-    for (int i = tid; i < wbytes; i += 64)
-        win[i] = (pos0 + i < len) ? payload[pos0 + i] : (uint8_t)0;
+    for (int i0 = tid; i0 < wbytes; i0 += 16 * 64) { // sixteen loads in flight
+        uint8_t v[16];
+#pragma unroll
+        for (int k = 0; k < 16; k++) {
+            const int i = i0 + k * 64;
+            v[k] = i < wbytes && pos0 + i < len ? payload[pos0 + i] : (uint8_t)0;
+        }
+#pragma unroll
+        for (int k = 0; k < 16; k++)
+            if (i0 + k * 64 < wbytes)
+                win[i0 + k * 64] = v[k];
+    }
+    // Up to here nothing depends on the kernels of this step: the state is what the step before left, and the step's first
+    // kernel (embedding, or the whole step in one launch) lets its successors start only when that is complete.
+    pdl_wait();
+    pdl_trigger(); // a successor that was launched to overlap this kernel may start on what does not depend on it
     __syncthreads();
 
     if (tid == 32) { // the copies, on a warp of their own: the walk does not stop to issue them

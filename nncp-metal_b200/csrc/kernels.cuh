@@ -234,10 +234,16 @@ residual_norm_vec_kernel(const T *__restrict__ a, const T *__restrict__ res, T *
                          float *__restrict__ stats, int rows, int D, int mode)
 {
     pdl_trigger();
-    pdl_wait();
     constexpr int W = RowVec<T>::W;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int r = blockIdx.x * 4 + warp;
+    // gain and bias are parameters, which no kernel of a pass writes (see gemm_tc_kernel's weights): on their way before the wait
+    float gv[NC][W], bv[NC][W];
+    if (mode != 0) {
+        vec_load_f32<NC, W>(g, lane, D, gv);
+        vec_load_f32<NC, W>(b, lane, D, bv);
+    }
+    pdl_wait();
     if (r >= rows)
         return;
     float v[NC][W];
@@ -257,9 +263,6 @@ residual_norm_vec_kernel(const T *__restrict__ a, const T *__restrict__ res, T *
         row_store<T, NC, W>(y + (size_t)r * D, lane, D, v);
         return;
     }
-    float gv[NC][W], bv[NC][W];
-    vec_load_f32<NC, W>(g, lane, D, gv);
-    vec_load_f32<NC, W>(b, lane, D, bv);
     norm_row<NC, W>(v, gv, bv, lane, D, mode, stats ? stats + 2 * r : nullptr);
     row_store<T, NC, W>(y + (size_t)r * D, lane, D, v);
 }

@@ -711,7 +711,8 @@ static int forward_range(nncu_model *m, int t0, int t1)
         const AttnPitch pt = {3 * HD, 3 * HD, 3 * HD, 3 * HD};
         NNCU_TRY(attn_forward_any<AT>(&s, at<AT>(a.qkv, (size_t)M * B * 3 * HD), at<AT>(a.qkv, HD),
                                       wf(m, o.w_r), m->W + o.b_r, a.o, a.lse, m->st, &pt,
-                                      (m->bf && o.w_r != NONE) ? m->Wb + o.w_r : nullptr, m->err_flag));
+                                      (m->bf && o.w_r != NONE) ? m->Wb + o.w_r : nullptr, m->err_flag,
+                                      t0 > 0)); // behind the first step the memory's keys and values are those of kernels before this step's
         // output projection, residual, post-LN (nncp.c:865-920)
         if (o.alpha != NONE) { // LN_COEF: the projection is kept as it is for the backward pass, tmp = alpha * it
             AT *ao = at<AT>(a.ao, (size_t)r0 * D);
