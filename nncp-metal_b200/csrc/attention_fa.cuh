@@ -289,7 +289,7 @@ template <int DK> struct FwdSmem {
 };
 
 template <int DK, bool WIDE> // WIDE: out takes 16-byte stores, an fp32 table 16-byte loads
-__global__ void __launch_bounds__(256, DK <= 64 ? 2 : 1) attn_fwd_kernel(const __grid_constant__ AttnArgs a)
+__global__ void __launch_bounds__(256, 2) attn_fwd_kernel(const __grid_constant__ AttnArgs a)
 {
     using SM = FwdSmem<DK>;
     constexpr int LD = SM::LD, NCH = DK >= 32 ? 2 : 1, NTC = DK / 8 / NCH; // column halves, 8-column groups in one
@@ -1035,6 +1035,304 @@ __global__ void __launch_bounds__(32) attn_one_warp_kernel(const __grid_constant
         a.lse[((size_t)b * a.H + h) * T + i] = m_run + logf(l);
 }
 
+// ---------------- forward, a group of queries, by TMA ----------------
+//
+// The same for head sizes 64 and 128 with tiles that arrive by TMA, issued by one thread, in 128-byte rows, chunk c of row r
+// at c ^ (r % 8) (tile_at): copies by every thread were a sixth of the instructions of the loop above.  Training
+// steps: 12 layers, 128 streams, 576 keys 10617 -> 10477 us; 20 layers, 320 keys 16416 -> 16320; 8 heads of 128 9654 -> 9579.  Table groups
+// that have to be rounded from fp32, or hold copies of row 0, are still written by all threads.
+template <int DK> struct FwdTmaSmem {
+    static constexpr int NS = DK / 64, TILE = NS * 8192;
+    static constexpr int Q = 0, K = TILE, V = K + 2 * TILE, R = V + 2 * TILE, ES = R + 3 * TILE, PF = ES + 8 * 16 * ESC * 4, MX = PF + 4 * 4 * 512,
+                         BRS = MX + 4 * 6 * 32 * 4;
+    static size_t bytes(int L) { return (size_t)BRS + br_bytes(L) + 1024; }
+};
+// s[nt][c] = 16 rows at `at` against 32 rows at `bt`; oa, ob: this lane's swizzled chunk of 16-wide step k (mod 4) in either
+template <int DK>
+__device__ __forceinline__ void product_16x32_at(float (&s)[4][4], uint32_t at, uint32_t bt, const uint32_t (&oa)[4], const uint32_t (&ob)[4])
+{
+#pragma unroll
+    for (int n = 0; n < 4; n++)
+#pragma unroll
+        for (int c = 0; c < 4; c++)
+            s[n][c] = 0.0f;
+#pragma unroll
+    for (int ks = 0; ks < DK / 16; ks++) {
+        uint32_t q[4];
+        ldsm4_at(q, at + (ks >> 2) * 8192 + oa[ks & 3]);
+#pragma unroll
+        for (int p = 0; p < 2; p++) {
+            uint32_t b[4];
+            ldsm4_at(b, bt + (ks >> 2) * 8192 + p * 2048 + ob[ks & 3]);
+            mma(s[2 * p], q, b[0], b[1]);
+            mma(s[2 * p + 1], q, b[2], b[3]);
+        }
+    }
+}
+template <int DK, typename W>
+__device__ __forceinline__ void skewed_positions_at(float (&e)[4][4], uint32_t Qt, W window, int qt, int hf, float *es, int lane, const uint32_t (&oa)[4],
+                                                    const uint32_t (&ob)[4])
+{
+    const int g = lane >> 2, t = lane & 3;
+    float x[6][4];
+#pragma unroll
+    for (int n = 0; n < 6; n++)
+#pragma unroll
+        for (int c = 0; c < 4; c++)
+            x[n][c] = 0.0f;
+#pragma unroll
+    for (int ks = 0; ks < DK / 16; ks++) {
+        uint32_t q[4];
+        ldsm4_at(q, Qt + (ks >> 2) * 8192 + oa[ks & 3]);
+#pragma unroll
+        for (int p = 0; p < 3; p++) {
+            uint32_t b[4];
+            ldsm4_at(b, window(2 * hf + 3 - qt + p) + (ks >> 2) * 8192 + ob[ks & 3]);
+            mma(x[2 * p], q, b[0], b[1]);
+            mma(x[2 * p + 1], q, b[2], b[3]);
+        }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int n = 0; n < 6; n++) {
+        *reinterpret_cast<float2 *>(es + g * ESC + n * 8 + 2 * t) = make_float2(x[n][0], x[n][1]);
+        *reinterpret_cast<float2 *>(es + (g + 8) * ESC + n * 8 + 2 * t) = make_float2(x[n][2], x[n][3]);
+    }
+    __syncwarp();
+#pragma unroll
+    for (int n = 0; n < 4; n++)
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            const int row = g + (c >> 1) * 8;
+            e[n][c] = es[row * ESC + n * 8 + 2 * t + (c & 1) + 15 - row];
+        }
+}
+
+template <int DK, bool WIDE> // WIDE: out takes 16-byte stores, an fp32 table 16-byte loads
+__global__ void __launch_bounds__(256, DK <= 64 ? 2 : 1) attn_fwd_tma_kernel(const __grid_constant__ AttnArgs a, const __grid_constant__ CUtensorMap map_q,
+                                                                                    const __grid_constant__ CUtensorMap map_kv,
+                                                                                    const __grid_constant__ CUtensorMap map_r)
+{
+    using SM = FwdTmaSmem<DK>;
+    constexpr int TILE = SM::TILE, NTC = DK / 16; // 8-column groups in one column half
+    extern __shared__ __align__(16) unsigned char smraw[];
+    __shared__ __align__(8) uint64_t bars[2];
+    __shared__ int abort_s, dummy;
+    unsigned char *sm = smraw + ((1024u - (smem_addr(smraw) & 1023u)) & 1023u);
+    const uint32_t base = smem_addr(sm), bar0 = smem_addr(bars);
+    float *brs = reinterpret_cast<float *>(sm + SM::BRS);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int qt = warp & 3, hf = warp >> 2;
+    const int b = blockIdx.x / a.H, h = blockIdx.x % a.H, HD = a.H * DK, T = a.T, M = a.M, L = a.L;
+    const int i0 = (a.t0 & ~63) + blockIdx.y * 64;
+    const Blocks blk = blocks_of(M, L, a.attn_len, max(i0, a.t0), min(i0 + 64, a.t1));
+    float *es = reinterpret_cast<float *>(sm + SM::ES) + warp * 16 * ESC;
+    // of this tile: [half][row A, row B][8] maxima, then [row A, row B][32] sums of half 0
+    float *mx = reinterpret_cast<float *>(sm + SM::MX) + qt * 6 * 32, *sums = mx + 32;
+    uint4 *pfs = reinterpret_cast<uint4 *>(sm + SM::PF) + qt * 4 * 32; // A fragments of the tile's probabilities, [16-key step][lane]
+    if (threadIdx.x == 0) {
+        abort_s = 0;
+        tc::mbar_init(bar0, 1);
+        tc::mbar_init(bar0 + 8, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    pdl_wait(); // no early trigger: successors resident beside these CTAs cost more than their launch (33 % of the op alone)
+    int *ef = a.err_flag ? a.err_flag : &dummy;
+    bool ok = true; // thread 0's waits: after one that ran out it issues no copy and waits no more
+
+    const bool fold = a.P < L; // rows below the table stand for row 0; otherwise no visible pair names one
+    auto group0 = [&](int gr) { return gr * KB - i0 + a.P - M - 64; }; // first table row of group gr: window rows 0-63 of block gr, 64-127 of block gr - 1
+    auto by_hand = [&](int gr) { return a.w_r && (!a.w_r16 || (fold && group0(gr) < 0)); };
+    auto group_by_hand = [&](int gr) {
+        const bf16 *w16 = reinterpret_cast<const bf16 *>(a.w_r16) + (size_t)h * a.P * DK;
+        const float *w32 = a.w_r + (size_t)h * a.P * DK;
+        for (int idx = threadIdx.x; idx < 64 * (DK / 8); idx += 256) {
+            const int r = idx / (DK / 8), c = idx % (DK / 8), x = min(max(group0(gr) + r, 0), a.P - 1);
+            bf16 *to = reinterpret_cast<bf16 *>(sm + SM::R + (gr % 3) * TILE + tile_at(r, c));
+            if (a.w_r16)
+                *reinterpret_cast<uint4 *>(to) = *reinterpret_cast<const uint4 *>(w16 + (size_t)x * DK + c * 8);
+            else
+                table_piece<WIDE>(to, w32 + (size_t)x * DK + c * 8);
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); // a later group may come by TMA to the same place
+    };
+    // block kb: its keys and values, the upper half of its window, and with the first block Q and the lower half
+    auto fetch = [&](int kb) {
+        const bool first = kb == blk.lo, lower = first && a.w_r && !by_hand(kb), upper = a.w_r && !by_hand(kb + 1);
+        if (threadIdx.x == 0 && ok) {
+            const uint32_t bar = bar0 + 8 * (kb & 1);
+            tc::mbar_expect_tx(bar, (uint32_t)((2 + (first ? 1 : 0) + (lower ? 1 : 0) + (upper ? 1 : 0)) * TILE));
+#pragma unroll
+            for (int n = 0; n < SM::NS; n++) {
+                if (first)
+                    tma_load_3d(base + SM::Q + n * 8192, &map_q, bar, h * DK + n * 64, b, i0);
+                tma_load_3d(base + SM::K + (kb & 1) * TILE + n * 8192, &map_kv, bar, h * DK + n * 64, b, kb * KB);
+                if (lower)
+                    tma_load_3d(base + SM::R + (kb % 3) * TILE + n * 8192, &map_r, bar, n * 64, group0(kb), h);
+                if (upper)
+                    tma_load_3d(base + SM::R + ((kb + 1) % 3) * TILE + n * 8192, &map_r, bar, n * 64, group0(kb + 1), h);
+                tma_load_3d(base + SM::V + (kb & 1) * TILE + n * 8192, &map_kv, bar, HD + h * DK + n * 64, b, kb * KB);
+            }
+        }
+        if (first && by_hand(kb))
+            group_by_hand(kb);
+        if (by_hand(kb + 1))
+            group_by_hand(kb + 1);
+    };
+    fetch(blk.lo);
+    load_br(brs, a, h, threadIdx.x, 256);
+    uint32_t oa[4], ob[4]; // swizzled chunks of this lane's rows: of an operand of 16 rows, and of one of 8 x 2
+#pragma unroll
+    for (int n = 0; n < 4; n++) {
+        oa[n] = (uint32_t)((lane & 15) * 128 + (((n * 2 + (lane >> 4)) ^ (lane & 7)) << 4));
+        ob[n] = (uint32_t)(((lane & 7) + (lane >> 4) * 8) * 128 + (((n * 2 + ((lane >> 3) & 1)) ^ (lane & 7)) << 4));
+    }
+    const uint32_t Qt = base + SM::Q + qt * 2048;
+    const int iA = i0 + qt * 16 + g, iB = iA + 8; // this thread's two rows
+    const bool active = i0 + qt * 16 < a.t1 && i0 + qt * 16 + 16 > a.t0;
+
+    float o[NTC][4], mA = -INFINITY, mB = -INFINITY, lA = 0.0f, lB = 0.0f;
+#pragma unroll
+    for (int n = 0; n < NTC; n++)
+#pragma unroll
+        for (int c = 0; c < 4; c++)
+            o[n][c] = 0.0f;
+
+    for (int kb = blk.lo; kb <= blk.hi; kb++) {
+        const int j0 = kb * KB;
+        if (threadIdx.x == 0)
+            ok = ok && tc::mbar_wait(bar0 + 8 * (kb & 1), (uint32_t)(((kb - blk.lo) >> 1) & 1), &abort_s, ef, 48);
+        __syncthreads(); // this block's tiles have landed, the one before has been read
+        if (kb < blk.hi)
+            fetch(kb + 1);
+        if (!active)
+            continue;
+        float s[4][4], mbA = -INFINITY, mbB = -INFINITY;
+        {
+            float e[4][4] = {};
+            product_16x32_at<DK>(s, Qt, base + SM::K + (kb & 1) * TILE + hf * 4096, oa, ob);
+            if (a.w_r)
+                skewed_positions_at<DK>(e, Qt, [&](int p) { return base + SM::R + ((kb + (p >> 2)) % 3) * TILE + (p & 3) * 2048; }, qt, hf, es, lane, oa, ob);
+            scores_16x32(s, e, brs, a, i0 + qt * 16, j0 + hf * 32, 1 << 30, lane);
+        }
+#pragma unroll
+        for (int n = 0; n < 4; n++) {
+            mbA = fmaxf(mbA, fmaxf(s[n][0], s[n][1]));
+            mbB = fmaxf(mbB, fmaxf(s[n][2], s[n][3]));
+        }
+        mbA = fmaxf(mbA, __shfl_xor_sync(0xffffffffu, mbA, 1));
+        mbB = fmaxf(mbB, __shfl_xor_sync(0xffffffffu, mbB, 1));
+        mbA = fmaxf(mbA, __shfl_xor_sync(0xffffffffu, mbA, 2));
+        mbB = fmaxf(mbB, __shfl_xor_sync(0xffffffffu, mbB, 2));
+        if (t == 0) {
+            mx[hf * 16 + g] = mbA;
+            mx[hf * 16 + 8 + g] = mbB;
+        }
+        asm volatile("bar.sync %0, 64;" ::"r"(1 + qt) : "memory");
+        mbA = fmaxf(mbA, mx[(hf ^ 1) * 16 + g]);
+        mbB = fmaxf(mbB, mx[(hf ^ 1) * 16 + 8 + g]);
+        const float nA = fmaxf(mA, mbA), nB = fmaxf(mB, mbB);
+        const float uA = nA == -INFINITY ? 0.0f : nA, uB = nB == -INFINITY ? 0.0f : nB;
+        const float scA = __expf(__fsub_rn(mA, uA)), scB = __expf(__fsub_rn(mB, uB));
+        mA = nA;
+        mB = nB;
+        float sA = 0.0f, sB = 0.0f, xA[4], xB[4];
+#pragma unroll
+        for (int n = 0; n < 4; n++) {
+            s[n][0] = __expf(__fsub_rn(s[n][0], uA));
+            s[n][1] = __expf(__fsub_rn(s[n][1], uA));
+            s[n][2] = __expf(__fsub_rn(s[n][2], uB));
+            s[n][3] = __expf(__fsub_rn(s[n][3], uB));
+            xA[n] = __fadd_rn(s[n][0], s[n][1]);
+            xB[n] = __fadd_rn(s[n][2], s[n][3]);
+            sA = __fadd_rn(sA, xA[n]);
+            sB = __fadd_rn(sB, xB[n]);
+        }
+#pragma unroll
+        for (int ks = 0; ks < 2; ks++)
+            pfs[(hf * 2 + ks) * 32 + lane] = make_uint4(pack2(s[2 * ks][0], s[2 * ks][1]), pack2(s[2 * ks][2], s[2 * ks][3]),
+                                                        pack2(s[2 * ks + 1][0], s[2 * ks + 1][1]), pack2(s[2 * ks + 1][2], s[2 * ks + 1][3]));
+        if (hf == 0) {
+            sums[lane] = sA;
+            sums[32 + lane] = sB;
+        }
+        asm volatile("bar.sync %0, 64;" ::"r"(1 + qt) : "memory");
+        if (hf == 1) { // the row's sum runs over the keys in order: half 1 carries on from half 0
+            sA = sums[lane];
+            sB = sums[32 + lane];
+#pragma unroll
+            for (int n = 0; n < 4; n++) {
+                sA = __fadd_rn(sA, xA[n]);
+                sB = __fadd_rn(sB, xB[n]);
+            }
+            lA = __fmaf_rn(lA, scA, sA);
+            lB = __fmaf_rn(lB, scB, sB);
+        }
+        {
+#pragma unroll
+            for (int n = 0; n < NTC; n++) {
+                o[n][0] = __fmul_rn(o[n][0], scA);
+                o[n][1] = __fmul_rn(o[n][1], scA);
+                o[n][2] = __fmul_rn(o[n][2], scB);
+                o[n][3] = __fmul_rn(o[n][3], scB);
+            }
+            const uint32_t vb = base + SM::V + (kb & 1) * TILE + ((lane & 7) + ((lane >> 3) & 1) * 8) * 128 + (DK == 128 ? hf * 8192 : 0);
+            const int vc = (DK == 64 ? hf * 4 : 0) + (lane >> 4);
+#pragma unroll
+            for (int ks = 0; ks < 4; ks++) {
+                const uint4 u = pfs[ks * 32 + lane];
+                const uint32_t pf[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+                for (int p = 0; p < NTC / 2; p++) {
+                    uint32_t bb[4];
+                    ldsm4t_at(bb, vb + ks * 2048 + (((vc + p * 2) ^ (lane & 7)) << 4));
+                    mma(o[2 * p], pf, bb[0], bb[1]);
+                    mma(o[2 * p + 1], pf, bb[2], bb[3]);
+                }
+            }
+        }
+    }
+    if (threadIdx.x == 0 && !ok) // copies still in flight land in this CTA's shared memory: both get a bounded chance to finish
+        for (uint32_t n = 0; n < 4; n++)
+            tc::mbar_wait(bar0 + 8 * (n & 1), n >> 1, &abort_s, ef, 48);
+    if (!active)
+        return;
+    if (hf == 1) {
+        lA = __fadd_rn(lA, __shfl_xor_sync(0xffffffffu, lA, 1));
+        lB = __fadd_rn(lB, __shfl_xor_sync(0xffffffffu, lB, 1));
+        lA = __fadd_rn(lA, __shfl_xor_sync(0xffffffffu, lA, 2));
+        lB = __fadd_rn(lB, __shfl_xor_sync(0xffffffffu, lB, 2));
+        sums[lane] = lA;
+        sums[32 + lane] = lB;
+    }
+    asm volatile("bar.sync %0, 64;" ::"r"(1 + qt) : "memory");
+    lA = sums[lane];
+    lB = sums[32 + lane];
+    const bool okA = iA >= a.t0 && iA < a.t1, okB = iB >= a.t0 && iB < a.t1;
+    {
+        const bool lost = *static_cast<volatile int *>(&abort_s); // a wait ran out: no result
+        const float rA = lost ? __int_as_float(0x7fffffff) : __fdiv_rn(1.0f, lA), rB = lost ? rA : __fdiv_rn(1.0f, lB);
+#pragma unroll
+        for (int n = 0; n < NTC; n++) {
+            o[n][0] = __fmul_rn(o[n][0], rA);
+            o[n][1] = __fmul_rn(o[n][1], rA);
+            o[n][2] = __fmul_rn(o[n][2], rB);
+            o[n][3] = __fmul_rn(o[n][3], rB);
+        }
+        bf16 *out = reinterpret_cast<bf16 *>(a.o) + ((size_t)iA * a.B + b) * HD + h * DK + hf * (DK / 2);
+        store_row<WIDE>(out, o, 0, t, okA);
+        store_row<WIDE>(out + (size_t)8 * a.B * HD, o, 2, t, okB);
+    }
+    if (hf == 0 && t == 0 && a.lse) {
+        float *lse = a.lse + ((size_t)b * a.H + h) * T;
+        if (okA)
+            lse[iA] = mA + logf(lA);
+        if (okB)
+            lse[iB] = mB + logf(lB);
+    }
+}
+
 // ---------------- backward ----------------
 //
 // One CTA of eight warps per (stream, head), key blocks in ascending order; per block
@@ -1457,9 +1755,23 @@ template <int DK> static int forward_dk(const AttnArgs &a, cudaStream_t st)
         return forward_one<DK>(a, st);
     static DeviceOnce once[2];
     const bool wide = aligned_to(a.o, 16) && aligned_to(a.w_r, 16);
-    auto kernel = wide ? attn_fwd_kernel<DK, true> : attn_fwd_kernel<DK, false>;
-    NNCU_TRY(smem_limit(once[wide], kernel, SMEM_MOST));
-    launch_kind(EDGE_ATTN, kernel, dim3(a.B * a.H, (a.t1 - (a.t0 & ~63) + 63) / 64), dim3(256), FwdSmem<DK>::bytes(a.L), st, a);
+    const dim3 grid(a.B * a.H, (a.t1 - (a.t0 & ~63) + 63) / 64);
+    if constexpr (DK >= 64) {
+        CUtensorMap q, kv, r;
+        const cuuint64_t B = a.B, T = a.T, L = a.L, qp = a.qp, kvp = a.kvp, H = a.H, P = a.P;
+        NNCU_TRY(tile_map(a.q, {H * DK, B, T}, {qp * 2, B * qp * 2}, true, &q));
+        NNCU_TRY(tile_map(a.kv, {2 * H * DK, B, L}, {kvp * 2, B * kvp * 2}, true, &kv));
+        r = kv;
+        if (a.w_r16)
+            NNCU_TRY(tile_map(a.w_r16, {DK, P, H}, {DK * 2, P * DK * 2}, false, &r));
+        auto kernel = wide ? attn_fwd_tma_kernel<DK, true> : attn_fwd_tma_kernel<DK, false>;
+        NNCU_TRY(smem_limit(once[wide], kernel, SMEM_MOST - 1024)); // its barriers are static
+        launch_kind(EDGE_ATTN, kernel, grid, dim3(256), FwdTmaSmem<DK>::bytes(a.L), st, a, q, kv, r);
+    } else {
+        auto kernel = wide ? attn_fwd_kernel<DK, true> : attn_fwd_kernel<DK, false>;
+        NNCU_TRY(smem_limit(once[wide], kernel, SMEM_MOST));
+        launch_kind(EDGE_ATTN, kernel, grid, dim3(256), FwdSmem<DK>::bytes(a.L), st, a);
+    }
     KERNEL_CHECK();
     return NNCU_OK;
 }
