@@ -25,6 +25,7 @@ struct AttnArgs {
     float *lse, *dwr_part, *dbr_part;
     int *err_flag; // raised when a bounded wait runs out, may be NULL
     int B, H, dk, T, M, L, P, attn_len, t0, t1, qchunk;
+    int sum;        // adjoint: dwr_part holds sums over the streams that a CTA takes (fab::Share), not one table a stream
     int ahead;      // one query: keys and values of other steps, and the tables, may be read before the wait for the predecessor
     int smem_pitch; // row pitch of the staged K and table rows (CUDA-core kernels)
     int qp, kvp, dqp, dkvp; // row pitches (elements) of q, kv, dq, dkv; K then V inside a kv row

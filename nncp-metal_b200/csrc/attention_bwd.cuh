@@ -142,14 +142,37 @@ __device__ __forceinline__ void tmem_ld_frag16(uint32_t taddr, uint32_t *r)
 __device__ __forceinline__ void fence_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void bar_compute() { asm volatile("bar.sync 1, 512;" ::: "memory"); }
 
+// The pairs, all streams of a head after another, in as even runs as there are CTAs: where CTA c starts, and the CTA that
+// has a place of the sequence.
+struct Share {
+    int q, r; // r CTAs with q + 1 pairs, the others with q
+    __host__ __device__ Share(int pairs, int ctas) : q(pairs / ctas), r(pairs % ctas) {}
+    __host__ __device__ int start(int c) const { return c * q + (c < r ? c : r); }
+    __host__ __device__ int cta_of(int at) const { return at < r * (q + 1) ? at / (q + 1) : r + (at - r * (q + 1)) / q; }
+};
+inline __host__ __device__ int ctas_of(int pairs) { return pairs < 148 ? pairs : 148; }
+// how many CTAs have pairs of head h: with AttnArgs::sum its table's partial sums are in that many slots
+inline __host__ __device__ int slots_of(int B, int H, int h)
+{
+    const Share s(B * H, ctas_of(B * H));
+    return s.cta_of(h * B + B - 1) - s.cta_of(h * B) + 1;
+}
+
 // the CTA's items (stream, head) and their key blocks as one sequence; each role steps through it on its own
-struct Walk {
-    int lo, nkb, H, item, n, kb, b, h; // n: items before this one
-    __device__ void at(int i)
+template <bool SUM> struct Walk {
+    int lo, nkb, B, H, start, step, item, n, kb, b, h; // n: items before this one
+    __device__ void at(int k)
     {
-        item = i;
-        b = i / H;
-        h = i - b * H;
+        const int i = start + k * step;
+        if (SUM) {
+            h = i / B;
+            b = i - h * B;
+        } else {
+            b = i / H;
+            h = i - b * H;
+        }
+        item = b * H + h;
+        n = k;
     }
     __device__ bool first() const { return kb == lo; }
     __device__ bool last() const { return kb == lo + nkb - 1; }
@@ -160,12 +183,11 @@ struct Walk {
             return;
         }
         kb = lo;
-        n++;
-        at(item + (int)gridDim.x);
+        at(n + 1);
     }
 };
 
-template <int DK, bool WIDE> // WIDE: out, w_r, dq, dkv and the table's partials take 16-byte accesses
+template <int DK, bool WIDE, bool SUM> // SUM: AttnArgs::sum; WIDE: out, w_r, dq, dkv and the table's partials take 16-byte accesses
 __global__ void __launch_bounds__(THREADS, 1)
 attn_bwd_tc_kernel(const __grid_constant__ AttnArgs a, const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_o,
                    const __grid_constant__ CUtensorMap map_kv, const __grid_constant__ CUtensorMap map_r,
@@ -190,16 +212,32 @@ attn_bwd_tc_kernel(const __grid_constant__ AttnArgs a, const __grid_constant__ C
     auto bar = [&](int i) { return bar0 + 8 * (uint32_t)i; };
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int B = a.B, HD = a.H * DK, T = a.T, M = a.M, L = a.L, P = a.P;
-    Walk wk;
+    Walk<SUM> wk;
     {
         const fa::Blocks all = fa::blocks_of(M, L, a.attn_len, 0, T); // in 64-key blocks
         wk.lo = wk.kb = all.lo / 2;
         wk.nkb = all.hi / 2 - wk.lo + 1;
+        wk.B = B;
         wk.H = a.H;
-        wk.n = 0;
-        wk.at(blockIdx.x);
     }
-    const int lo = wk.lo, n_items = (B * a.H - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x, G = n_items * wk.nkb;
+    int n_items;
+    if (SUM) {
+        const Share share(B * a.H, gridDim.x);
+        wk.start = share.start(blockIdx.x);
+        wk.step = 1;
+        n_items = share.start(blockIdx.x + 1) - wk.start;
+    } else {
+        wk.start = blockIdx.x;
+        wk.step = gridDim.x;
+        n_items = (B * a.H - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
+    }
+    wk.at(0);
+    const int lo = wk.lo, G = n_items * wk.nkb;
+    // where an item's table gradient goes; with a.sum all items of a head that this CTA has share a slot, and add to it but for the first
+    auto table_at = [&](int item, int h) {
+        return a.dwr_part + (SUM ? (size_t)((int)blockIdx.x - Share(B * a.H, gridDim.x).cta_of(h * B)) * a.H + h : (size_t)item) * P * DK;
+    };
+    auto adds = [&](int n, int b) { return SUM && n > 0 && b > 0; };
     constexpr int LB = NB - 1; // log2 NB
     constexpr bool STAGED = NB == 2 && WIDE; // dK and dV leave from the places of K and V by TMA
     auto window0 = [&](int kb) { return kb * KB + P - M - 64; }; // table row of window row 0
@@ -230,7 +268,7 @@ attn_bwd_tc_kernel(const __grid_constant__ AttnArgs a, const __grid_constant__ C
         if (lane == 0) {
             bool ok = true;
             // the results of block g out of the places of its K and V; `w` stands at it
-            auto store = [&](const Walk &w, int g) {
+            auto store = [&](const Walk<SUM> &w, int g) {
                 const int s = g & (NB - 1);
                 if (!(ok = mbar_wait(bar(FREE_KV + s), (uint32_t)((g >> LB) & 1), abort_s, ef, 62)))
                     return;
@@ -238,7 +276,7 @@ attn_bwd_tc_kernel(const __grid_constant__ AttnArgs a, const __grid_constant__ C
                 tma_store_3d(&map_dkv, sm0 + SM::V + s * SM::KT, HD + w.h * DK, w.b, w.kb * KB);
                 asm volatile("cp.async.bulk.commit_group;\n\tcp.async.bulk.wait_group.read 0;" ::: "memory");
             };
-            Walk ws = wk; // where the stores are
+            auto ws = wk; // where the stores are
             for (int g = 0; ok && g < G; g++, wk.next()) {
                 const int s = g & (NB - 1), b = wk.b, h = wk.h, kb = wk.kb, j0 = kb * KB;
                 if (wk.first()) {
@@ -295,7 +333,7 @@ attn_bwd_tc_kernel(const __grid_constant__ AttnArgs a, const __grid_constant__ C
                 return ok;
             };
             // scores, positions and dP of block g
-            Walk w1 = wk; // where phase1 is
+            auto w1 = wk; // where phase1 is
             auto phase1 = [&](int g) {
                 const int s = g & (NB - 1), n = w1.n, qs = n & (NB - 1);
                 const bool first = w1.first();
@@ -383,7 +421,9 @@ attn_bwd_tc_kernel(const __grid_constant__ AttnArgs a, const __grid_constant__ C
                     ok = mbar_wait(bar(ROWS_FREE + (n & 1)), (uint32_t)((n / 2 - 1) & 1), abort_s, ef, 69);
                 __syncwarp();
             }
-            const int item = blockIdx.x + n * gridDim.x, b = item / a.H, h = item - b * a.H;
+            auto of = wk;
+            of.at(n);
+            const int b = of.b, h = of.h, item = of.item;
             float *lses = reinterpret_cast<float *>(sm + SM::ROW) + (n & 1) * 128, *Dr = lses + 64;
             float *brs = reinterpret_cast<float *>(sm + SM::BRS) + (n & 1) * SM::br_floats(L);
             constexpr int LPR = DK / 8, RPW = 32 / LPR, IT = 32 / RPW; // lanes per row, rows at a time, times for a warp's 32 rows
@@ -442,8 +482,8 @@ attn_bwd_tc_kernel(const __grid_constant__ AttnArgs a, const __grid_constant__ C
                 fa::zero16<WIDE>(dkv + (size_t)j * B * a.dkvp + HD + c);
             }
             const int below = min(P, max(0, x_lo)), above = max(0, P - 1 - x_hi);
-            if (dwr0) {
-                float *dwr = dwr0 + (size_t)item * P * DK;
+            if (dwr0 && !adds(n, b)) {
+                float *dwr = table_at(item, h);
                 for (int idx = tid; idx < (below + above) * (DK / 4); idx += 64) {
                     const int k = idx / (DK / 4), x = k < below ? k : x_hi + 1 + k - below;
                     fa::zero16<WIDE>(dwr + (size_t)x * DK + (idx % (DK / 4)) * 4);
@@ -531,7 +571,7 @@ attn_bwd_tc_kernel(const __grid_constant__ AttnArgs a, const __grid_constant__ C
                 arrive(bar(i));
         };
         // the table window of block g, which `w` stands at, by ordinary stores (rounded from fp32, or with copies of row 0)
-        auto window_by_hand = [&](const Walk &w, int g) {
+        auto window_by_hand = [&](const Walk<SUM> &w, int g) {
             const int h = w.h, x0 = window0(w.kb);
             unsigned char *dst = sm + SM::R + (g & (NB - 1)) * SM::RT;
             const bf16 *w16 = reinterpret_cast<const bf16 *>(a.w_r16) + (size_t)h * P * DK;
@@ -585,7 +625,7 @@ attn_bwd_tc_kernel(const __grid_constant__ AttnArgs a, const __grid_constant__ C
         };
         float *pad = reinterpret_cast<float *>(sm + SM::PAD);
         // sums of table rows xb + 0 .. 127 out, as load_table has them
-        auto store_table = [&](float *dwr, int xb, const uint32_t *x) {
+        auto store_table = [&](float *dwr, int xb, const uint32_t *x, bool add) {
             if (fold && xb + qd * 32 <= 0) { // the same for the whole warp: rows at or below 0 go to this warp's share of row 0
 #pragma unroll
                 for (int c = 0; c < NC / 8; c++)
@@ -605,12 +645,20 @@ attn_bwd_tc_kernel(const __grid_constant__ AttnArgs a, const __grid_constant__ C
             }
             const int r0 = xb + qd * 32 + (lane >> 2), least = fold ? 1 : 0;
             float *dst = dwr + (ptrdiff_t)r0 * DK + cg * NC + 2 * t4;
+            auto rows = [&](auto f) {
 #pragma unroll
-            for (int k = 0; k < 4; k++)
-                if (r0 + 8 * k >= least && r0 + 8 * k < P)
+                for (int k = 0; k < 4; k++)
+                    if (r0 + 8 * k >= least && r0 + 8 * k < P)
 #pragma unroll
-                    for (int c = 0; c < NC / 8; c++)
-                        *reinterpret_cast<uint2 *>(dst + 8 * k * DK + 8 * c) = make_uint2(x[8 * c + 2 * k], x[8 * c + 2 * k + 1]);
+                        for (int c = 0; c < NC / 8; c++)
+                            f(dst + 8 * k * DK + 8 * c, x[8 * c + 2 * k], x[8 * c + 2 * k + 1]);
+            };
+            if (add) // no other thread has these places, so the sums are taken in the order of the items
+                rows([](float *p, uint32_t v0, uint32_t v1) {
+                    asm volatile("red.relaxed.gpu.global.add.v2.f32 [%0], {%1, %2};" ::"l"(p), "f"(__uint_as_float(v0)), "f"(__uint_as_float(v1)) : "memory");
+                });
+            else
+                rows([](float *p, uint32_t v0, uint32_t v1) { *reinterpret_cast<uint2 *>(p) = make_uint2(v0, v1); });
         };
         auto load_table = [&](uint32_t *x) {
 #pragma unroll
@@ -628,7 +676,8 @@ attn_bwd_tc_kernel(const __grid_constant__ AttnArgs a, const __grid_constant__ C
             const bool first = wk.first(), last = wk.last();
             const float *lses = reinterpret_cast<const float *>(sm + SM::ROW) + (n & 1) * 128 + cg * 16;
             const float *br = reinterpret_cast<const float *>(sm + SM::BRS) + (n & 1) * SM::br_floats(L) + BR_LO + j0 + jj + T - 1 - cg * 16;
-            float *dwr = dwr0 ? dwr0 + (size_t)wk.item * P * DK : nullptr;
+            float *dwr = dwr0 ? table_at(wk.item, h) : nullptr;
+            const bool add = adds(n, b);
             if (first) {
                 if (fold && dwr) { // own shares
                     for (int c = lane; c < NC; c += 32)
@@ -736,7 +785,7 @@ attn_bwd_tc_kernel(const __grid_constant__ AttnArgs a, const __grid_constant__ C
             if (last)
                 if (lane == 0)
                     arrive(bar(ROWS_FREE + (n & 1)));
-            Walk following = wk;
+            auto following = wk;
             following.next();
             const bool hand = g + 1 < G && by_hand(following.kb);
             if (NB == 2 && hand)
@@ -747,7 +796,7 @@ attn_bwd_tc_kernel(const __grid_constant__ AttnArgs a, const __grid_constant__ C
                 load_table(x);
             signal(TR_FREE);
             if (dwr)
-                store_table(dwr, window0(kb), x);
+                store_table(dwr, window0(kb), x, add);
             if constexpr (STAGED) { // into the places of V and K, which the producer sends out
                 auto park = [&](unsigned char *tile) {
                     unsigned char *row = tile + jj * 128;
@@ -800,13 +849,13 @@ attn_bwd_tc_kernel(const __grid_constant__ AttnArgs a, const __grid_constant__ C
                 if (dwr) {
                     if (qd < 2) { // the upper 64 rows of the last window
                         load_table(x);
-                        store_table(dwr, window0(kb) + 128, x);
+                        store_table(dwr, window0(kb) + 128, x, add);
                     }
                     if (fold) {
                         bar_compute();
                         if (window0(lo) <= 0)
                             for (int c = threadIdx.x; c < DK; c += CT)
-                                dwr[c] = (pad[c] + pad[DK + c]) + (pad[2 * DK + c] + pad[3 * DK + c]);
+                                dwr[c] = (add ? dwr[c] : 0.0f) + ((pad[c] + pad[DK + c]) + (pad[2 * DK + c] + pad[3 * DK + c]));
                         bar_compute();
                     }
                 }
@@ -835,6 +884,10 @@ static bool takes(const AttnArgs &a)
 {
     return a.dk == 64 ? Smem<64>::bytes(a.L) <= (size_t)SMEM_LIMIT : a.dk == 128 && Smem<128>::bytes(a.L) <= (size_t)SMEM_LIMIT;
 }
+// Table gradients added up by the CTA, in its own slot, instead of a table for each stream that the reduction reads again: where it
+// has four pairs or more.  The tables of 1024 pairs are 84 (320 rows) or 151 MB (576) a layer each way; steps of 20 layers 16196 -> 15999 us,
+// of 12 10469 -> 10359.  With 256 pairs, two to a CTA, it cost 0.5 % (2261 -> 2272 us): the tables stay in L2 and the added rows are slower.
+static bool sums(const AttnArgs &a) { return a.B * a.H >= 4 * 148; }
 template <int DK> static int launch(const AttnArgs &a, cudaStream_t st)
 {
     CUtensorMap q, o, kv, r, dkv;
@@ -850,10 +903,11 @@ template <int DK> static int launch(const AttnArgs &a, cudaStream_t st)
     dkv = kv;
     if (wide && Smem<DK>::NB == 2)
         NNCU_TRY(fa::tile_map(a.dkv, {2 * HD, B, L}, {(cuuint64_t)a.dkvp * 2, B * a.dkvp * 2}, true, &dkv, KB));
-    auto kernel = wide ? attn_bwd_tc_kernel<DK, true> : attn_bwd_tc_kernel<DK, false>;
-    static DeviceOnce once[2];
-    NNCU_TRY(smem_limit(once[wide], kernel, SMEM_LIMIT));
-    launch_kind(EDGE_ATTN, kernel, dim3(std::min(a.B * a.H, 148)), dim3(THREADS), Smem<DK>::bytes(a.L), st, a, q, o, kv, r, dkv);
+    auto kernel = a.sum ? (wide ? attn_bwd_tc_kernel<DK, true, true> : attn_bwd_tc_kernel<DK, false, true>)
+                        : (wide ? attn_bwd_tc_kernel<DK, true, false> : attn_bwd_tc_kernel<DK, false, false>);
+    static DeviceOnce once[4];
+    NNCU_TRY(smem_limit(once[2 * a.sum + wide], kernel, SMEM_LIMIT));
+    launch_kind(EDGE_ATTN, kernel, dim3(ctas_of(a.B * a.H)), dim3(THREADS), Smem<DK>::bytes(a.L), st, a, q, o, kv, r, dkv);
     KERNEL_CHECK();
     return NNCU_OK;
 }

@@ -1808,6 +1808,7 @@ static int backward(const AttnArgs &a, cudaStream_t st)
 
 namespace fab { // attention_bwd.cuh
 static bool takes(const AttnArgs &a);
+static bool sums(const AttnArgs &a);
 static int backward(const AttnArgs &a, cudaStream_t st);
 } // namespace fab
 
@@ -1829,11 +1830,12 @@ static int attn_forward_any(const nncu_attn_shape *s, const void *q, const void 
     return attn_forward_t<T>(s, q, kv, w_r, b_r, out, lse, st, pt);
 }
 
+// With `sums` dwr_part may come back as sums over streams in fewer parts (fab::slots_of); *sums says whether.
 template <typename T>
 static int attn_backward_any(const nncu_attn_shape *s, const void *q, const void *kv, const float *w_r,
                              const float *b_r, const void *out, const float *lse, const void *dout,
                              void *dq, void *dkv, float *dwr_part, float *dbr_part, cudaStream_t st,
-                             const AttnPitch *pt = nullptr, const void *w_r16 = nullptr, int *err_flag = nullptr)
+                             const AttnPitch *pt = nullptr, const void *w_r16 = nullptr, int *err_flag = nullptr, bool *sums = nullptr)
 {
     if (sizeof(T) == 2) {
         AttnArgs a = attn_args(s, pt);
@@ -1841,8 +1843,13 @@ static int attn_backward_any(const nncu_attn_shape *s, const void *q, const void
         a.err_flag = err_flag;
         a.q = q; a.kv = kv; a.w_r = w_r; a.b_r = b_r; a.out = out; a.lse = const_cast<float *>(lse);
         a.dout = dout; a.dq = dq; a.dkv = dkv; a.dwr_part = dwr_part; a.dbr_part = dbr_part;
-        if (fa::supported_bwd(a) && fa::fits(a.dk, a.L))
-            return fab::takes(a) ? fab::backward(a, st) : fa::backward(a, st);
+        if (fa::supported_bwd(a) && fa::fits(a.dk, a.L)) {
+            if (!fab::takes(a))
+                return fa::backward(a, st);
+            if (sums)
+                *sums = a.sum = fab::sums(a);
+            return fab::backward(a, st);
+        }
     }
     return attn_backward_t<T>(s, q, kv, w_r, b_r, out, lse, dout, dq, dkv, dwr_part, dbr_part, st, pt);
 }

@@ -416,6 +416,8 @@ __global__ void splitk_reduce_kernel(const float *__restrict__ ws, int ksplit, s
 //   0  out[c] = sum over parts p of part[p*stride + off + c], the parts dealt to 8 groups of
 //      consecutive parts whose sums are added in group order
 //   1  out[i] (+)= sum over parts (streams) in order of part[p*stride + i]
+//   2  the same for the position table, [n_parts streams] x [heads][off] values, whose heads are each summed over streams
+//      into fab::slots_of parts already
 // blk0 is the job's first block; a block finds its job by a short scan (the table is a kernel
 // argument, so the launch can sit in a captured graph).
 struct ReduceJob {
@@ -437,12 +439,15 @@ __global__ void __launch_bounds__(256) reduce_jobs_kernel(const __grid_constant_
         j++;
     const ReduceJob &jb = jobs.job[j];
     const int blk = blockIdx.x - jb.blk0;
-    if (jb.kind == 1) {
+    if (jb.kind >= 1) {
         const int i = blk * 256 + threadIdx.x;
         if (i < jb.n) {
+            int parts = jb.n_parts;
+            if (jb.kind == 2)
+                parts = fab::slots_of(parts, jb.n / jb.off, i / jb.off);
             float s = 0.0f;
 #pragma unroll 8 // eight parts' loads in flight
-            for (int p = 0; p < jb.n_parts; p++)
+            for (int p = 0; p < parts; p++)
                 s += jb.part[(size_t)p * jb.stride + i];
             jb.out[i] = jb.accumulate ? jb.out[i] + s : s;
         }

@@ -455,7 +455,7 @@ static int queue_reduction(nncu_model *m, int kind, const float *part, int n_par
     ReduceJob &j = m->rjobs.job[m->rjobs.n_jobs++];
     j.part = part; j.out = out; j.n_parts = n_parts; j.stride = stride; j.n = n; j.off = off; j.kind = kind;
     j.accumulate = accumulate; j.blk0 = m->rjob_blocks;
-    m->rjob_blocks += kind == 1 ? ceil_div(n, 256) : ceil_div(n, 32);
+    m->rjob_blocks += kind >= 1 ? ceil_div(n, 256) : ceil_div(n, 32);
     return NNCU_OK;
 }
 // out_k[c] = sum over parts of part[p*stride + off_k + c], up to three outputs
@@ -1043,16 +1043,17 @@ static int backward(nncu_model *m)
         NNCU_TRY(mm_tn(m, D, HD, TB, dt1, D, atc<AT>(a.o, 0), HD, gf(m, o.w_o)));
         NNCU_TRY(mm_nn(m, TB, HD, D, dt1, D, o.w_o, dof, HD, (const AT *)nullptr));
         nncu_attn_shape s = attn_shape(m, l, 0, m->T);
+        bool sums = false;
         NNCU_TRY(attn_backward_any<AT>(&s, at<AT>(a.qkv, (size_t)M * B * 3 * HD), at<AT>(a.qkv, HD), wf(m, o.w_r),
                                        m->W + o.b_r, a.o, a.lse, dof, dq, dkv, dwr_part, dbr_part, m->st,
-                                       &pt, (m->bf && o.w_r != NONE) ? m->Wb + o.w_r : nullptr, m->err_flag));
+                                       &pt, (m->bf && o.w_r != NONE) ? m->Wb + o.w_r : nullptr, m->err_flag, &sums));
         {
             // the partials are next written two layers on
             size_t nb = (size_t)m->H * m->L;
             NNCU_TRY(queue_reduction(m, 1, dbr_part, B, (int)nb, (int)nb, 0, gf(m, o.b_r), p.tied_b_r ? 1 : 0));
             if (o.w_r != NONE) {
                 size_t nw = (size_t)m->H * p.d_pos * m->dk;
-                NNCU_TRY(queue_reduction(m, 1, dwr_part, B, (int)nw, (int)nw, 0, gf(m, o.w_r), p.tied_w_r ? 1 : 0));
+                NNCU_TRY(queue_reduction(m, sums ? 2 : 1, dwr_part, B, (int)nw, (int)nw, p.d_pos * m->dk, gf(m, o.w_r), p.tied_w_r ? 1 : 0));
             }
         }
         // d[w_q ; w_kv] = [dq | dk | dv]^T [memory ; segment] in one contraction over all L*B rows

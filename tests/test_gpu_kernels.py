@@ -266,3 +266,32 @@ def test_attention_adjoint_on_128_key_blocks_bf16(pkg, oracle, B, H, dk, T, M, P
     """The persistent kernel of head sizes 64 and 128: whole and ragged key blocks, one query, more (stream, head) pairs
     than CTAs, tables that end inside the left pad, windows that leave whole blocks out."""
     _attn_case(pkg, oracle, B, H, dk, T, M, P, alen, True, 11)
+
+
+@pytest.mark.parametrize("kw", [
+    dict(n_head=8, n_streams=74, d_pos=64),                                       # four pairs to a CTA, heads that start in mid-CTA
+    dict(n_head=8, n_streams=75, d_pos=40),                                       # four or five; copies of table row 0
+    dict(n_head=9, n_streams=66, d_pos=70, mem_len=150, attn_len=[30]),           # a window: zero rows of the table
+    dict(n_head=12, n_streams=50, d_pos=33, d_key=128, n_layer=2, tied_w_r=1),    # one table of two layers
+    dict(n_head=200, n_streams=3, d_pos=64),                                      # several heads' ends in a CTA
+    dict(n_head=8, n_streams=73, d_pos=64)])                                      # a part for each stream
+def test_position_table_gradients_summed_over_streams(pkg, kw):
+    """The table's gradient where CTAs of the adjoint sum the streams they take, head by head against the fp32 engine.  Roundings of
+    2^-9 in the dozen bf16 stages of a layer and its adjoint stay within 5 %; a stream lost or counted twice is 1 / sqrt(75) = 12 %."""
+    base = dict(n_layer=1, d_model=128, d_key=64, d_inner=128, mem_len=40, seg_len=24, n_symbols=64, init_range=0.05)
+    p = [pkg.abi.make_params(use_bf16=b, **dict(base, **kw)) for b in (1, 0)]
+    rng, got = np.random.default_rng(6), []
+    ids, tg = (rng.integers(0, 64, (3, 24, p[0].n_streams)).astype(np.int32) for _ in range(2))
+    for q in p:
+        m = pkg.TrfModel(q)
+        m.reset()
+        for s in range(3):
+            m.eval(-1, ids[s], read=False)
+            m.eval_gradient(tg[s])
+            m.memory_shift()
+        got.append({n: m.get_grad(n).reshape(q.n_head, -1) for n in m.info if "w_r" in n})
+        m.close()
+    assert got[0]
+    for n in got[0]:
+        for a, b in zip(got[0][n], got[1][n]):
+            assert np.linalg.norm(a - b) < 0.05 * np.linalg.norm(b), n
