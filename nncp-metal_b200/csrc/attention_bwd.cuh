@@ -27,7 +27,8 @@
 //   warps 18, 19 D = dO . O and the log-sum-exp of the next item, b_r, column sums of dE (the b_r gradient)
 //
 // One CTA per SM walks the (stream, head) pairs; loads run ahead over their borders.  Every wait is bounded; a
-// compute warp whose wait ran out goes on without waiting (the barriers count on it) and dq becomes NaN.
+// compute warp whose wait ran out goes on without waiting (the barriers count on it), and every result of the CTA's
+// pairs becomes NaN.
 #pragma once
 #include "attention_fa.cuh"
 
@@ -61,6 +62,9 @@ template <int DK> struct Tmem {
                          R = Q + DK;
 };
 
+#ifndef NNCU_FAB_POLLS
+#define NNCU_FAB_POLLS (1u << 24)
+#endif
 // tc::mbar_wait by polling: the waits of a block are short
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int *abort_s, int *err_flag, int code)
 {
@@ -76,7 +80,7 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
                  "NNCU_DONE:\n\t"
                  "selp.u32 %0, 1, 0, p;\n\t}"
                  : "=r"(ok)
-                 : "r"(bar), "r"(parity), "r"(1u << 24)
+                 : "r"(bar), "r"(parity), "r"(NNCU_FAB_POLLS)
                  : "memory");
     if (!ok) {
         *abort_s = 1;
@@ -836,11 +840,6 @@ attn_bwd_tc_kernel(const __grid_constant__ AttnArgs a, const __grid_constant__ C
                 load_nc(TM::Q, x); // rows 0-63; the others are the products of what lies behind dS and dE
                 if (DK == 128)
                     signal(DRAINED);
-                if (*abort_s) {
-#pragma unroll
-                    for (int c = 0; c < NC; c++)
-                        x[c] = 0x7fffffffu;
-                }
                 bf16 *dq = reinterpret_cast<bf16 *>(a.dq) + (size_t)b * a.dqp + h * DK + cg * NC;
                 store_bf16(x, [&](int u) {
                     const int i = qd * 32 + lane4 + u;
@@ -867,9 +866,31 @@ attn_bwd_tc_kernel(const __grid_constant__ AttnArgs a, const __grid_constant__ C
     // common exit: nobody touches tensor memory or the barriers after this
     __syncwarp();
     __syncthreads();
-    if (*abort_s) { // a wait gave up: let copies and products that are still in flight finish before the CTA retires
+    if (*abort_s) { // a wait gave up: copies and products that are still in flight finish before the CTA retires, then there is no result
         for (int i = 0; i < 2000; i++)
             __nanosleep(500);
+        if (threadIdx.x == 16 * 32)
+            asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+        __syncthreads();
+        auto fill = [&](void *p, int words) {
+            for (int i = threadIdx.x; i < words; i += THREADS)
+                reinterpret_cast<uint32_t *>(p)[i] = 0x7fff7fffu; // NaN as fp32 and as two bf16
+        };
+        auto of = wk;
+        for (int n = 0; n < n_items; n++) {
+            of.at(n);
+            const int col = of.h * DK;
+            for (int i = 0; i < T; i++)
+                fill(reinterpret_cast<bf16 *>(a.dq) + ((size_t)i * B + of.b) * a.dqp + col, DK / 2);
+            for (int j = 0; j < L; j++) {
+                fill(reinterpret_cast<bf16 *>(a.dkv) + ((size_t)j * B + of.b) * a.dkvp + col, DK / 2);
+                fill(reinterpret_cast<bf16 *>(a.dkv) + ((size_t)j * B + of.b) * a.dkvp + HD + col, DK / 2);
+            }
+            if (dwr0)
+                fill(table_at(of.item, of.h), P * DK);
+            if (a.dbr_part)
+                fill(a.dbr_part + (size_t)of.item * L, L);
+        }
     }
     if (warp == 17) {
         fence_after_sync();

@@ -834,14 +834,16 @@ __global__ void __launch_bounds__(128) attn_one_tma_kernel(const __grid_constant
     }
     if (lane == 0 && !ok) { // copies still in flight land in this CTA's shared memory: both phases get a bounded chance to finish
         for (uint32_t parity = 0; parity < 2; parity++) {
-            tc::mbar_wait(bar_k, parity, &abort_s, ef, 44);
-            tc::mbar_wait(bar_v, parity, &abort_s, ef, 45);
+            tc::mbar_wait(bar_k, parity, &abort_s, ef, 44, tc::DRAIN_TRIES);
+            tc::mbar_wait(bar_v, parity, &abort_s, ef, 45, tc::DRAIN_TRIES);
         }
     }
     __syncwarp();
     l = __fadd_rn(l, __shfl_xor_sync(0xffffffffu, l, 1));
     l = __fadd_rn(l, __shfl_xor_sync(0xffffffffu, l, 2));
-    const float inv = *static_cast<volatile int *>(&abort_s) ? __int_as_float(0x7fffffff) : __fdiv_rn(1.0f, l); // a wait ran out: no result
+    if (*static_cast<volatile int *>(&abort_s)) // a wait ran out: no result
+        l = __int_as_float(0x7fffffff);
+    const float inv = __fdiv_rn(1.0f, l);
     bf16 *out = reinterpret_cast<bf16 *>(a.o) + ((size_t)i * a.B + b) * HD + h * DK;
 #pragma unroll
     for (int w = 0; w < MW; w++) {
@@ -1016,14 +1018,16 @@ __global__ void __launch_bounds__(32) attn_one_warp_kernel(const __grid_constant
     }
     if (lane == 0 && !ok) { // copies still in flight land in this CTA's shared memory: both phases get a bounded chance to finish
         for (uint32_t parity = 0; parity < 2; parity++) {
-            tc::mbar_wait(bar_k, parity, &abort_s, ef, 46);
-            tc::mbar_wait(bar_v, parity, &abort_s, ef, 47);
+            tc::mbar_wait(bar_k, parity, &abort_s, ef, 46, tc::DRAIN_TRIES);
+            tc::mbar_wait(bar_v, parity, &abort_s, ef, 47, tc::DRAIN_TRIES);
         }
     }
     __syncwarp();
     l = __fadd_rn(l, __shfl_xor_sync(0xffffffffu, l, 1));
     l = __fadd_rn(l, __shfl_xor_sync(0xffffffffu, l, 2));
-    const float inv = *static_cast<volatile int *>(&abort_s) ? __int_as_float(0x7fffffff) : __fdiv_rn(1.0f, l); // a wait ran out: no result
+    if (*static_cast<volatile int *>(&abort_s)) // a wait ran out: no result
+        l = __int_as_float(0x7fffffff);
+    const float inv = __fdiv_rn(1.0f, l);
     bf16 *out = reinterpret_cast<bf16 *>(a.o) + ((size_t)i * a.B + b) * HD + h * DK;
 #pragma unroll
     for (int m = 0; m < MT; m++)
@@ -1295,7 +1299,7 @@ __global__ void __launch_bounds__(256, DK <= 64 ? 2 : 1) attn_fwd_tma_kernel(con
     }
     if (threadIdx.x == 0 && !ok) // copies still in flight land in this CTA's shared memory: both get a bounded chance to finish
         for (uint32_t n = 0; n < 4; n++)
-            tc::mbar_wait(bar0 + 8 * (n & 1), n >> 1, &abort_s, ef, 48);
+            tc::mbar_wait(bar0 + 8 * (n & 1), n >> 1, &abort_s, ef, 48, tc::DRAIN_TRIES);
     if (!active)
         return;
     if (hf == 1) {
@@ -1310,9 +1314,10 @@ __global__ void __launch_bounds__(256, DK <= 64 ? 2 : 1) attn_fwd_tma_kernel(con
     lA = sums[lane];
     lB = sums[32 + lane];
     const bool okA = iA >= a.t0 && iA < a.t1, okB = iB >= a.t0 && iB < a.t1;
+    if (*static_cast<volatile int *>(&abort_s)) // a wait ran out: no result
+        lA = lB = __int_as_float(0x7fffffff);
     {
-        const bool lost = *static_cast<volatile int *>(&abort_s); // a wait ran out: no result
-        const float rA = lost ? __int_as_float(0x7fffffff) : __fdiv_rn(1.0f, lA), rB = lost ? rA : __fdiv_rn(1.0f, lB);
+        const float rA = __fdiv_rn(1.0f, lA), rB = __fdiv_rn(1.0f, lB);
 #pragma unroll
         for (int n = 0; n < NTC; n++) {
             o[n][0] = __fmul_rn(o[n][0], rA);

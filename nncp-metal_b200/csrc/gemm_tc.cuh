@@ -61,6 +61,7 @@ constexpr uint32_t WAIT_TRIES = 1u << 24;
 #else
 constexpr uint32_t WAIT_TRIES = 1u << 21;
 #endif
+constexpr uint32_t DRAIN_TRIES = 1u << 14; // for copies still in flight after a wait that ran out: a barrier that waits for none never completes
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int *abort_s,
                                           int *err_flag, int code, uint32_t tries = WAIT_TRIES)
 {
