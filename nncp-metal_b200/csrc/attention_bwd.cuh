@@ -285,7 +285,7 @@ attn_bwd_tc_kernel(const __grid_constant__ AttnArgs a, const __grid_constant__ C
                 const int s = g & (NB - 1), b = wk.b, h = wk.h, kb = wk.kb, j0 = kb * KB;
                 if (wk.first()) {
                     const int n = wk.n, qs = n & (NB - 1);
-                    if (n >= NB && !(ok = mbar_wait(bar(FREE_QO + qs), (uint32_t)(((n >> LB) - 1) & 1), abort_s, ef, 61)))
+                    if (n >= NB && !(ok = mbar_wait(bar(FREE_QO + qs), (uint32_t)(((n >> LB) - 1) & 1), abort_s, ef, 59)))
                         break;
                     mbar_expect_tx(bar(FULL_QO + qs), 2 * SM::QT);
                     const uint32_t dst = sm0 + SM::Q + qs * 2 * SM::QT;

@@ -157,3 +157,15 @@ int main(void)
     assert r.returncode == 0, (r.returncode, r.stderr)
     size, entries, n_sym = map(int, r.stdout.split())
     assert size == C.sizeof(pkg.host.FileParams) and entries > 256 and n_sym < 68
+
+
+def test_a_wait_code_names_one_file():
+    """nncu_last_error gives the code of the bounded wait that ran out: a code is used by one kernel file."""
+    csrc, files = os.path.join(ROOT, "nncp-metal_b200", "csrc"), {}
+    for name in sorted(os.listdir(csrc)):
+        text = open(os.path.join(csrc, name)).read()
+        calls = r"(?:wait|meet)\([^;{]*?, (\d+)(?:u|, [\w:]+)?\)|atomicExch\(err_flag, (\d+)\)"
+        for code in {a or b for a, b in re.findall(calls, text)} - {"0", "1u"}:
+            files.setdefault(int(code), []).append(name)
+    assert {1, 2, 3, 41, 44, 48, 51, 60, 61, 62, 78, 90} <= set(files)
+    assert {c: f for c, f in files.items() if len(f) > 1} == {}
