@@ -30,6 +30,7 @@
 // compute warp whose wait ran out goes on without waiting (the barriers count on it), and every result of the CTA's
 // pairs becomes NaN.
 #pragma once
+#include "attention_deal.h"
 #include "attention_fa.cuh"
 
 namespace fab {
@@ -900,10 +901,12 @@ attn_bwd_tc_kernel(const __grid_constant__ AttnArgs a, const __grid_constant__ C
 
 // ---------------- host side ----------------
 
-// Head sizes 64 and 128 whose two copies of b_r find room; other shapes stay with the warp-level kernel.
+// Head sizes 64 and 128 whose two copies of b_r find room, where it is the faster kernel; other shapes stay with the warp-level one.
 static bool takes(const AttnArgs &a)
 {
-    return a.dk == 64 ? Smem<64>::bytes(a.L) <= (size_t)SMEM_LIMIT : a.dk == 128 && Smem<128>::bytes(a.L) <= (size_t)SMEM_LIMIT;
+    const bool room = a.dk == 64 ? Smem<64>::bytes(a.L) <= (size_t)SMEM_LIMIT : a.dk == 128 && Smem<128>::bytes(a.L) <= (size_t)SMEM_LIMIT;
+    const fa::Blocks blk = fa::blocks_of(a.M, a.L, a.attn_len, 0, a.T);
+    return room && attn::adjoint_by_128(a.dk, (long)a.B * a.H, a.T, blk.lo, blk.hi);
 }
 // Table gradients added up by the CTA, in its own slot, instead of a table for each stream that the reduction reads again: where it
 // has four pairs or more.  The tables of 1024 pairs are 84 (320 rows) or 151 MB (576) a layer each way; steps of 20 layers 16196 -> 15999 us,

@@ -268,30 +268,47 @@ def test_attention_adjoint_on_128_key_blocks_bf16(pkg, oracle, B, H, dk, T, M, P
     _attn_case(pkg, oracle, B, H, dk, T, M, P, alen, True, 11)
 
 
+@pytest.mark.parametrize("B,H,dk,T,M,P,alen", [(40, 4, 64, 20, 30, 50, 0), (20, 8, 64, 64, 0, 40, 0), (40, 4, 64, 16, 150, 166, 0), (38, 4, 64, 9, 170, 100, 0),
+                                               (19, 8, 64, 33, 90, 123, 20), (37, 4, 64, 20, 30, 50, 0)])
+def test_attention_adjoint_of_short_windows_bf16(pkg, oracle, B, H, dk, T, M, P, alen):
+    """Head size 64, more pairs than SMs: one 64-key block, three of them for one tile of queries, two that a window puts into two
+    128-key blocks; and one block with a pair to an SM."""
+    _attn_case(pkg, oracle, B, H, dk, T, M, P, alen, True, 12)
+
+
 @pytest.mark.parametrize("kw", [
     dict(n_head=8, n_streams=74, d_pos=64),                                       # four pairs to a CTA, heads that start in mid-CTA
-    dict(n_head=8, n_streams=75, d_pos=40),                                       # four or five; copies of table row 0
-    dict(n_head=9, n_streams=66, d_pos=70, mem_len=150, attn_len=[30]),           # a window: zero rows of the table
+    dict(n_head=8, n_streams=75, d_pos=50),                                       # four or five; copies of table row 0
+    dict(n_head=9, n_streams=66, d_pos=324, mem_len=300, attn_len=[60]),          # a window: zero rows of the table
+    dict(n_head=9, n_streams=66, d_pos=310, mem_len=300, n_layer=4, attn_len=[60, 324, 90, 25]),  # layers in turn over the same partials
     dict(n_head=12, n_streams=50, d_pos=33, d_key=128, n_layer=2, tied_w_r=1),    # one table of two layers
     dict(n_head=200, n_streams=3, d_pos=64),                                      # several heads' ends in a CTA
     dict(n_head=8, n_streams=73, d_pos=64)])                                      # a part for each stream
 def test_position_table_gradients_summed_over_streams(pkg, kw):
-    """The table's gradient where CTAs of the adjoint sum the streams they take, head by head against the fp32 engine.  Roundings of
-    2^-9 in the dozen bf16 stages of a layer and its adjoint stay within 5 %; a stream lost or counted twice is 1 / sqrt(75) = 12 %."""
-    base = dict(n_layer=1, d_model=128, d_key=64, d_inner=128, mem_len=40, seg_len=24, n_symbols=64, init_range=0.05)
-    p = [pkg.abi.make_params(use_bf16=b, **dict(base, **kw)) for b in (1, 0)]
-    rng, got = np.random.default_rng(6), []
-    ids, tg = (rng.integers(0, 64, (3, 24, p[0].n_streams)).astype(np.int32) for _ in range(2))
-    for q in p:
-        m = pkg.TrfModel(q)
+    """The table's gradient where CTAs of the adjoint sum the streams they take, element by element against two models that have
+    half the streams each, which write a part for each stream.  Every row of activations and gradients has the same bits in both, so
+    what differs is the association of at most 75 fp32 parts (a layer): 75 x 2^-24 of the sum of their magnitudes, which for parts
+    of random sign is some sqrt(75) times the sum: 4e-5 of the head's largest element (2^-24 x 75 x 8.7), and a tied table's two layers
+    as much again.  A row that is lost, stale or counted twice is of the size of the others."""
+    base = dict(n_layer=1, d_model=128, d_key=64, d_inner=128, mem_len=60, seg_len=24, n_symbols=64, init_range=0.05, use_bf16=1)
+    kw = dict(base, **kw)
+    B, rng = kw.pop("n_streams"), np.random.default_rng(6)
+    ids, tg = (rng.integers(0, 64, (3, 24, B)).astype(np.int32) for _ in range(2))
+
+    def grads(s0, s1):
+        p = pkg.abi.make_params(n_streams=s1 - s0, n_streams_total=B, **kw)
+        m = pkg.TrfModel(p)
         m.reset()
         for s in range(3):
-            m.eval(-1, ids[s], read=False)
-            m.eval_gradient(tg[s])
+            m.eval(-1, np.ascontiguousarray(ids[s][:, s0:s1]), read=False)
+            m.eval_gradient(np.ascontiguousarray(tg[s][:, s0:s1]))
             m.memory_shift()
-        got.append({n: m.get_grad(n).reshape(q.n_head, -1) for n in m.info if "w_r" in n})
+        got = {n: m.get_grad(n).reshape(p.n_head, -1).astype(np.float64) for n in m.info if "w_r" in n}
         m.close()
-    assert got[0]
-    for n in got[0]:
-        for a, b in zip(got[0][n], got[1][n]):
-            assert np.linalg.norm(a - b) < 0.05 * np.linalg.norm(b), n
+        return got
+
+    whole, halves = grads(0, B), (grads(0, B // 2), grads(B // 2, B))
+    assert whole
+    for n in whole:
+        a, b = whole[n], halves[0][n] + halves[1][n]
+        assert (np.abs(a - b) <= 4e-5 * (1 + kw.get("tied_w_r", 0)) * np.abs(b).max(axis=1, keepdims=True)).all(), n
