@@ -15,6 +15,7 @@
 // butterflies combine them), so query row i gives the same bits whether it is
 // computed alone (one-symbol step) or with the whole segment.
 #pragma once
+#include "attention_deal.h"
 #include "common.cuh"
 
 struct AttnArgs {
@@ -261,9 +262,8 @@ template <int W, typename T> __device__ __forceinline__ void store_w(T *p, const
 // cluster's barrier every C-th part of the results; association and bits do not depend on C.  What bounds a CTA
 // is the rate of shared-memory reads, so every inner loop reads W = 4 elements per access (head sizes that are
 // a multiple of four; W = 1 otherwise) and each gradient row is a register tile of W columns.  One CTA per
-// (stream, head) left the chip to 16 CTAs (4 streams x 4 heads of 32, 32 queries over 64 keys: 29 us a launch; a step of two
-// such layers 208 -> 192 us with four) or to 128 of eight warps (16 x 8 heads: 27 us; a step of four layers 772 -> 739 us
-// with two, and eight queries a CTA in the forward kernel).
+// (stream, head) left the chip to 16 CTAs (4 streams x 4 heads of 32, 32 queries over 64 keys: 26 us a launch, 16.3 with
+// four; a step of two such layers 208 -> 192 us) or to 128 of eight warps (16 x 8 heads: 26.4 us, 24.6 with two).
 __device__ __forceinline__ uint32_t cluster_rank()
 {
     uint32_t r;
@@ -281,7 +281,7 @@ __device__ __forceinline__ void peer_store(uint32_t at, float v)
 {
     asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(at), "f"(v) : "memory");
 }
-template <typename T, int W>
+template <typename T, int W, bool CLUSTER> // CLUSTER: the grid's second dimension is a cluster, else it is one
 __global__ void __launch_bounds__(256) attn_bwd_kernel(AttnArgs a)
 {
     extern __shared__ __align__(16) unsigned char smraw[];
@@ -300,11 +300,11 @@ __global__ void __launch_bounds__(256) attn_bwd_kernel(AttnArgs a)
     float *Dr = dS + (size_t)Tn * (L + 1);              // [T]: D_i, later the row's sum over the left pad
     const int ls = L + 1;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int C = gridDim.y, rank = C > 1 ? (int)cluster_rank() : 0; // the cluster lies along y
+    const int C = CLUSTER ? gridDim.y : 1, rank = CLUSTER ? (int)cluster_rank() : 0; // the cluster lies along y
     const int b = blockIdx.x / a.H, h = blockIdx.x % a.H;
     const int HD = a.H * dk;
     const int tid = rank * blockDim.x + threadIdx.x, nthr = C * blockDim.x; // of the cluster
-    if (C > 1) // the others are there before anything is written to them
+    if constexpr (CLUSTER) // the others are there before anything is written to them
         asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");
     pdl_trigger();
     pdl_wait();
@@ -320,7 +320,7 @@ __global__ void __launch_bounds__(256) attn_bwd_kernel(AttnArgs a)
     if (a.w_r)
         stage_rows(Rs, ks, a.w_r + (size_t)h * P * dk, (size_t)dk, P, dk);
     __syncthreads();
-    if (C > 1)
+    if constexpr (CLUSTER)
         asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
     // P and dS, zero where the pair is masked
     for (int i = rank * 8 + warp; i < Tn; i += 8 * C) {
@@ -341,7 +341,7 @@ __global__ void __launch_bounds__(256) attn_bwd_kernel(AttnArgs a)
                 p = expf(score_ij<T>(i, j, Tn, L, P, dk, a.inv_sqrt, a.br_scale, qf, Ks, a.w_r ? Rs : nullptr, ks, a.b_r + (size_t)h * L) - lse);
                 d = p * (dot_q<T>(dof, Vs + (size_t)j * vs, dk) - D) * a.inv_sqrt;
             }
-            if (C == 1) {
+            if constexpr (!CLUSTER) {
                 Pm[(size_t)i * ls + j] = p;
                 dS[(size_t)i * ls + j] = d;
             } else {
@@ -354,10 +354,14 @@ __global__ void __launch_bounds__(256) attn_bwd_kernel(AttnArgs a)
                 pad += d;
         }
         pad = warp_sum(pad);
-        if (lane < C)
+        if constexpr (!CLUSTER) {
+            if (lane == 0)
+                Dr[i] = pad;
+        } else if (lane < C) {
             peer_store(peer_addr(Dr + i, lane), pad);
+        }
     }
-    if (C > 1)
+    if constexpr (CLUSTER)
         asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
     else
         __syncthreads();
@@ -525,15 +529,12 @@ static int attn_forward_t(const nncu_attn_shape *s, const void *q, const void *k
     AttnArgs a = attn_args(s, pt);
     a.q = q; a.kv = kv; a.w_r = w_r; a.b_r = b_r; a.o = out; a.lse = lse;
     const int nq = a.t1 - a.t0;
-    // Eight queries (one per warp) a CTA while four CTAs per SM take them all, else whole rounds of eight for two per
-    // SM (32 queries of 16 x 8 heads went in chunks of 11, two rounds of the warps)
-    const long heads = (long)a.B * a.H;
-    a.qchunk = heads * ceil_div(nq, 8) <= 4 * 148 ? 8 : (ceil_div(nq, max(1, ceil_div(2 * 148, heads))) + 7) & ~7;
-    const int chunks = ceil_div(nq, a.qchunk);
     size_t smem = 0;
     a.smem_pitch = fwd_pitch<T>(a, w_r != nullptr, smem);
     if (smem > 227 * 1024)
         return nncu_fail(NNCU_ERR_RANGE, "attention forward: %zu bytes of shared memory needed", smem);
+    a.qchunk = attn::queries_of_cta((long)a.B * a.H, nq, (long)smem);
+    const int chunks = ceil_div(nq, a.qchunk);
     static DeviceOnce once;
     NNCU_TRY(smem_limit(once, attn_fwd_kernel<T>, SMEM_MOST));
     launch_kind(EDGE_ATTN, attn_fwd_kernel<T>, dim3(a.B * a.H, chunks), dim3(256), smem, st, a);
@@ -556,13 +557,17 @@ static int attn_backward_t(const nncu_attn_shape *s, const void *q, const void *
     a.smem_pitch = bwd_pitch<T>(a, w_r != nullptr, smem);
     if (smem > 227 * 1024)
         return nncu_fail(NNCU_ERR_RANGE, "attention backward: %zu bytes of shared memory needed", smem);
-    auto kernel = a.dk % 4 == 0 ? attn_bwd_kernel<T, 4> : attn_bwd_kernel<T, 1>;
-    static DeviceOnce once[2];
-    NNCU_TRY(smem_limit(once[a.dk % 4 == 0 ? 0 : 1], kernel, SMEM_MOST));
-    // as many CTAs per (stream, head) as two to an SM hold, each with a query row for every warp
-    int C = 1;
-    while (C < 8 && 2 * C * a.B * a.H <= 2 * 148 && 2 * C * 8 <= a.T)
-        C *= 2;
+    const int C = attn::ctas_of_pair((long)a.B * a.H, a.T, (long)smem);
+    const bool vec = a.dk % 4 == 0;
+    auto kernel = C > 1 ? (vec ? attn_bwd_kernel<T, 4, true> : attn_bwd_kernel<T, 1, true>)
+                        : (vec ? attn_bwd_kernel<T, 4, false> : attn_bwd_kernel<T, 1, false>);
+    static DeviceOnce once[4];
+    NNCU_TRY(smem_limit(once[2 * (C > 1) + vec], kernel, SMEM_MOST));
+    if (C == 1) {
+        launch_kind(EDGE_ATTN, kernel, dim3(a.B * a.H), dim3(256), smem, st, a);
+        KERNEL_CHECK();
+        return NNCU_OK;
+    }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(a.B * a.H, C);
     cfg.blockDim = dim3(256);

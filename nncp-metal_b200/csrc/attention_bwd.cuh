@@ -30,7 +30,6 @@
 // compute warp whose wait ran out goes on without waiting (the barriers count on it), and every result of the CTA's
 // pairs becomes NaN.
 #pragma once
-#include "attention_deal.h"
 #include "attention_fa.cuh"
 
 namespace fab {
