@@ -442,13 +442,19 @@ __global__ void __launch_bounds__(256) reduce_jobs_kernel(const __grid_constant_
     if (jb.kind >= 1) {
         const int i = blk * 256 + threadIdx.x;
         if (i < jb.n) {
-            int parts = jb.n_parts;
-            if (jb.kind == 2)
-                parts = fab::slots_of(parts, jb.n / jb.off, i / jb.off);
+            // a loop for each kind: one over a number that either may have set is 5 to 35 % slower (148 parts of 8192 values
+            // 5.8 -> 7.7 us, 32 of 65536 2.4 -> 2.8)
             float s = 0.0f;
+            if (jb.kind == 1) {
 #pragma unroll 8 // eight parts' loads in flight
-            for (int p = 0; p < parts; p++)
-                s += jb.part[(size_t)p * jb.stride + i];
+                for (int p = 0; p < jb.n_parts; p++)
+                    s += jb.part[(size_t)p * jb.stride + i];
+            } else {
+                const int parts = fab::slots_of(jb.n_parts, jb.n / jb.off, i / jb.off);
+#pragma unroll 8
+                for (int p = 0; p < parts; p++)
+                    s += jb.part[(size_t)p * jb.stride + i];
+            }
             jb.out[i] = jb.accumulate ? jb.out[i] + s : s;
         }
         return;
