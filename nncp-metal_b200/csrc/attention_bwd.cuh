@@ -216,9 +216,13 @@ attn_bwd_tc_kernel(const __grid_constant__ AttnArgs a, const __grid_constant__ C
     auto bar = [&](int i) { return bar0 + 8 * (uint32_t)i; };
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int B = a.B, HD = a.H * DK, T = a.T, M = a.M, L = a.L, P = a.P;
+    // 64-key blocks with a visible pair.  The half of a first or last block that is none of them, and the table rows that only it
+    // meets, count as zeros, and their gradients are: what lies there need not be finite
+    const fa::Blocks all = fa::blocks_of(M, L, a.attn_len, 0, T);
+    auto seen = [&](int b64) { return b64 >= all.lo && b64 <= all.hi; };
+    auto met = [&](int g64) { return g64 >= all.lo && g64 <= all.hi + 1; }; // 64 rows of the window, 0-63 of block g64
     Walk<SUM> wk;
     {
-        const fa::Blocks all = fa::blocks_of(M, L, a.attn_len, 0, T); // in 64-key blocks
         wk.lo = wk.kb = all.lo / 2;
         wk.nkb = all.hi / 2 - wk.lo + 1;
         wk.B = B;
@@ -310,9 +314,9 @@ attn_bwd_tc_kernel(const __grid_constant__ AttnArgs a, const __grid_constant__ C
                 for (int c = 0; c < NA; c++)
 #pragma unroll
                     for (int p = 0; p < 2; p++) {
-                        fa::tma_load_3d(sm0 + SM::K + s * SM::KT + c * 16384 + p * 8192, &map_kv, bar(FULL_KV + s), h * DK + c * 64, b, j0 + p * 64);
-                        fa::tma_load_3d(sm0 + SM::V + s * SM::KT + c * 16384 + p * 8192, &map_kv, bar(FULL_KV + s), HD + h * DK + c * 64, b,
-                                        j0 + p * 64);
+                        const int j = seen(2 * kb + p) ? j0 + p * 64 : L; // rows from L on are zeros
+                        fa::tma_load_3d(sm0 + SM::K + s * SM::KT + c * 16384 + p * 8192, &map_kv, bar(FULL_KV + s), h * DK + c * 64, b, j);
+                        fa::tma_load_3d(sm0 + SM::V + s * SM::KT + c * 16384 + p * 8192, &map_kv, bar(FULL_KV + s), HD + h * DK + c * 64, b, j);
                     }
                 if (a.w_r && !by_hand(kb)) {
                     if (g >= NB && !(ok = mbar_wait(bar(FREE_R + s), (uint32_t)(((g >> LB) - 1) & 1), abort_s, ef, 60)))
@@ -322,7 +326,8 @@ attn_bwd_tc_kernel(const __grid_constant__ AttnArgs a, const __grid_constant__ C
                     for (int c = 0; c < NA; c++)
 #pragma unroll
                         for (int p = 0; p < 3; p++)
-                            fa::tma_load_3d(sm0 + SM::R + s * SM::RT + c * 24576 + p * 8192, &map_r, bar(FULL_R + s), c * 64, window0(kb) + p * 64, h);
+                            fa::tma_load_3d(sm0 + SM::R + s * SM::RT + c * 24576 + p * 8192, &map_r, bar(FULL_R + s), c * 64,
+                                            met(2 * kb + p) ? window0(kb) + p * 64 : P, h);
                 }
             }
             if constexpr (STAGED)
@@ -584,7 +589,9 @@ attn_bwd_tc_kernel(const __grid_constant__ AttnArgs a, const __grid_constant__ C
             for (int idx = threadIdx.x; idx < 192 * (DK / 8); idx += CT) {
                 const int r = idx / (DK / 8), c = idx % (DK / 8), x = min(max(x0 + r, 0), P - 1);
                 bf16 *at = reinterpret_cast<bf16 *>(dst + (c >> 3) * 24576 + r * 128 + (((c & 7) ^ (r & 7)) << 4));
-                if (a.w_r16)
+                if (!met(2 * w.kb + (r >> 6)))
+                    *reinterpret_cast<uint4 *>(at) = make_uint4(0u, 0u, 0u, 0u);
+                else if (a.w_r16)
                     *reinterpret_cast<uint4 *>(at) = *reinterpret_cast<const uint4 *>(w16 + (size_t)x * DK + c * 8);
                 else
                     fa::table_piece<WIDE>(at, w32 + (size_t)x * DK + c * 8);
@@ -796,8 +803,17 @@ attn_bwd_tc_kernel(const __grid_constant__ AttnArgs a, const __grid_constant__ C
                 window_by_hand(following, g + 1);
             uint32_t x[NC];
             meet(P2_DONE, g, 75);
-            if (dwr)
+            auto drop_unless = [&](bool there) { // the same for the whole warp
+                if (!there) {
+#pragma unroll
+                    for (int c = 0; c < NC; c++)
+                        x[c] = 0u;
+                }
+            };
+            if (dwr) {
                 load_table(x);
+                drop_unless(met(2 * kb + (qd >> 1)));
+            }
             signal(TR_FREE);
             if (dwr)
                 store_table(dwr, window0(kb), x, add);
@@ -814,8 +830,10 @@ attn_bwd_tc_kernel(const __grid_constant__ AttnArgs a, const __grid_constant__ C
                     }
                 };
                 load_nc(TM::V, x);
+                drop_unless(seen(2 * kb + (qd >> 1)));
                 park(sm + SM::V + s * SM::KT);
                 load_nc(TM::K, x);
+                drop_unless(seen(2 * kb + (qd >> 1)));
                 park(sm + SM::K + s * SM::KT);
                 fence_async();
                 signal(FREE_KV + s);
@@ -826,10 +844,12 @@ attn_bwd_tc_kernel(const __grid_constant__ AttnArgs a, const __grid_constant__ C
                     return j < L ? dkv + (size_t)j * B * a.dkvp + off : nullptr;
                 };
                 load_nc(TM::V, x);
+                drop_unless(seen(2 * kb + (qd >> 1)));
                 store_bf16(x, [&](int u) { return key_row(u, HD); });
                 load_nc(TM::K, x);
                 if (DK == 128 && !last)
                     signal(DRAINED);
+                drop_unless(seen(2 * kb + (qd >> 1)));
                 store_bf16(x, [&](int u) { return key_row(u, 0); });
             }
             if (last || (NB == 1 && hand))
@@ -848,6 +868,7 @@ attn_bwd_tc_kernel(const __grid_constant__ AttnArgs a, const __grid_constant__ C
                 if (dwr) {
                     if (qd < 2) { // the upper 64 rows of the last window
                         load_table(x);
+                        drop_unless(met(2 * kb + 2));
                         store_table(dwr, window0(kb) + 128, x, add);
                     }
                     if (fold) {

@@ -312,3 +312,65 @@ def test_position_table_gradients_summed_over_streams(pkg, kw):
     for n in whole:
         a, b = whole[n], halves[0][n] + halves[1][n]
         assert (np.abs(a - b) <= 4e-5 * (1 + kw.get("tied_w_r", 0)) * np.abs(b).max(axis=1, keepdims=True)).all(), n
+
+
+@pytest.mark.parametrize("dk,B,alen,P", [(64, 2, 60, 340), (64, 2, 60, 200), (128, 2, 60, 340), (128, 3, 60, 200), (64, 80, 60, 340)])
+def test_adjoint_reads_no_block_that_no_query_sees(pkg, dk, B, alen, P):
+    """A window whose first 64-key block is the upper half of a 128-key block (keys 192 on): what the keys before it, and the table
+    rows that only they would meet, hold does not matter, and their gradients are zeros even for queries that are not finite."""
+    lib = pkg.library()
+    H, T, M = 2, 40, 300
+    L, HD = T + M, H * dk
+    g = torch.Generator(device="cuda").manual_seed(dk + P)
+    q, dout = (torch.randn(T * B, HD, generator=g, device="cuda").bfloat16() for _ in range(2))
+    kv = torch.randn(L * B, 2 * HD, generator=g, device="cuda").bfloat16()
+    w_r, b_r = 0.1 * torch.randn(H, P, dk, generator=g, device="cuda"), 0.1 * torch.randn(H, L, generator=g, device="cuda")
+    shp = C.byref(pkg.abi.AttnShape(B, H, dk, T, M, P, alen, 0, T, float(np.sqrt(dk * 512.0)), 1))
+    unseen = 192 * B                      # rows of kv
+    unmet = max(0, 192 + P - M - 64)      # rows of the table below those of the first block's window
+
+    def run(fill, query=None):
+        k, w, x = kv.clone(), w_r.clone(), q.clone()
+        k[:unseen] = fill
+        w[:, 1:unmet] = fill              # row 0 stands for all rows before the table
+        if P == L:
+            w[:, :unmet] = fill
+        if query is not None:
+            x[query] = float("inf")
+        out, lse, dq, dkv = torch.zeros_like(q), torch.zeros(B * H, T, device="cuda"), torch.full_like(q, 7), torch.full_like(kv, 7)
+        pw, pb = torch.full((B, H, P, dk), 7.0, device="cuda"), torch.full((B, H, L), 7.0, device="cuda")
+        ptr = [C.c_void_p(t.data_ptr()) for t in (x, k, w, b_r, out, lse, dout, dq, dkv, pw, pb)]
+        assert lib.nncu_attention_forward(shp, *ptr[:6], None) == 0, lib.nncu_last_error()
+        assert lib.nncu_attention_backward(shp, *ptr, None) == 0, lib.nncu_last_error()
+        torch.cuda.synchronize()
+        return out, lse, dq, dkv, pw, pb
+
+    want = run(0.0)
+    assert all(t.isfinite().all() for t in want)
+    for fill in (float("nan"), float("inf")):
+        assert all(torch.equal(a, b) for a, b in zip(want, run(fill)))
+    got = run(0.0, query=5 * B)
+    assert (got[3][:unseen] == 0).all()
+    if P == L:
+        assert (got[4][:, :, :unmet] == 0).all()
+
+
+@pytest.mark.parametrize("dk", [64, 128])
+def test_table_rows_that_no_window_meets_do_not_matter_to_a_step(pkg, dk):
+    p = pkg.abi.make_params(n_layer=1, d_model=2 * dk, n_head=2, d_key=dk, d_inner=128, d_pos=340, mem_len=300, seg_len=40, n_streams=2, n_symbols=64,
+                            use_bf16=1, attn_len=[60], init_range=0.1)
+    rng = np.random.default_rng(4)
+    ids, tg = (rng.integers(0, 64, (40, 2)).astype(np.int32) for _ in range(2))
+    got = []
+    for fill in (0.0, float("nan")):
+        m = pkg.TrfModel(p)
+        w = m.get_param("w_r_0").reshape(2, 340, dk).copy()
+        w[:, :168] = fill
+        m.set_param("w_r_0", w.reshape(-1))
+        m.reset()
+        m.eval(-1, ids, read=False)
+        m.eval_gradient(tg)
+        got.append({n: m.get_grad(n) for n in m.info})
+        m.close()
+    for n in got[0]:
+        assert np.isfinite(got[0][n]).all() and np.array_equal(got[0][n], got[1][n]), n
