@@ -264,12 +264,6 @@ template <int W, typename T> __device__ __forceinline__ void store_w(T *p, const
 // a multiple of four; W = 1 otherwise) and each gradient row is a register tile of W columns.  One CTA per
 // (stream, head) left the chip to 16 CTAs (4 streams x 4 heads of 32, 32 queries over 64 keys: 26 us a launch, 16.3 with
 // four; a step of two such layers 208 -> 192 us) or to 128 of eight warps (16 x 8 heads: 26.4 us, 24.6 with two).
-__device__ __forceinline__ uint32_t cluster_rank()
-{
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
 // the address of `p` in the shared memory of CTA `rank` of the cluster
 __device__ __forceinline__ uint32_t peer_addr(const void *p, uint32_t rank)
 {
@@ -300,7 +294,7 @@ __global__ void __launch_bounds__(256) attn_bwd_kernel(AttnArgs a)
     float *Dr = dS + (size_t)Tn * (L + 1);              // [T]: D_i, later the row's sum over the left pad
     const int ls = L + 1;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int C = CLUSTER ? gridDim.y : 1, rank = CLUSTER ? (int)cluster_rank() : 0; // the cluster lies along y
+    const int C = CLUSTER ? gridDim.y : 1, rank = CLUSTER ? blockIdx.y : 0; // the cluster lies along y and is the whole of it
     const int b = blockIdx.x / a.H, h = blockIdx.x % a.H;
     const int HD = a.H * dk;
     const int tid = rank * blockDim.x + threadIdx.x, nthr = C * blockDim.x; // of the cluster
