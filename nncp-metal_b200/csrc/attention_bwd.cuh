@@ -30,6 +30,8 @@
 // compute warp whose wait ran out goes on without waiting (the barriers count on it), and every result of the CTA's
 // pairs becomes NaN.
 #pragma once
+#include <algorithm>
+
 #include "attention_fa.cuh"
 
 namespace fab {
@@ -958,3 +960,18 @@ template <int DK> static int launch(const AttnArgs &a, cudaStream_t st)
 static int backward(const AttnArgs &a, cudaStream_t st) { return a.dk == 64 ? launch<64>(a, st) : launch<128>(a, st); }
 
 } // namespace fab
+
+// How many tables attn_backward_any leaves in dwr_part for this shape when it may leave sums: the slots of the head with the
+// most CTAs, or one a stream.  Operands as a model places them, 16-byte aligned.
+static int attn_table_parts(const nncu_attn_shape *s, const AttnPitch *pt)
+{
+    AttnArgs a = attn_args(s, pt);
+    float lse; // supported_bwd asks that there be one
+    a.lse = &lse;
+    if (!s->dtype_bf16 || !fa::supported_bwd(a) || !fa::fits(a.dk, a.L) || !fab::takes(a) || !fab::sums(a))
+        return s->n_streams;
+    int most = 0;
+    for (int h = 0; h < a.H; h++)
+        most = std::max(most, fab::slots_of(a.B, a.H, h));
+    return most;
+}

@@ -1835,13 +1835,17 @@ static int attn_forward_any(const nncu_attn_shape *s, const void *q, const void 
     return attn_forward_t<T>(s, q, kv, w_r, b_r, out, lse, st, pt);
 }
 
-// With `sums` dwr_part may come back as sums over streams in fewer parts (fab::slots_of); *sums says whether.
+// With `sums` dwr_part may come back as sums over streams in fewer parts (fab::slots_of); *sums says whether.  It has room for
+// `parts` of them (attn_table_parts).
 template <typename T>
 static int attn_backward_any(const nncu_attn_shape *s, const void *q, const void *kv, const float *w_r,
                              const float *b_r, const void *out, const float *lse, const void *dout,
                              void *dq, void *dkv, float *dwr_part, float *dbr_part, cudaStream_t st,
-                             const AttnPitch *pt = nullptr, const void *w_r16 = nullptr, int *err_flag = nullptr, bool *sums = nullptr)
+                             const AttnPitch *pt = nullptr, const void *w_r16 = nullptr, int *err_flag = nullptr, bool *sums = nullptr, int parts = 0)
 {
+    const auto room = [&]() {
+        return sums && w_r && parts < s->n_streams ? nncu_fail(NNCU_ERR_INVALID, "attention backward: no room for a table a stream") : NNCU_OK;
+    };
     if (sizeof(T) == 2) {
         AttnArgs a = attn_args(s, pt);
         a.w_r16 = w_r ? w_r16 : nullptr;
@@ -1849,13 +1853,18 @@ static int attn_backward_any(const nncu_attn_shape *s, const void *q, const void
         a.q = q; a.kv = kv; a.w_r = w_r; a.b_r = b_r; a.out = out; a.lse = const_cast<float *>(lse);
         a.dout = dout; a.dq = dq; a.dkv = dkv; a.dwr_part = dwr_part; a.dbr_part = dbr_part;
         if (fa::supported_bwd(a) && fa::fits(a.dk, a.L)) {
-            if (!fab::takes(a))
+            if (!fab::takes(a)) {
+                NNCU_TRY(room());
                 return fa::backward(a, st);
+            }
             if (sums)
                 *sums = a.sum = fab::sums(a);
+            if (!a.sum)
+                NNCU_TRY(room());
             return fab::backward(a, st);
         }
     }
+    NNCU_TRY(room());
     return attn_backward_t<T>(s, q, kv, w_r, b_r, out, lse, dout, dq, dkv, dwr_part, dbr_part, st, pt);
 }
 

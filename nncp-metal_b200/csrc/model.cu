@@ -191,6 +191,7 @@ struct nncu_model {
     std::vector<LayerAct> act;
     void *xlast, *xf, *pool[POOLS], *dz, *dh, *dhp[2], *dof, *dqkv[2], *tA, *tB;
     float *st_f, *probs, *dwr_part[2], *dbr_part[2], *part, *logp, *loss_dev;
+    int table_parts = 0;    // tables in a dwr_part: one a stream, or the CTAs' sums (attn_table_parts)
     size_t part_floats = 0; // floats per region of `part`
     // Split-K workspaces: skw for products on the main stream (the output head's dX), skw_side for weight
     // gradients, which run on the side stream beside them.  Two regions, because nothing orders the head's
@@ -1046,7 +1047,7 @@ static int backward(nncu_model *m)
         bool sums = false;
         NNCU_TRY(attn_backward_any<AT>(&s, at<AT>(a.qkv, (size_t)M * B * 3 * HD), at<AT>(a.qkv, HD), wf(m, o.w_r),
                                        m->W + o.b_r, a.o, a.lse, dof, dq, dkv, dwr_part, dbr_part, m->st,
-                                       &pt, (m->bf && o.w_r != NONE) ? m->Wb + o.w_r : nullptr, m->err_flag, &sums));
+                                       &pt, (m->bf && o.w_r != NONE) ? m->Wb + o.w_r : nullptr, m->err_flag, &sums, m->table_parts));
         {
             // the partials are next written two layers on
             size_t nb = (size_t)m->H * m->L;
@@ -1509,7 +1510,12 @@ int nncu_create(const nncu_params *p, nncu_model **out)
     size_t max_n = (size_t)std::max(std::max(V, F1), std::max(3 * HD, D));
     size_t max_k = (size_t)std::max(std::max(F, D), HD);
     size_t oTA = m->use_tc ? take(max_n * LB * 2) : 0, oTB = m->use_tc ? take(max_k * LB * 2) : 0;
-    const size_t n_wr = slot((size_t)m->B * m->H * p->d_pos * m->dk * 4), n_br = slot((size_t)m->B * m->H * m->L * 4);
+    const AttnPitch qkv_pitch = {3 * HD, 3 * HD, 3 * HD, 3 * HD};
+    for (int l = 0; l < m->nl; l++) {
+        const nncu_attn_shape s = attn_shape(m, l, 0, m->T);
+        m->table_parts = std::max(m->table_parts, attn_table_parts(&s, &qkv_pitch));
+    }
+    const size_t n_wr = slot((size_t)m->table_parts * m->H * p->d_pos * m->dk * 4), n_br = slot((size_t)m->B * m->H * m->L * 4);
     size_t oWr = take(2 * n_wr), oBr = take(2 * n_br);
     size_t part_floats = std::max((size_t)ceil_div(TB, 64) * std::max(V, std::max(D, HD)), (size_t)ceil_div(TB, 8) * 3 * D);
     part_floats = std::max(part_floats, (size_t)ceil_div(TB, ACT_BWD_ROWS) * F1);

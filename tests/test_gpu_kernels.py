@@ -374,3 +374,21 @@ def test_table_rows_that_no_window_meets_do_not_matter_to_a_step(pkg, dk):
         m.close()
     for n in got[0]:
         assert np.isfinite(got[0][n]).all() and np.array_equal(got[0][n], got[1][n]), n
+
+
+def test_partial_tables_take_the_room_of_the_sums_that_are_kept(pkg):
+    """Many pairs, whose CTAs sum the table's gradient over their streams: a model's memory grows by a few tables with the
+    table's length (a table has the same weights, gradients and moments besides), not by one for each stream."""
+    def taken(d_pos):
+        kw = dict(n_layer=1, d_model=64, n_head=8, d_key=64, d_inner=64, d_pos=d_pos, mem_len=400, seg_len=32, n_streams=128, n_symbols=64, use_bf16=1)
+        m = pkg.TrfModel(pkg.abi.make_params(**kw))
+        m.close()
+        before = torch.cuda.mem_get_info()[0]
+        m = pkg.TrfModel(pkg.abi.make_params(**kw))
+        now = torch.cuda.mem_get_info()[0]
+        m.close()
+        return before - now
+
+    table = 8 * 431 * 64 * 4
+    # two sets of at most ceil(128 / 6) + 1 parts, and the copies of the parameter; allocations in pieces of 2 MB
+    assert taken(432) - taken(1) < (2 * 23 + 4) * table + 4 * 2 ** 20 < 128 * table
