@@ -229,7 +229,8 @@ def test_fp32_attention_by_clusters(pkg, oracle, B, H, dk, T, M, P, alen):
 
 
 @pytest.mark.parametrize("kw", [dict(n_layer=1), dict(n_layer=2), dict(n_layer=3), dict(n_layer=5, ln_flags=2 | 4 | 16, ff_act=2),
-                                dict(n_layer=3, use_bf16=0), dict(n_layer=4, use_bf16=0, tied_w_r=1, tied_b_r=1)])
+                                dict(n_layer=3, use_bf16=0), dict(n_layer=4, use_bf16=0, tied_w_r=1, tied_b_r=1),
+                                dict(n_layer=4, ln_flags=1 | 8), dict(n_layer=5, ln_flags=2 | 4 | 8, attn_len=[48, 20, 7, 33, 1])])
 def test_gradients_with_and_without_the_side_stream_are_the_same_bits(pkg, monkeypatch, kw):
     """Weight gradients and reductions run up to two layers behind the main stream, from buffers that layers take in
     turn: every gradient of several steps and models, against one stream."""
@@ -266,6 +267,15 @@ def test_attention_adjoint_on_128_key_blocks_bf16(pkg, oracle, B, H, dk, T, M, P
     """The persistent kernel of head sizes 64 and 128: whole and ragged key blocks, one query, more (stream, head) pairs
     than CTAs, tables that end inside the left pad, windows that leave whole blocks out."""
     _attn_case(pkg, oracle, B, H, dk, T, M, P, alen, True, 11)
+
+
+@pytest.mark.parametrize("B,H,dk,T,M,P,alen", [(1, 2, 64, 64, 1368, 1432, 0), (1, 2, 64, 64, 1369, 1433, 0), (1, 2, 64, 40, 1393, 700, 0), (2, 1, 64, 64, 1400, 1464, 200),
+                                               (1, 2, 128, 64, 1240, 1304, 0), (1, 2, 128, 64, 1241, 1305, 0), (1, 1, 128, 33, 1300, 500, 0),
+                                               (1, 2, 128, 64, 1250, 1314, 130)])
+def test_attention_adjoint_where_b_r_outgrows_its_place_bf16(pkg, oracle, B, H, dk, T, M, P, alen):
+    """The most keys whose two copies of b_r fit beside the tiles of 128 keys (1432 at head size 64, 1304 at 128), one more, and more than
+    that: the warp-level kernel, with tables that end inside the left pad and with windows."""
+    _attn_case(pkg, oracle, B, H, dk, T, M, P, alen, True, 13)
 
 
 @pytest.mark.parametrize("B,H,dk,T,M,P,alen", [(40, 4, 64, 20, 30, 50, 0), (20, 8, 64, 64, 0, 40, 0), (40, 4, 64, 16, 150, 166, 0), (38, 4, 64, 9, 170, 100, 0),
@@ -392,3 +402,40 @@ def test_partial_tables_take_the_room_of_the_sums_that_are_kept(pkg):
     table = 8 * 431 * 64 * 4
     # two sets of at most ceil(128 / 6) + 1 parts, and the copies of the parameter; allocations in pieces of 2 MB
     assert taken(432) - taken(1) < (2 * 23 + 4) * table + 4 * 2 ** 20 < 128 * table
+
+
+@pytest.mark.parametrize("kw", [
+    dict(d_model=256, n_head=4, d_key=64, n_streams=100),                           # a warp for every (stream, head)
+    dict(d_model=256, n_head=2, d_key=128, n_streams=130, attn_len=[90, 0, 30]),
+    dict(d_model=256, n_head=4, d_key=64, n_streams=5, d_pos=90),                   # four warps for one, tiles by TMA; copies of table row 0
+    dict(d_model=256, n_head=2, d_key=128, n_streams=3, ln_flags=2 | 4 | 16, ff_act=2),
+    dict(d_model=128, n_head=4, d_key=32, n_streams=6, mem_len=400, d_pos=412)])    # tiles by every thread, more than one round
+def test_device_decoder_over_several_key_blocks(pkg, kw):
+    """Steps of a decoder, launched to overlap one another, read the keys of earlier steps, the tables and the weights before they
+    wait: over memories of several key blocks, both memory twins and weights that have just been updated, the symbols are those of the
+    host's walk of a whole segment's trees, and probabilities and updated weights have that segment's bits."""
+    p = pkg.abi.make_params(**dict(dict(n_layer=3, d_inner=256, d_pos=162, mem_len=150, seg_len=12, n_symbols=300, use_bf16=1, init_range=0.2, lr=1e-3), **kw))
+    T, B, V, L = p.seg_len, p.n_streams, p.n_symbols, pkg.host.library()
+    rng = np.random.default_rng(9)
+    dev, ref, streams = pkg.TrfModel(p), pkg.TrfModel(p), [torch.cuda.Stream() for _ in range(2)]
+    for m, st in zip((dev, ref), streams):
+        m.set_stream(st.cuda_stream)
+        m.reset()
+    for seg in range(6):   # the third pass over a memory twin replays graphs
+        payload = rng.integers(0, 256, 40 * B, dtype=np.uint8).tobytes()
+        first = rng.integers(0, V, B).astype(np.int32)
+        dev.decoder_begin(payload)
+        got = dev.decode_steps(0, T, first)
+        dev.decoder_end()
+        ids = np.concatenate([first[None], got[:-1]])
+        assert np.array_equal(ref.eval(-1, ids), dev.read_probs(0, T))
+        buf = C.create_string_buffer(payload, len(payload))
+        hd, trees = L.nch_dec_new(buf, len(payload)), np.ascontiguousarray(ref.coder_trees(0, T))
+        want = [L.nch_read_sym_tree(hd, trees[i].ctypes.data_as(C.c_void_p), V) for i in range(T * B)]
+        L.nch_dec_free(hd)
+        assert np.array_equal(got.reshape(-1), want)
+        for m in (dev, ref):
+            m.eval_gradient(got)
+            m.update()
+        assert dev.weights_hash() == ref.weights_hash()
+    dev.close(); ref.close()

@@ -153,19 +153,19 @@ def _attn_case(pkg, oracle, B, H, dk, T, M, P, attn_len, bf16, seed):
     dt = torch.bfloat16 if bf16 else torch.float32
     dq_, dkv_, ddout = _dev(q, dt), _dev(kv, dt), _dev(dout, dt)
     dwr, dbr = _dev(w_r), _dev(b_r)
-    out = torch.zeros(T * B, H * dk, device="cuda", dtype=dt)
-    lse = torch.zeros(B * H, T, device="cuda")
+    # whatever was there: every value is written
+    new = lambda *shape, dtype=torch.float32: torch.full(shape, float("nan"), device="cuda", dtype=dtype)
+    out, lse = new(T * B, H * dk, dtype=dt), new(B * H, T)
     assert lib.nncu_attention_forward(C.byref(shp), dq_.data_ptr(), dkv_.data_ptr(), dwr.data_ptr(),
                                       dbr.data_ptr(), out.data_ptr(), lse.data_ptr(), None) == 0, \
         lib.nncu_last_error()
-    gq, gkv = torch.zeros_like(dq_), torch.zeros_like(dkv_)
-    pw = torch.zeros(B, H, P, dk, device="cuda")
-    pb = torch.zeros(B, H, L, device="cuda")
+    gq, gkv = torch.full_like(dq_, float("nan")), torch.full_like(dkv_, float("nan"))
+    pw, pb = new(B, H, P, dk), new(B, H, L)
     assert lib.nncu_attention_backward(C.byref(shp), dq_.data_ptr(), dkv_.data_ptr(), dwr.data_ptr(),
                                        dbr.data_ptr(), out.data_ptr(), lse.data_ptr(), ddout.data_ptr(),
                                        gq.data_ptr(), gkv.data_ptr(), pw.data_ptr(), pb.data_ptr(),
                                        None) == 0, lib.nncu_last_error()
-    gw, gb = torch.zeros(H, P, dk, device="cuda"), torch.zeros(H, L, device="cuda")
+    gw, gb = new(H, P, dk), new(H, L)
     assert lib.nncu_attention_reduce_tables(C.byref(shp), pw.data_ptr(), pb.data_ptr(), gw.data_ptr(),
                                             gb.data_ptr(), 0, None) == 0
     torch.cuda.synchronize()

@@ -210,7 +210,8 @@ def test_decoder_of_very_many_streams(pkg, B, V):
     dev.close(); ref.close()
 
 
-@pytest.mark.parametrize("dk,T,M,alen", [(16, 20, 300, 0), (32, 64, 500, 90), (64, 64, 836, 0), (64, 64, 600, 130), (128, 33, 500, 200)])
+@pytest.mark.parametrize("dk,T,M,alen", [(16, 20, 300, 0), (32, 64, 500, 90), (64, 64, 836, 0), (64, 64, 600, 130), (128, 33, 500, 200),
+                                           (64, 64, 1368, 0), (64, 64, 1369, 300), (128, 33, 1271, 0), (128, 33, 1272, 200)])
 def test_attention_of_operands_inside_larger_buffers(pkg, dk, T, M, alen):
     """An fp32 table, results and partials that start between 16-byte boundaries, as views of larger buffers do, with
     more keys than the CUDA-core kernels hold: the bits of the aligned call, segments and single queries."""
@@ -233,7 +234,7 @@ def test_attention_of_operands_inside_larger_buffers(pkg, dk, T, M, alen):
         table = place(w_r, off)
         out, one, dq, dkv = (place(torch.full_like(t, float("nan")), 2 * off) for t in (q, q, q, kv))
         lse = torch.zeros(B * H, T, device="cuda")
-        part, dbr = place(torch.full((B, H, P, dk), float("nan"), device="cuda"), 2 * off), torch.zeros(B, H, L, device="cuda")
+        part, dbr = place(torch.full((B, H, P, dk), float("nan"), device="cuda"), 2 * off), torch.full((B, H, L), float("nan"), device="cuda")
 
         def shape(t0, t1):
             return C.byref(pkg.abi.AttnShape(B, H, dk, T, M, P, alen, t0, t1, float(np.sqrt(dk * 512.0)), 1))
