@@ -486,7 +486,7 @@ attn_bwd_tc_kernel(const __grid_constant__ AttnArgs a, const __grid_constant__ C
                         brs[r0 + k * 64] = __fmul_rn(a.br_scale, v[k]);
             }
             bf16 *dkv = reinterpret_cast<bf16 *>(a.dkv) + (size_t)b * a.dkvp + h * DK;
-            const int j_lo = lo * KB, j_hi = (lo + wk.nkb) * KB, outside = j_lo + max(0, L - j_hi);
+            const int j_lo = STAGED ? lo * KB : all.lo * 64, j_hi = STAGED ? (lo + wk.nkb) * KB : (all.hi + 1) * 64, outside = j_lo + max(0, L - j_hi);
             for (int idx = tid; idx < outside * (DK / 8); idx += 64) {
                 const int k = idx / (DK / 8), j = k < j_lo ? k : j_hi + k - j_lo, c = (idx % (DK / 8)) * 8;
                 fa::zero16<WIDE>(dkv + (size_t)j * B * a.dkvp + c);
@@ -845,14 +845,16 @@ attn_bwd_tc_kernel(const __grid_constant__ AttnArgs a, const __grid_constant__ C
                     const int j = j0 + qd * 32 + lane4 + u;
                     return j < L ? dkv + (size_t)j * B * a.dkvp + off : nullptr;
                 };
-                load_nc(TM::V, x);
-                drop_unless(seen(2 * kb + (qd >> 1)));
-                store_bf16(x, [&](int u) { return key_row(u, HD); });
-                load_nc(TM::K, x);
+                const bool there = seen(2 * kb + (qd >> 1));
+                if (there) {
+                    load_nc(TM::V, x);
+                    store_bf16(x, [&](int u) { return key_row(u, HD); });
+                    load_nc(TM::K, x);
+                }
                 if (DK == 128 && !last)
                     signal(DRAINED);
-                drop_unless(seen(2 * kb + (qd >> 1)));
-                store_bf16(x, [&](int u) { return key_row(u, 0); });
+                if (there)
+                    store_bf16(x, [&](int u) { return key_row(u, 0); });
             }
             if (last || (NB == 1 && hand))
                 meet(DE_FREE, g, 78); // and everything else
