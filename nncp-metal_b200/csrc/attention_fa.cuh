@@ -857,7 +857,7 @@ __global__ void __launch_bounds__(128) attn_one_tma_kernel(const __grid_constant
         a.lse[((size_t)b * a.H + h) * T + i] = m_run + logf(l);
 }
 
-// Many streams and heads: a warp of its own for every (stream, head), a CTA each, up to nine on an SM.  The four warps
+// Many streams and heads: a warp of its own for every (stream, head), a CTA each, up to eight on an SM (four at head size 128).  The four warps
 // of the kernel above meet twice a round and its CTAs take turns at loading and at computing; here nothing
 // meets, K and the table rows of the next block are on their way as soon as the scores are taken and V as soon as
 // its products are, and 128 streams x 8 heads are one wave.  128 x 8 pairs of 576
@@ -1696,7 +1696,8 @@ inline bool supported_bwd(const AttnArgs &a)
     return supported(a) && a.T <= 64 && a.t0 == 0 && a.t1 == a.T && a.dqp % 8 == 0 && a.dkvp % 8 == 0 && aligned_to(a.dq, 4) &&
            aligned_to(a.dkv, 4) && aligned_to(a.dout, 16) && aligned_to(a.dwr_part, 8) && a.lse;
 }
-// shared memory both kernels of a shape need
+// Shared memory both kernels of a shape need.  At head sizes 64 and 128 the forward kernel by TMA needs a little less than
+// FwdSmem, which stays the line between what is taken and what goes to the CUDA-core kernels.
 inline bool fits(int dk, int L)
 {
     const size_t most = 227 * 1024;

@@ -343,7 +343,8 @@ static int mm_nn(nncu_model *m, int M, int Kin, int Nout, const bf16 *dY, long l
 // dW = dY^T X: G[Nout][Kin] = sum over R rows of dY[r][Nout] X[r][Kin]   (fp32 result)
 // The weight gradients are off the critical path of the backward pass (nothing downstream
 // reads them before the optimizer), so they go to a second stream: fork after the operands
-// exist, join once per layer before any operand buffer is reused.
+// exist; the main stream waits for a layer's operands only before they are written again, two layers on
+// (side_release), or at each layer where its gradients are exchanged or applied next (side_join).
 static cudaStream_t side_fork(nncu_model *m)
 {
     if (!m->overlap || g_nncu_prof)
@@ -437,7 +438,7 @@ static int mm_tn(nncu_model *m, int Nout, int Kin, int R, const bf16 *dY, long l
 
 // The column and stream reductions of the backward pass only write gradient buffers, which nobody
 // reads before the optimizer: they are queued and run as ONE launch per layer on the side stream
-// (flush_reductions, in front of the layer's join), instead of a 5 us launch each.
+// (flush_reductions, at the layer's end), instead of a 5 us launch each.
 static int flush_reductions(nncu_model *m)
 {
     if (m->rjobs.n_jobs == 0)
@@ -989,8 +990,8 @@ static int backward(nncu_model *m)
         } else if (o.ff_bias2 != NONE && !coef && !bias2_done) {
             NNCU_TRY(colsum<AT>(m, ds2, D, TB, D, gf(m, o.ff_bias2)));
         }
-        // LN_COEF: the branch sees alpha * ds2 (its own buffer: the weight-gradient GEMMs read it until the
-        // layer's join), the residual keeps ds2; the rows' shares of d alpha wait for the layer's reduction launch
+        // LN_COEF: the branch sees alpha * ds2 (its own buffer: the weight-gradient GEMMs read it, up to two
+        // layers on), the residual keeps ds2; the rows' shares of d alpha wait for the layer's reduction launch
         AT *dt2 = ds2;
         if (coef) {
             dt2 = reinterpret_cast<AT *>(m->dt_ff[half]);
@@ -1093,7 +1094,7 @@ static int backward(nncu_model *m)
             // layer l's slots are contiguous; tied tables live in layer 0, which is exchanged last
             const size_t lb = o.w_q, le = l + 1 < m->nl ? m->lo[l + 1].w_q : m->tail_begin;
             NNCU_TRY(exchange_update(m, lb, o.small, le));
-            if (l == m->nl - 1) // the output head's gradients have been complete since the first join
+            if (l == m->nl - 1) // the output head's gradients are complete since the join above
                 NNCU_TRY(exchange_update(m, m->embed_out, m->out_bias != NONE ? m->out_bias : m->n_floats, m->n_floats));
         }
         dx = dxn;
